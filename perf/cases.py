@@ -171,9 +171,84 @@ def work(case):
 
 
 def tolerance(case):
-    # measured against 64-bit arithmetic on the same quantised operands: 2e-4 .. 5e-4 with fp16 results (2e-3 where the
-    # activation quantiser meets rounding ties), 1.7e-3 .. 2.9e-3 with bf16 results
+    # four times what was measured against 64-bit arithmetic on the same quantised operands
     if case["kind"] == "mlp":
-        # 5e-3 .. 1.4e-2: rounding gate and up to fp16 moves int8 codes of the hidden activations by one step
-        return {"rel": 1.5e-2, "max": 0.15}
-    return {"rel": 2e-3 if case["dtype"] == "f16" else 8e-3, "max": 0.02}
+        # 5e-3 .. 1.3e-2: rounding gate and up to fp16, and the first sums, move int8 codes of the hidden activations
+        return {"rel": 4e-2, "max": 0.25}
+    if case["kind"] == "gemm":
+        # 2e-4 .. 3.4e-4 with fp16 results, 1.7e-3 with bf16 results
+        return {"rel": 1.5e-3 if case["dtype"] == "f16" else 7e-3, "max": 0.02}
+    # sums of normally distributed products cancel: 4e-4 .. 2.4e-3 with fp16 results, 1.7e-3 .. 2.9e-3 with bf16 results
+    return {"rel": 1e-2, "max": 0.06}
+
+
+# --------------------------------------------------------------------------------------------------------------
+# The same in 64 bits.  The integer codes of weights and activations are the format itself (their rule is defined in
+# fp32, as are the token scales; group scales are stored as fp16); sums, SiLU and scaling are float64.
+def _codes_of(w, group):
+    """Codes - 1 [N, K] in -1..2 and the stored fp16 scales [K/G, N] of a float weight [N, K]."""
+    N, K = w.shape
+    g = w.float().view(N, K // group, group)
+    scale = (g.abs().amax(dim=2).clamp_min(1e-9).double() / 1.5).float()
+    codes = torch.round(g / scale[:, :, None]).clamp_(-1, 2)
+    return codes.view(N, K), scale.t().to(torch.float16).contiguous()
+
+
+def _unpacked(w_packed, zero_point):
+    shifts = torch.tensor([6, 4, 2, 0], device=w_packed.device, dtype=torch.uint8)
+    return ((w_packed[:, :, None] >> shifts) & 3).view(w_packed.shape[0], -1).to(torch.float32) - zero_point
+
+
+def _quantized(x):
+    """Codes and scales of activations; the scale's and the quotient's rule is fp32."""
+    x = x.float()
+    s = (x.abs().amax(dim=1).double() / 127).float()
+    s = torch.where(s > 0, s, torch.ones_like(s))
+    return torch.round(x / s[:, None]).clamp_(-127, 127), s
+
+
+def _product(x_q, x_scale, codes, w_scale, group, columns=4096):
+    """float64 x_scale * sum over groups of w_scale * (x_q . codes), a block of output features at a time."""
+    xd = x_q.double()
+    out = []
+    for lo in range(0, codes.shape[0], columns):
+        c = codes[lo:lo + columns].double()
+        c = c * w_scale[:, lo:lo + columns].t().double().repeat_interleave(group, dim=1)
+        out.append(xd @ c.t())
+    return torch.cat(out, dim=1) * x_scale.double()[:, None]
+
+
+def exact(case, seed):
+    """What `run` returns, in float64 (None for the packed bytes of `load`, which are whole values)."""
+    g = _generator(seed)
+    kind, M, L, dt, G = case["kind"], case["M"], case["layers"], _DTYPES[case["dtype"]], case["group"]
+
+    def weight(N, K, std=None):
+        return _codes_of(_float_weight(g, N, K, K ** -0.5 if std is None else std), G)
+
+    def activations(K):
+        return _quantized(torch.randn(M, K, generator=g, device="cuda").to(dt).to(torch.float16))
+
+    if kind == "linear":
+        weights = [weight(case["N"], case["K"]) for _ in range(L)]
+        return [_product(*activations(case["K"]), *w, G) for w in weights]
+    if kind == "mlp":
+        hidden, inter = case["hidden"], case["inter"]
+        weights = [(weight(2 * inter, hidden), weight(hidden, inter, 1.5 * inter ** -0.5)) for _ in range(L)]
+        out = []
+        for gate_up, down in weights:
+            gu = _product(*activations(hidden), *gate_up, G)
+            h = torch.nn.functional.silu(gu[:, :inter]) * gu[:, inter:]
+            out.append(_product(*_quantized(h), *down, G))
+        return out
+    if kind == "gemm":
+        N, K, out = case["N"], case["K"], []
+        for _ in range(L):
+            w = torch.randint(0, 256, (N, K // 4), generator=g, device="cuda", dtype=torch.uint8)
+            s = torch.empty(K // G, N, device="cuda").uniform_(0.001, 0.01, generator=g).to(torch.float16)
+            x = torch.randint(-127, 128, (M, K), generator=g, device="cuda", dtype=torch.int8)
+            xs = torch.empty(M, device="cuda").uniform_(0.005, 0.02, generator=g)
+            out.append(_product(x, xs, _unpacked(w, case["zero_point"]), s, G))
+        return out
+    codes, scale = _codes_of(_float_weight(g, case["N"], case["K"], case["K"] ** -0.5).to(dt), G)
+    return {"w_packed": None, "w_scale": scale.double(), "y": _product(*activations(case["K"]), codes, scale, G)}
