@@ -109,6 +109,14 @@ int sk_w2a8_unrepack(const uint8_t* w_tiled, int64_t N, int64_t K, uint8_t* w_pa
 int sk_w2a8_plan_create(sk_w2a8_plan** plan, int device, int64_t N, int64_t K, int group_size,
                         int zero_point, const uint8_t* w, int w_layout, const void* w_scale_f16,
                         int out_dtype);
+/* The same plan in device memory the caller provides (sk_w2a8_plan_storage_bytes(...) bytes, 256-byte aligned, kept until
+ * the plan is destroyed and every launch made with it has completed) and without synchronising: the copies are made on
+ * `stream`, and the plan may be used there at once.  Use on another stream must be ordered after it by the caller.
+ * Creation and destruction neither allocate nor free device memory. */
+int64_t sk_w2a8_plan_storage_bytes(int device, int64_t N, int64_t K, int group_size, int w_layout);
+int sk_w2a8_plan_create_in(sk_w2a8_plan** plan, int device, int64_t N, int64_t K, int group_size, int zero_point,
+                           const uint8_t* w, int w_layout, const void* w_scale_f16, int out_dtype, void* storage,
+                           int64_t storage_bytes, sk_stream_t stream);
 int sk_w2a8_plan_destroy(sk_w2a8_plan* plan);
 int sk_w2a8_set_option(sk_w2a8_plan* plan, int key, int64_t value);
 /* What the plan was created with (any out-pointer may be NULL). */
@@ -184,6 +192,13 @@ int sk_w2a8_gemm_debug_partials(sk_w2a8_plan* plan, int64_t M, const int8_t* x_q
  * group_size % 4 == 0, K % group_size == 0, ld_w >= N.  Inputs must be finite. */
 int sk_w2a8_quantize_weight(const float* w, int64_t ld_w, int64_t K, int64_t N, int group_size, uint8_t* w_packed,
                             float* scale_f32, void* scale_f16, sk_stream_t stream);
+
+/* The same codes and fp16 scales from a weight the way a checkpoint holds it, [N, K] row-major (out-features first), in
+ * its own element type: 0 fp16, 1 bf16, 2 fp32 (widened exactly).  One pass, no transposed or fp32 copy.
+ *   w [N, ld_w]; group_size 16, 32, 64, 128, 256 or 512; K % group_size == 0; 16-byte aligned rows; w_packed 4-byte aligned.
+ * SK_ERR_UNAVAILABLE for other group sizes or alignments: sk_w2a8_quantize_weight takes those (transposed, as fp32). */
+int sk_w2a8_quantize_weight_rows(const void* w, int w_type, int64_t ld_w, int64_t N, int64_t K, int group_size,
+                                 uint8_t* w_packed, void* scale_f16, sk_stream_t stream);
 
 /* -------- activation side of the Llama MLP block -----------------------------------------------------
  * The reference has no activation quantiser (its prototype is fed ready-made e4m3 tensors,

@@ -36,6 +36,8 @@ SIGNATURES = {
     "sk_w2a8_repack": (_int, [_vp, _i64, _i64, _vp, _vp]),
     "sk_w2a8_unrepack": (_int, [_vp, _i64, _i64, _vp, _vp]),
     "sk_w2a8_plan_create": (_int, [ctypes.POINTER(_vp), _int, _i64, _i64, _int, _int, _vp, _int, _vp, _int]),
+    "sk_w2a8_plan_storage_bytes": (_i64, [_int, _i64, _i64, _int, _int]),
+    "sk_w2a8_plan_create_in": (_int, [ctypes.POINTER(_vp), _int, _i64, _i64, _int, _int, _vp, _int, _vp, _int, _vp, _i64, _vp]),
     "sk_w2a8_plan_destroy": (_int, [_vp]),
     "sk_w2a8_set_option": (_int, [_vp, _int, _i64]),
     "sk_w2a8_plan_info": (_int, [_vp, ctypes.POINTER(_i64), ctypes.POINTER(_i64), ctypes.POINTER(_int),
@@ -50,6 +52,7 @@ SIGNATURES = {
     "sk_w2a8_debug_stream_cut": (_int, [_i64, _int, _int, _i64, ctypes.POINTER(_i64), ctypes.POINTER(_i64), ctypes.POINTER(_int)]),
     "sk_sum_row_blocks": (_int, [_vp, _int, _i64, _i64, _i64, _i64, _vp, _i64, _int, _vp]),
     "sk_w2a8_quantize_weight": (_int, [_vp, _i64, _i64, _i64, _int, _vp, _vp, _vp, _vp]),
+    "sk_w2a8_quantize_weight_rows": (_int, [_vp, _int, _i64, _i64, _i64, _int, _vp, _vp, _vp]),
     "sk_w2a8_mlp_workspace_bytes": (_i64, [_vp, _vp, _i64]),
     "sk_w2a8_mlp_forward": (_int, [_vp, _vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _vp]),
     "sk_w2a8_mlp_static_scratch_bytes": (_i64, []),

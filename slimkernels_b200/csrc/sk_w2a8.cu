@@ -64,6 +64,51 @@ __global__ void repack_kernel(const uint8_t* __restrict__ w_packed, uint32_t* __
   }
 }
 
+// The same permutation for plan creation, with the scales of a group-size-128 weight tiled in the same launch: one CTA of
+// 128 threads per 4 KiB block, a thread takes one feature's 128 codes (two 16-byte loads, two 16-byte stores; the
+// source line's other three blocks are read by neighbouring CTAs and come from L2).  Rows 16-byte aligned, K % 128 == 0.
+__global__ void __launch_bounds__(128)
+tile_weight_kernel(const uint8_t* __restrict__ w_packed, uint8_t* __restrict__ w_tiled, const __half* __restrict__ w_scale,
+                   __half* __restrict__ w_scale_tiled, long long N, long long K, int k_blocks) {
+  const int r = threadIdx.x;
+  const long long T = blockIdx.y, B = blockIdx.x;
+  const long long block = T * k_blocks + B;
+  const long long n = T * 128 + r;
+  uint4 in[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
+  if (n < N) {
+    const uint4* src = reinterpret_cast<const uint4*>(w_packed + n * (K / 4) + B * 32);
+    in[0] = src[0];
+    in[1] = src[1];
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const uint32_t v[4] = {in[h].x, in[h].y, in[h].z, in[h].w};
+    uint32_t o[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const uint8_t b[4] = {static_cast<uint8_t>(v[c]), static_cast<uint8_t>(v[c] >> 8), static_cast<uint8_t>(v[c] >> 16),
+                            static_cast<uint8_t>(v[c] >> 24)};
+      o[c] = tiled_word_from_bytes(b);
+    }
+    *reinterpret_cast<uint4*>(w_tiled + block * 4096 + h * 2048 + r * 16) = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+  if (w_scale_tiled) w_scale_tiled[block * 128 + r] = n < N ? w_scale[static_cast<size_t>(B) * N + n] : __float2half(0.f);
+}
+
+// The scales of a group-size-128 plan in the order the decode kernels stream them: [n_tiles][k_blocks][128 features]
+// (rows past N are zero), so that the scales of a CTA's K range are one contiguous run.
+__global__ void tile_scales_kernel(const __half* __restrict__ w_scale, __half* __restrict__ tiled, long long N,
+                                   int k_blocks, long long total) {
+  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
+       i += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const int r = static_cast<int>(i % 128);
+    const long long t = i / 128;
+    const int kb = static_cast<int>(t % k_blocks);
+    const long long n = (t / k_blocks) * 128 + r;
+    tiled[i] = n < N ? w_scale[static_cast<size_t>(kb) * N + n] : __float2half(0.f);
+  }
+}
+
 __global__ void unrepack_kernel(const uint32_t* __restrict__ w_tiled, uint8_t* __restrict__ w_packed, long long N,
                                 long long K, int k_blocks, long long total_words) {
   const long long row_bytes = K / 4;
@@ -196,11 +241,12 @@ struct sk_w2a8_plan {
   int G = 128, zero_point = 1, out_dtype = SK_OUT_F16;
   int k_blocks = 0, n_tiles = 0, sm_count = 148;
   const uint8_t* w_rowmajor = nullptr;  // borrowed (may be null when created from a tiled buffer)
-  const uint8_t* w_tiled = nullptr;     // owned or borrowed
-  uint8_t* w_tiled_owned = nullptr;
+  const uint8_t* w_tiled = nullptr;     // in the plan's storage, or borrowed
   const __half* w_scale = nullptr;      // borrowed
   __half* w_scale_tiled = nullptr;      // device, owned: [n_tiles][k_blocks][128] copy of the scales (group size 128 only)
-  int* status = nullptr;                // device, owned
+  int* status = nullptr;                // device; first in the plan's storage, one block that also holds the tiled copies
+  bool external_storage = false;        // the buffers below live in the caller's storage (sk_w2a8_plan_create_in)
+  bool stream_owned = false;            // stream_scratch / stream_counters are the plan's own allocations
   // balanced-split decode kernel: scratch for the partial sums of tiles shared between CTAs, and their counters
   float* stream_scratch = nullptr;      // device, owned (null: that kernel is not available for this plan)
   int* stream_counters = nullptr;       // device, owned; zero between launches
@@ -444,8 +490,13 @@ static void stream_geometry(const sk_w2a8_plan* plan, int want_ctas, int* ctas_o
 // (Re)allocates the scratch buffer and the counters of the balanced-split decode kernel.  Not on the call path: plan
 // creation and sk_w2a8_set_option only.  The device of the plan is current.
 static int stream_setup(sk_w2a8_plan* plan, int want_ctas) {
-  if (plan->stream_scratch) { cudaFree(plan->stream_scratch); plan->stream_scratch = nullptr; }
-  if (plan->stream_counters) { cudaFree(plan->stream_counters); plan->stream_counters = nullptr; }
+  if (plan->stream_owned) {
+    if (plan->stream_scratch) cudaFree(plan->stream_scratch);
+    if (plan->stream_counters) cudaFree(plan->stream_counters);
+  }
+  plan->stream_scratch = nullptr;
+  plan->stream_counters = nullptr;
+  plan->stream_owned = false;
   plan->stream_ctas = plan->stream_slots = 0;
   if (plan->G != 128 || (plan->K % 256) != 0) return SK_OK;   // whole half stages only: the other decode kernel serves the rest
   int ctas = 0, slots = 0;
@@ -462,9 +513,42 @@ static int stream_setup(sk_w2a8_plan* plan, int want_ctas) {
     if (plan->stream_counters) { cudaFree(plan->stream_counters); plan->stream_counters = nullptr; }
     return cuda_fail(plan, e);
   }
+  plan->stream_owned = true;
   plan->stream_ctas = ctas;
   plan->stream_slots = slots;
   return SK_OK;
+}
+
+// Where a plan's buffers sit in one block of storage (256-byte aligned offsets; -1: the plan has no such buffer).
+struct PlanLayout {
+  long long status, w_tiled, w_scale_tiled, stream_scratch, stream_counters, total;
+  size_t counter_bytes;
+};
+static PlanLayout plan_layout(sk_w2a8_plan* plan, int w_layout) {
+  PlanLayout l;
+  long long o = 0;
+  auto take = [&o](long long bytes) {
+    const long long at = o;
+    o += (bytes + 255) & ~255LL;
+    return at;
+  };
+  const long long blocks = static_cast<long long>(plan->n_tiles) * plan->k_blocks;
+  l.status = take(sizeof(int));
+  l.w_tiled = w_layout == SK_WEIGHT_ROWMAJOR ? take(blocks * kWpBytes) : -1;
+  l.w_scale_tiled = plan->G == 128 ? take(blocks * kTileN * static_cast<long long>(sizeof(__half))) : -1;
+  l.stream_scratch = l.stream_counters = -1;
+  l.counter_bytes = 0;
+  // The balanced-split decode kernel's scratch is part of it only where that kernel is the default (large weight
+  // matrices, see choose()); elsewhere it is allocated on request (SK_OPT_KERNEL = 5 / SK_OPT_STREAM_CTAS, set-up calls).
+  if (plan->G == 128 && (plan->K % 256) == 0 && blocks >= 64LL * plan->sm_count) {
+    stream_geometry(plan, 0, &plan->stream_ctas, &plan->stream_slots);
+    l.counter_bytes = static_cast<size_t>(plan->n_tiles) * StreamTraits<32>::kEpiWarps * sizeof(int);
+    l.stream_scratch = take(static_cast<long long>(plan->n_tiles) * plan->stream_slots * StreamTraits<32>::kSlotFloats *
+                            static_cast<long long>(sizeof(float)));
+    l.stream_counters = take(static_cast<long long>(l.counter_bytes));
+  }
+  l.total = o;
+  return l;
 }
 
 constexpr int kPairStages = 6;
@@ -537,21 +621,6 @@ static int resolve_launch(const sk_w2a8_plan* plan, long long M, bool debug_part
   *out = ch;
   return SK_OK;
 }
-
-// The scales of a group-size-128 plan in the order the decode kernels stream them: [n_tiles][k_blocks][128 features]
-// (rows past N are zero), so that the scales of a CTA's K range are one contiguous run.
-__global__ void tile_scales_kernel(const __half* __restrict__ w_scale, __half* __restrict__ tiled, long long N,
-                                   int k_blocks, long long total) {
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int r = static_cast<int>(i % kTileN);
-    const long long t = i / kTileN;
-    const int kb = static_cast<int>(t % k_blocks);
-    const long long n = (t / k_blocks) * kTileN + r;
-    tiled[i] = n < N ? w_scale[static_cast<size_t>(kb) * N + n] : __float2half(0.f);
-  }
-}
-
 
 // Test aid: the expander's shared-memory image of one 128 x 128 weight block next to the image the TMA writes for the
 // same int8 values.  One CTA: (a) copies a 4 KiB tiled block into shared memory and expands it exactly as the general
@@ -859,6 +928,105 @@ static int repack_common(bool forward, const uint8_t* src, long long N, long lon
 // ================================================================================================
 // extern "C"
 // ================================================================================================
+// Plan creation behind both entry points.  storage == nullptr: one cudaMalloc'ed block, the work on the legacy default
+// stream, and the device synchronised before it returns.  Otherwise the caller's block, the work ordered on `stream`, and
+// no synchronisation.
+static int plan_create_common(sk_w2a8_plan** out, int device, int64_t N, int64_t K, int group_size, int zero_point,
+                              const uint8_t* w, int w_layout, const void* w_scale_f16, int out_dtype, void* storage,
+                              int64_t storage_bytes, cudaStream_t stream) {
+  if (!out) return SK_ERR_NULL_POINTER;
+  *out = nullptr;
+  if (!w || !w_scale_f16) return SK_ERR_NULL_POINTER;
+  if (N <= 0 || K <= 0 || N > (1LL << 30) || K > (1LL << 30)) return SK_ERR_BAD_SHAPE;
+  if (group_size <= 0 || (group_size % 32) != 0 || (K % group_size) != 0 || (K % 32) != 0) return SK_ERR_BAD_SHAPE;
+  if (!((group_size % 128) == 0 || (128 % group_size) == 0)) return SK_ERR_BAD_SHAPE;
+  if (zero_point < 0 || zero_point > 3) return SK_ERR_BAD_ARGUMENT;
+  if (out_dtype != SK_OUT_F16 && out_dtype != SK_OUT_BF16) return SK_ERR_BAD_ARGUMENT;
+  if (w_layout != SK_WEIGHT_ROWMAJOR && w_layout != SK_WEIGHT_TILED) return SK_ERR_BAD_ARGUMENT;
+  if ((reinterpret_cast<uintptr_t>(w_scale_f16) & 1) != 0) return SK_ERR_BAD_ALIGNMENT;
+  if (w_layout == SK_WEIGHT_TILED && (reinterpret_cast<uintptr_t>(w) & 15) != 0) return SK_ERR_BAD_ALIGNMENT;
+
+  int ndev = 0;
+  if (cudaGetDeviceCount(&ndev) != cudaSuccess) { (void)cudaGetLastError(); return SK_ERR_CUDA; }
+  if (device < 0 || device >= ndev) return SK_ERR_BAD_ARGUMENT;
+  int major = 0, sms = 0;
+  if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return SK_ERR_CUDA;
+  }
+  if (major != 10) return SK_ERR_UNSUPPORTED_ARCH;
+
+  sk_w2a8_plan* plan = new (std::nothrow) sk_w2a8_plan();
+  if (!plan) return SK_ERR_OUT_OF_MEMORY;
+  plan->device = device;
+  plan->N = N; plan->K = K; plan->G = group_size; plan->zero_point = zero_point; plan->out_dtype = out_dtype;
+  plan->k_blocks = static_cast<int>((K + 127) / 128);
+  plan->n_tiles = static_cast<int>((N + 127) / 128);
+  plan->sm_count = sms;
+  plan->w_scale = static_cast<const __half*>(w_scale_f16);
+  plan->external_storage = storage != nullptr;
+  const sk::PlanLayout l = sk::plan_layout(plan, w_layout);
+  if (storage && storage_bytes < l.total) { delete plan; return SK_ERR_BAD_SHAPE; }
+  plan->maps.reserve(sk::kMapCache + 1);   // the tensor-map cache never grows past kMapCache entries: no host reallocation on the call path
+
+  int cur = -1;
+  cudaGetDevice(&cur);
+  cudaError_t e = cur == device ? cudaSuccess : cudaSetDevice(device);
+  char* base = static_cast<char*>(storage);
+  if (e == cudaSuccess && !base) {
+    void* block = nullptr;
+    e = cudaMalloc(&block, static_cast<size_t>(l.total));
+    base = e == cudaSuccess ? static_cast<char*>(block) : nullptr;
+  }
+  int rc = e == cudaSuccess ? SK_OK : sk::cuda_fail(plan, e);
+  if (rc == SK_OK) {
+    plan->status = reinterpret_cast<int*>(base + l.status);
+    e = cudaMemsetAsync(plan->status, 0, sizeof(int), stream);
+    if (e == cudaSuccess && l.stream_counters >= 0) {
+      plan->stream_scratch = reinterpret_cast<float*>(base + l.stream_scratch);
+      plan->stream_counters = reinterpret_cast<int*>(base + l.stream_counters);
+      e = cudaMemsetAsync(plan->stream_counters, 0, l.counter_bytes, stream);
+    }
+    if (l.w_scale_tiled >= 0) plan->w_scale_tiled = reinterpret_cast<__half*>(base + l.w_scale_tiled);
+    // the decode kernels' copy of the scales is made once, here: later changes of w_scale_f16 are not seen by them
+    bool scales_tiled = plan->w_scale_tiled == nullptr;
+    if (w_layout == SK_WEIGHT_TILED) {
+      plan->w_tiled = w;
+    } else {
+      plan->w_rowmajor = w;
+      uint8_t* tiled = reinterpret_cast<uint8_t*>(base + l.w_tiled);
+      plan->w_tiled = tiled;
+      if (e == cudaSuccess) {
+        if ((K % 128) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 && ((K / 4) % 16) == 0 && plan->n_tiles <= 65535) {
+          sk::tile_weight_kernel<<<dim3(plan->k_blocks, plan->n_tiles), 128, 0, stream>>>(
+              w, tiled, plan->w_scale, plan->w_scale_tiled, N, K, plan->k_blocks);
+          e = cudaGetLastError();
+          scales_tiled = true;
+        } else {
+          rc = sk::repack_common(true, w, N, K, tiled, stream);
+        }
+      }
+    }
+    if (rc == SK_OK && e == cudaSuccess && !scales_tiled) {
+      const long long total = static_cast<long long>(plan->n_tiles) * plan->k_blocks * sk::kTileN;
+      const int blocks = static_cast<int>(total / 256 + 1 < 148 * 8 ? total / 256 + 1 : 148 * 8);
+      sk::tile_scales_kernel<<<blocks, 256, 0, stream>>>(plan->w_scale, plan->w_scale_tiled, N, plan->k_blocks, total);
+      e = cudaGetLastError();
+    }
+    if (rc == SK_OK && e == cudaSuccess && !storage) e = cudaDeviceSynchronize();
+    if (rc == SK_OK && e != cudaSuccess) rc = sk::cuda_fail(plan, e);
+  }
+  if (cur >= 0 && cur != device) (void)cudaSetDevice(cur);
+  if (rc != SK_OK) {
+    if (!storage && base) cudaFree(base);
+    delete plan;
+    return rc;
+  }
+  *out = plan;
+  return SK_OK;
+}
+
 extern "C" {
 
 int sk_w2a8_version(void) { return 100; }
@@ -896,111 +1064,45 @@ int sk_w2a8_unrepack(const uint8_t* w_tiled, int64_t N, int64_t K, uint8_t* w_pa
 
 int sk_w2a8_plan_create(sk_w2a8_plan** out, int device, int64_t N, int64_t K, int group_size, int zero_point,
                         const uint8_t* w, int w_layout, const void* w_scale_f16, int out_dtype) {
-  if (!out) return SK_ERR_NULL_POINTER;
-  *out = nullptr;
-  if (!w || !w_scale_f16) return SK_ERR_NULL_POINTER;
-  if (N <= 0 || K <= 0 || N > (1LL << 30) || K > (1LL << 30)) return SK_ERR_BAD_SHAPE;
-  if (group_size <= 0 || (group_size % 32) != 0 || (K % group_size) != 0 || (K % 32) != 0) return SK_ERR_BAD_SHAPE;
-  if (!((group_size % 128) == 0 || (128 % group_size) == 0)) return SK_ERR_BAD_SHAPE;
-  if (zero_point < 0 || zero_point > 3) return SK_ERR_BAD_ARGUMENT;
-  if (out_dtype != SK_OUT_F16 && out_dtype != SK_OUT_BF16) return SK_ERR_BAD_ARGUMENT;
-  if (w_layout != SK_WEIGHT_ROWMAJOR && w_layout != SK_WEIGHT_TILED) return SK_ERR_BAD_ARGUMENT;
-  if ((reinterpret_cast<uintptr_t>(w_scale_f16) & 1) != 0) return SK_ERR_BAD_ALIGNMENT;
-  if (w_layout == SK_WEIGHT_TILED && (reinterpret_cast<uintptr_t>(w) & 15) != 0) return SK_ERR_BAD_ALIGNMENT;
+  return plan_create_common(out, device, N, K, group_size, zero_point, w, w_layout, w_scale_f16, out_dtype, nullptr, 0, nullptr);
+}
 
-  int ndev = 0;
-  if (cudaGetDeviceCount(&ndev) != cudaSuccess) { (void)cudaGetLastError(); return SK_ERR_CUDA; }
-  if (device < 0 || device >= ndev) return SK_ERR_BAD_ARGUMENT;
-  int major = 0, sms = 0;
-  if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+int64_t sk_w2a8_plan_storage_bytes(int device, int64_t N, int64_t K, int group_size, int w_layout) {
+  if (N <= 0 || K <= 0 || N > (1LL << 30) || K > (1LL << 30) || group_size <= 0) return 0;
+  sk_w2a8_plan probe;
+  if (cudaDeviceGetAttribute(&probe.sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
     (void)cudaGetLastError();
-    return SK_ERR_CUDA;
+    return 0;
   }
-  if (major != 10) return SK_ERR_UNSUPPORTED_ARCH;
+  probe.N = N; probe.K = K; probe.G = group_size;
+  probe.k_blocks = static_cast<int>((K + 127) / 128);
+  probe.n_tiles = static_cast<int>((N + 127) / 128);
+  return sk::plan_layout(&probe, w_layout).total;
+}
 
-  sk_w2a8_plan* plan = new (std::nothrow) sk_w2a8_plan();
-  if (!plan) return SK_ERR_OUT_OF_MEMORY;
-  plan->device = device;
-  plan->N = N; plan->K = K; plan->G = group_size; plan->zero_point = zero_point; plan->out_dtype = out_dtype;
-  plan->k_blocks = static_cast<int>((K + 127) / 128);
-  plan->n_tiles = static_cast<int>((N + 127) / 128);
-  plan->sm_count = sms;
-  plan->w_scale = static_cast<const __half*>(w_scale_f16);
-  plan->maps.reserve(sk::kMapCache + 1);   // the tensor-map cache never grows past kMapCache entries: no host reallocation on the call path
-
-  int cur = -1;
-  cudaGetDevice(&cur);
-  cudaError_t e = cudaSetDevice(device);
-  int rc = SK_OK;
-  if (e != cudaSuccess) rc = sk::cuda_fail(plan, e);
-  if (rc == SK_OK) {
-    e = cudaMalloc(&plan->status, sizeof(int));
-    if (e != cudaSuccess) rc = sk::cuda_fail(plan, e);
-    else {
-      e = cudaMemset(plan->status, 0, sizeof(int));
-      if (e != cudaSuccess) rc = sk::cuda_fail(plan, e);
-    }
-  }
-  if (rc == SK_OK) {
-    if (w_layout == SK_WEIGHT_TILED) {
-      plan->w_tiled = w;
-    } else {
-      plan->w_rowmajor = w;
-      e = cudaMalloc(&plan->w_tiled_owned, static_cast<size_t>(sk_w2a8_tiled_bytes(N, K)));
-      if (e != cudaSuccess) rc = sk::cuda_fail(plan, e);
-      else {
-        rc = sk::repack_common(true, w, N, K, plan->w_tiled_owned, nullptr);
-        if (rc == SK_OK) {
-          e = cudaDeviceSynchronize();
-          if (e != cudaSuccess) rc = sk::cuda_fail(plan, e);
-        }
-        plan->w_tiled = plan->w_tiled_owned;
-      }
-    }
-  }
-  if (rc == SK_OK && group_size == 128) {
-    // the decode kernels' copy of the scales (made once, here: later changes of w_scale_f16 are not seen by them)
-    const long long total = static_cast<long long>(plan->n_tiles) * plan->k_blocks * sk::kTileN;
-    e = cudaMalloc(&plan->w_scale_tiled, static_cast<size_t>(total) * sizeof(__half));
-    if (e != cudaSuccess) { plan->w_scale_tiled = nullptr; rc = sk::cuda_fail(plan, e); }
-    else {
-      const int blocks = static_cast<int>(total / 256 + 1 < 148 * 8 ? total / 256 + 1 : 148 * 8);
-      sk::tile_scales_kernel<<<blocks, 256>>>(plan->w_scale, plan->w_scale_tiled, N, plan->k_blocks, total);
-      e = cudaGetLastError();
-      if (e == cudaSuccess) e = cudaDeviceSynchronize();
-      if (e != cudaSuccess) rc = sk::cuda_fail(plan, e);
-    }
-  }
-  // The balanced-split decode kernel's scratch is allocated here only where that kernel is the default (large weight
-  // matrices, see choose()); elsewhere on request (SK_OPT_KERNEL = 5 / SK_OPT_STREAM_CTAS, set-up calls).
-  if (rc == SK_OK && static_cast<long long>(plan->n_tiles) * plan->k_blocks >= 64LL * plan->sm_count)
-    rc = sk::stream_setup(plan, 0);
-  if (cur >= 0 && cur != device) (void)cudaSetDevice(cur);
-  if (rc != SK_OK) {
-    if (plan->status) cudaFree(plan->status);
-    if (plan->w_tiled_owned) cudaFree(plan->w_tiled_owned);
-    if (plan->stream_scratch) cudaFree(plan->stream_scratch);
-    if (plan->stream_counters) cudaFree(plan->stream_counters);
-    if (plan->w_scale_tiled) cudaFree(plan->w_scale_tiled);
-    delete plan;
-    return rc;
-  }
-  *out = plan;
-  return SK_OK;
+int sk_w2a8_plan_create_in(sk_w2a8_plan** out, int device, int64_t N, int64_t K, int group_size, int zero_point,
+                           const uint8_t* w, int w_layout, const void* w_scale_f16, int out_dtype, void* storage,
+                           int64_t storage_bytes, sk_stream_t stream) {
+  if (out) *out = nullptr;
+  if (!storage) return SK_ERR_NULL_POINTER;
+  if (reinterpret_cast<uintptr_t>(storage) & 255) return SK_ERR_BAD_ALIGNMENT;
+  return plan_create_common(out, device, N, K, group_size, zero_point, w, w_layout, w_scale_f16, out_dtype, storage, storage_bytes,
+                            static_cast<cudaStream_t>(stream));
 }
 
 int sk_w2a8_plan_destroy(sk_w2a8_plan* plan) {
   if (!plan) return SK_ERR_NULL_POINTER;
-  int cur = -1;
-  cudaGetDevice(&cur);
-  (void)cudaSetDevice(plan->device);
-  if (plan->status) cudaFree(plan->status);
-  if (plan->w_tiled_owned) cudaFree(plan->w_tiled_owned);
-  if (plan->stream_scratch) cudaFree(plan->stream_scratch);
-  if (plan->stream_counters) cudaFree(plan->stream_counters);
-  if (plan->w_scale_tiled) cudaFree(plan->w_scale_tiled);
-  if (cur >= 0 && cur != plan->device) (void)cudaSetDevice(cur);
+  if (!plan->external_storage || plan->stream_owned) {
+    int cur = -1;
+    cudaGetDevice(&cur);
+    (void)cudaSetDevice(plan->device);
+    if (plan->stream_owned) {
+      cudaFree(plan->stream_scratch);
+      cudaFree(plan->stream_counters);
+    }
+    if (!plan->external_storage && plan->status) cudaFree(plan->status);   // the block holds all the other buffers
+    if (cur >= 0 && cur != plan->device) (void)cudaSetDevice(cur);
+  }
   delete plan;
   return SK_OK;
 }
@@ -1246,6 +1348,31 @@ int sk_w2a8_quantize_weight(const float* w, int64_t ld_w, int64_t K, int64_t N, 
   }
   sk::quantize_pack_weight_kernel<<<grid, sk::kPrepCtaThreads, kPrepSmem, static_cast<cudaStream_t>(stream)>>>(
       w, ld_w, static_cast<int>(K), static_cast<int>(N), group_size, w_packed, scale_f32, static_cast<__half*>(scale_f16));
+  if (cudaGetLastError() != cudaSuccess) return SK_ERR_CUDA;
+  return SK_OK;
+}
+
+int sk_w2a8_quantize_weight_rows(const void* w, int w_type, int64_t ld_w, int64_t N, int64_t K, int group_size,
+                                 uint8_t* w_packed, void* scale_f16, sk_stream_t stream) {
+  if (!w || !w_packed || !scale_f16) return SK_ERR_NULL_POINTER;
+  if (w_type != sk::kRowsF16 && w_type != sk::kRowsBf16 && w_type != sk::kRowsF32) return SK_ERR_BAD_ARGUMENT;
+  if (K <= 0 || N <= 0 || group_size <= 0 || (group_size % 4) != 0 || (K % group_size) != 0 || ld_w < K ||
+      K > (1LL << 30) || N > (1LL << 30))
+    return SK_ERR_BAD_SHAPE;
+  if (reinterpret_cast<uintptr_t>(scale_f16) & 1) return SK_ERR_BAD_ALIGNMENT;
+  const int elem = w_type == sk::kRowsF32 ? 4 : 2;
+  const int64_t row_ctas = (N + sk::kRowsPerCta - 1) / sk::kRowsPerCta;
+  if (group_size < 16 || group_size > sk::kRowsChunk || (group_size & (group_size - 1)) != 0 || row_ctas > 65535 ||
+      (reinterpret_cast<uintptr_t>(w) & 15) || ((ld_w * elem) % 16) != 0 || (reinterpret_cast<uintptr_t>(w_packed) & 3))
+    return SK_ERR_UNAVAILABLE;
+  const dim3 grid(static_cast<unsigned>((K + sk::kRowsChunk - 1) / sk::kRowsChunk), static_cast<unsigned>(row_ctas));
+  auto* s16 = static_cast<__half*>(scale_f16);
+  const auto st = static_cast<cudaStream_t>(stream);
+  const int k = static_cast<int>(K), n = static_cast<int>(N);
+  constexpr int threads = 32 * sk::kRowsWarps;
+  if (w_type == sk::kRowsF16) sk::quantize_pack_rows_kernel<sk::kRowsF16><<<grid, threads, 0, st>>>(w, ld_w, k, n, group_size, w_packed, s16);
+  else if (w_type == sk::kRowsBf16) sk::quantize_pack_rows_kernel<sk::kRowsBf16><<<grid, threads, 0, st>>>(w, ld_w, k, n, group_size, w_packed, s16);
+  else sk::quantize_pack_rows_kernel<sk::kRowsF32><<<grid, threads, 0, st>>>(w, ld_w, k, n, group_size, w_packed, s16);
   if (cudaGetLastError() != cudaSuccess) return SK_ERR_CUDA;
   return SK_OK;
 }

@@ -2,9 +2,13 @@
 // Registers the ops of namespace `slimkernels` used by slimkernels_b200/torch/ops.py.
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <cuda_runtime.h>
 #include <torch/library.h>
 #include <torch/types.h>
 
+#include <algorithm>
+#include <atomic>
+#include <memory>
 #include <mutex>
 #include <vector>
 
@@ -16,9 +20,46 @@ void check(int rc, const char* what) {
   TORCH_CHECK(rc == SK_OK, "slimkernels::", what, " failed: ", sk_status_string(rc), " (", rc, ")");
 }
 
-sk_w2a8_plan* as_plan(int64_t handle) {
+// What a plan handle points to.  The plan's device buffers are one tensor from PyTorch's caching allocator and are filled
+// on the stream that is current at creation, so making and dropping a plan neither calls cudaMalloc / cudaFree nor
+// synchronises (both did, several times per plan: about 0.6 ms of a checkpoint layer's load).  Use on that stream is ordered by itself.
+// The first use on another stream waits for the filling on the host (once), and every use there is recorded with the
+// allocator, so that the memory is not handed out again before that stream is done with it.
+struct TorchPlan {
+  sk_w2a8_plan* plan = nullptr;
+  at::Tensor storage;
+  c10::cuda::CUDAStream home;
+  cudaEvent_t filled = nullptr;
+  std::atomic<bool> waited{false};
+  explicit TorchPlan(c10::cuda::CUDAStream s) : home(s) {}
+  ~TorchPlan() {
+    if (plan) sk_w2a8_plan_destroy(plan);
+    if (filled) cudaEventDestroy(filled);
+  }
+};
+
+TorchPlan* as_torch_plan(int64_t handle) {
   TORCH_CHECK(handle != 0, "slimkernels: null plan handle");
-  return reinterpret_cast<sk_w2a8_plan*>(static_cast<intptr_t>(handle));
+  return reinterpret_cast<TorchPlan*>(static_cast<intptr_t>(handle));
+}
+
+sk_w2a8_plan* as_plan(int64_t handle) { return as_torch_plan(handle)->plan; }
+
+// The plan, for a launch on `stream` (of the plan's device).
+sk_w2a8_plan* plan_on(int64_t handle, c10::cuda::CUDAStream stream) {
+  TorchPlan* t = as_torch_plan(handle);
+  if (stream != t->home) {
+    if (!t->waited.load(std::memory_order_acquire)) {
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;    // a capture elsewhere must not forbid the wait
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      const cudaError_t e = cudaEventSynchronize(t->filled);
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      TORCH_CHECK(e == cudaSuccess, "slimkernels: waiting for a plan failed: ", cudaGetErrorString(e));
+      t->waited.store(true, std::memory_order_release);
+    }
+    t->storage.record_stream(c10::Stream(stream));
+  }
+  return t->plan;
 }
 
 int64_t plan_create(const at::Tensor& w, const at::Tensor& w_scale, int64_t N, int64_t K, int64_t group_size,
@@ -35,15 +76,26 @@ int64_t plan_create(const at::Tensor& w, const at::Tensor& w_scale, int64_t N, i
     TORCH_CHECK(w.dim() == 2 && w.size(0) == N && w.size(1) * 4 == K, "w_packed must have shape [N, K/4]");
   }
   c10::cuda::CUDAGuard guard(w.device());
-  sk_w2a8_plan* plan = nullptr;
-  check(sk_w2a8_plan_create(&plan, w.get_device(), N, K, static_cast<int>(group_size), static_cast<int>(zero_point),
-                            w.data_ptr<uint8_t>(), tiled ? SK_WEIGHT_TILED : SK_WEIGHT_ROWMAJOR, w_scale.data_ptr(),
-                            bf16_out ? SK_OUT_BF16 : SK_OUT_F16),
+  const auto stream = at::cuda::getCurrentCUDAStream();
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  TORCH_CHECK(cudaStreamIsCapturing(stream.stream(), &capturing) == cudaSuccess && capturing == cudaStreamCaptureStatusNone,
+              "slimkernels::w2a8_plan_create: a plan cannot be made while its stream is being captured");
+  const int layout = tiled ? SK_WEIGHT_TILED : SK_WEIGHT_ROWMAJOR;
+  auto t = std::make_unique<TorchPlan>(stream);
+  // (arguments the plan refuses are refused before the storage is asked for)
+  const int64_t bytes = std::max<int64_t>(256, sk_w2a8_plan_storage_bytes(w.get_device(), N, K, static_cast<int>(group_size), layout));
+  t->storage = at::empty({bytes}, w.options().dtype(at::kByte));     // caching allocator: 512-byte aligned
+  check(sk_w2a8_plan_create_in(&t->plan, w.get_device(), N, K, static_cast<int>(group_size), static_cast<int>(zero_point),
+                               w.data_ptr<uint8_t>(), layout, w_scale.data_ptr(), bf16_out ? SK_OUT_BF16 : SK_OUT_F16,
+                               t->storage.data_ptr(), bytes, stream.stream()),
         "w2a8_plan_create");
-  return static_cast<int64_t>(reinterpret_cast<intptr_t>(plan));
+  TORCH_CHECK(cudaEventCreateWithFlags(&t->filled, cudaEventDisableTiming) == cudaSuccess &&
+                  cudaEventRecord(t->filled, stream.stream()) == cudaSuccess,
+              "slimkernels::w2a8_plan_create: recording an event failed");
+  return static_cast<int64_t>(reinterpret_cast<intptr_t>(t.release()));
 }
 
-void plan_destroy(int64_t handle) { check(sk_w2a8_plan_destroy(as_plan(handle)), "w2a8_plan_destroy"); }
+void plan_destroy(int64_t handle) { delete as_torch_plan(handle); }
 
 void plan_set_option(int64_t handle, int64_t key, int64_t value) {
   check(sk_w2a8_set_option(as_plan(handle), static_cast<int>(key), value), "w2a8_set_option");
@@ -73,7 +125,7 @@ void gemm_out(int64_t handle, const at::Tensor& x_q, const at::Tensor& x_scale, 
   if (M == 0) return;
   c10::cuda::CUDAGuard guard(x_q.device());
   auto stream = at::cuda::getCurrentCUDAStream();
-  check(sk_w2a8_gemm(as_plan(handle), M, x_q.data_ptr<int8_t>(), x_q.stride(0), x_scale.data_ptr<float>(),
+  check(sk_w2a8_gemm(plan_on(handle, stream), M, x_q.data_ptr<int8_t>(), x_q.stride(0), x_scale.data_ptr<float>(),
                      out.data_ptr(), out.stride(0), stream.stream()),
         "w2a8_gemm");
 }
@@ -91,7 +143,7 @@ void gemm_scatter(int64_t handle, const at::Tensor& x_q, const at::Tensor& x_sca
   for (int64_t v : out_ptrs) ptrs.push_back(reinterpret_cast<void*>(static_cast<intptr_t>(v)));
   c10::cuda::CUDAGuard guard(x_q.device());
   auto stream = at::cuda::getCurrentCUDAStream();
-  check(sk_w2a8_gemm_scatter(as_plan(handle), M, x_q.data_ptr<int8_t>(), x_q.stride(0), x_scale.data_ptr<float>(),
+  check(sk_w2a8_gemm_scatter(plan_on(handle, stream), M, x_q.data_ptr<int8_t>(), x_q.stride(0), x_scale.data_ptr<float>(),
                              ptrs.data(), static_cast<int>(ptrs.size()), ld_out, col_offset, stream.stream()),
         "w2a8_gemm_scatter");
 }
@@ -109,7 +161,7 @@ void gemm_rowscatter(int64_t handle, const at::Tensor& x_q, const at::Tensor& x_
   for (int64_t v : out_ptrs) ptrs.push_back(reinterpret_cast<void*>(static_cast<intptr_t>(v)));
   c10::cuda::CUDAGuard guard(x_q.device());
   auto stream = at::cuda::getCurrentCUDAStream();
-  check(sk_w2a8_gemm_rowscatter(as_plan(handle), M, x_q.data_ptr<int8_t>(), x_q.stride(0), x_scale.data_ptr<float>(),
+  check(sk_w2a8_gemm_rowscatter(plan_on(handle, stream), M, x_q.data_ptr<int8_t>(), x_q.stride(0), x_scale.data_ptr<float>(),
                                 ptrs.data(), static_cast<int>(ptrs.size()), rows_per_dest, dst_row0, ld_out,
                                 stream.stream()),
         "w2a8_gemm_rowscatter");
@@ -143,7 +195,7 @@ at::Tensor partials(int64_t handle, const at::Tensor& x_q, int64_t N, int64_t K,
   if (M == 0) return out;
   c10::cuda::CUDAGuard guard(x_q.device());
   auto stream = at::cuda::getCurrentCUDAStream();
-  check(sk_w2a8_gemm_debug_partials(as_plan(handle), M, x_q.data_ptr<int8_t>(), x_q.stride(0), out.data_ptr<int32_t>(),
+  check(sk_w2a8_gemm_debug_partials(plan_on(handle, stream), M, x_q.data_ptr<int8_t>(), x_q.stride(0), out.data_ptr<int32_t>(),
                                     stream.stream()),
         "w2a8_gemm_debug_partials");
   return out;
@@ -165,6 +217,31 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> quantize_weight(const at::Tensor&
                                 at::cuda::getCurrentCUDAStream().stream()),
         "w2a8_quantize_weight");
   return {packed, s16, s32};
+}
+
+// W[N, K] (fp16 / bf16 / fp32, out-features first) -> (w_packed uint8 [N, K/4], w_scale float16 [K/G, N])
+std::tuple<at::Tensor, at::Tensor> quantize_weight_rows(const at::Tensor& w_in, int64_t group_size) {
+  TORCH_CHECK(w_in.is_cuda() && w_in.dim() == 2, "w must be a 2-D CUDA tensor [N, K]");
+  const at::ScalarType t = w_in.scalar_type();
+  TORCH_CHECK(t == at::kHalf || t == at::kBFloat16 || t == at::kFloat, "w must be float16, bfloat16 or float32");
+  const int64_t N = w_in.size(0), K = w_in.size(1);
+  TORCH_CHECK(group_size > 0 && group_size % 4 == 0 && K % group_size == 0, "K must be a multiple of group_size (a multiple of 4)");
+  if (K > 0 && N > 0) {
+    const at::Tensor w = w_in.stride(1) == 1 && w_in.stride(0) >= K ? w_in : w_in.contiguous();
+    at::Tensor packed = at::empty({N, K / 4}, w.options().dtype(at::kByte));
+    at::Tensor s16 = at::empty({K / group_size, N}, w.options().dtype(at::kHalf));
+    c10::cuda::CUDAGuard guard(w.device());
+    const int rc = sk_w2a8_quantize_weight_rows(w.data_ptr(), t == at::kHalf ? 0 : t == at::kBFloat16 ? 1 : 2, N == 1 ? K : w.stride(0), N, K,
+                                                static_cast<int>(group_size), packed.data_ptr<uint8_t>(), s16.data_ptr(),
+                                                at::cuda::getCurrentCUDAStream().stream());
+    if (rc != SK_ERR_UNAVAILABLE) {
+      check(rc, "w2a8_quantize_weight_rows");
+      return {packed, s16};
+    }
+  }
+  // group sizes and alignments the row kernel does not take
+  auto [packed, s16, s32] = quantize_weight(w_in.to(at::kFloat).t().contiguous(), group_size);
+  return {packed, s16};
 }
 
 std::tuple<at::Tensor, at::Tensor> quantize_activation(const at::Tensor& x) {
@@ -205,8 +282,9 @@ at::Tensor mlp_forward(int64_t gate_up_plan, int64_t down_plan, const at::Tensor
   TORCH_CHECK(bytes > 0, "slimkernels::w2a8_mlp_forward: the two plans do not form an MLP block");
   at::Tensor ws = at::empty({bytes}, x.options().dtype(at::kByte));     // caching allocator: 512-byte aligned
   c10::cuda::CUDAGuard guard(x.device());
-  check(sk_w2a8_mlp_forward(as_plan(gate_up_plan), as_plan(down_plan), M, x.data_ptr(), x.stride(0), out.data_ptr(),
-                            out.stride(0), ws.data_ptr(), bytes, at::cuda::getCurrentCUDAStream().stream()),
+  const auto stream = at::cuda::getCurrentCUDAStream();
+  check(sk_w2a8_mlp_forward(plan_on(gate_up_plan, stream), plan_on(down_plan, stream), M, x.data_ptr(), x.stride(0),
+                            out.data_ptr(), out.stride(0), ws.data_ptr(), bytes, stream.stream()),
         "w2a8_mlp_forward");
   return out;
 }
@@ -264,19 +342,19 @@ struct CachedPlan {
   int64_t w_version, s_version;
   int64_t group_size, zero_point;
   bool bf16;
-  sk_w2a8_plan* plan;
+  int64_t plan;      // handle
 };
 std::mutex g_cache_mu;
-std::vector<CachedPlan> g_cache;
+std::vector<CachedPlan>& g_cache = *new std::vector<CachedPlan>();   // (never destroyed: CUDA may be gone by then)
 constexpr size_t kMaxCachedPlans = 512;
 
-sk_w2a8_plan* cached_plan(const at::Tensor& w_packed, const at::Tensor& w_scale, int64_t group_size, int64_t zero_point,
+int64_t cached_plan(const at::Tensor& w_packed, const at::Tensor& w_scale, int64_t group_size, int64_t zero_point,
                           bool bf16) {
   TORCH_CHECK(w_packed.is_cuda() && w_packed.scalar_type() == at::kByte && w_packed.is_contiguous() && w_packed.dim() == 2,
               "w_packed must be a contiguous 2-D CUDA uint8 tensor [N, K/4]");
   const int64_t N = w_packed.size(0), K = w_packed.size(1) * 4;
   std::lock_guard<std::mutex> lock(g_cache_mu);
-  sk_w2a8_plan* hit = nullptr;
+  int64_t hit = 0;
   for (size_t i = 0; i < g_cache.size();) {
     CachedPlan& e = g_cache[i];
     const bool dead = e.w.expired() || e.s.expired();
@@ -285,7 +363,7 @@ sk_w2a8_plan* cached_plan(const at::Tensor& w_packed, const at::Tensor& w_scale,
                       e.group_size == group_size && e.zero_point == zero_point && e.bf16 == bf16;
     const bool stale = same && (e.w_version != w_packed._version() || e.s_version != w_scale._version());
     if (dead || stale) {
-      sk_w2a8_plan_destroy(e.plan);
+      plan_destroy(e.plan);
       g_cache[i] = g_cache.back();
       g_cache.pop_back();
       continue;
@@ -295,14 +373,14 @@ sk_w2a8_plan* cached_plan(const at::Tensor& w_packed, const at::Tensor& w_scale,
   }
   if (hit) return hit;
   if (g_cache.size() >= kMaxCachedPlans) {      // oldest first
-    sk_w2a8_plan_destroy(g_cache.front().plan);
+    plan_destroy(g_cache.front().plan);
     g_cache.erase(g_cache.begin());
   }
   const int64_t handle = plan_create(w_packed, w_scale, N, K, group_size, zero_point, bf16, /*tiled=*/false);
   CachedPlan e{c10::weak_intrusive_ptr<c10::TensorImpl>(w_packed.getIntrusivePtr()),
                c10::weak_intrusive_ptr<c10::TensorImpl>(w_scale.getIntrusivePtr()),
                w_packed.data_ptr(), w_scale.data_ptr(), w_packed._version(), w_scale._version(),
-               group_size, zero_point, bf16, as_plan(handle)};
+               group_size, zero_point, bf16, handle};
   g_cache.push_back(e);
   return e.plan;
 }
@@ -311,14 +389,14 @@ at::Tensor w2a8_gemm_op(const at::Tensor& x_q, const at::Tensor& x_scale, const 
                         const at::Tensor& w_scale, int64_t group_size, int64_t zero_point, at::ScalarType out_dtype) {
   TORCH_CHECK(out_dtype == at::kHalf || out_dtype == at::kBFloat16, "out_dtype must be float16 or bfloat16");
   const bool bf16 = out_dtype == at::kBFloat16;
-  sk_w2a8_plan* plan = cached_plan(w_packed, w_scale, group_size, zero_point, bf16);
-  return gemm(static_cast<int64_t>(reinterpret_cast<intptr_t>(plan)), x_q, x_scale, w_packed.size(0), w_packed.size(1) * 4, bf16);
+  const int64_t plan = cached_plan(w_packed, w_scale, group_size, zero_point, bf16);
+  return gemm(plan, x_q, x_scale, w_packed.size(0), w_packed.size(1) * 4, bf16);
 }
 
 at::Tensor w2a8_partials_op(const at::Tensor& x_q, const at::Tensor& w_packed, const at::Tensor& w_scale,
                             int64_t group_size, int64_t zero_point) {
-  sk_w2a8_plan* plan = cached_plan(w_packed, w_scale, group_size, zero_point, false);
-  return partials(static_cast<int64_t>(reinterpret_cast<intptr_t>(plan)), x_q, w_packed.size(0), w_packed.size(1) * 4, group_size);
+  const int64_t plan = cached_plan(w_packed, w_scale, group_size, zero_point, false);
+  return partials(plan, x_q, w_packed.size(0), w_packed.size(1) * 4, group_size);
 }
 
 int64_t cached_plan_count() {
@@ -348,6 +426,7 @@ TORCH_LIBRARY(slimkernels, m) {
   m.def("w2a8_plan_launch_floor_probe(int plan, Tensor on_device_of, int M) -> ()", &launch_floor_probe);
   m.def("quantize_activation_int8(Tensor x) -> (Tensor, Tensor)", &quantize_activation);
   m.def("w2a8_quantize_weight(Tensor w_kn, int group_size) -> (Tensor, Tensor, Tensor)", &quantize_weight);
+  m.def("w2a8_quantize_weight_rows(Tensor w_nk, int group_size) -> (Tensor, Tensor)", &quantize_weight_rows);
   m.def("silu_mul_quantize_int8(Tensor gate_up) -> (Tensor, Tensor)", &silu_mul_quantize);
   m.def("w2a8_mlp_forward(int gate_up_plan, int down_plan, Tensor x, int hidden_out, bool bf16_out) -> Tensor", &mlp_forward);
   m.def("w2a8_repack(Tensor w_packed) -> Tensor", &repack);

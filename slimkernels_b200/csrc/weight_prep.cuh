@@ -161,4 +161,119 @@ quantize_pack_weight_kernel(const float* __restrict__ w, long long ld_w, int K, 
   }
 }
 
+// ------------------------------------------------------------------------------------------------
+// The same codes and scales from a weight the way a checkpoint holds it: [N, K] row-major (out-features first) in fp16,
+// bf16 or fp32, so a scale group is a run of consecutive elements.  One pass: the element type is widened in registers
+// (exact), nothing is transposed, no fp32 copy is made.
+//
+// A warp takes 512 elements of a row (16 per lane), a group is 1 .. 32 neighbouring lanes; four rows per warp keep 8 (16
+// for fp32) 16-byte loads in flight per lane.  A CTA covers 32 rows x 512 columns; its scales are collected in shared
+// memory because they are stored group-major ([K / G, N]): 64-byte runs instead of scattered halves.
+// A 11008 x 4096 fp16 weight loaded and used once (W2A8Linear.from_float, plan, first GEMM) took 861 us through an fp32
+// copy, its transpose and a plan that allocated and synchronised; 63 us with this pass and a plan in given storage.
+// Requires G = 16 .. 512, a power of two; K % G == 0; rows 16-byte aligned.
+//
+// The quantiser compares instead of dividing.  With q = fl(x / s):  code = clip(rint(q) + 1, 0, 3) = [q >= -1/2] + [q > 1/2]
+// + [q >= 3/2]  (ties to even: -1/2 -> 0, 1/2 -> 0, 3/2 -> 2).
+//   * fl(x / s) > 1/2  <=>  x > s / 2: s / 2 is exact (s >= 1e-9 / 1.5 is normal), and the next float above it divided by
+//     s lies at least half an ulp above 1/2, so it rounds above 1/2.  The same for -1/2.
+//   * fl(x / s) is monotonic in x, so q >= 3/2 has a smallest x too; it is within two floats of fl(1.5 s) and found there
+//     with the division itself, once per group.
+// (s = inf, from an infinite weight, takes quantize_code.)
+// ------------------------------------------------------------------------------------------------
+constexpr int kRowsChunk = 512;          // elements of a row per warp
+constexpr int kRowsPerWarp = 4;
+constexpr int kRowsWarps = 8;
+constexpr int kRowsPerCta = kRowsPerWarp * kRowsWarps;
+
+__device__ __forceinline__ float threehalves_threshold(float s) {
+  const int c = __float_as_int(1.5f * s);
+  float t = __int_as_float(0x7fc00000);            // (never met: q < 3/2 for every x)
+#pragma unroll
+  for (int d = 1; d >= -2; --d) {
+    const float x = __int_as_float(c + d);
+    if (__fdiv_rn(x, s) >= 1.5f) t = x;
+  }
+  return t;
+}
+
+enum : int { kRowsF16 = 0, kRowsBf16 = 1, kRowsF32 = 2 };
+template <int TYPE> struct RowVec { static constexpr int kVecs = TYPE == kRowsF32 ? 4 : 2; uint4 v[kVecs]; };   // 16 elements
+template <int TYPE>
+__device__ __forceinline__ float row_element(const RowVec<TYPE>& r, int i) {   // i is a compile-time constant after unrolling
+  if constexpr (TYPE == kRowsF32) {
+    const uint32_t w[4] = {r.v[i >> 2].x, r.v[i >> 2].y, r.v[i >> 2].z, r.v[i >> 2].w};
+    return __uint_as_float(w[i & 3]);
+  } else {
+    const uint32_t w[4] = {r.v[i >> 3].x, r.v[i >> 3].y, r.v[i >> 3].z, r.v[i >> 3].w};
+    const uint32_t h = w[(i >> 1) & 3];
+    if constexpr (TYPE == kRowsBf16) return __uint_as_float((i & 1) ? (h & 0xffff0000u) : (h << 16));
+    else return __half2float(__ushort_as_half(static_cast<unsigned short>((i & 1) ? (h >> 16) : (h & 0xffffu))));
+  }
+}
+
+template <int TYPE>
+__global__ void __launch_bounds__(32 * kRowsWarps)
+quantize_pack_rows_kernel(const void* __restrict__ w, long long ld_w, int K, int N, int G, uint8_t* __restrict__ w_packed,
+                          __half* __restrict__ scale_f16) {
+  constexpr int kElem = TYPE == kRowsF32 ? 4 : 2;
+  __shared__ __half scales[kRowsChunk / 16][kRowsPerCta];      // [group of the chunk][row]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int k0 = blockIdx.x * kRowsChunk;
+  const int k = k0 + lane * 16;
+  const int lanes = G >> 4;                                    // lanes per group
+  const int n_cta = blockIdx.y * kRowsPerCta;
+  const int n_warp = n_cta + warp * kRowsPerWarp;
+  const bool k_ok = k < K;                                     // (whole groups: K % G == 0)
+  RowVec<TYPE> rows[kRowsPerWarp];
+#pragma unroll
+  for (int r = 0; r < kRowsPerWarp; ++r) {
+    const int n = n_warp + r;
+    if (k_ok && n < N) {
+      const uint4* src = reinterpret_cast<const uint4*>(static_cast<const uint8_t*>(w) +
+                                                        (static_cast<long long>(n) * ld_w + k) * kElem);
+#pragma unroll
+      for (int i = 0; i < RowVec<TYPE>::kVecs; ++i) rows[r].v[i] = __ldcs(src + i);
+    } else {
+#pragma unroll
+      for (int i = 0; i < RowVec<TYPE>::kVecs; ++i) rows[r].v[i] = make_uint4(0u, 0u, 0u, 0u);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < kRowsPerWarp; ++r) {
+    float x[16];
+    float amax = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      x[i] = row_element<TYPE>(rows[r], i);
+      amax = fmaxf(amax, fabsf(x[i]));
+    }
+    for (int o = 1; o < lanes; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    const float s = __fdiv_rn(fmaxf(amax, 1e-9f), 1.5f);
+    const float half = 0.5f * s;
+    const float t3 = threehalves_threshold(s);
+    uint32_t word = 0;
+    if (s < __int_as_float(0x7f800000)) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const uint32_t code = (x[i] >= -half ? 1u : 0u) + (x[i] > half ? 1u : 0u) + (x[i] >= t3 ? 1u : 0u);
+        word |= code << (8 * (i >> 2) + 6 - 2 * (i & 3));
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) word |= quantize_code(x[i], s) << (8 * (i >> 2) + 6 - 2 * (i & 3));
+    }
+    const int n = n_warp + r;
+    if (k_ok && n < N) *reinterpret_cast<uint32_t*>(w_packed + static_cast<long long>(n) * (K / 4) + k / 4) = word;
+    if ((lane & (lanes - 1)) == 0) scales[lane / lanes][warp * kRowsPerWarp + r] = __float2half_rn(s);
+  }
+  __syncthreads();
+  const int g0 = k0 / G;
+  const int groups = min(32 / lanes, (K - k0) / G);
+  for (int i = threadIdx.x; i < groups * kRowsPerCta; i += 32 * kRowsWarps) {
+    const int g = i / kRowsPerCta, r = i % kRowsPerCta;
+    if (n_cta + r < N) scale_f16[static_cast<long long>(g0 + g) * N + n_cta + r] = scales[g][r];
+  }
+}
+
 }  // namespace sk

@@ -50,8 +50,11 @@ class W2A8Linear(nn.Module):
     @classmethod
     def from_float(cls, weight_out_in, group_size=128, device="cuda", out_dtype=torch.float16):
         """Quantise a float weight [out_features, in_features] with the reference's rule, on the GPU."""
-        w_kn = weight_out_in.detach().to(device=device, dtype=torch.float32).t().contiguous()
-        w_packed, w_scale = prepare_weight_gpu(w_kn, group_size)
+        load_extension()
+        w = weight_out_in.detach().to(device=device)
+        if w.dtype not in (torch.float16, torch.bfloat16, torch.float32):
+            w = w.to(torch.float32)
+        w_packed, w_scale = torch.ops.slimkernels.w2a8_quantize_weight_rows(w, group_size)
         return cls(w_packed, w_scale, group_size, 1, out_dtype)
 
     def plan(self) -> W2A8Plan:
