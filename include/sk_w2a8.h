@@ -207,6 +207,9 @@ int sk_w2a8_quantize_weight_rows(const void* w, int w_type, int64_t ld_w, int64_
  * x fp16 [M, ld_x] -> x_q int8 [M, ld_q], x_scale fp32 [M].  K % 8 == 0, rows 16-byte aligned. */
 int sk_quantize_activation_int8(const void* x_f16, int64_t ld_x, int64_t M, int64_t K, int8_t* x_q, int64_t ld_q,
                                 float* x_scale, sk_stream_t stream);
+/* The same with x in fp16 (x_bf16 = 0) or bf16 (1; each value is first rounded to fp16, on the way in). */
+int sk_quantize_activation_int8_from(const void* x, int x_bf16, int64_t ld_x, int64_t M, int64_t K, int8_t* x_q, int64_t ld_q,
+                                     float* x_scale, sk_stream_t stream);
 /* gate_up fp16 [M, ld_gu] (gate = columns [0, I), up = [I, 2I)) -> h = SiLU(gate) * up in fp32, quantised as
  * above to h_q int8 [M, ld_q], h_scale fp32 [M].  I % 8 == 0. */
 int sk_silu_mul_quantize_int8(const void* gate_up_f16, int64_t ld_gu, int64_t M, int64_t I, int8_t* h_q,
@@ -218,6 +221,10 @@ int sk_silu_mul_quantize_int8(const void* gate_up_f16, int64_t ld_gu, int64_t M,
 int64_t sk_w2a8_mlp_workspace_bytes(const sk_w2a8_plan* gate_up, const sk_w2a8_plan* down, int64_t M);
 int sk_w2a8_mlp_forward(sk_w2a8_plan* gate_up, sk_w2a8_plan* down, int64_t M, const void* x_f16, int64_t ld_x,
                         void* out, int64_t ld_out, void* workspace, int64_t workspace_bytes, sk_stream_t stream);
+
+/* The same with x in fp16 (x_bf16 = 0) or bf16 (1), as sk_quantize_activation_int8_from takes it. */
+int sk_w2a8_mlp_forward_from(sk_w2a8_plan* gate_up, sk_w2a8_plan* down, int64_t M, const void* x, int x_bf16, int64_t ld_x,
+                             void* out, int64_t ld_out, void* workspace, int64_t workspace_bytes, sk_stream_t stream);
 
 /* The MLP block for hosts that must not allocate device memory while serving.  It has no counterpart in the
  * reference.  Some embedders hand the GPU's memory to another owner at start-up (an inference server's arena, a

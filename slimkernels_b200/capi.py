@@ -47,6 +47,7 @@ SIGNATURES = {
     "sk_w2a8_gemm_rowscatter": (_int, [_vp, _i64, _vp, _i64, _vp, ctypes.POINTER(_vp), _int, _i64, _i64, _i64, _vp]),
     "sk_w2a8_gemm_debug_partials": (_int, [_vp, _i64, _vp, _i64, _vp, _vp]),
     "sk_quantize_activation_int8": (_int, [_vp, _i64, _i64, _i64, _vp, _i64, _vp, _vp]),
+    "sk_quantize_activation_int8_from": (_int, [_vp, _int, _i64, _i64, _i64, _vp, _i64, _vp, _vp]),
     "sk_silu_mul_quantize_int8": (_int, [_vp, _i64, _i64, _i64, _vp, _i64, _vp, _vp]),
     "sk_w2a8_debug_expander_image": (_int, [_vp, _int, _vp, _vp, _vp, _vp, _vp, _vp]),
     "sk_w2a8_debug_stream_cut": (_int, [_i64, _int, _int, _i64, ctypes.POINTER(_i64), ctypes.POINTER(_i64), ctypes.POINTER(_int)]),
@@ -55,6 +56,7 @@ SIGNATURES = {
     "sk_w2a8_quantize_weight_rows": (_int, [_vp, _int, _i64, _i64, _i64, _int, _vp, _vp, _vp]),
     "sk_w2a8_mlp_workspace_bytes": (_i64, [_vp, _vp, _i64]),
     "sk_w2a8_mlp_forward": (_int, [_vp, _vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _vp]),
+    "sk_w2a8_mlp_forward_from": (_int, [_vp, _vp, _i64, _vp, _int, _i64, _vp, _i64, _vp, _i64, _vp]),
     "sk_w2a8_mlp_static_scratch_bytes": (_i64, []),
     "sk_w2a8_mlp_forward_static": (_int, [_vp, _vp, _i64, _vp, _i64, _vp, _i64, _vp]),
     "sk_w2a8_last_device_status": (_int, [_vp, ctypes.POINTER(_int)]),

@@ -59,11 +59,27 @@ __device__ __forceinline__ uint32_t quantize_one_fast(float x, float s, float r)
   return __float_as_uint(big) & 0xffu;
 }
 
-// x fp16 [M, ld_x] -> x_q int8 [M, ld_q], x_scale fp32 [M].  K % 8 == 0, rows 16-byte aligned.
+// (16 bf16 tokens through 12288 x 4096: 27.8 us a layer with the separate pass and Python between the calls, 14.5 in one)
+// 8 activations as fp16: bf16 inputs are rounded to fp16 here, in registers (the fp16 values are what the quantiser's rule
+// is stated on), which replaces a conversion pass over the activations and its launch.
+template <bool BF16>
+__device__ __forceinline__ uint4 as_half8(uint4 v) {
+  if constexpr (!BF16) return v;
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  uint32_t o[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const __half2 h = __floats2half2_rn(__uint_as_float(w[j] << 16), __uint_as_float(w[j] & 0xffff0000u));
+    o[j] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+// x fp16 (or bf16) [M, ld_x] -> x_q int8 [M, ld_q], x_scale fp32 [M].  K % 8 == 0, rows 16-byte aligned.
 // Each thread keeps its 8-element vectors of the row in registers (up to kMaxVec of them); longer rows are re-read.
-template <int kMaxVec>
+template <int kMaxVec, bool BF16>
 __global__ void __launch_bounds__(kActThreads)
-quantize_activation_kernel(const __half* __restrict__ x, long long ld_x, int8_t* __restrict__ x_q, long long ld_q,
+quantize_activation_kernel(const uint16_t* __restrict__ x, long long ld_x, int8_t* __restrict__ x_q, long long ld_q,
                            float* __restrict__ x_scale, int K) {
   __shared__ float red[kActThreads / 32];
   act_launch_dependents();
@@ -77,7 +93,7 @@ quantize_activation_kernel(const __half* __restrict__ x, long long ld_x, int8_t*
   for (int i = 0; i < kMaxVec; ++i) {
     const int v = threadIdx.x + i * kActThreads;
     if (v < nvec) {
-      keep[i] = row[v];
+      keep[i] = as_half8<BF16>(row[v]);
       const __half2* h = reinterpret_cast<const __half2*>(&keep[i]);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -87,7 +103,7 @@ quantize_activation_kernel(const __half* __restrict__ x, long long ld_x, int8_t*
     }
   }
   for (int v = threadIdx.x + kMaxVec * kActThreads; v < nvec; v += kActThreads) {   // rows longer than the cache
-    const uint4 t = row[v];
+    const uint4 t = as_half8<BF16>(row[v]);
     const __half2* h = reinterpret_cast<const __half2*>(&t);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -117,7 +133,7 @@ quantize_activation_kernel(const __half* __restrict__ x, long long ld_x, int8_t*
     const int v = threadIdx.x + i * kActThreads;
     if (v < nvec) emit(v, keep[i]);
   }
-  for (int v = threadIdx.x + kMaxVec * kActThreads; v < nvec; v += kActThreads) emit(v, row[v]);
+  for (int v = threadIdx.x + kMaxVec * kActThreads; v < nvec; v += kActThreads) emit(v, as_half8<BF16>(row[v]));
 }
 
 // gate_up fp16 [M, ld_gu] with gate = columns [0, I), up = columns [I, 2I)  ->  h = SiLU(gate) * up (fp32),

@@ -1379,30 +1379,35 @@ int sk_w2a8_quantize_weight_rows(const void* w, int w_type, int64_t ld_w, int64_
 
 int sk_quantize_activation_int8(const void* x_f16, int64_t ld_x, int64_t M, int64_t K, int8_t* x_q, int64_t ld_q,
                                 float* x_scale, sk_stream_t stream) {
-  if (!x_f16 || !x_q || !x_scale) return SK_ERR_NULL_POINTER;
+  return sk_quantize_activation_int8_from(x_f16, 0, ld_x, M, K, x_q, ld_q, x_scale, stream);
+}
+
+int sk_quantize_activation_int8_from(const void* x, int x_bf16, int64_t ld_x, int64_t M, int64_t K, int8_t* x_q, int64_t ld_q,
+                                     float* x_scale, sk_stream_t stream) {
+  if (!x || !x_q || !x_scale) return SK_ERR_NULL_POINTER;
   if (M <= 0 || K <= 0 || (K % 8) != 0 || ld_x < K || ld_q < K || M > 0x7fffffffLL) return SK_ERR_BAD_SHAPE;
-  if ((reinterpret_cast<uintptr_t>(x_f16) & 15) || (ld_x % 8) || (reinterpret_cast<uintptr_t>(x_q) & 7) || (ld_q % 8))
+  if ((reinterpret_cast<uintptr_t>(x) & 15) || (ld_x % 8) || (reinterpret_cast<uintptr_t>(x_q) & 7) || (ld_q % 8))
     return SK_ERR_BAD_ALIGNMENT;
-  auto st = static_cast<cudaStream_t>(stream);
-  const __half* x = static_cast<const __half*>(x_f16);
-  const dim3 grid(static_cast<unsigned>(M));
   // launched as a programmatic dependent launch: the kernel waits for its inputs itself (griddepcontrol.wait) and
   // lets the kernel behind it start its set-up early
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
+  cfg.gridDim = dim3(static_cast<unsigned>(M));
   cfg.blockDim = dim3(sk::kActThreads, 1, 1);
-  cfg.stream = st;
+  cfg.stream = static_cast<cudaStream_t>(stream);
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  const uint16_t* src = static_cast<const uint16_t*>(x);
   const long long ldx = ld_x, ldq = ld_q;
   const int k = static_cast<int>(K);
-  cudaError_t le;
-  if (K <= 8 * sk::kActThreads * 2) le = cudaLaunchKernelEx(&cfg, sk::quantize_activation_kernel<2>, x, ldx, x_q, ldq, x_scale, k);
-  else if (K <= 8 * sk::kActThreads * 4) le = cudaLaunchKernelEx(&cfg, sk::quantize_activation_kernel<4>, x, ldx, x_q, ldq, x_scale, k);
-  else le = cudaLaunchKernelEx(&cfg, sk::quantize_activation_kernel<8>, x, ldx, x_q, ldq, x_scale, k);
+  const int vecs = K <= 8 * sk::kActThreads * 2 ? 2 : K <= 8 * sk::kActThreads * 4 ? 4 : 8;
+  auto kern = x_bf16 ? (vecs == 2 ? sk::quantize_activation_kernel<2, true> : vecs == 4 ? sk::quantize_activation_kernel<4, true>
+                                                                                        : sk::quantize_activation_kernel<8, true>)
+                     : (vecs == 2 ? sk::quantize_activation_kernel<2, false> : vecs == 4 ? sk::quantize_activation_kernel<4, false>
+                                                                                         : sk::quantize_activation_kernel<8, false>);
+  const cudaError_t le = cudaLaunchKernelEx(&cfg, kern, src, ldx, x_q, ldq, x_scale, k);
   if (le != cudaSuccess) { (void)cudaGetLastError(); return SK_ERR_CUDA; }
   if (cudaGetLastError() != cudaSuccess) return SK_ERR_CUDA;
   return SK_OK;
@@ -1470,7 +1475,7 @@ inline MlpLayout mlp_layout(int64_t M, int64_t hidden, int64_t inter) {
   return l;
 }
 // The caller has made the plans' device current: the two side kernels launch on the current device.
-int mlp_run(sk_w2a8_plan* gu, sk_w2a8_plan* down, int64_t M, const void* x, int64_t ld_x, void* out, int64_t ld_out,
+int mlp_run(sk_w2a8_plan* gu, sk_w2a8_plan* down, int64_t M, const void* x, int x_bf16, int64_t ld_x, void* out, int64_t ld_out,
             char* ws, sk_stream_t stream) {
   const int64_t hidden = gu->K, inter = down->K;
   const MlpLayout l = mlp_layout(M, hidden, inter);
@@ -1479,7 +1484,7 @@ int mlp_run(sk_w2a8_plan* gu, sk_w2a8_plan* down, int64_t M, const void* x, int6
   void* gate_up = ws + l.gate_up;
   int8_t* h_q = reinterpret_cast<int8_t*>(ws + l.h_q);
   float* h_scale = reinterpret_cast<float*>(ws + l.h_scale);
-  int rc = sk_quantize_activation_int8(x, ld_x, M, hidden, x_q, hidden, x_scale, stream);
+  int rc = sk_quantize_activation_int8_from(x, x_bf16, ld_x, M, hidden, x_q, hidden, x_scale, stream);
   if (rc == SK_OK) rc = sk_w2a8_gemm(gu, M, x_q, hidden, x_scale, gate_up, 2 * inter, stream);
   if (rc == SK_OK) rc = sk_silu_mul_quantize_int8(gate_up, 2 * inter, M, inter, h_q, inter, h_scale, stream);
   if (rc == SK_OK) rc = sk_w2a8_gemm(down, M, h_q, inter, h_scale, out, ld_out, stream);
@@ -1502,9 +1507,14 @@ int64_t sk_w2a8_mlp_workspace_bytes(const sk_w2a8_plan* gate_up, const sk_w2a8_p
 
 int sk_w2a8_mlp_forward(sk_w2a8_plan* gate_up, sk_w2a8_plan* down, int64_t M, const void* x_f16, int64_t ld_x,
                         void* out, int64_t ld_out, void* workspace, int64_t workspace_bytes, sk_stream_t stream) {
+  return sk_w2a8_mlp_forward_from(gate_up, down, M, x_f16, 0, ld_x, out, ld_out, workspace, workspace_bytes, stream);
+}
+
+int sk_w2a8_mlp_forward_from(sk_w2a8_plan* gate_up, sk_w2a8_plan* down, int64_t M, const void* x, int x_bf16, int64_t ld_x,
+                             void* out, int64_t ld_out, void* workspace, int64_t workspace_bytes, sk_stream_t stream) {
   int rc = mlp_check(gate_up, down, M);
   if (rc != SK_OK) return rc;
-  if (!x_f16 || !out || !workspace) return SK_ERR_NULL_POINTER;
+  if (!x || !out || !workspace) return SK_ERR_NULL_POINTER;
   if (reinterpret_cast<uintptr_t>(workspace) & 255) return SK_ERR_BAD_ALIGNMENT;
   if (workspace_bytes < static_cast<int64_t>(mlp_layout(M, gate_up->K, down->K).total)) return SK_ERR_BAD_SHAPE;
   // a plan is bound to one device: run there whatever device the calling thread has current, and put that back
@@ -1512,7 +1522,7 @@ int sk_w2a8_mlp_forward(sk_w2a8_plan* gate_up, sk_w2a8_plan* down, int64_t M, co
   int cur = -1;
   if (cudaGetDevice(&cur) != cudaSuccess) return sk::cuda_fail(gate_up, cudaGetLastError());
   if (cur != dev && cudaSetDevice(dev) != cudaSuccess) return sk::cuda_fail(gate_up, cudaGetLastError());
-  rc = mlp_run(gate_up, down, M, x_f16, ld_x, out, ld_out, static_cast<char*>(workspace), stream);
+  rc = mlp_run(gate_up, down, M, x, x_bf16, ld_x, out, ld_out, static_cast<char*>(workspace), stream);
   if (cur != dev) (void)cudaSetDevice(cur);
   return rc;
 }
@@ -1556,7 +1566,7 @@ int sk_w2a8_mlp_forward_static(sk_w2a8_plan* gate_up, sk_w2a8_plan* down, int64_
     }
     scratch = g_static_addr[dev];
   }
-  rc = mlp_run(gate_up, down, M, x_f16, ld_x, out, ld_out, static_cast<char*>(scratch), stream);
+  rc = mlp_run(gate_up, down, M, x_f16, 0, ld_x, out, ld_out, static_cast<char*>(scratch), stream);
   if (cur != dev) (void)cudaSetDevice(cur);
   return rc;
 }

@@ -272,9 +272,7 @@ std::tuple<at::Tensor, at::Tensor> silu_mul_quantize(const at::Tensor& gate_up) 
   return {q, s};
 }
 
-at::Tensor mlp_forward(int64_t gate_up_plan, int64_t down_plan, const at::Tensor& x, int64_t hidden_out, bool bf16_out) {
-  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kHalf && x.dim() == 2 && x.stride(1) == 1,
-              "x must be a 2-D CUDA float16 tensor with unit inner stride");
+at::Tensor mlp_run(int64_t gate_up_plan, int64_t down_plan, const at::Tensor& x, bool x_bf16, int64_t hidden_out, bool bf16_out) {
   const int64_t M = x.size(0);
   at::Tensor out = at::empty({M, hidden_out}, x.options().dtype(bf16_out ? at::kBFloat16 : at::kHalf));
   if (M == 0) return out;
@@ -283,10 +281,69 @@ at::Tensor mlp_forward(int64_t gate_up_plan, int64_t down_plan, const at::Tensor
   at::Tensor ws = at::empty({bytes}, x.options().dtype(at::kByte));     // caching allocator: 512-byte aligned
   c10::cuda::CUDAGuard guard(x.device());
   const auto stream = at::cuda::getCurrentCUDAStream();
-  check(sk_w2a8_mlp_forward(plan_on(gate_up_plan, stream), plan_on(down_plan, stream), M, x.data_ptr(), x.stride(0),
-                            out.data_ptr(), out.stride(0), ws.data_ptr(), bytes, stream.stream()),
+  check(sk_w2a8_mlp_forward_from(plan_on(gate_up_plan, stream), plan_on(down_plan, stream), M, x.data_ptr(), x_bf16, x.stride(0),
+                                 out.data_ptr(), out.stride(0), ws.data_ptr(), bytes, stream.stream()),
         "w2a8_mlp_forward");
   return out;
+}
+
+at::Tensor mlp_forward(int64_t gate_up_plan, int64_t down_plan, const at::Tensor& x, int64_t hidden_out, bool bf16_out) {
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kHalf && x.dim() == 2 && x.stride(1) == 1,
+              "x must be a 2-D CUDA float16 tensor with unit inner stride");
+  return mlp_run(gate_up_plan, down_plan, x, false, hidden_out, bf16_out);
+}
+
+// Activations of any leading shape as the 2-D matrix a quantiser reads: fp16, or bf16 whose rows it can read as they are;
+// anything else is converted to fp16 first.
+at::Tensor activation_rows(const at::Tensor& x, bool* is_bf16) {
+  TORCH_CHECK(x.is_cuda() && x.dim() >= 1, "x must be a CUDA tensor [..., K]");
+  at::Tensor x2 = x.dim() == 2 ? x : x.reshape({-1, x.size(-1)});
+  *is_bf16 = x2.scalar_type() == at::kBFloat16 && x2.stride(1) == 1 && x2.stride(0) >= x2.size(1) && x2.stride(0) % 8 == 0 &&
+             (reinterpret_cast<uintptr_t>(x2.data_ptr()) & 15) == 0;
+  if (!*is_bf16) x2 = x2.to(at::kHalf);
+  TORCH_CHECK(x2.stride(1) == 1, "x must have unit inner stride");
+  return x2;
+}
+
+at::Tensor with_leading_shape(const at::Tensor& y, const at::Tensor& x) {
+  if (x.dim() == 2) return y;
+  std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
+  shape.back() = y.size(1);
+  return y.reshape(shape);
+}
+
+// x [..., K] (fp16 / bf16 / other floats) -> [..., N]: quantise the tokens, one GEMM.  The whole of W2A8Linear's forward in
+// one call: at decode sizes the host work of its pieces took longer than the GPU's.
+at::Tensor linear_forward(int64_t handle, const at::Tensor& x, int64_t N, int64_t K, bool bf16_out) {
+  bool x_bf16 = false;
+  const at::Tensor x2 = activation_rows(x, &x_bf16);
+  const int64_t M = x2.size(0);
+  TORCH_CHECK(x2.size(1) == K, "x must have ", K, " features, got ", x2.size(1));
+  int64_t plan_n = 0, plan_k = 0;
+  int plan_dtype = 0, plan_dev = 0;
+  check(sk_w2a8_plan_info(as_plan(handle), &plan_n, &plan_k, nullptr, nullptr, &plan_dtype, &plan_dev), "w2a8_plan_info");
+  TORCH_CHECK(N == plan_n && K == plan_k && bf16_out == (plan_dtype == SK_OUT_BF16), "the plan is for another weight");
+  TORCH_CHECK(x2.get_device() == plan_dev, "tensors must live on the plan's device ", plan_dev);
+  c10::cuda::CUDAGuard guard(x2.device());
+  at::Tensor out = at::empty({M, N}, x2.options().dtype(bf16_out ? at::kBFloat16 : at::kHalf));
+  if (M > 0) {
+    const int64_t scales = (M * K + 255) / 256 * 256;
+    at::Tensor ws = at::empty({scales + 4 * M}, x2.options().dtype(at::kByte));   // int8 rows, then their scales
+    int8_t* x_q = static_cast<int8_t*>(ws.data_ptr());
+    float* x_scale = reinterpret_cast<float*>(x_q + scales);
+    const auto stream = at::cuda::getCurrentCUDAStream();
+    check(sk_quantize_activation_int8_from(x2.data_ptr(), x_bf16, x2.stride(0), M, K, x_q, K, x_scale, stream.stream()),
+          "quantize_activation_int8");
+    check(sk_w2a8_gemm(plan_on(handle, stream), M, x_q, K, x_scale, out.data_ptr(), out.stride(0), stream.stream()), "w2a8_gemm");
+  }
+  return with_leading_shape(out, x);
+}
+
+// x [..., hidden] -> [..., hidden]: the MLP block, from activations as linear_forward takes them.
+at::Tensor mlp_block(int64_t gate_up_plan, int64_t down_plan, const at::Tensor& x, int64_t hidden_out, bool bf16_out) {
+  bool x_bf16 = false;
+  const at::Tensor x2 = activation_rows(x, &x_bf16);
+  return with_leading_shape(mlp_run(gate_up_plan, down_plan, x2, x_bf16, hidden_out, bf16_out), x);
 }
 
 // [token tile, split-K, CTAs, kernel kind] of the launch the plan makes for M tokens
@@ -429,6 +486,8 @@ TORCH_LIBRARY(slimkernels, m) {
   m.def("w2a8_quantize_weight_rows(Tensor w_nk, int group_size) -> (Tensor, Tensor)", &quantize_weight_rows);
   m.def("silu_mul_quantize_int8(Tensor gate_up) -> (Tensor, Tensor)", &silu_mul_quantize);
   m.def("w2a8_mlp_forward(int gate_up_plan, int down_plan, Tensor x, int hidden_out, bool bf16_out) -> Tensor", &mlp_forward);
+  m.def("w2a8_linear_forward(int plan, Tensor x, int N, int K, bool bf16_out) -> Tensor", &linear_forward);
+  m.def("w2a8_mlp_block(int gate_up_plan, int down_plan, Tensor x, int hidden_out, bool bf16_out) -> Tensor", &mlp_block);
   m.def("w2a8_repack(Tensor w_packed) -> Tensor", &repack);
   m.def("w2a8_unrepack(Tensor w_tiled, int N, int K) -> Tensor", &unrepack);
 }

@@ -72,10 +72,8 @@ class W2A8Linear(nn.Module):
         return self.plan().gemm(x_q, x_scale)
 
     def forward(self, x):
-        shape = x.shape
-        x2 = x.reshape(-1, shape[-1]).to(torch.float16)
-        x_q, x_scale = quantize_activation_int8(x2)
-        return self.plan().gemm(x_q, x_scale).reshape(*shape[:-1], self.out_features)
+        plan = self.plan()
+        return torch.ops.slimkernels.w2a8_linear_forward.default(plan._h, x, plan.N, plan.K, plan._bf16)
 
 
 class W2A8LlamaMLP(nn.Module):
@@ -89,9 +87,5 @@ class W2A8LlamaMLP(nn.Module):
         self.gate_up, self.down = gate_up, down
 
     def forward(self, x):
-        shape = x.shape
-        x2 = x.reshape(-1, shape[-1]).to(torch.float16)
         gate_up_plan, down_plan = self.gate_up.plan(), self.down.plan()      # also loads the extension
-        y = torch.ops.slimkernels.w2a8_mlp_forward(gate_up_plan._h, down_plan._h, x2,
-                                                   self.down.out_features, self.down.out_dtype == torch.bfloat16)
-        return y.reshape(*shape[:-1], self.down.out_features)
+        return torch.ops.slimkernels.w2a8_mlp_block.default(gate_up_plan._h, down_plan._h, x, down_plan.N, down_plan._bf16)

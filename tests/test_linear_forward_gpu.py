@@ -1,0 +1,101 @@
+"""W2A8Linear / W2A8LlamaMLP forward in one native call: the same bits as its pieces for every activation layout, and plans
+used on other streams than the one they were made on."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _need_gpu(built_libs):
+    if not torch.cuda.is_available():
+        pytest.fail("GPU tests selected but no CUDA device is visible")
+
+
+def _linear(N, K, G=128, out_dtype=torch.float16, seed=0):
+    from slimkernels_b200.torch import W2A8Linear
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return W2A8Linear.from_float(torch.randn(N, K, generator=g, device="cuda") * 0.05, G, out_dtype=out_dtype)
+
+
+def _by_pieces(lin, x):
+    from slimkernels_b200.torch import quantize_activation_int8
+    x_q, x_s = quantize_activation_int8(x.reshape(-1, x.shape[-1]).to(torch.float16).contiguous())
+    return lin.plan().gemm(x_q, x_s).reshape(*x.shape[:-1], lin.out_features)
+
+
+@pytest.mark.parametrize("K", [128, 4096, 8320, 18432])            # 2, 4 and 8 vectors per thread, and rows read twice
+@pytest.mark.parametrize("M", [1, 5, 40])
+def test_bf16_activations_are_rounded_to_fp16_on_the_way_in(M, K):
+    lin = _linear(136, K, out_dtype=torch.bfloat16)
+    x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    x[0, :4] = torch.tensor([1e30, -3e38, 1e-30, 6e-8])            # beyond fp16 on both sides
+    torch.testing.assert_close(lin(x), _by_pieces(lin, x), rtol=0, atol=0, equal_nan=True)
+    x[0, :2] = 3.0
+    assert torch.equal(lin(x), _by_pieces(lin, x))
+
+
+def test_layouts_and_shapes():
+    lin = _linear(136, 512)
+    for dtype in (torch.float16, torch.bfloat16, torch.float32):
+        base = torch.randn(4, 6, 1040, device="cuda").to(dtype)
+        views = [base[..., 3:515], base[..., 8:520], base[:, :, ::2][..., :512], base[0, 0, :512].expand(3, 512),
+                 base[0, :, :512], base[0, 0, :512], base[:0, :, :512]]
+        for x in views:
+            if dtype == torch.float16 and (x.data_ptr() % 16 or (x.dim() == 2 and x.stride(0) == 0) or x.stride(-1) != 1):
+                continue                                           # fp16 rows are read where they are: refused before, too
+            y = lin(x)
+            assert y.shape == (*x.shape[:-1], 136) and torch.equal(y, _by_pieces(lin, x))
+    with pytest.raises(RuntimeError):
+        lin(torch.randn(4, 256, device="cuda"))
+    with pytest.raises(RuntimeError):
+        lin(torch.randn(4, 512))
+    with pytest.raises(RuntimeError):
+        lin(torch.randn(512, 4, device="cuda").half().t())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+def test_mlp_takes_the_same_activations(dtype):
+    from slimkernels_b200.torch import W2A8LlamaMLP
+    mlp = W2A8LlamaMLP(_linear(768, 256), _linear(256, 384, seed=1))
+    x = torch.randn(2, 9, 256, device="cuda").to(dtype)
+    want = torch.ops.slimkernels.w2a8_mlp_forward(mlp.gate_up.plan()._h, mlp.down.plan()._h, x.reshape(-1, 256).half(), 256, False)
+    assert torch.equal(mlp(x), want.reshape(2, 9, 256))
+
+
+def test_plan_used_on_another_stream_and_dropped_there():
+    """A plan made on one stream, used at once on another, and dropped while that stream still works: its memory is not
+    handed out before the stream is done with it."""
+    want, x = None, torch.randn(8, 4096, device="cuda").half()
+    side = torch.cuda.Stream()
+    for i in range(6):
+        lin = _linear(4096, 4096, seed=3)
+        with torch.cuda.stream(side):
+            for w in (lin.w_packed, lin.w_scale, x):
+                w.record_stream(side)
+            side.wait_stream(torch.cuda.default_stream())
+            ys = [lin(x) for _ in range(8)]
+        del lin
+        junk = torch.full((8 << 20,), 0xFF, dtype=torch.uint8, device="cuda")     # takes a freed block, if there is one
+        side.synchronize()
+        if want is None:
+            want = ys[0].clone()
+        assert all(torch.equal(y, want) for y in ys)
+        del junk
+
+
+def test_plan_is_refused_under_capture():
+    lin = _linear(256, 256)
+    x = torch.randn(2, 256, device="cuda").half()
+    graph = torch.cuda.CUDAGraph()
+    with pytest.raises(RuntimeError):
+        with torch.cuda.graph(graph):
+            lin(x)                                                 # the plan would be made inside the capture
+    torch.cuda.synchronize()
+    y = lin(x)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        z = lin(x)                                                 # made before (on another stream): captured
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, z)
