@@ -65,7 +65,8 @@ typedef enum sk_option {
                              range of the WHOLE problem into equal CTA ranges, two CTAs per SM (the default for M <= 32
                              with group size 128 and K a multiple of 256; else 3 is taken).  Partial sums of tiles that
                              two or more CTAs share meet in a scratch buffer owned by the plan, so calls on one plan
-                             must not run concurrently (they must not anyway, see above). */
+                             must not run concurrently (they must not anyway, see above),
+                             6 direct decode kernel (weights from HBM to registers to mma.sync; taken by itself for small M) */
   SK_OPT_TOKEN_TILE = 2,  /* tokens per CTA tile: 0 auto, or 16 / 32 / 64 / 128 / 192 / 256 */
   SK_OPT_SPLIT_K = 3,     /* CTAs (one cluster) sharing the K range of one tile: 0 auto, 1, 2, 4, 8 */
   SK_OPT_TMA_STORE = 6,   /* general kernel, one CTA per tile: 0 auto (= 2), 1 vector stores by the epilogue threads, 2 one TMA
@@ -100,8 +101,7 @@ int sk_w2a8_unrepack(const uint8_t* w_tiled, int64_t N, int64_t K, uint8_t* w_pa
  * Binds one weight matrix to a device: validates shapes/alignment, builds the tiled weight copy (or
  * borrows one), allocates a 4-byte device status word.  Stands where gemm_tn builds its tilers, smem
  * layouts and tensor maps on every call (wgmma_sm90_W2A8.cu:448-466).  Synchronises `device` once.
- * With group size 128 the plan also makes a private copy of the scales in the order its decode kernels
- * stream them, and -- for weight matrices large enough that the balanced-split decode kernel is their default, or
+ * The plan also makes a private copy of the scales in the order its decode kernels stream them, and -- for weight matrices large enough that the balanced-split decode kernel is their default, or
  * on the first SK_OPT_KERNEL = 5 / SK_OPT_STREAM_CTAS request -- a scratch buffer for that kernel's partial sums
  * (3-20 MiB):
  * w_scale_f16 must still outlive the plan (the other kernels read it), and a change of its contents
@@ -253,9 +253,13 @@ int sk_w2a8_last_device_status(sk_w2a8_plan* plan, int* device_status);
 /* Names the role and the wait behind a device status code (static string). */
 const char* sk_device_status_string(int device_status);
 int sk_w2a8_last_cuda_error(const sk_w2a8_plan* plan);
-/* Describes the launch the plan would make for M tokens: token tile, split-K factor, CTAs, kernel kind. */
+/* Describes the launch the plan's tensor-memory kernels (1, 3, 4, 5) make for M tokens, which is what the options below force
+ * and the integer partial sums come from: token tile, split-K factor, CTAs, kernel kind. */
 int sk_w2a8_query_launch(sk_w2a8_plan* plan, int64_t M, int* token_tile, int* split_k, int* ctas,
                          int* kernel_kind);
+/* The same for the launch sk_w2a8_gemm really makes with the plan's options: where the direct decode kernel (6) takes the
+ * call, that; elsewhere the tcgen05 launch above, with the tile and split it is given for M. */
+int sk_w2a8_query_route(sk_w2a8_plan* plan, int64_t M, int* token_tile, int* split_k, int* ctas, int* kernel_kind);
 /* Measurement aid (decode-sized M only, else SK_ERR_UNAVAILABLE): launches an EMPTY kernel with the grid, cluster,
  * block size, shared memory and launch attributes sk_w2a8_gemm would use for M tokens, doing only the fixed per-CTA
  * work (barrier set-up, tensor-memory allocation and release, the barriers).  Timed as a chain in a CUDA graph it gives

@@ -27,6 +27,7 @@ SK_WEIGHT_ROWMAJOR, SK_WEIGHT_TILED = 0, 1
 SK_OPT_KERNEL, SK_OPT_TOKEN_TILE, SK_OPT_SPLIT_K, SK_OPT_PERSISTENT, SK_OPT_DEPENDENT_LAUNCH, SK_OPT_TMA_STORE = 1, 2, 3, 4, 5, 6
 SK_OPT_WAIT_LIMIT_CYCLES, SK_OPT_TEST_SKIP_COPY, SK_OPT_STREAM_CTAS = 7, 8, 9
 KERNEL_AUTO, KERNEL_TCGEN05, KERNEL_CUDA_CORE, KERNEL_TCGEN05_DECODE, KERNEL_TCGEN05_PAIR, KERNEL_TCGEN05_DECODE_BALANCED = 0, 1, 2, 3, 4, 5
+KERNEL_DIRECT = 6
 
 _i64, _int, _vp = ctypes.c_int64, ctypes.c_int, ctypes.c_void_p
 
@@ -64,6 +65,8 @@ SIGNATURES = {
     "sk_device_status_string": (ctypes.c_char_p, [_int]),
     "sk_w2a8_query_launch": (_int, [_vp, _i64, ctypes.POINTER(_int), ctypes.POINTER(_int), ctypes.POINTER(_int),
                                     ctypes.POINTER(_int)]),
+    "sk_w2a8_query_route": (_int, [_vp, _i64, ctypes.POINTER(_int), ctypes.POINTER(_int), ctypes.POINTER(_int),
+                                   ctypes.POINTER(_int)]),
     "sk_w2a8_launch_floor_probe": (_int, [_vp, _i64, _vp]),
     "sk_status_string": (ctypes.c_char_p, [_int]),
     "sk_w2a8_version": (_int, []),
@@ -136,6 +139,12 @@ class Plan:
         if rc not in (SK_OK, SK_ERR_DEVICE_TIMEOUT):
             raise SkError(rc, "sk_w2a8_last_device_status")
         return v.value
+
+    def query_route(self, M: int):
+        t, s, c, k = _int(0), _int(0), _int(0), _int(0)
+        check(load().sk_w2a8_query_route(self._h, M, ctypes.byref(t), ctypes.byref(s), ctypes.byref(c),
+                                         ctypes.byref(k)), "sk_w2a8_query_route")
+        return {"token_tile": t.value, "split_k": s.value, "ctas": c.value, "kernel": k.value}
 
     def query_launch(self, M: int):
         t, s, c, k = _int(), _int(), _int(), _int()

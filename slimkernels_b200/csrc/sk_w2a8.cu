@@ -14,6 +14,7 @@
 #include "w2a8_umma.cuh"
 #include "w2a8_decode.cuh"
 #include "w2a8_stream.cuh"
+#include "w2a8_direct.cuh"
 #include "w2a8_pair.cuh"
 #include "weight_prep.cuh"
 
@@ -95,17 +96,17 @@ tile_weight_kernel(const uint8_t* __restrict__ w_packed, uint8_t* __restrict__ w
   if (w_scale_tiled) w_scale_tiled[block * 128 + r] = n < N ? w_scale[static_cast<size_t>(B) * N + n] : __float2half(0.f);
 }
 
-// The scales of a group-size-128 plan in the order the decode kernels stream them: [n_tiles][k_blocks][128 features]
-// (rows past N are zero), so that the scales of a CTA's K range are one contiguous run.
+// The scales in the order the decode kernels stream them: [n_tiles][groups][128 features] (rows past N are zero), so that
+// the scales of a CTA's K range are one contiguous run.
 __global__ void tile_scales_kernel(const __half* __restrict__ w_scale, __half* __restrict__ tiled, long long N,
-                                   int k_blocks, long long total) {
+                                   int groups, long long total) {
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const int r = static_cast<int>(i % 128);
     const long long t = i / 128;
-    const int kb = static_cast<int>(t % k_blocks);
-    const long long n = (t / k_blocks) * 128 + r;
-    tiled[i] = n < N ? w_scale[static_cast<size_t>(kb) * N + n] : __float2half(0.f);
+    const int g = static_cast<int>(t % groups);
+    const long long n = (t / groups) * 128 + r;
+    tiled[i] = n < N ? w_scale[static_cast<size_t>(g) * N + n] : __float2half(0.f);
   }
 }
 
@@ -243,7 +244,7 @@ struct sk_w2a8_plan {
   const uint8_t* w_rowmajor = nullptr;  // borrowed (may be null when created from a tiled buffer)
   const uint8_t* w_tiled = nullptr;     // in the plan's storage, or borrowed
   const __half* w_scale = nullptr;      // borrowed
-  __half* w_scale_tiled = nullptr;      // device, owned: [n_tiles][k_blocks][128] copy of the scales (group size 128 only)
+  __half* w_scale_tiled = nullptr;      // in the plan's storage: [n_tiles][K / G][128] copy of the scales
   int* status = nullptr;                // device; first in the plan's storage, one block that also holds the tiled copies
   bool external_storage = false;        // the buffers below live in the caller's storage (sk_w2a8_plan_create_in)
   bool stream_owned = false;            // stream_scratch / stream_counters are the plan's own allocations
@@ -297,7 +298,7 @@ static LaunchChoice choose(const sk_w2a8_plan* plan, long long M) {
   // global round trips -- costs more than the even load saves.  Its 32-token variant is slower throughout.
   const bool stream_pays = stream_ok && c.token_tile == 16 &&
                            static_cast<long long>(plan->n_tiles) * plan->k_blocks >= 64LL * plan->sm_count;
-  c.kernel = plan->opt_kernel ? plan->opt_kernel : (stream_pays ? 5 : decode_ok ? 3 : 1);
+  c.kernel = plan->opt_kernel && plan->opt_kernel != 6 ? plan->opt_kernel : (stream_pays ? 5 : decode_ok ? 3 : 1);
   if (c.kernel == 5 && !stream_ok) c.kernel = 3;
   if (c.kernel == 3 && !decode_ok) c.kernel = 1;
   const int groups = static_cast<int>(plan->K / plan->G);
@@ -535,7 +536,7 @@ static PlanLayout plan_layout(sk_w2a8_plan* plan, int w_layout) {
   const long long blocks = static_cast<long long>(plan->n_tiles) * plan->k_blocks;
   l.status = take(sizeof(int));
   l.w_tiled = w_layout == SK_WEIGHT_ROWMAJOR ? take(blocks * kWpBytes) : -1;
-  l.w_scale_tiled = plan->G == 128 ? take(blocks * kTileN * static_cast<long long>(sizeof(__half))) : -1;
+  l.w_scale_tiled = take(static_cast<long long>(plan->n_tiles) * (plan->K / plan->G) * kTileN * static_cast<long long>(sizeof(__half)));
   l.stream_scratch = l.stream_counters = -1;
   l.counter_bytes = 0;
   // The balanced-split decode kernel's scratch is part of it only where that kernel is the default (large weight
@@ -549,6 +550,143 @@ static PlanLayout plan_layout(sk_w2a8_plan* plan, int w_layout) {
   }
   l.total = o;
   return l;
+}
+
+// ---------------------------------------------------------------------------------------------- direct decode kernel (6)
+struct DirectChoice {
+  int mt, nt, warps;          // 16-feature tiles per CTA, 8-token tiles per CTA, warps
+  int split;                  // CTAs (one cluster) sharing the K range of a tile
+  int ctas;
+  bool deep;                  // all CTAs resident at once, three per SM
+};
+
+template <int MT, int NT, int WARPS, int DEPTH, int MIN_CTAS, int GPB>
+static int launch_direct(sk_w2a8_plan* plan, const DirectParams& prm, int split, cudaStream_t stream) {
+  using T = DirectTraits<MT, NT, WARPS, DEPTH, GPB>;
+  auto kern = w2a8_direct_kernel<MT, NT, WARPS, DEPTH, MIN_CTAS, GPB>;
+  if constexpr (T::kDynamicBytes > 48 * 1024) {
+    static int configured_device_mask[64] = {0};
+    if (plan->device < 64 && !configured_device_mask[plan->device]) {
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, T::kDynamicBytes);
+      if (e != cudaSuccess) return cuda_fail(plan, e);
+      configured_device_mask[plan->device] = 1;
+    }
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>((plan->N + T::kFeatures - 1) / T::kFeatures),
+                     static_cast<unsigned>((prm.M + T::kTokens - 1) / T::kTokens), static_cast<unsigned>(split));
+  cfg.blockDim = dim3(T::kThreads, 1, 1);
+  cfg.dynamicSmemBytes = T::kDynamicBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  int na = 0;
+  if (split > 1) {
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = 1;
+    attr[na].val.clusterDim.y = 1;
+    attr[na].val.clusterDim.z = static_cast<unsigned>(split);
+    ++na;
+  }
+  if (plan->opt_pdl != 1) {   // programmatic dependent launch, as for the other decode kernels
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = na;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, prm);
+  if (e != cudaSuccess) return cuda_fail(plan, e);
+  return SK_OK;
+}
+
+// Serves small calls unless an option asks for another kernel (or for its failure-path hook).  Its time grows with the
+// tokens, the tcgen05 kernels' hardly does up to a tile, so the line lies where weights x tokens per SM get large (us, this
+// kernel against the better tcgen05 one, group size 128):
+//   * up to 24 tokens always: 24 x 57344 x 8192 64 / 80, 24 x 22016 x 4096 17.1 / 17.3, 24 x 4096 x 4096 4.9 / 7.6;
+//   * up to 32 tokens below 16 K blocks of a feature tile per SM: 32 x 4096 x 4096 5.9 / 7.8, but 32 x 22016 x 4096 24 / 17.5;
+//     with other group sizes always (64: 32 x 22016 x 4096 29 / 52);
+//   * up to 128 tokens below 8 such blocks per SM, the weight counted once per 32 tokens: 64 x 2048 x 1024 3.4 / 8.4,
+//     64 x 512 x 16384 6.9 / 10.6, but 64 x 4096 x 4096 11.6 / 9.2.
+// The shape of a CTA:
+//   * 64 features and 4 warps once that gives two CTAs per SM: 1 x 22016 x 4096 6.9, with 8 warps 8.8;
+//   * 64 features and 8 warps (8 tokens), 64 and 4 with the K range split (16 tokens) while there is a CTA of 64 per SM:
+//     1 x 12288 x 4096 4.9 against 5.3 with 32 features;
+//   * else, and from 24 tokens on, 32 features: 64 x 24 sums do not leave registers for three CTAs per SM;
+//   * the K range is split over a cluster while the CTAs fit the SMs' slots and every warp keeps four K blocks: 1 x 4096 x
+//     11008 in two halves 5.9, but 1 x 4096 x 4096 whole 2.7, in halves 3.7 (the cluster barriers cost more).
+static bool choose_direct(const sk_w2a8_plan* plan, long long M, DirectChoice* out) {
+  const bool forced = plan->opt_kernel == 6;
+  if (!forced && (plan->opt_kernel || plan->opt_token_tile || plan->opt_split_k || plan->opt_persistent || plan->opt_skip_copy || M > 128))
+    return false;
+  DirectChoice c;
+  c.nt = M <= 8 ? 1 : M <= 16 ? 2 : M <= 24 ? 3 : 4;
+  const long long sms = plan->sm_count;
+  const long long token_tiles = (M + 8 * c.nt - 1) / (8 * c.nt);
+  const long long work = static_cast<long long>(plan->n_tiles) * plan->k_blocks * token_tiles;
+  if (token_tiles > 65535) return false;
+  if (!forced && c.nt == 4 && !(M <= 32 && (plan->G != 128 || work < 16 * sms)) && work > 8 * sms) return false;
+  const long long per_64 = (plan->N + 63) / 64, per_32 = (plan->N + 31) / 32;
+  int slots;                                   // CTAs an SM holds
+  if (plan->G < 128) { c.mt = 2; c.warps = 4; slots = 4; }
+  else if (per_64 >= 2 * sms && (c.nt < 3 || per_64 >= 4 * sms)) { c.mt = 4; c.warps = 4; slots = 2; }
+  else if (per_64 >= sms && c.nt <= 2) { c.mt = 4; c.warps = c.nt == 1 ? 8 : 4; slots = c.nt == 1 ? 2 : 3; }
+  else if (per_32 >= 2 * sms) { c.mt = 2; c.warps = 4; slots = 3; }
+  else { c.mt = 2; c.warps = 8; slots = c.nt <= 2 ? 2 : 1; }
+  const long long tiles = (c.mt == 4 ? per_64 : per_32) * token_tiles;
+  c.split = 1;
+  if (plan->opt_split_k) c.split = plan->opt_split_k;
+  else
+    while (c.split < 8 && tiles * (2 * c.split) <= slots * sms && plan->k_blocks / (2 * c.split * c.warps) >= 4) c.split *= 2;
+  if (c.split > plan->k_blocks) c.split = 1;
+  c.ctas = static_cast<int>(tiles * c.split);
+  c.deep = tiles * c.split <= 3 * sms;
+  *out = c;
+  return true;
+}
+
+// <16-feature tiles, 8-token tiles, warps, K blocks in flight per warp, CTAs per SM that registers are kept for, groups per
+// K block>.  With 4 warps and one token tile, three CTAs of six blocks in flight where they all fit at once (1 x 22016 x 4096
+// 6.9 us; four of four blocks 8.5), else four of four (1 x 57344 x 8192 27.7; 30.0).
+static int dispatch_direct(sk_w2a8_plan* plan, const DirectChoice& c, const DirectParams& prm, cudaStream_t stream) {
+  if (plan->G == 64) {
+    switch (c.nt) {
+      case 1: return launch_direct<2, 1, 4, 4, 4, 2>(plan, prm, c.split, stream);
+      case 2: return launch_direct<2, 2, 4, 4, 4, 2>(plan, prm, c.split, stream);
+      case 3: return launch_direct<2, 3, 4, 4, 2, 2>(plan, prm, c.split, stream);
+      default: return launch_direct<2, 4, 4, 4, 2, 2>(plan, prm, c.split, stream);
+    }
+  }
+  if (plan->G == 32) {
+    switch (c.nt) {
+      case 1: return launch_direct<2, 1, 4, 4, 4, 4>(plan, prm, c.split, stream);
+      case 2: return launch_direct<2, 2, 4, 4, 3, 4>(plan, prm, c.split, stream);
+      case 3: return launch_direct<2, 3, 4, 4, 2, 4>(plan, prm, c.split, stream);
+      default: return launch_direct<2, 4, 4, 4, 2, 4>(plan, prm, c.split, stream);
+    }
+  }
+  if (c.mt == 4 && c.warps == 8) return launch_direct<4, 1, 8, 4, 2, 1>(plan, prm, c.split, stream);
+  if (c.mt == 4) {
+    switch (c.nt) {
+      case 1: return c.deep ? launch_direct<4, 1, 4, 6, 3, 1>(plan, prm, c.split, stream) : launch_direct<4, 1, 4, 4, 4, 1>(plan, prm, c.split, stream);
+      case 2: return launch_direct<4, 2, 4, 4, 3, 1>(plan, prm, c.split, stream);
+      case 3: return launch_direct<4, 3, 4, 4, 2, 1>(plan, prm, c.split, stream);
+      default: return launch_direct<4, 4, 4, 4, 2, 1>(plan, prm, c.split, stream);
+    }
+  }
+  if (c.warps == 4) {
+    switch (c.nt) {
+      case 1: return launch_direct<2, 1, 4, 6, 4, 1>(plan, prm, c.split, stream);
+      case 2: return launch_direct<2, 2, 4, 6, 4, 1>(plan, prm, c.split, stream);
+      case 3: return launch_direct<2, 3, 4, 6, 3, 1>(plan, prm, c.split, stream);
+      default: return launch_direct<2, 4, 4, 6, 3, 1>(plan, prm, c.split, stream);
+    }
+  }
+  switch (c.nt) {
+    case 1: return launch_direct<2, 1, 8, 4, 2, 1>(plan, prm, c.split, stream);
+    case 2: return launch_direct<2, 2, 8, 4, 2, 1>(plan, prm, c.split, stream);
+    case 3: return launch_direct<2, 3, 8, 4, 1, 1>(plan, prm, c.split, stream);
+    default: return launch_direct<2, 4, 8, 4, 1, 1>(plan, prm, c.split, stream);
+  }
 }
 
 constexpr int kPairStages = 6;
@@ -788,6 +926,30 @@ static int run_gemm(sk_w2a8_plan* plan, long long M, const int8_t* x_q, long lon
     if (cur != plan->device) (void)cudaSetDevice(cur);
     return rc;
   }
+  DirectChoice dc;
+  if (!partials && scatter_rows == 0 && choose_direct(plan, M, &dc)) {
+    DirectParams prm;
+    prm.w_tiled = plan->w_tiled;
+    prm.w_scale_tiled = plan->w_scale_tiled;
+    prm.x_q = x_q;
+    prm.x_scale = x_scale;
+    prm.out = out;
+    prm.n_extra = n_extra;
+    for (int i = 0; i < 7; ++i) prm.out_extra[i] = i < n_extra ? extra_outs[i] : nullptr;
+    prm.ld_x = ld_x;
+    prm.ld_out = ld_out;
+    prm.M = static_cast<int>(M);
+    prm.N = static_cast<int>(plan->N);
+    prm.K = static_cast<int>(plan->K);
+    prm.groups = static_cast<int>(plan->K / plan->G);
+    prm.k_blocks = plan->k_blocks;
+    prm.blocks_per_group = plan->G / 128;
+    prm.zero_point = plan->zero_point;
+    prm.out_bf16 = plan->out_dtype == SK_OUT_BF16;
+    rc = dispatch_direct(plan, dc, prm, stream);
+    if (cur != plan->device) (void)cudaSetDevice(cur);
+    return rc;
+  }
   if (scatter_rows > 0 && (ch.kernel != 1 || ch.split_k != 1 || (scatter_rows % ch.token_tile) != 0)) {
     // row scatter is the general kernel's: every token tile must belong to one destination
     if (cur != plan->device) (void)cudaSetDevice(cur);
@@ -988,9 +1150,9 @@ static int plan_create_common(sk_w2a8_plan** out, int device, int64_t N, int64_t
       plan->stream_counters = reinterpret_cast<int*>(base + l.stream_counters);
       e = cudaMemsetAsync(plan->stream_counters, 0, l.counter_bytes, stream);
     }
-    if (l.w_scale_tiled >= 0) plan->w_scale_tiled = reinterpret_cast<__half*>(base + l.w_scale_tiled);
+    plan->w_scale_tiled = reinterpret_cast<__half*>(base + l.w_scale_tiled);
     // the decode kernels' copy of the scales is made once, here: later changes of w_scale_f16 are not seen by them
-    bool scales_tiled = plan->w_scale_tiled == nullptr;
+    bool scales_tiled = false;
     if (w_layout == SK_WEIGHT_TILED) {
       plan->w_tiled = w;
     } else {
@@ -1000,18 +1162,19 @@ static int plan_create_common(sk_w2a8_plan** out, int device, int64_t N, int64_t
       if (e == cudaSuccess) {
         if ((K % 128) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 && ((K / 4) % 16) == 0 && plan->n_tiles <= 65535) {
           sk::tile_weight_kernel<<<dim3(plan->k_blocks, plan->n_tiles), 128, 0, stream>>>(
-              w, tiled, plan->w_scale, plan->w_scale_tiled, N, K, plan->k_blocks);
+              w, tiled, plan->w_scale, group_size == 128 ? plan->w_scale_tiled : nullptr, N, K, plan->k_blocks);
           e = cudaGetLastError();
-          scales_tiled = true;
+          scales_tiled = group_size == 128;
         } else {
           rc = sk::repack_common(true, w, N, K, tiled, stream);
         }
       }
     }
     if (rc == SK_OK && e == cudaSuccess && !scales_tiled) {
-      const long long total = static_cast<long long>(plan->n_tiles) * plan->k_blocks * sk::kTileN;
+      const int groups = static_cast<int>(K / group_size);
+      const long long total = static_cast<long long>(plan->n_tiles) * groups * sk::kTileN;
       const int blocks = static_cast<int>(total / 256 + 1 < 148 * 8 ? total / 256 + 1 : 148 * 8);
-      sk::tile_scales_kernel<<<blocks, 256, 0, stream>>>(plan->w_scale, plan->w_scale_tiled, N, plan->k_blocks, total);
+      sk::tile_scales_kernel<<<blocks, 256, 0, stream>>>(plan->w_scale, plan->w_scale_tiled, N, groups, total);
       e = cudaGetLastError();
     }
     if (rc == SK_OK && e == cudaSuccess && !storage) e = cudaDeviceSynchronize();
@@ -1123,7 +1286,7 @@ int sk_w2a8_set_option(sk_w2a8_plan* plan, int key, int64_t value) {
   if (!plan) return SK_ERR_NULL_POINTER;
   switch (key) {
     case SK_OPT_KERNEL:
-      if (value < 0 || value > 5) return SK_ERR_BAD_ARGUMENT;
+      if (value < 0 || value > 6) return SK_ERR_BAD_ARGUMENT;
       if (value == 2 && !plan->w_rowmajor) return SK_ERR_UNAVAILABLE;
       if (value == 5 && !plan->stream_scratch) {   // first request on a plan that did not get the scratch at creation
         int cur = -1;
@@ -1309,6 +1472,17 @@ const char* sk_device_status_string(int device_status) {
     case sk::kStStreamSlots: return "epilogue: a tile is shared by more CTAs than the scratch buffer has slots for";
     default: return "unknown device status";
   }
+}
+
+int sk_w2a8_query_route(sk_w2a8_plan* plan, int64_t M, int* token_tile, int* split_k, int* ctas, int* kernel_kind) {
+  const int rc = sk_w2a8_query_launch(plan, M, token_tile, split_k, ctas, kernel_kind);
+  sk::DirectChoice d;
+  if (rc != SK_OK || !sk::choose_direct(plan, M, &d)) return rc;
+  if (token_tile) *token_tile = 8 * d.nt;
+  if (split_k) *split_k = d.split;
+  if (ctas) *ctas = d.ctas;
+  if (kernel_kind) *kernel_kind = 6;
+  return SK_OK;
 }
 
 int sk_w2a8_query_launch(sk_w2a8_plan* plan, int64_t M, int* token_tile, int* split_k, int* ctas, int* kernel_kind) {

@@ -353,6 +353,13 @@ std::vector<int64_t> query_launch(int64_t handle, int64_t M) {
   return {t, sp, c, k};
 }
 
+// the same for the launch w2a8_plan_gemm really makes
+std::vector<int64_t> query_route(int64_t handle, int64_t M) {
+  int t = 0, sp = 0, c = 0, k = 0;
+  check(sk_w2a8_query_route(as_plan(handle), M, &t, &sp, &c, &k), "w2a8_query_route");
+  return {t, sp, c, k};
+}
+
 void launch_floor_probe(int64_t handle, const at::Tensor& on_device_of, int64_t M) {
   c10::cuda::CUDAGuard guard(on_device_of.device());
   check(sk_w2a8_launch_floor_probe(as_plan(handle), M, at::cuda::getCurrentCUDAStream().stream()), "w2a8_launch_floor_probe");
@@ -480,6 +487,7 @@ TORCH_LIBRARY(slimkernels, m) {
   m.def("w2a8_plan_partials(int plan, Tensor x_q, int N, int K, int group_size) -> Tensor", &partials);
   m.def("w2a8_plan_device_status(int plan) -> int", &device_status);
   m.def("w2a8_plan_query_launch(int plan, int M) -> int[]", &query_launch);
+  m.def("w2a8_plan_query_route(int plan, int M) -> int[]", &query_route);
   m.def("w2a8_plan_launch_floor_probe(int plan, Tensor on_device_of, int M) -> ()", &launch_floor_probe);
   m.def("quantize_activation_int8(Tensor x) -> (Tensor, Tensor)", &quantize_activation);
   m.def("w2a8_quantize_weight(Tensor w_kn, int group_size) -> (Tensor, Tensor, Tensor)", &quantize_weight);

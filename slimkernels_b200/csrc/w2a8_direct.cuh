@@ -1,0 +1,362 @@
+// Decode GEMM without tensor memory: 2-bit weights go from HBM through a small ring of each warp's own into registers,
+// where two mask operations and a shift per word make them the operands of warp-level integer MMAs.
+//
+// For a handful of tokens the GEMM is one pass over the packed weights, and a call lasts a few microseconds: what
+// bounds it is how soon the first weights are asked for, how many bytes are in flight, and how long the last ones take
+// to turn into outputs.  The tcgen05 kernels pay for their roles there: set-up, four hand-overs per K block, a
+// tensor-memory round trip per scale group.  Here a warp owns 16 * MT output features and every WARPS-th 128-wide K block
+// of its CTA's range, and shares nothing with the others until the end:
+//   * cp.async brings whole blocks (2 KiB of codes at MT = 4, their scales) into DEPTH slots; nobody else reads them, so
+//     the only synchronisation is the warp's own wait for its oldest group;
+//   * a word holds 16 codes, two to a nibble.  w & 0x03030303 and (w >> 4) & 0x03030303 are four int8 codes each; with
+//     the mask 0x0C0C0C0C they are four codes times 4, and their products go to accumulators of their own, weighed 1/4 at
+//     the end.  Five operations per 16 codes (a byte-permute look-up needs nine, and prmt issues at half rate);
+//   * those four registers ARE A fragments of mma.sync m16n8k32: lane (g, q) holds features g and g + 8.  The K order
+//     inside an MMA is free as long as both operands use the same one, so the activations are read as they lie (two 16-byte
+//     loads per lane and 8 tokens) and four byte permutes per 16 codes put them in the masks' order;
+//   * the zero point is taken off per token, not per code: zero point x sum of the token's codes is a row of the same MMAs
+//     whose A operand is the zero point everywhere;
+//   * the exact int32 sums start at the bits of 1.5 * 2^23, so that they read as floats: an FMA, a subtraction and an FMA
+//     per value join the two accumulators, take the biases off and scale, all exact up to the last one.
+// The CTA's warps add their sums in shared memory in warp order, the CTAs of a cluster (split K) in rank order through
+// distributed shared memory: fixed orders, repeated launches are bit-identical.
+//
+// Measured, cold weights, tokens x features x K (before: the better tcgen05 decode kernel):
+//   1 x 4096 x 4096 3.0 us (6.2), 1 x 22016 x 4096 7.5 us (15.1), 8 x 57344 x 8192 28.5 us = 4.4 TB/s (52.7),
+//   16 x 22016 x 4096 10.7 us (15.2); group size 64: 8 x 22016 x 4096 11.9 us (44.9); group size 32: 14.8 us (48.6).
+// mma.sync s8 issues an m16n8k32 every 8 cycles per sub-core, 1.15 POP/s in all: from about 32 tokens on the tcgen05
+// kernels win on large weights (see choose_direct).
+#pragma once
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include "ptx_sm100.cuh"
+
+namespace sk {
+
+struct DirectParams {
+  const uint8_t* w_tiled;     // [n_tiles][k_blocks][4096]
+  const __half* w_scale_tiled;  // [n_tiles][groups][128], zero past N
+  const int8_t* x_q;          // [M, ld_x]
+  const float* x_scale;       // [M]
+  void* out;                  // [M, ld_out] half or bf16
+  void* out_extra[7];         // further destinations (peer GPUs' buffers), same ld_out
+  int n_extra;
+  long long ld_x, ld_out;
+  int M, N;
+  int K, groups;              // groups = K / G
+  int k_blocks;               // ceil(K / 128)
+  int blocks_per_group;       // G / 128 (group sizes 64 and 32 are the kernel's GPB = 128 / G instead)
+  int zero_point;
+  int out_bf16;
+};
+
+template <int MT, int NT, int WARPS, int DEPTH, int GPB>
+struct DirectTraits {
+  static constexpr int kFeatures = 16 * MT;        // output features per CTA
+  static constexpr int kTokens = 8 * NT;           // tokens per CTA
+  static constexpr int kThreads = 32 * WARPS;
+  // one warp's copy of a K block: the two halves of the features' codes (the second 64 bytes out of step, so that the four
+  // lanes of a feature read different banks), then their scales
+  static constexpr int kHalfBytes = 16 * kFeatures;
+  static constexpr int kOffHalf = kHalfBytes + 64;
+  static constexpr int kOffScales = kOffHalf + kHalfBytes;
+  static constexpr int kStageBytes = kOffScales + GPB * 2 * kFeatures;
+  static constexpr int kWarpBytes = DEPTH * kStageBytes;
+  static constexpr int kPitch = kFeatures + 4;     // floats per token in the reduction buffer: stores are conflict-free
+  static constexpr int kRedBytes = WARPS * kTokens * kPitch * 4;    // takes the rings' place
+  static constexpr int kDynamicBytes = WARPS * kWarpBytes > kRedBytes ? WARPS * kWarpBytes : kRedBytes;
+  static_assert(128 % kFeatures == 0, "a CTA's features lie in one weight tile");
+  static_assert(GPB * 2 * MT <= 32 && kStageBytes % 16 == 0, "one 16-byte piece of the scales per lane");
+};
+
+// d = a . b + c on 16 features x 8 tokens x 32 codes
+__device__ __forceinline__ void mma_s8_16832(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                             uint32_t b1, const int (&c)[4]) {
+  asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %11, %12, %13};"
+      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]));
+}
+// (volatile: never moved above griddepcontrol.wait)
+__device__ __forceinline__ uint4 ld_global_v4(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {   // L2 only: packed weights are read once
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ uint2 ld_shared_v2(uint32_t addr) {
+  uint2 v;
+  asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t ld_shared_b32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ float ld_shared_half(uint32_t addr) {
+  unsigned short v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr) : "memory");
+  return __half2float(__ushort_as_half(v));
+}
+
+template <int MT, int NT, int WARPS, int DEPTH, int MIN_CTAS, int GPB = 1>
+__global__ void __launch_bounds__(32 * WARPS, MIN_CTAS) w2a8_direct_kernel(const DirectParams p) {
+  using T = DirectTraits<MT, NT, WARPS, DEPTH, GPB>;
+  extern __shared__ __align__(16) uint8_t direct_smem[];
+  float* red = reinterpret_cast<float*>(direct_smem);   // after the main loop: [WARPS][kTokens][kPitch]
+  grid_dep_launch_dependents();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, q = lane & 3;
+  const int n0 = blockIdx.x * T::kFeatures;
+  const int m0 = blockIdx.y * T::kTokens;
+  const int splits = gridDim.z, rank = blockIdx.z; // a cluster spans the grid's z dimension
+  const int kb_end = static_cast<int>(static_cast<long long>(p.k_blocks) * (rank + 1) / splits);
+  const int kb0 = static_cast<int>(static_cast<long long>(p.k_blocks) * rank / splits) + warp;
+  // This warp's blocks are kb0, kb0 + WARPS, ...: `count` of them, walked in a ring that starts elsewhere in every CTA, so
+  // that the CTAs do not all ask L2 for the same activations at the same time.
+  const int count = kb0 < kb_end ? (kb_end - kb0 + WARPS - 1) / WARPS : 0;
+  const int first = count > 1 ? static_cast<int>(blockIdx.x % static_cast<unsigned>(count)) : 0;
+
+  // ---- weights and scales: DEPTH blocks in flight per warp
+  const size_t tile = static_cast<size_t>(n0 >> 7);
+  const uint8_t* w_src = p.w_tiled + (tile * p.k_blocks + kb0) * 4096 + ((n0 & 127) + (lane & 15)) * 16;
+  const uint8_t* s_src = reinterpret_cast<const uint8_t*>(p.w_scale_tiled) + tile * p.groups * 256 + (n0 & 127) * 2 +
+                         (lane % (2 * MT)) * 16;
+  const uint32_t ring = smem_u32(direct_smem) + warp * T::kWarpBytes;
+  int idx_fetch = first, to_fetch = count;
+  uint32_t slot_fetch = ring;
+  auto fetch = [&]() {
+    if (to_fetch > 0) {
+      const uint8_t* w = w_src + static_cast<size_t>(idx_fetch) * (WARPS * 4096);
+      // piece i of a lane: 16 rows of one half per half-warp
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        const int piece = 2 * i + (lane >> 4);     // 16-row group of the two halves' 2 * MT
+        const int half = piece / MT, rows = (piece % MT) * 16;
+        cp_async16(slot_fetch + half * T::kOffHalf + (rows + (lane & 15)) * 16, w + half * 2048 + rows * 16);
+      }
+      if (lane < GPB * 2 * MT) {
+        const int kb = kb0 + idx_fetch * WARPS;
+        const int group = GPB > 1 ? min(kb * GPB + lane / (2 * MT), p.groups - 1)
+                                  : p.blocks_per_group == 1 ? kb : kb / p.blocks_per_group;
+        cp_async16(slot_fetch + T::kOffScales + lane * 16, s_src + static_cast<size_t>(group) * 256);
+      }
+      --to_fetch;
+      if (++idx_fetch == count) idx_fetch = 0;
+    }
+    cp_async_commit();                             // (an empty group when there is nothing left: the waits count groups)
+    slot_fetch += T::kStageBytes;
+    if (slot_fetch == ring + T::kWarpBytes) slot_fetch = ring;
+  };
+#pragma unroll
+  for (int d = 0; d < DEPTH; ++d) fetch();
+
+  const uint32_t zp4x = static_cast<uint32_t>(p.zero_point) * 0x01010101u;
+  const int bias[4] = {0x4B400000, 0x4B400000, 0x4B400000, 0x4B400000};   // as a float 12582912 = 1.5 * 2^23
+  const int8_t* x_lane[NT];
+#pragma unroll
+  for (int t = 0; t < NT; ++t) x_lane[t] = p.x_q + min(m0 + 8 * t + g, p.M - 1) * p.ld_x + kb0 * 128 + (GPB == 1 ? 32 : 16) * q;
+  float acc[MT][NT][4];
+#pragma unroll
+  for (int i = 0; i < MT; ++i)
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[i][t][c] = 0.f;
+
+  // weights and scales were written by the plan; activations and outputs belong to the kernels before this one
+  grid_dep_wait();
+
+  uint4 xn[NT][2];                                 // the next block's activations
+  int idx_x = first, to_fetch_x = count;
+  auto fetch_x = [&]() {
+    if (to_fetch_x > 0) {
+      const int at = idx_x * (WARPS * 128);
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        if constexpr (GPB == 1) {
+          xn[t][0] = ld_global_v4(x_lane[t] + at);
+          xn[t][1] = ld_global_v4(x_lane[t] + at + 16);
+        } else {           // K ends inside the last block: what lies past it is read as zero (16-byte pieces: K % 32 == 0)
+          const int k = kb0 * 128 + at + 16 * q;
+          xn[t][0] = k < p.K ? ld_global_v4(x_lane[t] + at) : make_uint4(0u, 0u, 0u, 0u);
+          xn[t][1] = k + 64 < p.K ? ld_global_v4(x_lane[t] + at + 64) : make_uint4(0u, 0u, 0u, 0u);
+        }
+      }
+      --to_fetch_x;
+      if (++idx_x == count) idx_x = 0;
+    }
+  };
+  fetch_x();
+  // A lane's two words of a feature's block: GPB 1 adjacent ones (codes 32 q .. 32 q + 31), else word q of either half
+  // (codes 16 q .. and 64 + 16 q ..), so that a half -- one or two scale groups -- is one K step of the warp's MMAs.
+  const uint32_t w_off = (GPB == 1 ? (q >> 1) * T::kOffHalf + (q & 1) * 8 : q * 4) + g * 16;
+  uint32_t slot = ring;
+#pragma unroll 1
+  for (int left = count; left > 0; --left) {
+    cp_async_wait<DEPTH - 1>();
+    __syncwarp();
+    uint2 wv[2 * MT];
+    float sv[GPB][2 * MT];
+#pragma unroll
+    for (int j = 0; j < 2 * MT; ++j) {
+      if constexpr (GPB == 1) wv[j] = ld_shared_v2(slot + w_off + j * 128);
+      else wv[j] = make_uint2(ld_shared_b32(slot + w_off + j * 128), ld_shared_b32(slot + w_off + T::kOffHalf + j * 128));
+    }
+#pragma unroll
+    for (int b = 0; b < GPB; ++b)
+#pragma unroll
+      for (int j = 0; j < 2 * MT; ++j) sv[b][j] = ld_shared_half(slot + T::kOffScales + b * 2 * T::kFeatures + (8 * j + g) * 2);
+    __syncwarp();
+    fetch();                                   // into the slot just read
+    slot += T::kStageBytes;
+    if (slot == ring + T::kWarpBytes) slot = ring;
+    // B fragments in the order the masks below pick a word's codes: {0,2,8,10}, {1,3,9,11} | {4,6,12,14}, {5,7,13,15}
+    uint32_t b_lo[NT][2][2], b_hi[NT][2][2];
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        b_lo[t][h][0] = prmt(xn[t][h].x, xn[t][h].z, 0x6420u);
+        b_lo[t][h][1] = prmt(xn[t][h].x, xn[t][h].z, 0x7531u);
+        b_hi[t][h][0] = prmt(xn[t][h].y, xn[t][h].w, 0x6420u);
+        b_hi[t][h][1] = prmt(xn[t][h].y, xn[t][h].w, 0x7531u);
+      }
+    fetch_x();
+    if constexpr (GPB == 1) {
+      // zero point x sum of the token's codes, the same for every feature: one more row of MMAs, whose columns are the
+      // accumulators' columns; together with what the two biases below add up to
+      float off[NT][2];
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        int z[4];
+        mma_s8_16832(z, zp4x, zp4x, zp4x, zp4x, b_lo[t][0][0], b_lo[t][0][1], bias);
+        mma_s8_16832(z, zp4x, zp4x, zp4x, zp4x, b_hi[t][0][0], b_hi[t][0][1], z);
+        mma_s8_16832(z, zp4x, zp4x, zp4x, zp4x, b_lo[t][1][0], b_lo[t][1][1], z);
+        mma_s8_16832(z, zp4x, zp4x, zp4x, zp4x, b_hi[t][1][0], b_hi[t][1][1], z);
+        off[t][0] = __int_as_float(z[0]) + 3145728.f;      // 12582912 + zp sum + 3145728: integers below 2^24, exact
+        off[t][1] = __int_as_float(z[1]) + 3145728.f;
+      }
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        const uint2 lo = wv[2 * i], hi = wv[2 * i + 1];
+        const float s_lo = sv[0][2 * i], s_hi = sv[0][2 * i + 1];
+        constexpr uint32_t m0x = 0x03030303u, m4x = 0x0C0C0C0Cu;
+        const uint32_t lx4 = lo.x >> 4, ly4 = lo.y >> 4, hx4 = hi.x >> 4, hy4 = hi.y >> 4;
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          int l0[4], l1[4], h0[4], h1[4];
+          mma_s8_16832(l0, lo.x & m0x, hi.x & m0x, lx4 & m0x, hx4 & m0x, b_lo[t][0][0], b_lo[t][0][1], bias);
+          mma_s8_16832(h0, lo.x & m4x, hi.x & m4x, lx4 & m4x, hx4 & m4x, b_hi[t][0][0], b_hi[t][0][1], bias);
+          mma_s8_16832(l1, lo.y & m0x, hi.y & m0x, ly4 & m0x, hy4 & m0x, b_lo[t][1][0], b_lo[t][1][1], l0);
+          mma_s8_16832(h1, lo.y & m4x, hi.y & m4x, ly4 & m4x, hy4 & m4x, b_hi[t][1][0], b_hi[t][1][1], h0);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            // (12582912 + L) + (12582912 + 4 H) / 4 = 15728640 + L + H: integers below 2^24, exact
+            const float v = fmaf(0.25f, __int_as_float(h1[c]), __int_as_float(l1[c])) - off[t][c & 1];
+            acc[i][t][c] = fmaf(c < 2 ? s_lo : s_hi, v, acc[i][t][c]);
+          }
+        }
+      }
+    } else {
+      constexpr int kSub = GPB / 2;            // scale groups per half block: one, or the lanes q < 2 and q >= 2
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int sub = 0; sub < kSub; ++sub) {
+          const bool mine = kSub == 1 || (q >> 1) == sub;   // the other group's activations count as zero
+          uint32_t bl[NT][2], bh[NT][2];
+          float off[NT][2];
+#pragma unroll
+          for (int t = 0; t < NT; ++t) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              bl[t][e] = mine ? b_lo[t][h][e] : 0u;
+              bh[t][e] = mine ? b_hi[t][h][e] : 0u;
+            }
+            int z[4];
+            mma_s8_16832(z, zp4x, zp4x, zp4x, zp4x, bl[t][0], bl[t][1], bias);
+            mma_s8_16832(z, zp4x, zp4x, zp4x, zp4x, bh[t][0], bh[t][1], z);
+            off[t][0] = __int_as_float(z[0]) + 3145728.f;
+            off[t][1] = __int_as_float(z[1]) + 3145728.f;
+          }
+#pragma unroll
+          for (int i = 0; i < MT; ++i) {
+            const uint32_t lo = h == 0 ? wv[2 * i].x : wv[2 * i].y;
+            const uint32_t hi = h == 0 ? wv[2 * i + 1].x : wv[2 * i + 1].y;
+            const float s_lo = sv[h * kSub + sub][2 * i], s_hi = sv[h * kSub + sub][2 * i + 1];
+            constexpr uint32_t m0x = 0x03030303u, m4x = 0x0C0C0C0Cu;
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+              int l0[4], h0[4];
+              mma_s8_16832(l0, lo & m0x, hi & m0x, (lo >> 4) & m0x, (hi >> 4) & m0x, bl[t][0], bl[t][1], bias);
+              mma_s8_16832(h0, lo & m4x, hi & m4x, (lo >> 4) & m4x, (hi >> 4) & m4x, bh[t][0], bh[t][1], bias);
+#pragma unroll
+              for (int c = 0; c < 4; ++c) {
+                const float v = fmaf(0.25f, __int_as_float(h0[c]), __int_as_float(l0[c])) - off[t][c & 1];
+                acc[i][t][c] = fmaf(c < 2 ? s_lo : s_hi, v, acc[i][t][c]);
+              }
+            }
+          }
+        }
+    }
+  }
+
+  cp_async_wait<0>();
+  __syncthreads();                                 // every warp is done with its ring
+  // the warps' sums meet in shared memory: element (token, feature) of warp w at red[(w * kTokens + token) * kPitch + feature]
+  float* mine = red + warp * T::kTokens * T::kPitch;
+#pragma unroll
+  for (int i = 0; i < MT; ++i)
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+      float* r = mine + (8 * t + 2 * q) * T::kPitch + 16 * i + g;
+      r[0] = acc[i][t][0];
+      r[T::kPitch] = acc[i][t][1];
+      r[8] = acc[i][t][2];
+      r[T::kPitch + 8] = acc[i][t][3];
+    }
+  __syncthreads();
+  auto store = [&](int tok, int f, float sum) {
+    const int m = m0 + tok, n = n0 + f;
+    if (m >= p.M || n >= p.N) return;
+    const float y = sum * __ldg(p.x_scale + m);
+    const uint16_t bits = p.out_bf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(y)) : __half_as_ushort(__float2half_rn(y));
+    const size_t at = static_cast<size_t>(m) * p.ld_out + n;
+    reinterpret_cast<uint16_t*>(p.out)[at] = bits;
+    for (int e = 0; e < p.n_extra; ++e) reinterpret_cast<uint16_t*>(p.out_extra[e])[at] = bits;
+  };
+  const int tokens = min(T::kTokens, p.M - m0);
+  for (int i = threadIdx.x; i < tokens * T::kFeatures; i += T::kThreads) {
+    const int tok = i / T::kFeatures, f = i % T::kFeatures;
+    float* r = red + tok * T::kPitch + f;
+    float sum = r[0];
+#pragma unroll
+    for (int w = 1; w < WARPS; ++w) sum += r[w * T::kTokens * T::kPitch];
+    if (splits == 1) store(tok, f, sum);
+    else r[0] = sum;                               // (this thread alone reads and writes the element)
+  }
+  if (splits > 1) {
+    cluster_sync_all();
+    for (int i = rank * T::kThreads + threadIdx.x; i < tokens * T::kFeatures; i += splits * T::kThreads) {
+      const int tok = i / T::kFeatures, f = i % T::kFeatures;
+      const uint32_t local = smem_u32(red + tok * T::kPitch + f);
+      float part[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) part[r] = r < splits ? ld_dsmem_f32(map_to_cta(local, r)) : 0.f;
+      float sum = part[0];
+#pragma unroll
+      for (int r = 1; r < 8; ++r) sum += part[r];
+      store(tok, f, sum);
+    }
+    cluster_sync_all();                            // peers may still be reading this CTA's shared memory until here
+  }
+}
+
+}  // namespace sk

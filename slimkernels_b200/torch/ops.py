@@ -122,9 +122,14 @@ class W2A8Plan:
         """Launches the empty kernel with the launch geometry of a decode-sized GEMM (measurement aid)."""
         torch.ops.slimkernels.w2a8_plan_launch_floor_probe(self._h, self._w, int(M))
 
+    def query_route(self, M: int) -> dict:
+        """The launch gemm() makes for M tokens, as query_launch words it; kernel 6 is the direct decode kernel."""
+        t, s, c, k = torch.ops.slimkernels.w2a8_plan_query_route(self._h, int(M))
+        return {"token_tile": t, "split_k": s, "ctas": c, "kernel": k}
+
     def query_launch(self, M: int) -> dict:
-        """The launch the plan makes for M tokens: token tile, split-K factor, CTAs and kernel kind
-        (1 general tcgen05 kernel, 2 CUDA-core checker, 3 decode tcgen05 kernel)."""
+        """The launch the plan's tcgen05 kernels make for M tokens: token tile, split-K factor, CTAs and kernel kind
+        (1 general tcgen05 kernel, 2 CUDA-core checker, 3 / 5 decode tcgen05 kernels)."""
         t, s, c, k = torch.ops.slimkernels.w2a8_plan_query_launch(self._h, int(M))
         return {"token_tile": t, "split_k": s, "ctas": c, "kernel": k}
 
