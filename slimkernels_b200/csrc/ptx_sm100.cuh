@@ -270,6 +270,13 @@ __device__ __forceinline__ float ld_dsmem_f32(uint32_t cluster_addr) {
   return v;
 }
 
+__device__ __forceinline__ float4 ld_dsmem_f32x4(uint32_t cluster_addr) {   // 16-byte aligned
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(cluster_addr) : "memory");
+  return v;
+}
+
 __device__ __forceinline__ void st_dsmem_f32(uint32_t cluster_addr, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(cluster_addr), "f"(v) : "memory");
 }

@@ -321,8 +321,7 @@ static LaunchChoice choose(const sk_w2a8_plan* plan, long long M) {
       while (s < 8 && tiles * (2 * s) <= capacity && groups / (2 * s) >= min_groups) s *= 2;
     c.split_k = s;
   }
-  if (c.split_k > groups) c.split_k = 1;
-  if (c.token_tile > 64) c.split_k = 1;   // the cluster reduction buffer is sized for small token tiles
+  if (c.split_k > groups || c.token_tile == 192) c.split_k = 1;
   // Decode kernel, one token tile, more feature tiles than SMs (but fewer than CTA slots): with one CTA per tile a
   // few SMs carry two whole tiles and everybody waits for them.  Mixed launch instead: one CTA per tile for as many
   // tiles as there are SMs (rounded down to whole clusters of four), the tiles beyond that split 4 ways (or 2 ways,
@@ -358,12 +357,12 @@ static LaunchChoice choose(const sk_w2a8_plan* plan, long long M) {
 }
 
 template <int BLOCK_M, int EPI_WGS, int EXP_WARPS, int LSTAGES, int ESTAGES, int ACC_BUFS, bool DUMP, bool A_TMEM = false,
-          bool PERSIST = false>
+          bool PERSIST = false, bool SPLIT = false, bool OTHER_G = false>
 static int launch_umma(sk_w2a8_plan* plan, const CUtensorMap& map, const CUtensorMap& out_map,
                        const ExtraOutMaps& extra_maps, const GemmParams& prm, int m_tiles, int split_k,
                        int persistent_ctas, cudaStream_t stream) {
   using L = KernelTraits<BLOCK_M, EPI_WGS, EXP_WARPS, LSTAGES, ESTAGES, ACC_BUFS, A_TMEM, PERSIST>;
-  auto kern = w2a8_umma_kernel<BLOCK_M, EPI_WGS, EXP_WARPS, LSTAGES, ESTAGES, ACC_BUFS, DUMP, A_TMEM, PERSIST>;
+  auto kern = w2a8_umma_kernel<BLOCK_M, EPI_WGS, EXP_WARPS, LSTAGES, ESTAGES, ACC_BUFS, DUMP, A_TMEM, PERSIST, SPLIT, OTHER_G>;
   static int configured_device_mask[64] = {0};
   if (plan->device < 64 && !configured_device_mask[plan->device]) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamicBytes);
@@ -375,15 +374,24 @@ static int launch_umma(sk_w2a8_plan* plan, const CUtensorMap& map, const CUtenso
   cfg.blockDim = dim3(L::kThreads, 1, 1);
   cfg.dynamicSmemBytes = L::kDynamicBytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  int na = 0;
   if (split_k > 1) {
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = split_k;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = 1;
+    attr[na].val.clusterDim.y = 1;
+    attr[na].val.clusterDim.z = split_k;
+    ++na;
   }
+  // as for the decode kernels; where the tiles take several waves, set-up is nothing and early CTAs of the next kernel in
+  // the last wave's free slots cost 2 % (the MLP block of 4096 tokens: 704 us without, 721 with)
+  if (!DUMP && plan->opt_pdl != 1 && prm.small_grid) {
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = na;
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, map, out_map, extra_maps, prm);
   if (e != cudaSuccess) return cuda_fail(plan, e);
   return SK_OK;
@@ -737,6 +745,19 @@ static bool running_sum_fits(const sk_w2a8_plan* plan, int token_tile, int split
   return k_per_buf * 127 * mx < (1LL << 22);
 }
 
+// The general kernel's accumulator bias for a launch: the smallest power of two above what a running sum can reach.
+static uint32_t accumulator_bias(const sk_w2a8_plan* plan, int token_tile, int split_k) {
+  const long long per_block = plan->G < 128 ? 128 / plan->G : 1;
+  long long groups_cta = (plan->K / plan->G + split_k - 1) / split_k;
+  groups_cta = (groups_cta + per_block - 1) / per_block * per_block;      // (a CTA's range is whole K blocks)
+  const int ab = acc_bufs_of(token_tile, 1);
+  const int mx = plan->zero_point > 3 - plan->zero_point ? plan->zero_point : 3 - plan->zero_point;
+  const long long most = ((groups_cta + ab - 1) / ab) * plan->G * 128 * mx;
+  uint32_t bias = 1u << 8;
+  while (bias < (1u << 22) && static_cast<long long>(bias) <= most) bias <<= 1;
+  return bias;
+}
+
 // The launch run_gemm makes for M tokens: the heuristic choice, then the depth check.  A K range too deep for the two
 // accumulator buffers of the 256-token tile falls back to 128 tokens (four buffers, half the depth per buffer);
 // beyond that the call is refused.
@@ -758,6 +779,47 @@ static int resolve_launch(const sk_w2a8_plan* plan, long long M, bool debug_part
   }
   *out = ch;
   return SK_OK;
+}
+
+// The token tile and K split the general kernel runs M > 32 tokens with: of the tiles up to the heuristic one's size and
+// the splits the K range allows, the pair that a simple model gives the least time,
+//     waves x (set-up and output + K blocks per CTA x time per K block + cluster reduction),
+// with the constants below fitted to sweeps on B200 (one CTA per SM; they hold within 10 % from 32 to 1376 CTAs).  It replaces "the smallest tile that holds
+// M", which left most SMs idle wherever there are few tiles: 96 x 4096 x 11008 38.4 us on 32 CTAs, 15.3 as 128 tokens split 4
+// ways; 256 x 4096 x 4096 22.4, 13.7 as 64-token tiles; 512 x 4096 x 11008 50.7, 35.2 as 128-token tiles (in part the
+// expanders' second group, see w2a8_umma.cuh).
+// The launch that resolve_launch names stays where the model sees less than 5 % in it, where its depth check moved it to
+// another tile, and where an option forces any part of it.  What is refused is decided before, on that launch.
+static void refine_launch(const sk_w2a8_plan* plan, long long M, LaunchChoice* ch) {
+  if (ch->kernel != 1 || plan->opt_kernel || plan->opt_token_tile || plan->opt_split_k || plan->opt_persistent) return;
+  if (ch->token_tile != (M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256)) return;
+  struct Tile { int tokens; double us_cta, us_256, us_128, us_64, us_32, us_split; };   // per CTA, per K block by group size, per reduction
+  constexpr Tile kTiles[] = {{64, 3.4, 0.50, 0.285, 0.575, 1.04, 3.6}, {128, 4.0, 0.56, 0.365, 0.68, 1.14, 3.8}, {256, 5.3, 0.61, 0.43, 0.87, 1.8, 0.0}};
+  const int sms = plan->sm_count;
+  auto model = [&](const Tile& t, int split) {
+    const long long ctas = static_cast<long long>(plan->n_tiles) * ((M + t.tokens - 1) / t.tokens) * split;
+    const long long waves = (ctas + sms - 1) / sms;
+    const double us = plan->G > 128 ? t.us_256 : plan->G == 128 ? t.us_128 : plan->G == 64 ? t.us_64 : t.us_32;
+    return waves * (t.us_cta + ((plan->k_blocks + split - 1) / split) * us + (split > 1 ? t.us_split : 0.0));
+  };
+  const Tile* best = nullptr;
+  int best_split = 0;
+  double best_us = 0.0, now_us = 0.0;
+  for (const Tile& t : kTiles) {
+    if (t.tokens > ch->token_tile) continue;
+    for (int split = 1; split <= 8; split *= 2) {
+      if (split > 1 && (plan->k_blocks / split < 4 || t.tokens == 256)) continue;   // (256: the reduction takes longer than it saves)
+      if (!running_sum_fits(plan, t.tokens, split, 1)) continue;
+      const double us = model(t, split);
+      if (t.tokens == ch->token_tile && split == ch->split_k) now_us = us;
+      if (!best || us < best_us) { best = &t; best_split = split; best_us = us; }
+    }
+  }
+  if (!best || now_us == 0.0 || best_us > 0.95 * now_us) return;
+  ch->token_tile = best->tokens;
+  ch->split_k = best_split;
+  ch->persistent = 0;
+  ch->ctas = static_cast<int>(plan->n_tiles * ((M + best->tokens - 1) / best->tokens) * best_split);
 }
 
 // Test aid: the expander's shared-memory image of one 128 x 128 weight block next to the image the TMA writes for the
@@ -827,28 +889,49 @@ __global__ void diff_partials_kernel(int32_t* __restrict__ partials, int groups,
     for (int g = groups - 1; g >= acc_bufs; --g) partials[g * mn + i] -= partials[(g - acc_bufs) * mn + i];
 }
 
-template <bool DUMP>
+// <tokens, epilogue warpgroups, expander warps, load stages, expanded stages, accumulator buffers>
+template <bool SPLIT, bool OTHER_G>
+static int dispatch_umma_tile(sk_w2a8_plan* plan, int token_tile, const CUtensorMap& map, const CUtensorMap& out_map,
+                              const ExtraOutMaps& extra_maps, const GemmParams& prm, int m_tiles, int split_k, cudaStream_t stream) {
+  switch (token_tile) {
+    case 16: return launch_umma<16, 1, 8, 4, 4, kAccBufsSmall, false, false, false, SPLIT, OTHER_G>(plan, map, out_map, extra_maps, prm, m_tiles, split_k, 0, stream);
+    case 32: return launch_umma<32, 1, 4, 4, 4, kAccBufsSmall, false, false, false, SPLIT, OTHER_G>(plan, map, out_map, extra_maps, prm, m_tiles, split_k, 0, stream);
+    case 64: return launch_umma<64, 1, 8, 6, 6, kAccBufsSmall, false, false, false, SPLIT, OTHER_G>(plan, map, out_map, extra_maps, prm, m_tiles, split_k, 0, stream);
+    case 128: return launch_umma<128, 2, 8, 6, 6, kAccBufsSmall, false, false, false, SPLIT, OTHER_G>(plan, map, out_map, extra_maps, prm, m_tiles, split_k, 0, stream);
+    case 256: return launch_umma<256, 2, 4, 4, 4, kAccBufs256, false, false, false, SPLIT, OTHER_G>(plan, map, out_map, extra_maps, prm, m_tiles, split_k, 0, stream);
+    default: return SK_ERR_BAD_ARGUMENT;
+  }
+}
+
 static int dispatch_umma(sk_w2a8_plan* plan, int token_tile, const CUtensorMap& map, const CUtensorMap& out_map,
                          const ExtraOutMaps& extra_maps, const GemmParams& prm, int m_tiles, int split_k,
                          int persistent_ctas, cudaStream_t stream) {
+  if (persistent_ctas > 0 && token_tile == 128)
+    return launch_umma<128, 2, 4, 4, 4, kAccBufsSmall, false, false, true>(plan, map, out_map, extra_maps, prm, m_tiles, 1, persistent_ctas, stream);
+  if (persistent_ctas > 0 && token_tile == 256)
+    return launch_umma<256, 2, 4, 4, 2, kAccBufs256, false, false, true>(plan, map, out_map, extra_maps, prm, m_tiles, 1, persistent_ctas, stream);
+  // 192 tokens: the expanded weights live in tensor memory (2 x 192 accumulator columns + 4 x 32 weight columns;
+  // no expanded-weight ring in shared memory, so the load ring is 6 stages deep)
+  if (token_tile == 192)
+    return launch_umma<192, 2, 4, 6, 4, kAccBufs256, false, true>(plan, map, out_map, extra_maps, prm, m_tiles, 1, 0, stream);
+  const bool other = plan->G != 128;
+  if (split_k > 1)
+    return other ? dispatch_umma_tile<true, true>(plan, token_tile, map, out_map, extra_maps, prm, m_tiles, split_k, stream)
+                 : dispatch_umma_tile<true, false>(plan, token_tile, map, out_map, extra_maps, prm, m_tiles, split_k, stream);
+  return other ? dispatch_umma_tile<false, true>(plan, token_tile, map, out_map, extra_maps, prm, m_tiles, 1, stream)
+               : dispatch_umma_tile<false, false>(plan, token_tile, map, out_map, extra_maps, prm, m_tiles, 1, stream);
+}
+
+// The debug variants: they store the integer partial sums instead of the scaled output.
+static int dispatch_umma_dump(sk_w2a8_plan* plan, int token_tile, const CUtensorMap& map, const ExtraOutMaps& extra_maps,
+                              const GemmParams& prm, int m_tiles, cudaStream_t stream) {
   switch (token_tile) {
-    // <tokens, epilogue warpgroups, expander warps, load stages, expanded stages, accumulator buffers>
-    case 16: return launch_umma<16, 1, 8, 4, 4, kAccBufsSmall, DUMP>(plan, map, out_map, extra_maps, prm, m_tiles, split_k, persistent_ctas, stream);
-    case 32: return launch_umma<32, 1, 4, 4, 4, kAccBufsSmall, DUMP>(plan, map, out_map, extra_maps, prm, m_tiles, split_k, persistent_ctas, stream);
-    case 64: return launch_umma<64, 1, 4, 6, 6, kAccBufsSmall, DUMP>(plan, map, out_map, extra_maps, prm, m_tiles, split_k, persistent_ctas, stream);
-    case 128:
-      if constexpr (!DUMP)
-        if (persistent_ctas > 0)
-          return launch_umma<128, 2, 4, 4, 4, kAccBufsSmall, false, false, true>(plan, map, out_map, extra_maps, prm, m_tiles, 1, persistent_ctas, stream);
-      return launch_umma<128, 2, 4, 4, 4, kAccBufsSmall, DUMP>(plan, map, out_map, extra_maps, prm, m_tiles, split_k, persistent_ctas, stream);
-    // 192 tokens: the expanded weights live in tensor memory (2 x 192 accumulator columns + 4 x 32 weight columns;
-    // no expanded-weight ring in shared memory, so the load ring is 7 stages deep)
-    case 192: return launch_umma<192, 2, 4, 7, 4, kAccBufs256, DUMP, true>(plan, map, out_map, extra_maps, prm, m_tiles, split_k, persistent_ctas, stream);
-    case 256:
-      if constexpr (!DUMP)
-        if (persistent_ctas > 0)
-          return launch_umma<256, 2, 4, 4, 2, kAccBufs256, false, false, true>(plan, map, out_map, extra_maps, prm, m_tiles, 1, persistent_ctas, stream);
-      return launch_umma<256, 2, 4, 4, 4, kAccBufs256, DUMP>(plan, map, out_map, extra_maps, prm, m_tiles, split_k, persistent_ctas, stream);
+    case 16: return launch_umma<16, 1, 8, 4, 4, kAccBufsSmall, true>(plan, map, map, extra_maps, prm, m_tiles, 1, 0, stream);
+    case 32: return launch_umma<32, 1, 4, 4, 4, kAccBufsSmall, true>(plan, map, map, extra_maps, prm, m_tiles, 1, 0, stream);
+    case 64: return launch_umma<64, 1, 8, 6, 6, kAccBufsSmall, true>(plan, map, map, extra_maps, prm, m_tiles, 1, 0, stream);
+    case 128: return launch_umma<128, 2, 8, 6, 6, kAccBufsSmall, true>(plan, map, map, extra_maps, prm, m_tiles, 1, 0, stream);
+    case 192: return launch_umma<192, 2, 4, 6, 4, kAccBufs256, true, true>(plan, map, map, extra_maps, prm, m_tiles, 1, 0, stream);
+    case 256: return launch_umma<256, 2, 4, 4, 4, kAccBufs256, true>(plan, map, map, extra_maps, prm, m_tiles, 1, 0, stream);
     default: return SK_ERR_BAD_ARGUMENT;
   }
 }
@@ -955,6 +1038,7 @@ static int run_gemm(sk_w2a8_plan* plan, long long M, const int8_t* x_q, long lon
     if (cur != plan->device) (void)cudaSetDevice(cur);
     return SK_ERR_UNAVAILABLE;
   }
+  if (!partials) refine_launch(plan, M, &ch);
   if (ch.kernel == 2) {
     if (!plan->w_rowmajor || n_extra > 0) rc = SK_ERR_UNAVAILABLE;
     else {
@@ -990,6 +1074,8 @@ static int run_gemm(sk_w2a8_plan* plan, long long M, const int8_t* x_q, long lon
       prm.k_blocks = plan->k_blocks;
       prm.steps_per_group = plan->G / 32;
       prm.groups = static_cast<int>(plan->K / plan->G);
+      prm.small_grid = ch.ctas <= 2 * plan->sm_count;
+      prm.acc_bias = accumulator_bias(plan, ch.token_tile, partials ? 1 : ch.split_k);
       prm.zero_point = plan->zero_point;
       prm.out_bf16 = plan->out_dtype == SK_OUT_BF16;
       prm.wait_limit = plan->opt_wait_limit > 0 ? plan->opt_wait_limit : kWaitLimitCycles;
@@ -1041,7 +1127,7 @@ static int run_gemm(sk_w2a8_plan* plan, long long M, const int8_t* x_q, long lon
           rc = ch.token_tile == 16 ? launch_decode<16, true>(plan, map, prm, m_tiles, 1, stream)
                                    : launch_decode<32, true>(plan, map, prm, m_tiles, 1, stream);
         else if (ch.kernel == 4) rc = launch_pair<true>(plan, map, out_map, extra_maps, prm, m_tiles, stream);
-        else rc = dispatch_umma<true>(plan, ch.token_tile, map, out_map, extra_maps, prm, m_tiles, 1, 0, stream);
+        else rc = dispatch_umma_dump(plan, ch.token_tile, map, extra_maps, prm, m_tiles, stream);
         if (rc == SK_OK) {
           const long long mn = M * plan->N;
           const int blocks = static_cast<int>(mn / 256 + 1 < 148 * 8 ? mn / 256 + 1 : 148 * 8);
@@ -1056,7 +1142,7 @@ static int run_gemm(sk_w2a8_plan* plan, long long M, const int8_t* x_q, long lon
         rc = ch.token_tile == 16 ? launch_decode<16, false>(plan, map, prm, m_tiles, ch.split_k, stream, ch.mix_split ? ch.ctas : 0)
                                  : launch_decode<32, false>(plan, map, prm, m_tiles, ch.split_k, stream, ch.mix_split ? ch.ctas : 0);
       else if (ch.kernel == 4) rc = launch_pair<false>(plan, map, out_map, extra_maps, prm, m_tiles, stream);
-      else rc = dispatch_umma<false>(plan, ch.token_tile, map, out_map, extra_maps, prm, m_tiles, ch.split_k, persist ? ch.ctas : 0, stream);
+      else rc = dispatch_umma(plan, ch.token_tile, map, out_map, extra_maps, prm, m_tiles, ch.split_k, persist ? ch.ctas : 0, stream);
     }
   }
   if (cur != plan->device) (void)cudaSetDevice(cur);
@@ -1476,8 +1562,17 @@ const char* sk_device_status_string(int device_status) {
 
 int sk_w2a8_query_route(sk_w2a8_plan* plan, int64_t M, int* token_tile, int* split_k, int* ctas, int* kernel_kind) {
   const int rc = sk_w2a8_query_launch(plan, M, token_tile, split_k, ctas, kernel_kind);
+  if (rc != SK_OK) return rc;
   sk::DirectChoice d;
-  if (rc != SK_OK || !sk::choose_direct(plan, M, &d)) return rc;
+  if (!sk::choose_direct(plan, M, &d)) {
+    sk::LaunchChoice c;
+    (void)sk::resolve_launch(plan, M, false, &c);
+    sk::refine_launch(plan, M, &c);
+    if (token_tile) *token_tile = c.token_tile;
+    if (split_k) *split_k = c.split_k;
+    if (ctas) *ctas = c.ctas;
+    return SK_OK;
+  }
   if (token_tile) *token_tile = 8 * d.nt;
   if (split_k) *split_k = d.split;
   if (ctas) *ctas = d.ctas;

@@ -154,7 +154,7 @@ w2a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
   const int n0 = n_tile * kTileN;
   const int m0 = tc.m_tile * BLOCK_M;
   const int kb_end = p.groups;                         // group size 128: one K block per scale group
-  const uint32_t bias = 1u << 22;
+  const uint32_t bias = p.acc_bias;   // (the same as the general kernel's: same bits)
 
   // ---------------------------------------------------------------- set-up
   if (threadIdx.x == 0) SK_TRACE_EVENT(4, 0);

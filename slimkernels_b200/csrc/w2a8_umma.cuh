@@ -17,7 +17,7 @@
 //      output's alignment rules that out).
 //
 // Integer -> float without a conversion instruction, and without ever resetting an accumulator:
-//   * every accumulator buffer is pre-set ONCE per tile to the bias B = 2^22 and the MMAs always accumulate, so
+//   * every accumulator buffer is pre-set ONCE per tile to a bias B <= 2^22 and the MMAs always accumulate, so
 //     after group g buffer b = g mod ACC_BUFS holds the running sum  D_g = B + sum_{g' <= g, g' = g mod ACC_BUFS} P_g'
 //     with 0 < D < 2^23 (the host refuses K ranges whose running sums could leave that interval);
 //   * read as an IEEE float those bits are the denormal D * 2^-149, exactly;
@@ -106,6 +106,8 @@ struct GemmParams {
   int n_tiles;                // ceil(N / 128)
   int num_tiles;              // n_tiles * token tiles
   long long wait_limit;       // SM cycles after which a wait inside the kernel gives up (kWaitLimitCycles by default)
+  uint32_t acc_bias;          // general kernel: what the accumulators start at (a power of two, at most 2^22)
+  int small_grid;             // general kernel: let the next kernel in the stream start its set-up early
   int fault_skip_kb;          // failure-path test hook: the producer leaves out the copies of this K block of its
                               // range (-1: off), so that the waits for them run into the limit
   int mix_tiles1;             // decode kernel with clusters, mixed launch: tiles that get a CTA of their own (multiple of 4)
@@ -127,7 +129,12 @@ struct KernelTraits {
   static constexpr int kThreads = kWarps * 32;
   static constexpr int kEpiThreads = EPI_WGS * 128;
   static constexpr int kExpThreads = EXP_WARPS * 32;
-  static constexpr int kRowsPerExpThread = EXP_WARPS == 2 ? 2 : 1;   // with 8 warps a thread expands half a row
+  static constexpr int kRowsPerExpThread = EXP_WARPS == 2 ? 2 : 1;
+  // Eight expander warps: the 16-token tile gives every thread half a row; the others take K blocks in turn, four warps a
+  // block.  One block's wait -> load -> expand -> store -> proxy fence -> arrive is a serial chain of ~800 cycles, which
+  // paced the 64- and 128-token tiles with four warps (0.43 and 0.54 us per K block, three times their MMAs).
+  static constexpr bool kHalfRows = EXP_WARPS == 8 && BLOCK_M == 16;
+  static constexpr int kExpGroups = EXP_WARPS == 8 && !kHalfRows ? 2 : 1;
   static constexpr int kColsPerWg = BLOCK_M / EPI_WGS;           // accumulators per epilogue thread
   static constexpr int kChunk = kColsPerWg >= 32 ? 32 : 16;      // TMEM columns per tcgen05.ld
   static constexpr int kNumChunks = kColsPerWg / kChunk;
@@ -168,7 +175,7 @@ struct KernelTraits {
   // With fewer expanded stages than load stages (a deep load ring hides the TMA latency; expanded stages cost
   // 16 KB of shared memory or 32 TMEM columns each) a separate "expanded stage free" barrier is needed.
   static constexpr bool kTied = (ESTAGES == LSTAGES);
-  static_assert(ESTAGES <= LSTAGES, "expanded stages");
+  static_assert(ESTAGES <= LSTAGES && LSTAGES % 2 == 0 && ESTAGES % 2 == 0, "even rings: see the issuers");
   // Register budgets.  With two epilogue warpgroups the epilogue threads hold kColsPerWg accumulators plus two
   // sets of TMEM-load registers and take registers from the other warpgroup(s) with setmaxnreg.  The CTA's pool
   // is what it was given at launch (kLaunchRegs per thread); setmaxnreg.inc BLOCKS until the pool can serve it,
@@ -180,8 +187,9 @@ struct KernelTraits {
   static constexpr int kLaunchRegs = (65536 / kThreads) / 8 * 8;
   static constexpr bool kBig = kColsPerWg > 96;
   static constexpr int kEpiRegs = kBig ? 224 : 168;
-  static constexpr int kExpRegs = kBig ? 32 : 88;                         // warpgroup holding the expander warps
-  static constexpr int kCtlRegs = kBig ? (kThreads == 384 ? 56 : 32) : 88;   // warpgroup holding producer + MMA warps
+  static constexpr int kOtherRegs = EXP_WARPS == 8 ? 48 : 88;             // (640 threads, 96 at launch -> epilogue 168, others 48)
+  static constexpr int kExpRegs = kBig ? 32 : kOtherRegs;                 // warpgroup holding the expander warps
+  static constexpr int kCtlRegs = kBig ? (kThreads == 384 ? 56 : 32) : kOtherRegs;   // warpgroup holding producer + MMA warps
   static constexpr int kExpWgThreads = (EXP_WARPS == 4) ? 128 : 0;        // expanders have a warpgroup of their own
   static_assert(!kUseSetMaxNReg ||
                     kEpiThreads * kEpiRegs + kExpWgThreads * kExpRegs +
@@ -316,7 +324,7 @@ __device__ __forceinline__ void tmem_fill_chunk(uint32_t taddr, uint32_t value) 
 }
 
 template <int BLOCK_M, int EPI_WGS, int EXP_WARPS, int LSTAGES, int ESTAGES, int ACC_BUFS, bool DUMP, bool A_TMEM = false,
-          bool PERSIST = false>
+          bool PERSIST = false, bool SPLIT = false, bool OTHER_G = false>
 __global__ void __launch_bounds__(KernelTraits<BLOCK_M, EPI_WGS, EXP_WARPS, LSTAGES, ESTAGES, ACC_BUFS, A_TMEM, PERSIST>::kThreads,
                                   KernelTraits<BLOCK_M, EPI_WGS, EXP_WARPS, LSTAGES, ESTAGES, ACC_BUFS, A_TMEM, PERSIST>::kMinBlocks)
 w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_out,
@@ -345,10 +353,11 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + T::kOffMisc + 4);
   const WaitCtx ctx{abort_flag, p.status, p.wait_limit};
 
+  if (p.small_grid) grid_dep_launch_dependents();
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int split = blockIdx.z;
-  const int num_splits = gridDim.z;
+  const int split = SPLIT ? blockIdx.z : 0;        // (a kernel of its own: the reduction costs the others registers)
+  const int num_splits = SPLIT ? gridDim.z : 1;
   // Tiles are numbered feature-tile fastest.  A persistent CTA walks tiles blockIdx.x, blockIdx.x + gridDim.x, ...:
   // its rings, barrier phases and accumulator buffers simply carry on from one tile to the next, so the loads,
   // the expansion and the MMAs of the next tile start while the epilogue still writes the previous one.
@@ -357,29 +366,36 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
   const int tile_step = PERSIST ? static_cast<int>(gridDim.x) : 1;
 
   // K range of this CTA, in whole scale groups.
-  const int groups_per_split = (p.groups + num_splits - 1) / num_splits;
+  int groups_per_split = (p.groups + num_splits - 1) / num_splits;
+  if (SPLIT && OTHER_G && p.steps_per_group < 4) { // ... and in whole K blocks
+    const int per_block = 4 / p.steps_per_group;
+    groups_per_split = (groups_per_split + per_block - 1) / per_block * per_block;
+  }
   const int g_begin = min(split * groups_per_split, p.groups);
   const int g_end = min(g_begin + groups_per_split, p.groups);
   const int ks_begin = g_begin * p.steps_per_group;
   const int ks_end = g_end * p.steps_per_group;
   const int kb_begin = ks_begin / 4;
-  const int kb_end = (ks_end + 3) / 4;
+  const int kb_end = g_end > g_begin ? (ks_end + 3) / 4 : kb_begin;   // (a CTA of a cluster may have no groups)
 
-  // running sums stay inside (-2^22, 2^22): checked on the host (kMaxKPerAccBuf)
-  const uint32_t bias = 1u << 22;
+  // Running sums stay inside (-bias, bias), bias <= 2^22: checked on the host, which picks the smallest such power of two.
+  // The scaled sums are rounded at the bias's size until it is taken off, so a smaller one is accuracy for nothing: 2^18
+  // instead of 2^22 for 4096 codes in four buffers.
+  const uint32_t bias = p.acc_bias;
 
   // ---------------------------------------------------------------- set-up
   if (threadIdx.x == 0) SK_TRACE_EVENT(4, 0);
   // Every mbarrier counts ONE arrival per participating warp (lane 0, after __syncwarp): arrivals on one
   // barrier are serialised shared-memory atomics.
   if (threadIdx.x == 0) {
+    const int readers = OTHER_G && p.steps_per_group < 4 ? 2 : 1;   // issuing warps that read a stage
     for (int i = 0; i < LSTAGES; ++i) {
       mbar_init(bar_ld_full + 8 * i, 1);           // TMA transaction bytes
-      mbar_init(bar_ld_empty + 8 * i, 1);          // tcgen05.commit of the MMAs that read the stage
+      mbar_init(bar_ld_empty + 8 * i, readers);    // tcgen05.commit of the MMAs that read the stage
     }
     for (int i = 0; i < ESTAGES; ++i) {
-      mbar_init(bar_ex_full + 8 * i, EXP_WARPS);   // expanded weights of the stage are in place
-      mbar_init(bar_ex_empty + 8 * i, 1);          // commit of the MMAs that read them (untied rings only)
+      mbar_init(bar_ex_full + 8 * i, EXP_WARPS / T::kExpGroups);   // expanded weights of the stage are in place
+      mbar_init(bar_ex_empty + 8 * i, readers);    // commit of the MMAs that read them (untied rings only)
     }
     for (int i = 0; i < ACC_BUFS; ++i) { mbar_init(bar_acc_full + 8 * i, 1); mbar_init(bar_acc_empty + 8 * i, T::kEpiWarps); }
     *abort_flag = 0;
@@ -397,6 +413,9 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
   __syncthreads();
   tcgen05_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  // Programmatic dependent launch: the set-up above overlaps the tail of the previous kernel in the stream, which has to
+  // be complete before anything it wrote is read or its inputs are overwritten.
+  grid_dep_wait();
   if (threadIdx.x == 0) SK_TRACE_EVENT(4, 1);
 
   if (warp >= kExpWarp0) {
@@ -463,7 +482,52 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       int l = 0, e = 0, ab = 0;                 // load stage, expanded stage, accumulator buffer
       uint32_t lph = 0, eph = 0, aph = 0;       // their phases
       bool ok = true;
-      if (p.steps_per_group == 4) {
+      if constexpr (OTHER_G) {
+        // Group sizes other than 128 (a kernel of its own: the issuing warps of the 256-token tile have 32 registers).
+        // 64 and 32: a 128-wide K block holds two or four groups, and an issuer takes those whose accumulator buffers have its
+        // parity, in every block, so that it sees every phase of the barriers that it waits on: a parity wait that skips a
+        // phase can succeed one phase early.  (For the same reason the rings have even lengths where the issuers take blocks
+        // in turn.)  Both issuers read a block, so its "free" barriers count both.
+        // 256, 384, ...: a group spans blocks; one issuer.
+        const int steps = p.steps_per_group;                  // 1, 2 or a multiple of 8 (in blocks: 4)
+        const int per_block = steps < 4 ? 4 / steps : 1;      // groups per block
+        const int blocks = steps < 4 ? 1 : steps / 4;         // blocks per group
+        if (per_block > 1 || mma_id == 0)
+        for (int kb = kb_begin, buf = mma_id & (per_block > 1 ? 1 : 0), pos = 0; kb < kb_end; ++kb) {
+          ok = wait_bounded(bar_ld_full + 8 * l, lph, ctx, kStMmaLdFull) &&
+               wait_bounded(bar_ex_full + 8 * e, eph, ctx, kStMmaExFull);
+          const int n_groups = per_block > 1 ? min(per_block, g_end - kb * per_block) : 1;    // (the last block may be short)
+          for (int i = per_block > 1 ? mma_id : 0; i < n_groups && ok; i += 2) {
+            if (pos == 0) ok = wait_bounded(bar_acc_empty + 8 * buf, aph, ctx, kStMmaAccEmpty);
+            if (!ok) break;
+            tcgen05_fence_after_sync();
+            const bool last = pos == blocks - 1;
+            if (elect_one()) {
+              const uint64_t a_desc = a_desc0 + static_cast<uint64_t>(e * (kWxBytes >> 4) + 2 * i * steps);
+              const uint64_t b_desc = b_desc0 + static_cast<uint64_t>(l * (T::kXBytes >> 4) + 2 * i * steps);
+              const uint32_t d = tmem_base + buf * BLOCK_M;
+#pragma unroll
+              for (int s = 0; s < 4; ++s)
+                if (s < steps) umma_i8(d, a_desc + 2 * s, b_desc + 2 * s, idesc, 1u);
+              if (last) umma_commit(bar_acc_full + 8 * buf);
+            }
+            __syncwarp();
+            pos = last ? 0 : pos + 1;
+            if (last) {                                       // the issuer's next buffer
+              buf += per_block > 1 ? 2 : 1;
+              if (buf >= ACC_BUFS) { buf -= ACC_BUFS; aph ^= 1; }
+            }
+          }
+          if (!ok) break;
+          if (elect_one()) {
+            umma_commit(bar_ld_empty + 8 * l);
+            if constexpr (!T::kTied) umma_commit(bar_ex_empty + 8 * e);
+          }
+          __syncwarp();
+          if (++l == LSTAGES) { l = 0; lph ^= 1; }
+          if (++e == ESTAGES) { e = 0; eph ^= 1; }
+        }
+      } else if (p.steps_per_group == 4) {
         // one K block == one scale group: four MMAs and three commits per iteration, nothing else
         int turn = 0;                             // whose group this is (alternates over all K blocks of all tiles)
         for (int tile = tile_first; tile < tile_end && ok; tile += tile_step)
@@ -523,7 +587,8 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
           if (++ab == ACC_BUFS) { ab = 0; aph ^= 1; }
         }
       } else {
-        // general group sizes (32, 64, 256, ...): one issuer, tracking the position inside the group per 32-wide K step
+        // other group sizes in the debug, persistent and 192-token kernels: one issuer, tracking the position inside the group
+        // per 32-wide K step
         int pos = 0;
         if (mma_id == 0)
         for (int tile = tile_first; tile < tile_end && ok; tile += tile_step)
@@ -572,8 +637,9 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       __syncwarp();
     } else if (warp < kProducerWarp) {
       // ============================================================ expanders (one or two weight rows per thread)
-      const int et = threadIdx.x - kExpWarp0 * 32;             // expander thread index
-      constexpr bool kHalfRows = (EXP_WARPS == 8);             // 8 warps: a thread expands half a row
+      const int exp_group = (warp - kExpWarp0) / (EXP_WARPS / T::kExpGroups);
+      const int et = threadIdx.x - kExpWarp0 * 32 - exp_group * (T::kExpThreads / T::kExpGroups);   // thread index in the group
+      constexpr bool kHalfRows = T::kHalfRows;
       const int row0 = kHalfRows ? (et >> 1) : et * T::kRowsPerExpThread;
       const int half = kHalfRows ? (et & 1) : 0;
       const int zp = p.zero_point;
@@ -591,8 +657,17 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         wp_off[rr] = T::kOffWp + row * 16 + half * 2048;
       }
       bool ok = true;
+      int turn = 0;                                            // whose K block this is
       for (int tile = tile_first; tile < tile_end && ok; tile += tile_step)
       for (int kb = kb_begin; kb < kb_end; ++kb) {
+        if constexpr (T::kExpGroups > 1) {
+          turn ^= 1;
+          if (turn == exp_group) {                             // (group 0 starts: turn is 1 for the first block)
+            if (++l == LSTAGES) { l = 0; lph ^= 1; }
+            if (++e == ESTAGES) { e = 0; eph ^= 1; }
+            continue;
+          }
+        }
         // The loads below must not be issued before the wait has been seen to succeed: a load that does not depend
         // on the poll's predicate can be served before the barrier state is sampled and return stale bytes.
         ok = wait_bounded(bar_ld_full + 8 * l, lph, ctx, kStExpanderFull);
@@ -861,7 +936,7 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         xs_s[j] = (m0 + j < p.M) ? __ldg(p.x_scale + m0 + j) * kScaleDown : 0.f;
       named_barrier_sync(1, T::kEpiThreads);
       if (threadIdx.x == 0) SK_TRACE_EVENT(4, 2);
-      if (num_splits == 1) {
+      if constexpr (!SPLIT) {
         uint16_t* st = reinterpret_cast<uint16_t*>(smem);   // [BLOCK_M][128] in the output dtype
         if (p.out_bf16) stage_tokens<kCols, true>(acc, 0, xs_s + col0, st + col0 * kTileN + row);
         else stage_tokens<kCols, false>(acc, 0, xs_s + col0, st + col0 * kTileN + row);
@@ -915,41 +990,54 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     }
   }
 
-  if constexpr (!DUMP) {
-    if (num_splits > 1) {
+  if constexpr (!DUMP && SPLIT) {
+    {
       // split-K: fixed-order reduction over the cluster through distributed shared memory
       const float kScaleDown = 5.62949953421312e14f;
       __syncwarp();
       cluster_sync_all();
       if (warp < T::kEpiWarps) {
+        // A warp takes a token row, a lane four of its features: 16-byte remote loads, every CTA's in flight before the
+        // first is added, in rank order (deterministic).  (One float per thread and load left this phase latency-bound:
+        // 128 tokens over 4 CTAs were 16 dependent round trips of ~700 cycles.)
         const float* red = reinterpret_cast<const float*>(smem);
-        const uint32_t my_rank = cluster_ctarank();
-        const int row = threadIdx.x & 127;
-        const int wg = warp >> 2;
+        const int my_rank = static_cast<int>(cluster_ctarank());
         const TileCoord tc = tile_coord(tile_first, p.n_tiles, p.num_tiles);   // split-K CTAs own exactly one tile
-        const int n0 = tc.n_tile * kTileN;
+        const int n = tc.n_tile * kTileN + 4 * lane;
         const int m0 = tc.m_tile * BLOCK_M;
-        const int n = n0 + row;
-        uint16_t* outp = reinterpret_cast<uint16_t*>(p.out);
-        // token rows are dealt round-robin to (cluster rank, epilogue warpgroup); every remote load of a row
-        // is issued before the first is consumed, and the sum runs in rank order (deterministic)
-        for (int j = static_cast<int>(my_rank) * EPI_WGS + wg; j < BLOCK_M; j += num_splits * EPI_WGS) {
+        const bool vec_ok = n + 4 <= p.N && (p.ld_out % 4) == 0;
+#pragma unroll 2
+        for (int j = my_rank * T::kEpiWarps + warp; j < BLOCK_M; j += num_splits * T::kEpiWarps) {
           const int m = m0 + j;
           if (m >= p.M) break;
-          const uint32_t local = smem_u32(red + j * kTileN + row);
-          float part[8];
+          const uint32_t local = smem_u32(red + j * kTileN + 4 * lane);
+          float4 part[8];
 #pragma unroll
-          for (int r = 0; r < 8; ++r) part[r] = (r < num_splits) ? ld_dsmem_f32(map_to_cta(local, r)) : 0.f;
-          float sum = 0.f;
+          for (int r = 0; r < 8; ++r)
+            part[r] = r < num_splits ? ld_dsmem_f32x4(map_to_cta(local, r)) : make_float4(0.f, 0.f, 0.f, 0.f);
+          const float xs = __ldg(p.x_scale + m) * kScaleDown;
+          float y[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-          for (int r = 0; r < 8; ++r) sum += part[r];
-          const float y = sum * (__ldg(p.x_scale + m) * kScaleDown);
-          if (n < p.N) {
-            const uint16_t bits = p.out_bf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(y))
-                                             : __half_as_ushort(__float2half_rn(y));
-            outp[static_cast<size_t>(m) * p.ld_out + n] = bits;
-            for (int d = 0; d < p.n_extra; ++d)
-              reinterpret_cast<uint16_t*>(p.out_extra[d])[static_cast<size_t>(m) * p.ld_out + n] = bits;
+          for (int r = 0; r < 8; ++r) { y[0] += part[r].x; y[1] += part[r].y; y[2] += part[r].z; y[3] += part[r].w; }
+          uint16_t bits[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            bits[i] = p.out_bf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(y[i] * xs)) : __half_as_ushort(__float2half_rn(y[i] * xs));
+          int d_first = 0, d_last = p.n_extra, m_dst = m;
+          if (p.scatter_rows > 0) {                  // row scatter: the row's one destination, and its place there
+            d_first = d_last = m / p.scatter_rows;
+            m_dst = p.scatter_row0 + (m - d_first * p.scatter_rows);
+          }
+          for (int d = d_first; d <= d_last; ++d) {
+            uint16_t* o = reinterpret_cast<uint16_t*>(d == 0 ? p.out : p.out_extra[d - 1]) + static_cast<size_t>(m_dst) * p.ld_out + n;
+            if (vec_ok && (reinterpret_cast<uintptr_t>(o) & 7) == 0) {
+              *reinterpret_cast<uint2*>(o) = make_uint2(bits[0] | (static_cast<uint32_t>(bits[1]) << 16),
+                                                        bits[2] | (static_cast<uint32_t>(bits[3]) << 16));
+            } else {
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                if (n + i < p.N) o[i] = bits[i];
+            }
           }
         }
       }
