@@ -210,6 +210,12 @@ int sk_quantize_activation_int8(const void* x_f16, int64_t ld_x, int64_t M, int6
 /* The same with x in fp16 (x_bf16 = 0) or bf16 (1; each value is first rounded to fp16, on the way in). */
 int sk_quantize_activation_int8_from(const void* x, int x_bf16, int64_t ld_x, int64_t M, int64_t K, int8_t* x_q, int64_t ld_q,
                                      float* x_scale, sk_stream_t stream);
+/* A whole linear layer on float activations (x as above): quantise, then the GEMM.  A few tokens go through one kernel that
+ * quantises them itself (same bits) and needs no workspace; sk_w2a8_linear_workspace_bytes says what a call with M tokens
+ * needs (256-byte aligned device memory, 0: none). */
+int64_t sk_w2a8_linear_workspace_bytes(const sk_w2a8_plan* plan, int64_t M);
+int sk_w2a8_linear(sk_w2a8_plan* plan, int64_t M, const void* x, int x_bf16, int64_t ld_x, void* out, int64_t ld_out,
+                   void* workspace, int64_t workspace_bytes, sk_stream_t stream);
 /* gate_up fp16 [M, ld_gu] (gate = columns [0, I), up = [I, 2I)) -> h = SiLU(gate) * up in fp32, quantised as
  * above to h_q int8 [M, ld_q], h_scale fp32 [M].  I % 8 == 0. */
 int sk_silu_mul_quantize_int8(const void* gate_up_f16, int64_t ld_gu, int64_t M, int64_t I, int8_t* h_q,

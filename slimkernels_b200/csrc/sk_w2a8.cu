@@ -568,14 +568,19 @@ struct DirectChoice {
   bool deep;                  // all CTAs resident at once, three per SM
 };
 
-template <int MT, int NT, int WARPS, int DEPTH, int MIN_CTAS, int GPB>
+// Activations the direct kernel quantises itself: at most this many elements in all.  Every CTA reads them, so the limit is
+// what a CTA can read and convert in less time than a launch (one token through 4096 x 4096, a whole call: 9.4 us against 12.6).
+constexpr long long kDirectQuantElements = 8192;
+
+template <int MT, int NT, int WARPS, int DEPTH, int MIN_CTAS, int GPB, bool QUANT = false>
 static int launch_direct(sk_w2a8_plan* plan, const DirectParams& prm, int split, cudaStream_t stream) {
   using T = DirectTraits<MT, NT, WARPS, DEPTH, GPB>;
-  auto kern = w2a8_direct_kernel<MT, NT, WARPS, DEPTH, MIN_CTAS, GPB>;
-  if constexpr (T::kDynamicBytes > 48 * 1024) {
+  auto kern = w2a8_direct_kernel<MT, NT, WARPS, DEPTH, MIN_CTAS, GPB, QUANT>;
+  constexpr int kMaxQuant = QUANT ? static_cast<int>(kDirectQuantElements) + 8 * (128 + 16) : 0;   // (a rank's range rounds up to a block)
+  if constexpr (T::kQuantOffset + kMaxQuant > 48 * 1024) {
     static int configured_device_mask[64] = {0};
     if (plan->device < 64 && !configured_device_mask[plan->device]) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, T::kDynamicBytes);
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, T::kQuantOffset + kMaxQuant);
       if (e != cudaSuccess) return cuda_fail(plan, e);
       configured_device_mask[plan->device] = 1;
     }
@@ -584,7 +589,7 @@ static int launch_direct(sk_w2a8_plan* plan, const DirectParams& prm, int split,
   cfg.gridDim = dim3(static_cast<unsigned>((plan->N + T::kFeatures - 1) / T::kFeatures),
                      static_cast<unsigned>((prm.M + T::kTokens - 1) / T::kTokens), static_cast<unsigned>(split));
   cfg.blockDim = dim3(T::kThreads, 1, 1);
-  cfg.dynamicSmemBytes = T::kDynamicBytes;
+  cfg.dynamicSmemBytes = QUANT ? T::kQuantOffset + prm.M * ((prm.k_blocks + split - 1) / split * 128 + 16) : T::kDynamicBytes;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   int na = 0;
@@ -695,6 +700,17 @@ static int dispatch_direct(sk_w2a8_plan* plan, const DirectChoice& c, const Dire
     case 3: return launch_direct<2, 3, 8, 4, 1, 1>(plan, prm, c.split, stream);
     default: return launch_direct<2, 4, 8, 4, 1, 1>(plan, prm, c.split, stream);
   }
+}
+
+// The same with the activations quantised inside (up to 8 tokens, group sizes from 128 on).
+static bool direct_quantises(const sk_w2a8_plan* plan, long long M, const DirectChoice& c) {
+  return c.nt == 1 && plan->G >= 128 && M <= 8 && M * plan->K <= kDirectQuantElements;
+}
+static int dispatch_direct_quant(sk_w2a8_plan* plan, const DirectChoice& c, const DirectParams& prm, cudaStream_t stream) {
+  if (c.mt == 4 && c.warps == 8) return launch_direct<4, 1, 8, 4, 2, 1, true>(plan, prm, c.split, stream);
+  if (c.mt == 4)
+    return c.deep ? launch_direct<4, 1, 4, 6, 3, 1, true>(plan, prm, c.split, stream) : launch_direct<4, 1, 4, 4, 4, 1, true>(plan, prm, c.split, stream);
+  return c.warps == 4 ? launch_direct<2, 1, 4, 6, 4, 1, true>(plan, prm, c.split, stream) : launch_direct<2, 1, 8, 4, 2, 1, true>(plan, prm, c.split, stream);
 }
 
 constexpr int kPairStages = 6;
@@ -984,6 +1000,23 @@ static int get_out_map(sk_w2a8_plan* plan, const void* out, long long M, long lo
   return SK_OK;
 }
 
+static DirectParams direct_params(const sk_w2a8_plan* plan, long long M, void* out, long long ld_out) {
+  DirectParams prm = {};
+  prm.w_tiled = plan->w_tiled;
+  prm.w_scale_tiled = plan->w_scale_tiled;
+  prm.out = out;
+  prm.ld_out = ld_out;
+  prm.M = static_cast<int>(M);
+  prm.N = static_cast<int>(plan->N);
+  prm.K = static_cast<int>(plan->K);
+  prm.groups = static_cast<int>(plan->K / plan->G);
+  prm.k_blocks = plan->k_blocks;
+  prm.blocks_per_group = plan->G / 128;
+  prm.zero_point = plan->zero_point;
+  prm.out_bf16 = plan->out_dtype == SK_OUT_BF16;
+  return prm;
+}
+
 static int run_gemm(sk_w2a8_plan* plan, long long M, const int8_t* x_q, long long ld_x, const float* x_scale,
                     void* out, long long ld_out, int32_t* partials, cudaStream_t stream,
                     void* const* extra_outs = nullptr, int n_extra = 0, long long scatter_rows = 0,
@@ -1011,24 +1044,12 @@ static int run_gemm(sk_w2a8_plan* plan, long long M, const int8_t* x_q, long lon
   }
   DirectChoice dc;
   if (!partials && scatter_rows == 0 && choose_direct(plan, M, &dc)) {
-    DirectParams prm;
-    prm.w_tiled = plan->w_tiled;
-    prm.w_scale_tiled = plan->w_scale_tiled;
+    DirectParams prm = direct_params(plan, M, out, ld_out);
     prm.x_q = x_q;
     prm.x_scale = x_scale;
-    prm.out = out;
-    prm.n_extra = n_extra;
-    for (int i = 0; i < 7; ++i) prm.out_extra[i] = i < n_extra ? extra_outs[i] : nullptr;
     prm.ld_x = ld_x;
-    prm.ld_out = ld_out;
-    prm.M = static_cast<int>(M);
-    prm.N = static_cast<int>(plan->N);
-    prm.K = static_cast<int>(plan->K);
-    prm.groups = static_cast<int>(plan->K / plan->G);
-    prm.k_blocks = plan->k_blocks;
-    prm.blocks_per_group = plan->G / 128;
-    prm.zero_point = plan->zero_point;
-    prm.out_bf16 = plan->out_dtype == SK_OUT_BF16;
+    prm.n_extra = n_extra;
+    for (int i = 0; i < n_extra; ++i) prm.out_extra[i] = extra_outs[i];
     rc = dispatch_direct(plan, dc, prm, stream);
     if (cur != plan->device) (void)cudaSetDevice(cur);
     return rc;
@@ -1148,6 +1169,13 @@ static int run_gemm(sk_w2a8_plan* plan, long long M, const int8_t* x_q, long lon
   if (cur != plan->device) (void)cudaSetDevice(cur);
   return rc;
 }
+
+// Whether sk_w2a8_linear on M tokens is one kernel that quantises its activations itself.
+static bool linear_is_one_kernel(const sk_w2a8_plan* plan, long long M, DirectChoice* dc) {
+  LaunchChoice ch;
+  return M > 0 && resolve_launch(plan, M, false, &ch) == SK_OK && choose_direct(plan, M, dc) && direct_quantises(plan, M, *dc);
+}
+static size_t linear_scale_offset(long long M, long long K) { return (static_cast<size_t>(M) * K + 255) & ~static_cast<size_t>(255); }
 
 static int repack_common(bool forward, const uint8_t* src, long long N, long long K, uint8_t* dst,
                          cudaStream_t stream) {
@@ -1433,6 +1461,44 @@ int sk_w2a8_set_option(sk_w2a8_plan* plan, int key, int64_t value) {
 int sk_w2a8_gemm(sk_w2a8_plan* plan, int64_t M, const int8_t* x_q, int64_t ld_x, const float* x_scale, void* out,
                  int64_t ld_out, sk_stream_t stream) {
   return sk::run_gemm(plan, M, x_q, ld_x, x_scale, out, ld_out, nullptr, static_cast<cudaStream_t>(stream));
+}
+
+int64_t sk_w2a8_linear_workspace_bytes(const sk_w2a8_plan* plan, int64_t M) {
+  if (!plan || M <= 0) return 0;
+  sk::DirectChoice dc;
+  if (sk::linear_is_one_kernel(plan, M, &dc)) return 0;
+  return static_cast<int64_t>(sk::linear_scale_offset(M, plan->K)) + 4 * M;
+}
+
+int sk_w2a8_linear(sk_w2a8_plan* plan, int64_t M, const void* x, int x_bf16, int64_t ld_x, void* out, int64_t ld_out,
+                   void* workspace, int64_t workspace_bytes, sk_stream_t stream) {
+  if (!plan || !x || !out) return SK_ERR_NULL_POINTER;
+  if (M <= 0 || M > 0x7fffffffLL / 2 || ld_x < plan->K || ld_out < plan->N) return SK_ERR_BAD_SHAPE;
+  if ((reinterpret_cast<uintptr_t>(x) & 15) || (ld_x % 8) || (reinterpret_cast<uintptr_t>(out) & 1)) return SK_ERR_BAD_ALIGNMENT;
+  int cur = -1;
+  cudaError_t e = cudaGetDevice(&cur);
+  if (e == cudaSuccess && cur != plan->device) e = cudaSetDevice(plan->device);
+  if (e != cudaSuccess) return sk::cuda_fail(plan, e);
+  int rc;
+  sk::DirectChoice dc;
+  if (sk::linear_is_one_kernel(plan, M, &dc)) {
+    sk::DirectParams prm = sk::direct_params(plan, M, out, ld_out);
+    prm.x_float = static_cast<const uint16_t*>(x);
+    prm.ld_float = ld_x;
+    prm.float_bf16 = x_bf16;
+    rc = sk::dispatch_direct_quant(plan, dc, prm, static_cast<cudaStream_t>(stream));
+  } else if (!workspace) {
+    rc = SK_ERR_NULL_POINTER;
+  } else if (workspace_bytes < static_cast<int64_t>(sk::linear_scale_offset(M, plan->K)) + 4 * M) {
+    rc = SK_ERR_BAD_SHAPE;
+  } else {
+    int8_t* x_q = static_cast<int8_t*>(workspace);
+    float* x_scale = reinterpret_cast<float*>(x_q + sk::linear_scale_offset(M, plan->K));
+    rc = sk_quantize_activation_int8_from(x, x_bf16, ld_x, M, plan->K, x_q, plan->K, x_scale, stream);
+    if (rc == SK_OK) rc = sk::run_gemm(plan, M, x_q, plan->K, x_scale, out, ld_out, nullptr, static_cast<cudaStream_t>(stream));
+  }
+  if (cur != plan->device) (void)cudaSetDevice(cur);
+  return rc;
 }
 
 int sk_w2a8_gemm_scatter(sk_w2a8_plan* plan, int64_t M, const int8_t* x_q, int64_t ld_x, const float* x_scale,
@@ -1748,13 +1814,11 @@ int mlp_run(sk_w2a8_plan* gu, sk_w2a8_plan* down, int64_t M, const void* x, int 
             char* ws, sk_stream_t stream) {
   const int64_t hidden = gu->K, inter = down->K;
   const MlpLayout l = mlp_layout(M, hidden, inter);
-  int8_t* x_q = reinterpret_cast<int8_t*>(ws + l.x_q);
-  float* x_scale = reinterpret_cast<float*>(ws + l.x_scale);
   void* gate_up = ws + l.gate_up;
   int8_t* h_q = reinterpret_cast<int8_t*>(ws + l.h_q);
   float* h_scale = reinterpret_cast<float*>(ws + l.h_scale);
-  int rc = sk_quantize_activation_int8_from(x, x_bf16, ld_x, M, hidden, x_q, hidden, x_scale, stream);
-  if (rc == SK_OK) rc = sk_w2a8_gemm(gu, M, x_q, hidden, x_scale, gate_up, 2 * inter, stream);
+  // (int8 activations and their scales lie next to each other at the start of the workspace)
+  int rc = sk_w2a8_linear(gu, M, x, x_bf16, ld_x, gate_up, 2 * inter, ws + l.x_q, static_cast<int64_t>(l.gate_up - l.x_q), stream);
   if (rc == SK_OK) rc = sk_silu_mul_quantize_int8(gate_up, 2 * inter, M, inter, h_q, inter, h_scale, stream);
   if (rc == SK_OK) rc = sk_w2a8_gemm(down, M, h_q, inter, h_scale, out, ld_out, stream);
   return rc;

@@ -327,14 +327,13 @@ at::Tensor linear_forward(int64_t handle, const at::Tensor& x, int64_t N, int64_
   c10::cuda::CUDAGuard guard(x2.device());
   at::Tensor out = at::empty({M, N}, x2.options().dtype(bf16_out ? at::kBFloat16 : at::kHalf));
   if (M > 0) {
-    const int64_t scales = (M * K + 255) / 256 * 256;
-    at::Tensor ws = at::empty({scales + 4 * M}, x2.options().dtype(at::kByte));   // int8 rows, then their scales
-    int8_t* x_q = static_cast<int8_t*>(ws.data_ptr());
-    float* x_scale = reinterpret_cast<float*>(x_q + scales);
+    const int64_t bytes = sk_w2a8_linear_workspace_bytes(as_plan(handle), M);
+    at::Tensor ws;
+    if (bytes > 0) ws = at::empty({bytes}, x2.options().dtype(at::kByte));     // int8 rows, then their scales
     const auto stream = at::cuda::getCurrentCUDAStream();
-    check(sk_quantize_activation_int8_from(x2.data_ptr(), x_bf16, x2.stride(0), M, K, x_q, K, x_scale, stream.stream()),
-          "quantize_activation_int8");
-    check(sk_w2a8_gemm(plan_on(handle, stream), M, x_q, K, x_scale, out.data_ptr(), out.stride(0), stream.stream()), "w2a8_gemm");
+    check(sk_w2a8_linear(plan_on(handle, stream), M, x2.data_ptr(), x_bf16, x2.stride(0), out.data_ptr(), out.stride(0),
+                         bytes > 0 ? ws.data_ptr() : nullptr, bytes, stream.stream()),
+          "w2a8_linear");
   }
   return with_leading_shape(out, x);
 }

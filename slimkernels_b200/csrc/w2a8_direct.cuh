@@ -30,6 +30,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include "activation.cuh"   // the quantiser's rule
 #include "ptx_sm100.cuh"
 
 namespace sk {
@@ -49,6 +50,10 @@ struct DirectParams {
   int blocks_per_group;       // G / 128 (group sizes 64 and 32 are the kernel's GPB = 128 / G instead)
   int zero_point;
   int out_bf16;
+  // kernels that quantise their activations themselves (x_q, ld_x and x_scale are not used then)
+  const uint16_t* x_float;    // [M, ld_float] fp16 or bf16, rows 16-byte aligned
+  long long ld_float;
+  int float_bf16;
 };
 
 template <int MT, int NT, int WARPS, int DEPTH, int GPB>
@@ -66,6 +71,7 @@ struct DirectTraits {
   static constexpr int kPitch = kFeatures + 4;     // floats per token in the reduction buffer: stores are conflict-free
   static constexpr int kRedBytes = WARPS * kTokens * kPitch * 4;    // takes the rings' place
   static constexpr int kDynamicBytes = WARPS * kWarpBytes > kRedBytes ? WARPS * kWarpBytes : kRedBytes;
+  static constexpr int kQuantOffset = (kDynamicBytes + 15) / 16 * 16;   // int8 activations of kernels that quantise them
   static_assert(128 % kFeatures == 0, "a CTA's features lie in one weight tile");
   static_assert(GPB * 2 * MT <= 32 && kStageBytes % 16 == 0, "one 16-byte piece of the scales per lane");
 };
@@ -105,7 +111,7 @@ __device__ __forceinline__ float ld_shared_half(uint32_t addr) {
   return __half2float(__ushort_as_half(v));
 }
 
-template <int MT, int NT, int WARPS, int DEPTH, int MIN_CTAS, int GPB = 1>
+template <int MT, int NT, int WARPS, int DEPTH, int MIN_CTAS, int GPB = 1, bool QUANT = false>
 __global__ void __launch_bounds__(32 * WARPS, MIN_CTAS) w2a8_direct_kernel(const DirectParams p) {
   using T = DirectTraits<MT, NT, WARPS, DEPTH, GPB>;
   extern __shared__ __align__(16) uint8_t direct_smem[];
@@ -160,8 +166,9 @@ __global__ void __launch_bounds__(32 * WARPS, MIN_CTAS) w2a8_direct_kernel(const
   const uint32_t zp4x = static_cast<uint32_t>(p.zero_point) * 0x01010101u;
   const int bias[4] = {0x4B400000, 0x4B400000, 0x4B400000, 0x4B400000};   // as a float 12582912 = 1.5 * 2^23
   const int8_t* x_lane[NT];
+  if constexpr (!QUANT)
 #pragma unroll
-  for (int t = 0; t < NT; ++t) x_lane[t] = p.x_q + min(m0 + 8 * t + g, p.M - 1) * p.ld_x + kb0 * 128 + (GPB == 1 ? 32 : 16) * q;
+    for (int t = 0; t < NT; ++t) x_lane[t] = p.x_q + min(m0 + 8 * t + g, p.M - 1) * p.ld_x + kb0 * 128 + (GPB == 1 ? 32 : 16) * q;
   float acc[MT][NT][4];
 #pragma unroll
   for (int i = 0; i < MT; ++i)
@@ -173,6 +180,65 @@ __global__ void __launch_bounds__(32 * WARPS, MIN_CTAS) w2a8_direct_kernel(const
   // weights and scales were written by the plan; activations and outputs belong to the kernels before this one
   grid_dep_wait();
 
+  const int kb_first = kb0 - warp;                 // the CTA's range is [kb_first, kb_end)
+  uint32_t xs_lane = 0;                            // QUANT: this lane's token in shared memory, at the warp's first block
+  const float* q_scale = nullptr;
+  if constexpr (QUANT) {
+    // The activations of the CTA's K range as int8 behind the rings, by the quantiser's rule: the row's largest value (the
+    // whole row's), its scale, then the range.  Every CTA reads the rows again -- a few KiB from L2 -- which costs less than a
+    // kernel before this one whose only product is those bytes.
+    static_assert(NT == 1 && GPB == 1, "few tokens");
+    __shared__ float part[T::kTokens][WARPS];
+    __shared__ float scale_s[T::kTokens];
+    const int tokens = min(T::kTokens, p.M - m0);
+    const int nvec = p.K / 8;
+    auto row8 = [&](int tok, int v) {
+      const uint4 u = ld_global_v4(p.x_float + (m0 + tok) * p.ld_float + 8 * v);
+      return p.float_bf16 ? as_half8<true>(u) : u;
+    };
+    for (int tok = 0; tok < tokens; ++tok) {
+      float amax = 0.f;
+#pragma unroll 4
+      for (int v = threadIdx.x; v < nvec; v += T::kThreads) {
+        const uint4 u = row8(tok, v);
+        const __half2* h = reinterpret_cast<const __half2*>(&u);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 f = __half22float2(h[j]);
+          amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
+        }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+      if (lane == 0) part[tok][warp] = amax;
+    }
+    __syncthreads();
+    const int pitch = (kb_end - kb_first) * 128 + 16;    // 16 bytes on: a quarter-warp reads two tokens from different banks
+    uint8_t* xq_s = direct_smem + T::kQuantOffset;
+    for (int tok = 0; tok < tokens; ++tok) {
+      float amax = 0.f;
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) amax = fmaxf(amax, part[tok][w]);
+      const float s = amax > 0.f ? amax / 127.f : 1.f;
+      const float r = 1.f / s;
+      if (threadIdx.x == 0) scale_s[tok] = s;
+      for (int v = threadIdx.x; v < (kb_end - kb_first) * 16; v += T::kThreads) {
+        const uint4 u = row8(tok, kb_first * 16 + v);
+        const __half2* h = reinterpret_cast<const __half2*>(&u);
+        uint32_t w[2] = {0u, 0u};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 f = __half22float2(h[j]);
+          w[j >> 1] |= (quantize_one_fast(f.x, s, r) | (quantize_one_fast(f.y, s, r) << 8)) << (16 * (j & 1));
+        }
+        *reinterpret_cast<uint2*>(xq_s + tok * pitch + 8 * v) = make_uint2(w[0], w[1]);
+      }
+    }
+    __syncthreads();
+    q_scale = scale_s;
+    xs_lane = smem_u32(xq_s) + min(g, tokens - 1) * pitch + warp * 128 + 32 * q;
+  }
+
   uint4 xn[NT][2];                                 // the next block's activations
   int idx_x = first, to_fetch_x = count;
   auto fetch_x = [&]() {
@@ -180,7 +246,10 @@ __global__ void __launch_bounds__(32 * WARPS, MIN_CTAS) w2a8_direct_kernel(const
       const int at = idx_x * (WARPS * 128);
 #pragma unroll
       for (int t = 0; t < NT; ++t) {
-        if constexpr (GPB == 1) {
+        if constexpr (QUANT) {
+          xn[t][0] = ld_shared_v4(xs_lane + at);
+          xn[t][1] = ld_shared_v4(xs_lane + at + 16);
+        } else if constexpr (GPB == 1) {
           xn[t][0] = ld_global_v4(x_lane[t] + at);
           xn[t][1] = ld_global_v4(x_lane[t] + at + 16);
         } else {           // K ends inside the last block: what lies past it is read as zero (16-byte pieces: K % 32 == 0)
@@ -326,7 +395,7 @@ __global__ void __launch_bounds__(32 * WARPS, MIN_CTAS) w2a8_direct_kernel(const
   auto store = [&](int tok, int f, float sum) {
     const int m = m0 + tok, n = n0 + f;
     if (m >= p.M || n >= p.N) return;
-    const float y = sum * __ldg(p.x_scale + m);
+    const float y = sum * (QUANT ? q_scale[tok] : __ldg(p.x_scale + m));
     const uint16_t bits = p.out_bf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(y)) : __half_as_ushort(__float2half_rn(y));
     const size_t at = static_cast<size_t>(m) * p.ld_out + n;
     reinterpret_cast<uint16_t*>(p.out)[at] = bits;

@@ -99,3 +99,20 @@ def test_plan_is_refused_under_capture():
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(y, z)
+
+
+@pytest.mark.parametrize("G", [128, 256])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("M,N,K", [(1, 40, 256), (1, 4096, 4096), (1, 512, 8192), (2, 4096, 4096), (3, 300, 2560), (8, 136, 1024),
+                                   (1, 22016, 1024), (1, 57344, 512), (1, 12288, 768), (1, 4096, 8448)])
+def test_activations_quantised_inside_the_gemm(M, N, K, G, dtype):
+    """Few tokens: one kernel, the same bits as the quantiser followed by the GEMM (the last size is one over its limit)."""
+    lin = _linear(N, K, G, out_dtype=dtype)
+    for scale in (1.0, 0.0):
+        x = (torch.randn(M, K, device="cuda") * scale).to(dtype)
+        if M > 1:
+            x[1] = 0
+        assert torch.equal(lin(x), _by_pieces(lin, x))
+    wide = torch.randn(M, K + 24, device="cuda").to(dtype)[:, 16:16 + K]
+    if M > 1 and wide.data_ptr() % 16 == 0:
+        assert torch.equal(lin(wide), _by_pieces(lin, wide))
