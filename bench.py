@@ -426,14 +426,15 @@ def prefill_sweep(dev, peaks):
 
 
 def kernel_description(plan, M):
-    """Names the kernel the plan launches for M tokens, from sk_w2a8_query_launch (nothing is assumed here)."""
-    q = plan.query_launch(M)
+    """Names the kernel the plan launches for M tokens, from sk_w2a8_query_route (nothing is assumed here)."""
+    q = plan.query_route(M)
     kind = {1: "w2a8_umma_kernel (tcgen05.mma kind::i8, weights expanded to int8 in shared memory)",
             2: "w2a8_simt_kernel (CUDA cores)",
             3: "w2a8_decode_kernel (tcgen05.mma kind::i8, weights expanded into tensor memory, split-K over a cluster)",
             5: "w2a8_stream_kernel (tcgen05.mma kind::i8, weights expanded into tensor memory, K range of the whole "
                "problem cut into equal CTA ranges)",
-            4: "w2a8_pair_kernel (tcgen05.mma cta_group::2 kind::i8, two CTAs share one token tile)"}.get(q["kernel"], "?")
+            4: "w2a8_pair_kernel (tcgen05.mma cta_group::2 kind::i8, two CTAs share one token tile)",
+            6: "w2a8_direct_kernel (mma.sync s8, weights expanded in registers, split-K over warps and a cluster)"}.get(q["kernel"], "?")
     return f"{kind}: token tile {q['token_tile']}, split-K {q['split_k']}, {q['ctas']} CTAs", q
 
 

@@ -565,7 +565,6 @@ struct DirectChoice {
   int mt, nt, warps;          // 16-feature tiles per CTA, 8-token tiles per CTA, warps
   int split;                  // CTAs (one cluster) sharing the K range of a tile
   int ctas;
-  bool deep;                  // all CTAs resident at once, three per SM
 };
 
 // Activations the direct kernel quantises itself: at most this many elements in all.  Every CTA reads them, so the limit is
@@ -615,16 +614,16 @@ static int launch_direct(sk_w2a8_plan* plan, const DirectParams& prm, int split,
 // Serves small calls unless an option asks for another kernel (or for its failure-path hook).  Its time grows with the
 // tokens, the tcgen05 kernels' hardly does up to a tile, so the line lies where weights x tokens per SM get large (us, this
 // kernel against the better tcgen05 one, group size 128):
-//   * up to 24 tokens always: 24 x 57344 x 8192 64 / 80, 24 x 22016 x 4096 17.1 / 17.3, 24 x 4096 x 4096 4.9 / 7.6;
-//   * up to 32 tokens below 16 K blocks of a feature tile per SM: 32 x 4096 x 4096 5.9 / 7.8, but 32 x 22016 x 4096 24 / 17.5;
+//   * up to 24 tokens always: 24 x 57344 x 8192 61 / 80, 24 x 22016 x 4096 15.3 / 17.0, 24 x 4096 x 4096 4.5 / 7.6;
+//   * up to 32 tokens below 24 K blocks of a feature tile per SM: 32 x 4096 x 11008 10.4 / 11.5, but 32 x 22016 x 4096 22 / 17.4;
 //     with other group sizes always (64: 32 x 22016 x 4096 29 / 52);
 //   * up to 128 tokens below 8 such blocks per SM, the weight counted once per 32 tokens: 64 x 2048 x 1024 3.4 / 8.4,
 //     64 x 512 x 16384 6.9 / 10.6, but 64 x 4096 x 4096 11.6 / 9.2.
 // The shape of a CTA:
-//   * 64 features and 4 warps once that gives two CTAs per SM: 1 x 22016 x 4096 6.9, with 8 warps 8.8;
-//   * 64 features and 8 warps (8 tokens), 64 and 4 with the K range split (16 tokens) while there is a CTA of 64 per SM:
-//     1 x 12288 x 4096 4.9 against 5.3 with 32 features;
-//   * else, and from 24 tokens on, 32 features: 64 x 24 sums do not leave registers for three CTAs per SM;
+//   * 64 features and 4 warps from four such CTAs per SM on (two for 16 tokens): 8 x 57344 x 8192 28.7;
+//   * else 32 features and 4 warps from two of those per SM on: 8 x 22016 x 4096 7.2 (9.3 with 64), 24 tokens 15.1 (16.4); with 8
+//     tokens and one CTA of 64 per SM, 64 features and 8 warps: 8 x 12288 x 4096 5.2;
+//   * else 32 features and 8 warps;
 //   * the K range is split over a cluster while the CTAs fit the SMs' slots and every warp keeps four K blocks: 1 x 4096 x
 //     11008 in two halves 5.9, but 1 x 4096 x 4096 whole 2.7, in halves 3.7 (the cluster barriers cost more).
 static bool choose_direct(const sk_w2a8_plan* plan, long long M, DirectChoice* out) {
@@ -637,13 +636,13 @@ static bool choose_direct(const sk_w2a8_plan* plan, long long M, DirectChoice* o
   const long long token_tiles = (M + 8 * c.nt - 1) / (8 * c.nt);
   const long long work = static_cast<long long>(plan->n_tiles) * plan->k_blocks * token_tiles;
   if (token_tiles > 65535) return false;
-  if (!forced && c.nt == 4 && !(M <= 32 && (plan->G != 128 || work < 16 * sms)) && work > 8 * sms) return false;
+  if (!forced && c.nt == 4 && !(M <= 32 && (plan->G != 128 || work < 24 * sms)) && work > 8 * sms) return false;
   const long long per_64 = (plan->N + 63) / 64, per_32 = (plan->N + 31) / 32;
   int slots;                                   // CTAs an SM holds
   if (plan->G < 128) { c.mt = 2; c.warps = 4; slots = 4; }
-  else if (per_64 >= 2 * sms && (c.nt < 3 || per_64 >= 4 * sms)) { c.mt = 4; c.warps = 4; slots = 2; }
-  else if (per_64 >= sms && c.nt <= 2) { c.mt = 4; c.warps = c.nt == 1 ? 8 : 4; slots = c.nt == 1 ? 2 : 3; }
-  else if (per_32 >= 2 * sms) { c.mt = 2; c.warps = 4; slots = 3; }
+  else if (c.nt != 3 && per_64 >= (c.nt == 2 ? 2 : 4) * sms) { c.mt = 4; c.warps = 4; slots = 2; }
+  else if (c.nt == 1 && per_64 >= sms && per_64 < 2 * sms) { c.mt = 4; c.warps = 8; slots = 2; }
+  else if (per_32 >= 2 * sms) { c.mt = 2; c.warps = 4; slots = 2; }
   else { c.mt = 2; c.warps = 8; slots = c.nt <= 2 ? 2 : 1; }
   const long long tiles = (c.mt == 4 ? per_64 : per_32) * token_tiles;
   c.split = 1;
@@ -652,14 +651,12 @@ static bool choose_direct(const sk_w2a8_plan* plan, long long M, DirectChoice* o
     while (c.split < 8 && tiles * (2 * c.split) <= slots * sms && plan->k_blocks / (2 * c.split * c.warps) >= 4) c.split *= 2;
   if (c.split > plan->k_blocks) c.split = 1;
   c.ctas = static_cast<int>(tiles * c.split);
-  c.deep = tiles * c.split <= 3 * sms;
   *out = c;
   return true;
 }
 
 // <16-feature tiles, 8-token tiles, warps, K blocks in flight per warp, CTAs per SM that registers are kept for, groups per
-// K block>.  With 4 warps and one token tile, three CTAs of six blocks in flight where they all fit at once (1 x 22016 x 4096
-// 6.9 us; four of four blocks 8.5), else four of four (1 x 57344 x 8192 27.7; 30.0).
+// K block>
 static int dispatch_direct(sk_w2a8_plan* plan, const DirectChoice& c, const DirectParams& prm, cudaStream_t stream) {
   if (plan->G == 64) {
     switch (c.nt) {
@@ -680,18 +677,17 @@ static int dispatch_direct(sk_w2a8_plan* plan, const DirectChoice& c, const Dire
   if (c.mt == 4 && c.warps == 8) return launch_direct<4, 1, 8, 4, 2, 1>(plan, prm, c.split, stream);
   if (c.mt == 4) {
     switch (c.nt) {
-      case 1: return c.deep ? launch_direct<4, 1, 4, 6, 3, 1>(plan, prm, c.split, stream) : launch_direct<4, 1, 4, 4, 4, 1>(plan, prm, c.split, stream);
-      case 2: return launch_direct<4, 2, 4, 4, 3, 1>(plan, prm, c.split, stream);
-      case 3: return launch_direct<4, 3, 4, 4, 2, 1>(plan, prm, c.split, stream);
+      case 1: return launch_direct<4, 1, 4, 4, 3, 1>(plan, prm, c.split, stream);
+      case 2: return launch_direct<4, 2, 4, 6, 3, 1>(plan, prm, c.split, stream);
       default: return launch_direct<4, 4, 4, 4, 2, 1>(plan, prm, c.split, stream);
     }
   }
   if (c.warps == 4) {
     switch (c.nt) {
-      case 1: return launch_direct<2, 1, 4, 6, 4, 1>(plan, prm, c.split, stream);
+      case 1: return launch_direct<2, 1, 4, 4, 4, 1>(plan, prm, c.split, stream);
       case 2: return launch_direct<2, 2, 4, 6, 4, 1>(plan, prm, c.split, stream);
       case 3: return launch_direct<2, 3, 4, 6, 3, 1>(plan, prm, c.split, stream);
-      default: return launch_direct<2, 4, 4, 6, 3, 1>(plan, prm, c.split, stream);
+      default: return launch_direct<2, 4, 4, 4, 2, 1>(plan, prm, c.split, stream);
     }
   }
   switch (c.nt) {
@@ -708,9 +704,8 @@ static bool direct_quantises(const sk_w2a8_plan* plan, long long M, const Direct
 }
 static int dispatch_direct_quant(sk_w2a8_plan* plan, const DirectChoice& c, const DirectParams& prm, cudaStream_t stream) {
   if (c.mt == 4 && c.warps == 8) return launch_direct<4, 1, 8, 4, 2, 1, true>(plan, prm, c.split, stream);
-  if (c.mt == 4)
-    return c.deep ? launch_direct<4, 1, 4, 6, 3, 1, true>(plan, prm, c.split, stream) : launch_direct<4, 1, 4, 4, 4, 1, true>(plan, prm, c.split, stream);
-  return c.warps == 4 ? launch_direct<2, 1, 4, 6, 4, 1, true>(plan, prm, c.split, stream) : launch_direct<2, 1, 8, 4, 2, 1, true>(plan, prm, c.split, stream);
+  if (c.mt == 4) return launch_direct<4, 1, 4, 4, 3, 1, true>(plan, prm, c.split, stream);
+  return c.warps == 4 ? launch_direct<2, 1, 4, 4, 4, 1, true>(plan, prm, c.split, stream) : launch_direct<2, 1, 8, 4, 2, 1, true>(plan, prm, c.split, stream);
 }
 
 constexpr int kPairStages = 6;

@@ -8,23 +8,23 @@
 // of its CTA's range, and shares nothing with the others until the end:
 //   * cp.async brings whole blocks (2 KiB of codes at MT = 4, their scales) into DEPTH slots; nobody else reads them, so
 //     the only synchronisation is the warp's own wait for its oldest group;
-//   * a word holds 16 codes, two to a nibble.  w & 0x03030303 and (w >> 4) & 0x03030303 are four int8 codes each; with
-//     the mask 0x0C0C0C0C they are four codes times 4, and their products go to accumulators of their own, weighed 1/4 at
-//     the end.  Five operations per 16 codes (a byte-permute look-up needs nine, and prmt issues at half rate);
+//   * a word holds 16 codes.  code - zero point fits two bits of two's complement (or its negative does: see the kernel), and
+//     in the top two bits of a byte that is 64 times its value as int8: a shift and one three-input logic operation take four
+//     codes of a word (a byte-permute look-up needs nine operations per 16 codes instead of seven, and prmt issues at half
+//     rate; masking without a shift, with the zero point as further rows of MMAs, five, but a quarter more MMAs);
 //   * those four registers ARE A fragments of mma.sync m16n8k32: lane (g, q) holds features g and g + 8.  The K order
 //     inside an MMA is free as long as both operands use the same one, so the activations are read as they lie (two 16-byte
-//     loads per lane and 8 tokens) and four byte permutes per 16 codes put them in the masks' order;
-//   * the zero point is taken off per token, not per code: zero point x sum of the token's codes is a row of the same MMAs
-//     whose A operand is the zero point everywhere;
-//   * the exact int32 sums start at the bits of 1.5 * 2^23, so that they read as floats: an FMA, a subtraction and an FMA
-//     per value join the two accumulators, take the biases off and scale, all exact up to the last one.
+//     loads per lane and 8 tokens) and four byte permutes per 16 codes put them in the words' order;
+//   * the exact int32 sums start at the bits of 1.5 * 2^23, so that they read as floats: a subtraction and an FMA per value
+//     take the bias off and scale, exact up to the last rounding.
 // The CTA's warps add their sums in shared memory in warp order, the CTAs of a cluster (split K) in rank order through
 // distributed shared memory: fixed orders, repeated launches are bit-identical.
 //
 // Measured, cold weights, tokens x features x K (before: the better tcgen05 decode kernel):
-//   1 x 4096 x 4096 3.0 us (6.2), 1 x 22016 x 4096 7.5 us (15.1), 8 x 57344 x 8192 28.5 us = 4.4 TB/s (52.7),
-//   16 x 22016 x 4096 10.7 us (15.2); group size 64: 8 x 22016 x 4096 11.9 us (44.9); group size 32: 14.8 us (48.6).
-// mma.sync s8 issues an m16n8k32 every 8 cycles per sub-core, 1.15 POP/s in all: from about 32 tokens on the tcgen05
+//   8 x 4096 x 4096 2.8 us (6.1), 8 x 22016 x 4096 7.2 us (15.1), 8 x 57344 x 8192 28.7 us = 4.3 TB/s (52.7),
+//   16 x 12288 x 4096 8.0 us (10.4), 24 x 4096 x 11008 8.9 us (12.5); group size 64: 8 x 22016 x 4096 11.4 us (46.5).
+// mma.sync s8 issues an m16n8k32 every 8 cycles per sub-core, 1.15 POP/s in all, but two or three warps per sub-core do not
+// keep it busy (a third of the cycles at 24 tokens), and few CTAs fill whole waves badly: from about 32 tokens on the tcgen05
 // kernels win on large weights (see choose_direct).
 #pragma once
 #include <cuda_bf16.h>
@@ -83,6 +83,18 @@ __device__ __forceinline__ void mma_s8_16832(int (&d)[4], uint32_t a0, uint32_t 
       : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]));
 }
+// The 16 codes of a tiled word as four registers of int8, code k of a nibble pair in the top two bits of its byte: f[0] codes
+// {0, 2, 8, 10}, f[1] {4, 6, 12, 14}, f[2] {1, 3, 9, 11}, f[3] {5, 7, 13, 15} (a shift and a three-input logic operation each).
+struct CodeBytes {
+  uint32_t f[4];
+  __device__ __forceinline__ CodeBytes(uint32_t w, uint32_t flip) {
+    constexpr uint32_t kTop = 0xC0C0C0C0u;
+    f[0] = ((w << 6) ^ flip) & kTop;
+    f[1] = ((w << 4) ^ flip) & kTop;
+    f[2] = ((w << 2) ^ flip) & kTop;
+    f[3] = (w ^ flip) & kTop;
+  }
+};
 // (volatile: never moved above griddepcontrol.wait)
 __device__ __forceinline__ uint4 ld_global_v4(const void* p) {
   uint4 v;
@@ -163,7 +175,13 @@ __global__ void __launch_bounds__(32 * WARPS, MIN_CTAS) w2a8_direct_kernel(const
 #pragma unroll
   for (int d = 0; d < DEPTH; ++d) fetch();
 
-  const uint32_t zp4x = static_cast<uint32_t>(p.zero_point) * 0x01010101u;
+  // code - zp as two's complement in the top two bits of a byte is 64 times its value: for zp 2 the code with its upper bit
+  // flipped, for zp 1 the code with its lower bit flipped is 1 - code (the scale takes the sign).  Zero points 0 and 3 do not fit
+  // two bits: they are zp 2 plus a multiple of the token's sum of codes, another row of MMAs.
+  const uint32_t flip = p.zero_point == 1 ? 0x55555555u : 0xAAAAAAAAu;
+  const float unit = p.zero_point == 1 ? -0.015625f : 0.015625f;
+  const bool offset = p.zero_point == 0 || p.zero_point == 3;
+  const uint32_t offset4x = p.zero_point == 0 ? 0x80808080u : 0x40404040u;     // -64 * 2, or -64 * -1
   const int bias[4] = {0x4B400000, 0x4B400000, 0x4B400000, 0x4B400000};   // as a float 12582912 = 1.5 * 2^23
   const int8_t* x_lane[NT];
   if constexpr (!QUANT)
@@ -281,7 +299,7 @@ __global__ void __launch_bounds__(32 * WARPS, MIN_CTAS) w2a8_direct_kernel(const
 #pragma unroll
     for (int b = 0; b < GPB; ++b)
 #pragma unroll
-      for (int j = 0; j < 2 * MT; ++j) sv[b][j] = ld_shared_half(slot + T::kOffScales + b * 2 * T::kFeatures + (8 * j + g) * 2);
+      for (int j = 0; j < 2 * MT; ++j) sv[b][j] = unit * ld_shared_half(slot + T::kOffScales + b * 2 * T::kFeatures + (8 * j + g) * 2);
     __syncwarp();
     fetch();                                   // into the slot just read
     slot += T::kStageBytes;
@@ -299,38 +317,35 @@ __global__ void __launch_bounds__(32 * WARPS, MIN_CTAS) w2a8_direct_kernel(const
       }
     fetch_x();
     if constexpr (GPB == 1) {
-      // zero point x sum of the token's codes, the same for every feature: one more row of MMAs, whose columns are the
-      // accumulators' columns; together with what the two biases below add up to
-      float off[NT][2];
+      float off[NT][2];                            // the bias, and what zero points 0 and 3 add per token
 #pragma unroll
       for (int t = 0; t < NT; ++t) {
-        int z[4];
-        mma_s8_16832(z, zp4x, zp4x, zp4x, zp4x, b_lo[t][0][0], b_lo[t][0][1], bias);
-        mma_s8_16832(z, zp4x, zp4x, zp4x, zp4x, b_hi[t][0][0], b_hi[t][0][1], z);
-        mma_s8_16832(z, zp4x, zp4x, zp4x, zp4x, b_lo[t][1][0], b_lo[t][1][1], z);
-        mma_s8_16832(z, zp4x, zp4x, zp4x, zp4x, b_hi[t][1][0], b_hi[t][1][1], z);
-        off[t][0] = __int_as_float(z[0]) + 3145728.f;      // 12582912 + zp sum + 3145728: integers below 2^24, exact
-        off[t][1] = __int_as_float(z[1]) + 3145728.f;
+        off[t][0] = off[t][1] = 12582912.f;
+        if (offset) {
+          int z[4];
+          mma_s8_16832(z, offset4x, offset4x, offset4x, offset4x, b_lo[t][0][0], b_lo[t][0][1], bias);
+          mma_s8_16832(z, offset4x, offset4x, offset4x, offset4x, b_hi[t][0][0], b_hi[t][0][1], z);
+          mma_s8_16832(z, offset4x, offset4x, offset4x, offset4x, b_lo[t][1][0], b_lo[t][1][1], z);
+          mma_s8_16832(z, offset4x, offset4x, offset4x, offset4x, b_hi[t][1][0], b_hi[t][1][1], z);
+          off[t][0] = __int_as_float(z[0]);
+          off[t][1] = __int_as_float(z[1]);
+        }
       }
 #pragma unroll
       for (int i = 0; i < MT; ++i) {
         const uint2 lo = wv[2 * i], hi = wv[2 * i + 1];
         const float s_lo = sv[0][2 * i], s_hi = sv[0][2 * i + 1];
-        constexpr uint32_t m0x = 0x03030303u, m4x = 0x0C0C0C0Cu;
-        const uint32_t lx4 = lo.x >> 4, ly4 = lo.y >> 4, hx4 = hi.x >> 4, hy4 = hi.y >> 4;
+        const CodeBytes lx(lo.x, flip), ly(lo.y, flip), hx(hi.x, flip), hy(hi.y, flip);
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
-          int l0[4], l1[4], h0[4], h1[4];
-          mma_s8_16832(l0, lo.x & m0x, hi.x & m0x, lx4 & m0x, hx4 & m0x, b_lo[t][0][0], b_lo[t][0][1], bias);
-          mma_s8_16832(h0, lo.x & m4x, hi.x & m4x, lx4 & m4x, hx4 & m4x, b_hi[t][0][0], b_hi[t][0][1], bias);
-          mma_s8_16832(l1, lo.y & m0x, hi.y & m0x, ly4 & m0x, hy4 & m0x, b_lo[t][1][0], b_lo[t][1][1], l0);
-          mma_s8_16832(h1, lo.y & m4x, hi.y & m4x, ly4 & m4x, hy4 & m4x, b_hi[t][1][0], b_hi[t][1][1], h0);
+          int c[4];
+          mma_s8_16832(c, lx.f[0], hx.f[0], lx.f[2], hx.f[2], b_lo[t][0][0], b_lo[t][0][1], bias);
+          mma_s8_16832(c, lx.f[1], hx.f[1], lx.f[3], hx.f[3], b_hi[t][0][0], b_hi[t][0][1], c);
+          mma_s8_16832(c, ly.f[0], hy.f[0], ly.f[2], hy.f[2], b_lo[t][1][0], b_lo[t][1][1], c);
+          mma_s8_16832(c, ly.f[1], hy.f[1], ly.f[3], hy.f[3], b_hi[t][1][0], b_hi[t][1][1], c);
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            // (12582912 + L) + (12582912 + 4 H) / 4 = 15728640 + L + H: integers below 2^24, exact
-            const float v = fmaf(0.25f, __int_as_float(h1[c]), __int_as_float(l1[c])) - off[t][c & 1];
-            acc[i][t][c] = fmaf(c < 2 ? s_lo : s_hi, v, acc[i][t][c]);
-          }
+          for (int k = 0; k < 4; ++k)
+            acc[i][t][k] = fmaf(k < 2 ? s_lo : s_hi, __int_as_float(c[k]) - off[t][k & 1], acc[i][t][k]);
         }
       }
     } else {
@@ -349,28 +364,29 @@ __global__ void __launch_bounds__(32 * WARPS, MIN_CTAS) w2a8_direct_kernel(const
               bl[t][e] = mine ? b_lo[t][h][e] : 0u;
               bh[t][e] = mine ? b_hi[t][h][e] : 0u;
             }
-            int z[4];
-            mma_s8_16832(z, zp4x, zp4x, zp4x, zp4x, bl[t][0], bl[t][1], bias);
-            mma_s8_16832(z, zp4x, zp4x, zp4x, zp4x, bh[t][0], bh[t][1], z);
-            off[t][0] = __int_as_float(z[0]) + 3145728.f;
-            off[t][1] = __int_as_float(z[1]) + 3145728.f;
+            off[t][0] = off[t][1] = 12582912.f;
+            if (offset) {
+              int z[4];
+              mma_s8_16832(z, offset4x, offset4x, offset4x, offset4x, bl[t][0], bl[t][1], bias);
+              mma_s8_16832(z, offset4x, offset4x, offset4x, offset4x, bh[t][0], bh[t][1], z);
+              off[t][0] = __int_as_float(z[0]);
+              off[t][1] = __int_as_float(z[1]);
+            }
           }
 #pragma unroll
           for (int i = 0; i < MT; ++i) {
             const uint32_t lo = h == 0 ? wv[2 * i].x : wv[2 * i].y;
             const uint32_t hi = h == 0 ? wv[2 * i + 1].x : wv[2 * i + 1].y;
             const float s_lo = sv[h * kSub + sub][2 * i], s_hi = sv[h * kSub + sub][2 * i + 1];
-            constexpr uint32_t m0x = 0x03030303u, m4x = 0x0C0C0C0Cu;
+            const CodeBytes lb(lo, flip), hb(hi, flip);
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
-              int l0[4], h0[4];
-              mma_s8_16832(l0, lo & m0x, hi & m0x, (lo >> 4) & m0x, (hi >> 4) & m0x, bl[t][0], bl[t][1], bias);
-              mma_s8_16832(h0, lo & m4x, hi & m4x, (lo >> 4) & m4x, (hi >> 4) & m4x, bh[t][0], bh[t][1], bias);
+              int c[4];
+              mma_s8_16832(c, lb.f[0], hb.f[0], lb.f[2], hb.f[2], bl[t][0], bl[t][1], bias);
+              mma_s8_16832(c, lb.f[1], hb.f[1], lb.f[3], hb.f[3], bh[t][0], bh[t][1], c);
 #pragma unroll
-              for (int c = 0; c < 4; ++c) {
-                const float v = fmaf(0.25f, __int_as_float(h0[c]), __int_as_float(l0[c])) - off[t][c & 1];
-                acc[i][t][c] = fmaf(c < 2 ? s_lo : s_hi, v, acc[i][t][c]);
-              }
+              for (int k = 0; k < 4; ++k)
+                acc[i][t][k] = fmaf(k < 2 ? s_lo : s_hi, __int_as_float(c[k]) - off[t][k & 1], acc[i][t][k]);
             }
           }
         }
