@@ -567,7 +567,7 @@ struct DirectChoice {
   int ctas;
 };
 
-// Activations the direct kernel quantises itself: at most this many elements in all.  Every CTA reads them, so the limit is
+// Activations the direct kernel quantises itself: at most this many elements in all, and no more than two CTAs per SM.  Every CTA reads them, so the limit is
 // what a CTA can read and convert in less time than a launch (one token through 4096 x 4096, a whole call: 9.4 us against 12.6).
 constexpr long long kDirectQuantElements = 8192;
 
@@ -700,7 +700,7 @@ static int dispatch_direct(sk_w2a8_plan* plan, const DirectChoice& c, const Dire
 
 // The same with the activations quantised inside (up to 8 tokens, group sizes from 128 on).
 static bool direct_quantises(const sk_w2a8_plan* plan, long long M, const DirectChoice& c) {
-  return c.nt == 1 && plan->G >= 128 && M <= 8 && M * plan->K <= kDirectQuantElements;
+  return c.nt == 1 && plan->G >= 128 && M <= 8 && M * plan->K <= kDirectQuantElements && c.ctas <= 2 * plan->sm_count;
 }
 static int dispatch_direct_quant(sk_w2a8_plan* plan, const DirectChoice& c, const DirectParams& prm, cudaStream_t stream) {
   if (c.mt == 4 && c.warps == 8) return launch_direct<4, 1, 8, 4, 2, 1, true>(plan, prm, c.split, stream);
@@ -1737,6 +1737,12 @@ int sk_quantize_activation_int8_from(const void* x, int x_bf16, int64_t ld_x, in
                                                                                         : sk::quantize_activation_kernel<8, true>)
                      : (vecs == 2 ? sk::quantize_activation_kernel<2, false> : vecs == 4 ? sk::quantize_activation_kernel<4, false>
                                                                                          : sk::quantize_activation_kernel<8, false>);
+  if (M <= 2 * 148 && K > 8 * sk::kActThreads) {      // few rows: more threads per row
+    const bool half = K <= 8 * 512;
+    cfg.blockDim = dim3(half ? 512 : 1024, 1, 1);
+    kern = x_bf16 ? (half ? sk::quantize_activation_kernel<1, true, 512> : sk::quantize_activation_kernel<2, true, 1024>)
+                  : (half ? sk::quantize_activation_kernel<1, false, 512> : sk::quantize_activation_kernel<2, false, 1024>);
+  }
   const cudaError_t le = cudaLaunchKernelEx(&cfg, kern, src, ldx, x_q, ldq, x_scale, k);
   if (le != cudaSuccess) { (void)cudaGetLastError(); return SK_ERR_CUDA; }
   if (cudaGetLastError() != cudaSuccess) return SK_ERR_CUDA;
@@ -1753,9 +1759,13 @@ int sk_silu_mul_quantize_int8(const void* gate_up_f16, int64_t ld_gu, int64_t M,
   const auto st = static_cast<cudaStream_t>(stream);
   const __half* gu = static_cast<const __half*>(gate_up_f16);
   // one pass over HBM: the row split over a cluster of 1..8 CTAs whose threads keep their fp32 values in registers
+  // As many CTAs as the row needs, whether or not that is a power of two: 11008 features are 3 x 1.8 vectors per thread, in
+  // four CTAs a third of the second vectors' threads would idle (12 us of 697 of the MLP block of 4096 tokens).  Few rows leave SMs
+  // idle instead: then up to eight CTAs, one vector per thread.
   const long long per_cta = 8LL * sk::kActThreads * sk::kClusterVecs;
-  int csize = 1;
-  while (csize < 8 && I > per_cta * csize) csize *= 2;
+  int csize = static_cast<int>(I / per_cta < 8 ? (I + per_cta - 1) / per_cta : 9);
+  if (csize <= 8 && M * 8 <= 148) csize = static_cast<int>((I + 8LL * sk::kActThreads - 1) / (8LL * sk::kActThreads));
+  if (csize > 8) csize = 8;
   if (I <= per_cta * csize) {
     for (int64_t m0 = 0; m0 < M; m0 += 65535) {       // gridDim.y holds at most 65535 rows per launch
       const int64_t rows = M - m0 < 65535 ? M - m0 : 65535;
