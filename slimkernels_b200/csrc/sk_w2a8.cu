@@ -1253,12 +1253,6 @@ static int plan_create_common(sk_w2a8_plan** out, int device, int64_t N, int64_t
   int rc = e == cudaSuccess ? SK_OK : sk::cuda_fail(plan, e);
   if (rc == SK_OK) {
     plan->status = reinterpret_cast<int*>(base + l.status);
-    e = cudaMemsetAsync(plan->status, 0, sizeof(int), stream);
-    if (e == cudaSuccess && l.stream_counters >= 0) {
-      plan->stream_scratch = reinterpret_cast<float*>(base + l.stream_scratch);
-      plan->stream_counters = reinterpret_cast<int*>(base + l.stream_counters);
-      e = cudaMemsetAsync(plan->stream_counters, 0, l.counter_bytes, stream);
-    }
     plan->w_scale_tiled = reinterpret_cast<__half*>(base + l.w_scale_tiled);
     // the decode kernels' copy of the scales is made once, here: later changes of w_scale_f16 are not seen by them
     bool scales_tiled = false;
@@ -1286,6 +1280,15 @@ static int plan_create_common(sk_w2a8_plan** out, int device, int64_t N, int64_t
       sk::tile_scales_kernel<<<blocks, 256, 0, stream>>>(plan->w_scale, plan->w_scale_tiled, N, groups, total);
       e = cudaGetLastError();
     }
+    if (rc == SK_OK && e == cudaSuccess && l.stream_counters >= 0) {
+      plan->stream_scratch = reinterpret_cast<float*>(base + l.stream_scratch);
+      plan->stream_counters = reinterpret_cast<int*>(base + l.stream_counters);
+      e = cudaMemsetAsync(plan->stream_counters, 0, l.counter_bytes, stream);
+    }
+    // Last, and not only for its own sake: decode kernels are dependent launches that read the copies before they wait for the
+    // kernel in front of them.  Were that a kernel above, they could start when its last CTA exits, before its stores are
+    // sure to be visible; this operation starts only after those kernels are complete.
+    if (rc == SK_OK && e == cudaSuccess) e = cudaMemsetAsync(plan->status, 0, sizeof(int), stream);
     if (rc == SK_OK && e == cudaSuccess && !storage) e = cudaDeviceSynchronize();
     if (rc == SK_OK && e != cudaSuccess) rc = sk::cuda_fail(plan, e);
   }

@@ -116,3 +116,15 @@ def test_activations_quantised_inside_the_gemm(M, N, K, G, dtype):
     wide = torch.randn(M, K + 24, device="cuda").to(dtype)[:, 16:16 + K]
     if M > 1 and wide.data_ptr() % 16 == 0:
         assert torch.equal(lin(wide), _by_pieces(lin, wide))
+
+
+def test_plan_used_at_once_after_it_is_made():
+    """The GEMM behind a plan's copies in the stream reads them before it waits for the kernel in front of it."""
+    x = torch.randn(1, 4096, device="cuda").half()
+    w = [torch.randn(1024, 4096, device="cuda").half() for _ in range(2)]
+    from slimkernels_b200.torch import W2A8Linear
+    want = [W2A8Linear.from_float(v, 128)(x).clone() for v in w]
+    torch.cuda.synchronize()
+    got = [W2A8Linear.from_float(w[i % 2], 128)(x) for i in range(60)]      # storage of dropped plans comes round again
+    for i, y in enumerate(got):
+        assert torch.equal(y, want[i % 2])
