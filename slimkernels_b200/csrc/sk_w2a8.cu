@@ -687,7 +687,7 @@ static int dispatch_direct(sk_w2a8_plan* plan, const DirectChoice& c, const Dire
       case 1: return launch_direct<2, 1, 4, 4, 4, 1>(plan, prm, c.split, stream);
       case 2: return launch_direct<2, 2, 4, 6, 4, 1>(plan, prm, c.split, stream);
       case 3: return launch_direct<2, 3, 4, 6, 3, 1>(plan, prm, c.split, stream);
-      default: return launch_direct<2, 4, 4, 4, 2, 1>(plan, prm, c.split, stream);
+      default: return launch_direct<2, 4, 4, 6, 3, 1>(plan, prm, c.split, stream);    // 32 x 12288 x 4096 11.5; two CTAs of four blocks 15.2
     }
   }
   switch (c.nt) {
