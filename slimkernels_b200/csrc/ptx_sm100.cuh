@@ -292,6 +292,13 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, const uint4& v) {
                : "memory");
 }
 
+// What a kernel before this one wrote, read after grid_dep_wait: volatile, so that the load stays behind it.
+__device__ __forceinline__ float ld_global_f32(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
+
 // Programmatic dependent launch.  launch_dependents: the next kernel in the stream (if it was launched with the
 // programmatic-serialization attribute) may start being scheduled now; wait: every kernel this one depends on has
 // completed and its memory is visible.  Both are no-ops for a kernel launched without the attribute.

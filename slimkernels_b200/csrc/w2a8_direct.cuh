@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(32 * WARPS, MIN_CTAS) w2a8_direct_kernel(const
   auto store = [&](int tok, int f, float sum) {
     const int m = m0 + tok, n = n0 + f;
     if (m >= p.M || n >= p.N) return;
-    const float y = sum * (QUANT ? q_scale[tok] : __ldg(p.x_scale + m));
+    const float y = sum * (QUANT ? q_scale[tok] : ld_global_f32(p.x_scale + m));
     const uint16_t bits = p.out_bf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(y)) : __half_as_ushort(__float2half_rn(y));
     const size_t at = static_cast<size_t>(m) * p.ld_out + n;
     reinterpret_cast<uint16_t*>(p.out)[at] = bits;

@@ -766,7 +766,7 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       // x_scale * 2^49 of this tile's tokens; read after the named barrier that precedes the output.  The buffer
       // of the tile before last is free: every epilogue thread passed that tile's barrier before it got here.
       for (int j = threadIdx.x; j < BLOCK_M; j += T::kEpiThreads)
-        xs_tile[j] = (m0 + j < p.M) ? __ldg(p.x_scale + m0 + j) * 5.62949953421312e14f : 0.f;
+        xs_tile[j] = (m0 + j < p.M) ? ld_global_f32(p.x_scale + m0 + j) * 5.62949953421312e14f : 0.f;
       tile_parity ^= 1;
     }
 
@@ -933,7 +933,7 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       // reuse it to transpose the tile.  All epilogue threads must be past their last TMEM read first.
       float* xs_s = reinterpret_cast<float*>(smem + T::kOffXs);
       for (int j = threadIdx.x; j < BLOCK_M; j += T::kEpiThreads)
-        xs_s[j] = (m0 + j < p.M) ? __ldg(p.x_scale + m0 + j) * kScaleDown : 0.f;
+        xs_s[j] = (m0 + j < p.M) ? ld_global_f32(p.x_scale + m0 + j) * kScaleDown : 0.f;
       named_barrier_sync(1, T::kEpiThreads);
       if (threadIdx.x == 0) SK_TRACE_EVENT(4, 2);
       if constexpr (!SPLIT) {
@@ -1015,7 +1015,7 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
 #pragma unroll
           for (int r = 0; r < 8; ++r)
             part[r] = r < num_splits ? ld_dsmem_f32x4(map_to_cta(local, r)) : make_float4(0.f, 0.f, 0.f, 0.f);
-          const float xs = __ldg(p.x_scale + m) * kScaleDown;
+          const float xs = ld_global_f32(p.x_scale + m) * kScaleDown;
           float y[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
           for (int r = 0; r < 8; ++r) { y[0] += part[r].x; y[1] += part[r].y; y[2] += part[r].z; y[3] += part[r].w; }
