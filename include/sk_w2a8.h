@@ -62,16 +62,16 @@ typedef enum sk_option {
                              of its K range, summed over a cluster (group size 128; used for token tiles 16 / 32, else 1 is
                              taken), 4 prefill tcgen05 kernel on pairs of CTAs (cta_group::2; group size 128, token tile 256, an
                              even number of 128-feature tiles, else 1 is taken), 5 decode tcgen05 kernel that cuts the K
-                             range of the WHOLE problem into equal CTA ranges, two CTAs per SM (the default for M <= 32
-                             with group size 128 and K a multiple of 256; else 3 is taken).  Partial sums of tiles that
+                             range of the WHOLE problem into equal CTA ranges, two CTAs per SM (one token tile, group size
+                             128 and K a multiple of 256; else 3 is taken).  Partial sums of tiles that
                              two or more CTAs share meet in a scratch buffer owned by the plan, so calls on one plan
                              must not run concurrently (they must not anyway, see above),
                              6 direct decode kernel (weights from HBM to registers to mma.sync; taken by itself for small M) */
   SK_OPT_TOKEN_TILE = 2,  /* tokens per CTA tile: 0 auto, or 16 / 32 / 64 / 128 / 192 / 256 */
-  SK_OPT_SPLIT_K = 3,     /* CTAs (one cluster) sharing the K range of one tile: 0 auto, 1, 2, 4, 8 */
+  SK_OPT_SPLIT_K = 3,     /* CTAs (one cluster) sharing the K range of one tile: 0 auto, 1, 2, 4, 8 (token tile 192: always 1) */
   SK_OPT_TMA_STORE = 6,   /* general kernel, one CTA per tile: 0 auto (= 2), 1 vector stores by the epilogue threads, 2 one TMA
                              store per destination where alignment allows (16-byte base, pitch % 8 == 0, N % 8 == 0) */
-  SK_OPT_DEPENDENT_LAUNCH = 5, /* decode kernels: 0 auto (= 2), 1 plain launch, 2 programmatic dependent launch: the
+  SK_OPT_DEPENDENT_LAUNCH = 5, /* decode kernels, general kernel up to two waves: 0 auto (= 2), 1 plain launch, 2 programmatic dependent launch: the
                              kernel's set-up and first weight copies overlap the tail of the previous kernel in the
                              stream; it waits for that kernel before it reads activations or writes outputs */
   SK_OPT_PERSISTENT = 4,  /* 0 auto (= 1), 1 one CTA per tile, 2 one resident set of CTAs walks all tiles (token tiles
