@@ -96,16 +96,16 @@ tile_weight_kernel(const uint8_t* __restrict__ w_packed, uint8_t* __restrict__ w
   if (w_scale_tiled) w_scale_tiled[block * 128 + r] = n < N ? w_scale[static_cast<size_t>(B) * N + n] : __float2half(0.f);
 }
 
-// The scales in the order the decode kernels stream them: [n_tiles][groups][128 features] (rows past N are zero), so that
-// the scales of a CTA's K range are one contiguous run.
+// The scales of a group-size-128 weight in the order the split decode kernel (3) streams them: [n_tiles][k_blocks][128
+// features] (rows past N are zero), so that the scales of a CTA's K range are one contiguous run.
 __global__ void tile_scales_kernel(const __half* __restrict__ w_scale, __half* __restrict__ tiled, long long N,
-                                   int groups, long long total) {
+                                   int k_blocks, long long total) {
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const int r = static_cast<int>(i % 128);
     const long long t = i / 128;
-    const int g = static_cast<int>(t % groups);
-    const long long n = (t / groups) * 128 + r;
+    const int g = static_cast<int>(t % k_blocks);
+    const long long n = (t / k_blocks) * 128 + r;
     tiled[i] = n < N ? w_scale[static_cast<size_t>(g) * N + n] : __float2half(0.f);
   }
 }
@@ -244,7 +244,7 @@ struct sk_w2a8_plan {
   const uint8_t* w_rowmajor = nullptr;  // borrowed (may be null when created from a tiled buffer)
   const uint8_t* w_tiled = nullptr;     // in the plan's storage, or borrowed
   const __half* w_scale = nullptr;      // borrowed
-  __half* w_scale_tiled = nullptr;      // in the plan's storage: [n_tiles][K / G][128] copy of the scales
+  __half* w_scale_tiled = nullptr;      // in the plan's storage, group size 128: [n_tiles][k_blocks][128] copy of the scales
   int* status = nullptr;                // device; first in the plan's storage, one block that also holds the tiled copies
   bool external_storage = false;        // the buffers below live in the caller's storage (sk_w2a8_plan_create_in)
   bool stream_owned = false;            // stream_scratch / stream_counters are the plan's own allocations
@@ -544,7 +544,7 @@ static PlanLayout plan_layout(sk_w2a8_plan* plan, int w_layout) {
   const long long blocks = static_cast<long long>(plan->n_tiles) * plan->k_blocks;
   l.status = take(sizeof(int));
   l.w_tiled = w_layout == SK_WEIGHT_ROWMAJOR ? take(blocks * kWpBytes) : -1;
-  l.w_scale_tiled = take(static_cast<long long>(plan->n_tiles) * (plan->K / plan->G) * kTileN * static_cast<long long>(sizeof(__half)));
+  l.w_scale_tiled = plan->G == 128 ? take(blocks * kTileN * static_cast<long long>(sizeof(__half))) : -1;
   l.stream_scratch = l.stream_counters = -1;
   l.counter_bytes = 0;
   // The balanced-split decode kernel's scratch is part of it only where that kernel is the default (large weight
@@ -571,10 +571,14 @@ struct DirectChoice {
 // what a CTA can read and convert in less time than a launch (one token through 4096 x 4096, a whole call: 9.4 us against 12.6).
 constexpr long long kDirectQuantElements = 8192;
 
-template <int MT, int NT, int WARPS, int DEPTH, int MIN_CTAS, int GPB, bool QUANT = false>
+// Whether the kernel takes the scales from the plan's copy: only where the decode kernels, which do, served these calls too.  A
+// caller who rewrites the scales in stream order finds them read live everywhere else, as the general kernel does.
+static bool direct_reads_copy(const sk_w2a8_plan* plan, long long M) { return plan->G == 128 && M <= 32; }
+
+template <int MT, int NT, int WARPS, int DEPTH, int MIN_CTAS, int GPB, bool LIVE, bool QUANT = false>
 static int launch_direct(sk_w2a8_plan* plan, const DirectParams& prm, int split, cudaStream_t stream) {
-  using T = DirectTraits<MT, NT, WARPS, DEPTH, GPB>;
-  auto kern = w2a8_direct_kernel<MT, NT, WARPS, DEPTH, MIN_CTAS, GPB, QUANT>;
+  using T = DirectTraits<MT, NT, WARPS, DEPTH, GPB, LIVE>;
+  auto kern = w2a8_direct_kernel<MT, NT, WARPS, DEPTH, MIN_CTAS, GPB, LIVE, QUANT>;
   constexpr int kMaxQuant = QUANT ? static_cast<int>(kDirectQuantElements) + 8 * (128 + 16) : 0;   // (a rank's range rounds up to a block)
   if constexpr (T::kQuantOffset + kMaxQuant > 48 * 1024) {
     static int configured_device_mask[64] = {0};
@@ -611,13 +615,14 @@ static int launch_direct(sk_w2a8_plan* plan, const DirectParams& prm, int split,
   return SK_OK;
 }
 
-// Serves small calls unless an option asks for another kernel (or for its failure-path hook).  Its time grows with the
+// Serves small calls unless an option asks for another kernel (or for its failure-path hook), or scales that are read live do
+// not start on a word.  Its time grows with the
 // tokens, the tcgen05 kernels' hardly does up to a tile, so the line lies where weights x tokens per SM get large (us, this
 // kernel against the better tcgen05 one, group size 128):
 //   * up to 24 tokens always: 24 x 57344 x 8192 61 / 80, 24 x 22016 x 4096 15.3 / 17.0, 24 x 4096 x 4096 4.5 / 7.6;
 //   * up to 32 tokens below 24 K blocks of a feature tile per SM: 32 x 4096 x 11008 10.4 / 11.5, but 32 x 22016 x 4096 22 / 17.4;
 //     with other group sizes always (64: 32 x 22016 x 4096 29 / 52);
-//   * up to 128 tokens below 8 such blocks per SM, the weight counted once per 32 tokens: 64 x 2048 x 1024 3.4 / 8.4,
+//   * up to 128 tokens below 8 such blocks per SM, the weight counted once per 32 tokens: 64 x 2048 x 1024 3.8 / 8.4,
 //     64 x 512 x 16384 6.9 / 10.6, but 64 x 4096 x 4096 11.6 / 9.2.
 // The shape of a CTA:
 //   * 64 features and 4 warps from four such CTAs per SM on (two for 16 tokens): 8 x 57344 x 8192 28.7;
@@ -630,6 +635,7 @@ static bool choose_direct(const sk_w2a8_plan* plan, long long M, DirectChoice* o
   const bool forced = plan->opt_kernel == 6;
   if (!forced && (plan->opt_kernel || plan->opt_token_tile || plan->opt_split_k || plan->opt_persistent || plan->opt_skip_copy || M > 128))
     return false;
+  if ((reinterpret_cast<uintptr_t>(plan->w_scale) & 3) && !direct_reads_copy(plan, M)) return false;
   DirectChoice c;
   c.nt = M <= 8 ? 1 : M <= 16 ? 2 : M <= 24 ? 3 : 4;
   const long long sms = plan->sm_count;
@@ -656,56 +662,62 @@ static bool choose_direct(const sk_w2a8_plan* plan, long long M, DirectChoice* o
 }
 
 // <16-feature tiles, 8-token tiles, warps, K blocks in flight per warp, CTAs per SM that registers are kept for, groups per
-// K block>
-static int dispatch_direct(sk_w2a8_plan* plan, const DirectChoice& c, const DirectParams& prm, cudaStream_t stream) {
-  if (plan->G == 64) {
-    switch (c.nt) {
-      case 1: return launch_direct<2, 1, 4, 4, 4, 2>(plan, prm, c.split, stream);
-      case 2: return launch_direct<2, 2, 4, 4, 4, 2>(plan, prm, c.split, stream);
-      case 3: return launch_direct<2, 3, 4, 4, 2, 2>(plan, prm, c.split, stream);
-      default: return launch_direct<2, 4, 4, 4, 2, 2>(plan, prm, c.split, stream);
-    }
+// K block, scales read from the caller's buffer>
+template <int GPB>
+static int dispatch_direct_small_groups(sk_w2a8_plan* plan, const DirectChoice& c, const DirectParams& prm, cudaStream_t stream) {
+  switch (c.nt) {
+    case 1: return launch_direct<2, 1, 4, 4, GPB == 2 ? 5 : 4, GPB, true>(plan, prm, c.split, stream);
+    case 2: return launch_direct<2, 2, 4, 4, GPB == 2 ? 4 : 3, GPB, true>(plan, prm, c.split, stream);
+    case 3: return launch_direct<2, 3, 4, 4, 2, GPB, true>(plan, prm, c.split, stream);
+    default: return launch_direct<2, 4, 4, 4, 2, GPB, true>(plan, prm, c.split, stream);
   }
-  if (plan->G == 32) {
-    switch (c.nt) {
-      case 1: return launch_direct<2, 1, 4, 4, 4, 4>(plan, prm, c.split, stream);
-      case 2: return launch_direct<2, 2, 4, 4, 3, 4>(plan, prm, c.split, stream);
-      case 3: return launch_direct<2, 3, 4, 4, 2, 4>(plan, prm, c.split, stream);
-      default: return launch_direct<2, 4, 4, 4, 2, 4>(plan, prm, c.split, stream);
-    }
-  }
-  if (c.mt == 4 && c.warps == 8) return launch_direct<4, 1, 8, 4, 2, 1>(plan, prm, c.split, stream);
+}
+template <bool LIVE>
+static int dispatch_direct_blocks(sk_w2a8_plan* plan, const DirectChoice& c, const DirectParams& prm, cudaStream_t stream) {
+  if (c.mt == 4 && c.warps == 8) return launch_direct<4, 1, 8, 4, 2, 1, LIVE>(plan, prm, c.split, stream);
   if (c.mt == 4) {
     switch (c.nt) {
-      case 1: return launch_direct<4, 1, 4, 4, 3, 1>(plan, prm, c.split, stream);
-      case 2: return launch_direct<4, 2, 4, 6, 3, 1>(plan, prm, c.split, stream);
-      default: return launch_direct<4, 4, 4, 4, 2, 1>(plan, prm, c.split, stream);
+      case 1: return launch_direct<4, 1, 4, 4, 3, 1, LIVE>(plan, prm, c.split, stream);
+      case 2: return launch_direct<4, 2, 4, 6, 3, 1, LIVE>(plan, prm, c.split, stream);
+      default: return launch_direct<4, 4, 4, 4, 2, 1, LIVE>(plan, prm, c.split, stream);
     }
   }
   if (c.warps == 4) {
     switch (c.nt) {
-      case 1: return launch_direct<2, 1, 4, 4, 4, 1>(plan, prm, c.split, stream);
-      case 2: return launch_direct<2, 2, 4, 6, 4, 1>(plan, prm, c.split, stream);
-      case 3: return launch_direct<2, 3, 4, 6, 3, 1>(plan, prm, c.split, stream);
-      default: return launch_direct<2, 4, 4, 6, 3, 1>(plan, prm, c.split, stream);    // 32 x 12288 x 4096 11.5; two CTAs of four blocks 15.2
+      case 1: return launch_direct<2, 1, 4, 4, LIVE ? 5 : 4, 1, LIVE>(plan, prm, c.split, stream);   // (five CTAs per SM either way)
+      case 2: return launch_direct<2, 2, 4, 6, 4, 1, LIVE>(plan, prm, c.split, stream);
+      case 3: return launch_direct<2, 3, 4, 6, 3, 1, LIVE>(plan, prm, c.split, stream);
+      default: return launch_direct<2, 4, 4, 6, 3, 1, LIVE>(plan, prm, c.split, stream);    // 32 x 12288 x 4096 11.5; two CTAs of four blocks 15.2
     }
   }
   switch (c.nt) {
-    case 1: return launch_direct<2, 1, 8, 4, 2, 1>(plan, prm, c.split, stream);
-    case 2: return launch_direct<2, 2, 8, 4, 2, 1>(plan, prm, c.split, stream);
-    case 3: return launch_direct<2, 3, 8, 4, 1, 1>(plan, prm, c.split, stream);
-    default: return launch_direct<2, 4, 8, 4, 1, 1>(plan, prm, c.split, stream);
+    case 1: return launch_direct<2, 1, 8, 4, 2, 1, LIVE>(plan, prm, c.split, stream);
+    case 2: return launch_direct<2, 2, 8, 4, 2, 1, LIVE>(plan, prm, c.split, stream);
+    case 3: return launch_direct<2, 3, 8, 4, 1, 1, LIVE>(plan, prm, c.split, stream);
+    default: return launch_direct<2, 4, 8, 4, 1, 1, LIVE>(plan, prm, c.split, stream);
   }
+}
+static int dispatch_direct(sk_w2a8_plan* plan, const DirectChoice& c, const DirectParams& prm, cudaStream_t stream) {
+  if (plan->G == 64) return dispatch_direct_small_groups<2>(plan, c, prm, stream);
+  if (plan->G == 32) return dispatch_direct_small_groups<4>(plan, c, prm, stream);
+  return direct_reads_copy(plan, prm.M) ? dispatch_direct_blocks<false>(plan, c, prm, stream)
+                                        : dispatch_direct_blocks<true>(plan, c, prm, stream);
 }
 
 // The same with the activations quantised inside (up to 8 tokens, group sizes from 128 on).
 static bool direct_quantises(const sk_w2a8_plan* plan, long long M, const DirectChoice& c) {
   return c.nt == 1 && plan->G >= 128 && M <= 8 && M * plan->K <= kDirectQuantElements && c.ctas <= 2 * plan->sm_count;
 }
+template <bool LIVE>
+static int dispatch_direct_quant_blocks(sk_w2a8_plan* plan, const DirectChoice& c, const DirectParams& prm, cudaStream_t stream) {
+  if (c.mt == 4 && c.warps == 8) return launch_direct<4, 1, 8, 4, 2, 1, LIVE, true>(plan, prm, c.split, stream);
+  if (c.mt == 4) return launch_direct<4, 1, 4, 4, 3, 1, LIVE, true>(plan, prm, c.split, stream);
+  return c.warps == 4 ? launch_direct<2, 1, 4, 4, LIVE ? 5 : 4, 1, LIVE, true>(plan, prm, c.split, stream)
+                      : launch_direct<2, 1, 8, 4, 2, 1, LIVE, true>(plan, prm, c.split, stream);
+}
 static int dispatch_direct_quant(sk_w2a8_plan* plan, const DirectChoice& c, const DirectParams& prm, cudaStream_t stream) {
-  if (c.mt == 4 && c.warps == 8) return launch_direct<4, 1, 8, 4, 2, 1, true>(plan, prm, c.split, stream);
-  if (c.mt == 4) return launch_direct<4, 1, 4, 4, 3, 1, true>(plan, prm, c.split, stream);
-  return c.warps == 4 ? launch_direct<2, 1, 4, 4, 4, 1, true>(plan, prm, c.split, stream) : launch_direct<2, 1, 8, 4, 2, 1, true>(plan, prm, c.split, stream);
+  return direct_reads_copy(plan, prm.M) ? dispatch_direct_quant_blocks<false>(plan, c, prm, stream)
+                                        : dispatch_direct_quant_blocks<true>(plan, c, prm, stream);
 }
 
 constexpr int kPairStages = 6;
@@ -999,6 +1011,11 @@ static DirectParams direct_params(const sk_w2a8_plan* plan, long long M, void* o
   DirectParams prm = {};
   prm.w_tiled = plan->w_tiled;
   prm.w_scale_tiled = plan->w_scale_tiled;
+  prm.w_scale = plan->w_scale;
+  prm.scale_pieces = (reinterpret_cast<uintptr_t>(plan->w_scale) & 15) == 0 && plan->N % 8 == 0;
+  // Borrowed codes are read behind the dependent-launch wait wherever the kernel that took these calls before did, so that a
+  // buffer refilled in stream order is seen; the decode kernels (one tile of up to 32 tokens, group size 128) do not wait.
+  prm.weights_late = plan->w_rowmajor == nullptr && !direct_reads_copy(plan, M);
   prm.out = out;
   prm.ld_out = ld_out;
   prm.M = static_cast<int>(M);
@@ -1253,9 +1270,9 @@ static int plan_create_common(sk_w2a8_plan** out, int device, int64_t N, int64_t
   int rc = e == cudaSuccess ? SK_OK : sk::cuda_fail(plan, e);
   if (rc == SK_OK) {
     plan->status = reinterpret_cast<int*>(base + l.status);
-    plan->w_scale_tiled = reinterpret_cast<__half*>(base + l.w_scale_tiled);
-    // the decode kernels' copy of the scales is made once, here: later changes of w_scale_f16 are not seen by them
-    bool scales_tiled = false;
+    if (l.w_scale_tiled >= 0) plan->w_scale_tiled = reinterpret_cast<__half*>(base + l.w_scale_tiled);
+    // kernel 3's copy of the scales is made once, here: later changes of w_scale_f16 are not seen by it
+    bool scales_tiled = plan->w_scale_tiled == nullptr;
     if (w_layout == SK_WEIGHT_TILED) {
       plan->w_tiled = w;
     } else {
@@ -1265,19 +1282,18 @@ static int plan_create_common(sk_w2a8_plan** out, int device, int64_t N, int64_t
       if (e == cudaSuccess) {
         if ((K % 128) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 && ((K / 4) % 16) == 0 && plan->n_tiles <= 65535) {
           sk::tile_weight_kernel<<<dim3(plan->k_blocks, plan->n_tiles), 128, 0, stream>>>(
-              w, tiled, plan->w_scale, group_size == 128 ? plan->w_scale_tiled : nullptr, N, K, plan->k_blocks);
+              w, tiled, plan->w_scale, plan->w_scale_tiled, N, K, plan->k_blocks);
           e = cudaGetLastError();
-          scales_tiled = group_size == 128;
+          scales_tiled = true;
         } else {
           rc = sk::repack_common(true, w, N, K, tiled, stream);
         }
       }
     }
     if (rc == SK_OK && e == cudaSuccess && !scales_tiled) {
-      const int groups = static_cast<int>(K / group_size);
-      const long long total = static_cast<long long>(plan->n_tiles) * groups * sk::kTileN;
+      const long long total = static_cast<long long>(plan->n_tiles) * plan->k_blocks * sk::kTileN;
       const int blocks = static_cast<int>(total / 256 + 1 < 148 * 8 ? total / 256 + 1 : 148 * 8);
-      sk::tile_scales_kernel<<<blocks, 256, 0, stream>>>(plan->w_scale, plan->w_scale_tiled, N, groups, total);
+      sk::tile_scales_kernel<<<blocks, 256, 0, stream>>>(plan->w_scale, plan->w_scale_tiled, N, plan->k_blocks, total);
       e = cudaGetLastError();
     }
     if (rc == SK_OK && e == cudaSuccess && l.stream_counters >= 0) {

@@ -22,7 +22,7 @@
 //
 // Measured, cold weights, tokens x features x K (before: the better tcgen05 decode kernel):
 //   8 x 4096 x 4096 2.8 us (6.1), 8 x 22016 x 4096 7.2 us (15.1), 8 x 57344 x 8192 28.7 us = 4.3 TB/s (52.7),
-//   16 x 12288 x 4096 8.0 us (10.4), 24 x 4096 x 11008 8.9 us (12.5); group size 64: 8 x 22016 x 4096 11.4 us (46.5).
+//   16 x 12288 x 4096 8.0 us (10.4), 24 x 4096 x 11008 8.9 us (12.5); group size 64: 8 x 22016 x 4096 10.1 us (46.5).
 // mma.sync s8 issues an m16n8k32 every 8 cycles per sub-core, 1.15 POP/s in all, but two or three warps per sub-core do not
 // keep it busy (a third of the cycles at 24 tokens), and few CTAs fill whole waves badly: from about 32 tokens on the tcgen05
 // kernels win on large weights (see choose_direct).
@@ -37,7 +37,11 @@ namespace sk {
 
 struct DirectParams {
   const uint8_t* w_tiled;     // [n_tiles][k_blocks][4096]
-  const __half* w_scale_tiled;  // [n_tiles][groups][128], zero past N
+  const __half* w_scale_tiled;  // [n_tiles][groups][128], zero past N: the plan's copy
+  // kernels with LIVE scales read these instead, behind the dependent-launch wait
+  const __half* w_scale;      // [groups][N], the caller's, 4-byte aligned
+  int scale_pieces;           // 1: its rows are whole 16-byte pieces (base 16-byte aligned, N % 8 == 0)
+  int weights_late;           // 1: the codes, too, are read behind that wait (a borrowed buffer)
   const int8_t* x_q;          // [M, ld_x]
   const float* x_scale;       // [M]
   void* out;                  // [M, ld_out] half or bf16
@@ -56,17 +60,18 @@ struct DirectParams {
   int float_bf16;
 };
 
-template <int MT, int NT, int WARPS, int DEPTH, int GPB>
+template <int MT, int NT, int WARPS, int DEPTH, int GPB, bool LIVE>
 struct DirectTraits {
   static constexpr int kFeatures = 16 * MT;        // output features per CTA
   static constexpr int kTokens = 8 * NT;           // tokens per CTA
   static constexpr int kThreads = 32 * WARPS;
   // one warp's copy of a K block: the two halves of the features' codes (the second 64 bytes out of step, so that the four
-  // lanes of a feature read different banks), then their scales
+  // lanes of a feature read different banks), then their scales (LIVE: and room for a row that starts mid-word)
   static constexpr int kHalfBytes = 16 * kFeatures;
   static constexpr int kOffHalf = kHalfBytes + 64;
   static constexpr int kOffScales = kOffHalf + kHalfBytes;
-  static constexpr int kStageBytes = kOffScales + GPB * 2 * kFeatures;
+  static constexpr int kScalePitch = 2 * kFeatures + (LIVE ? 16 : 0);
+  static constexpr int kStageBytes = kOffScales + GPB * kScalePitch;
   static constexpr int kWarpBytes = DEPTH * kStageBytes;
   static constexpr int kPitch = kFeatures + 4;     // floats per token in the reduction buffer: stores are conflict-free
   static constexpr int kRedBytes = WARPS * kTokens * kPitch * 4;    // takes the rings' place
@@ -104,7 +109,12 @@ __device__ __forceinline__ uint4 ld_global_v4(const void* p) {
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {   // L2 only: packed weights are read once
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, int bytes) {   // (the rest of the word is zero)
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ uint2 ld_shared_v2(uint32_t addr) {
@@ -123,9 +133,10 @@ __device__ __forceinline__ float ld_shared_half(uint32_t addr) {
   return __half2float(__ushort_as_half(v));
 }
 
-template <int MT, int NT, int WARPS, int DEPTH, int MIN_CTAS, int GPB = 1, bool QUANT = false>
+template <int MT, int NT, int WARPS, int DEPTH, int MIN_CTAS, int GPB, bool LIVE, bool QUANT = false>
 __global__ void __launch_bounds__(32 * WARPS, MIN_CTAS) w2a8_direct_kernel(const DirectParams p) {
-  using T = DirectTraits<MT, NT, WARPS, DEPTH, GPB>;
+  using T = DirectTraits<MT, NT, WARPS, DEPTH, GPB, LIVE>;
+  static_assert(LIVE || GPB == 1, "the plan has a copy of the scales for group size 128 only");
   extern __shared__ __align__(16) uint8_t direct_smem[];
   float* red = reinterpret_cast<float*>(direct_smem);   // after the main loop: [WARPS][kTokens][kPitch]
   grid_dep_launch_dependents();
@@ -144,36 +155,92 @@ __global__ void __launch_bounds__(32 * WARPS, MIN_CTAS) w2a8_direct_kernel(const
   // ---- weights and scales: DEPTH blocks in flight per warp
   const size_t tile = static_cast<size_t>(n0 >> 7);
   const uint8_t* w_src = p.w_tiled + (tile * p.k_blocks + kb0) * 4096 + ((n0 & 127) + (lane & 15)) * 16;
+  const uint32_t ring = smem_u32(direct_smem) + warp * T::kWarpBytes;
+  auto fetch_weights = [&](int idx, uint32_t slot) {
+    const uint8_t* w = w_src + static_cast<size_t>(idx) * (WARPS * 4096);
+    // piece i of a lane: 16 rows of one half per half-warp
+#pragma unroll
+    for (int i = 0; i < MT; ++i) {
+      const int piece = 2 * i + (lane >> 4);       // 16-row group of the two halves' 2 * MT
+      const int half = piece / MT, rows = (piece % MT) * 16;
+      cp_async16(slot + half * T::kOffHalf + (rows + (lane & 15)) * 16, w + half * 2048 + rows * 16);
+    }
+  };
+  // Where the scales come from (16 bytes per lane and block, unless a row is cut otherwise):
+  //   * the plan's copy, a block's features together, for group size 128 and up to 32 tokens.  It is constant and is fetched
+  //     with the codes, before the wait below;
+  //   * LIVE: the caller's [groups][N], as it is when the call runs, so behind that wait.  The kernel that served group sizes
+  //     other than 128 and more than 32 tokens before this one read it then, too.  It costs about a microsecond, most of
+  //     it the first loads' latency behind the wait: 8 x 22016 x 4096 with group size 64 8.8 us from a copy, 10.1 from the rows,
+  //     8 x 4096 x 4096 with 256 3.1 and 4.3.  That is why the copy stays where it may.  Rows that are not whole 16-byte pieces take words from the one that holds their first scale on:
+  //     with N odd every other row starts in the middle of it (scale_shift).
   const uint8_t* s_src = reinterpret_cast<const uint8_t*>(p.w_scale_tiled) + tile * p.groups * 256 + (n0 & 127) * 2 +
                          (lane % (2 * MT)) * 16;
-  const uint32_t ring = smem_u32(direct_smem) + warp * T::kWarpBytes;
+  auto group_of = [&](int idx, int b) {            // the scale group of part b of a block
+    const int kb = kb0 + idx * WARPS;
+    return GPB > 1 ? min(kb * GPB + b, p.groups - 1) : !LIVE || p.blocks_per_group == 1 ? kb : kb / p.blocks_per_group;
+  };
+  const uint8_t* s_base = reinterpret_cast<const uint8_t*>(p.w_scale) + 2 * n0;
+  // (pieces past N are left out: those features are not stored)
+  const bool s_lane = lane < GPB * 2 * MT && (!LIVE || n0 + (lane % (2 * MT)) * 8 < p.N);
+  auto piece_src = [&](int idx) {
+    if constexpr (!LIVE) return s_src + static_cast<size_t>(group_of(idx, 0)) * 256;
+    return s_base + static_cast<size_t>(group_of(idx, lane / (2 * MT))) * (2 * static_cast<size_t>(p.N)) + (lane % (2 * MT)) * 16;
+  };
+  const uint32_t piece_dst = T::kOffScales + (LIVE ? (lane / (2 * MT)) * T::kScalePitch + (lane % (2 * MT)) * 16 : lane * 16);
+  auto fetch_scale_words = [&](int idx, uint32_t slot) {
+    constexpr int kWords = T::kFeatures / 2 + 1;
+    const long long end = 2LL * p.groups * p.N - 2 * n0;       // of the buffer, from s_base
+#pragma unroll 1
+    for (int i = lane; i < GPB * kWords; i += 32) {
+      const int b = i / kWords, w = i % kWords;
+      const long long o = ((2LL * group_of(idx, b) * p.N) & ~3LL) + 4 * w;      // (n0 is even: rows of even N start on words)
+      if (o < end) cp_async4(slot + T::kOffScales + b * T::kScalePitch + 4 * w, s_base + o, end - o < 4 ? 2 : 4);
+    }
+  };
   int idx_fetch = first, to_fetch = count;
   uint32_t slot_fetch = ring;
-  auto fetch = [&]() {
-    if (to_fetch > 0) {
-      const uint8_t* w = w_src + static_cast<size_t>(idx_fetch) * (WARPS * 4096);
-      // piece i of a lane: 16 rows of one half per half-warp
-#pragma unroll
-      for (int i = 0; i < MT; ++i) {
-        const int piece = 2 * i + (lane >> 4);     // 16-row group of the two halves' 2 * MT
-        const int half = piece / MT, rows = (piece % MT) * 16;
-        cp_async16(slot_fetch + half * T::kOffHalf + (rows + (lane & 15)) * 16, w + half * 2048 + rows * 16);
-      }
-      if (lane < GPB * 2 * MT) {
-        const int kb = kb0 + idx_fetch * WARPS;
-        const int group = GPB > 1 ? min(kb * GPB + lane / (2 * MT), p.groups - 1)
-                                  : p.blocks_per_group == 1 ? kb : kb / p.blocks_per_group;
-        cp_async16(slot_fetch + T::kOffScales + lane * 16, s_src + static_cast<size_t>(group) * 256);
-      }
-      --to_fetch;
-      if (++idx_fetch == count) idx_fetch = 0;
-    }
-    cp_async_commit();                             // (an empty group when there is nothing left: the waits count groups)
+  auto advance = [&]() {
+    --to_fetch;
+    if (++idx_fetch == count) idx_fetch = 0;
+  };
+  auto next_slot = [&]() {
     slot_fetch += T::kStageBytes;
     if (slot_fetch == ring + T::kWarpBytes) slot_fetch = ring;
   };
+  auto fetch = [&]() {
+    if (to_fetch > 0) {
+      fetch_weights(idx_fetch, slot_fetch);
+      if (!LIVE || p.scale_pieces) {
+        if (s_lane) cp_async16(slot_fetch + piece_dst, piece_src(idx_fetch));
+      } else {
+        fetch_scale_words(idx_fetch, slot_fetch);
+      }
+      advance();
+    }
+    cp_async_commit();                             // (an empty group when there is nothing left: the waits count groups)
+    next_slot();
+  };
+  // The first DEPTH blocks: the plan's codes go out at once, a borrowed buffer's behind the wait.  Live scales are pulled into
+  // L2 meanwhile.
+  if (LIVE && p.weights_late) grid_dep_wait();
 #pragma unroll
-  for (int d = 0; d < DEPTH; ++d) fetch();
+  for (int d = 0; d < DEPTH; ++d) {
+    if constexpr (!LIVE) {
+      fetch();
+    } else {
+      if (to_fetch > 0) {
+        fetch_weights(idx_fetch, slot_fetch);
+        if (lane < 2 * GPB) {                      // both ends of each group's row
+          const size_t row = static_cast<size_t>(group_of(idx_fetch, lane >> 1)) * (2 * static_cast<size_t>(p.N));
+          prefetch_l2(s_base + row + 2 * ((lane & 1) ? min(T::kFeatures, p.N - n0) - 1 : 0));
+        }
+        advance();
+      }
+      cp_async_commit();
+      next_slot();
+    }
+  }
 
   // code - zp as two's complement in the top two bits of a byte is 64 times its value: for zp 2 the code with its upper bit
   // flipped, for zp 1 the code with its lower bit flipped is 1 - code (the scale takes the sign).  Zero points 0 and 3 do not fit
@@ -195,8 +262,16 @@ __global__ void __launch_bounds__(32 * WARPS, MIN_CTAS) w2a8_direct_kernel(const
 #pragma unroll
       for (int c = 0; c < 4; ++c) acc[i][t][c] = 0.f;
 
-  // weights and scales were written by the plan; activations and outputs belong to the kernels before this one
+  // the plan wrote its codes and copies; live scales, activations and outputs may belong to the kernels before this one
   grid_dep_wait();
+  // The first blocks' scales with plain loads: as copies behind those of the codes they would hold up the first block until
+  // all DEPTH have landed (groups complete in order).
+  uint4 s_first[DEPTH];
+  if (LIVE && p.scale_pieces) {
+#pragma unroll
+    for (int d = 0; d < DEPTH; ++d)
+      if (s_lane && d < count) s_first[d] = ld_global_v4(piece_src(first + d < count ? first + d : first + d - count));
+  }
 
   const int kb_first = kb0 - warp;                 // the CTA's range is [kb_first, kb_end)
   uint32_t xs_lane = 0;                            // QUANT: this lane's token in shared memory, at the warp's first block
@@ -281,6 +356,15 @@ __global__ void __launch_bounds__(32 * WARPS, MIN_CTAS) w2a8_direct_kernel(const
     }
   };
   fetch_x();
+  if (!LIVE) {
+  } else if (p.scale_pieces) {
+#pragma unroll
+    for (int d = 0; d < DEPTH; ++d)
+      if (s_lane && d < count) st_shared_v4(ring + d * T::kStageBytes + piece_dst, s_first[d]);
+  } else {
+    for (int d = 0; d < min(DEPTH, count); ++d) fetch_scale_words(first + d < count ? first + d : first + d - count, ring + d * T::kStageBytes);
+    cp_async_wait_all();
+  }
   // A lane's two words of a feature's block: GPB 1 adjacent ones (codes 32 q .. 32 q + 31), else word q of either half
   // (codes 16 q .. and 64 + 16 q ..), so that a half -- one or two scale groups -- is one K step of the warp's MMAs.
   const uint32_t w_off = (GPB == 1 ? (q >> 1) * T::kOffHalf + (q & 1) * 8 : q * 4) + g * 16;
@@ -296,10 +380,14 @@ __global__ void __launch_bounds__(32 * WARPS, MIN_CTAS) w2a8_direct_kernel(const
       if constexpr (GPB == 1) wv[j] = ld_shared_v2(slot + w_off + j * 128);
       else wv[j] = make_uint2(ld_shared_b32(slot + w_off + j * 128), ld_shared_b32(slot + w_off + T::kOffHalf + j * 128));
     }
+    const int idx_now = idx_x > 0 ? idx_x - 1 : count - 1;     // (fetch_x is one block ahead)
 #pragma unroll
-    for (int b = 0; b < GPB; ++b)
+    for (int b = 0; b < GPB; ++b) {
+      const uint32_t scale_shift = LIVE && (p.N & 1) ? (group_of(idx_now, b) & 1) * 2 : 0;
 #pragma unroll
-      for (int j = 0; j < 2 * MT; ++j) sv[b][j] = unit * ld_shared_half(slot + T::kOffScales + b * 2 * T::kFeatures + (8 * j + g) * 2);
+      for (int j = 0; j < 2 * MT; ++j)
+        sv[b][j] = unit * ld_shared_half(slot + T::kOffScales + scale_shift + b * T::kScalePitch + (8 * j + g) * 2);
+    }
     __syncwarp();
     fetch();                                   // into the slot just read
     slot += T::kStageBytes;
