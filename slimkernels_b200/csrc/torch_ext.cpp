@@ -1,6 +1,7 @@
 // PyTorch C++ extension: marshals tensors into the C ABI of include/sk_w2a8.h.  No kernels live here.
 // Registers the ops of namespace `slimkernels` used by slimkernels_b200/torch/ops.py.
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <cuda_runtime.h>
 #include <torch/library.h>
@@ -23,20 +24,54 @@ void check(int rc, const char* what) {
 // What a plan handle points to.  The plan's device buffers are one tensor from PyTorch's caching allocator and are filled
 // on the stream that is current at creation, so making and dropping a plan neither calls cudaMalloc / cudaFree nor
 // synchronises (both did, several times per plan: about 0.6 ms of a checkpoint layer's load).  Use on that stream is ordered by itself.
-// The first use on another stream waits for the filling on the host (once), and every use there is recorded with the
-// allocator, so that the memory is not handed out again before that stream is done with it.
+// The first use on another stream waits for the filling on the host (once).
+//
+// Dropping a plan does not wait for its launches either, so the memory that they read must not be handed out before they
+// are done: every use on another stream records that stream with the allocator, for the plan's own buffers and for the
+// caller's codes and scales, which launches read where they lie; the plan's own stream is recorded for those two when it
+// is made and when it is dropped.  (They are held weakly: a plan does not keep its weight alive.)  Where the allocator
+// cannot know -- launches captured in a graph run whenever it is replayed, and memory may not be the allocator's -- dropping
+// the plan waits for the device.
 struct TorchPlan {
   sk_w2a8_plan* plan = nullptr;
   at::Tensor storage;
+  std::vector<c10::weak_intrusive_ptr<c10::StorageImpl>> borrowed;      // codes and scales
   c10::cuda::CUDAStream home;
   cudaEvent_t filled = nullptr;
   std::atomic<bool> waited{false};
+  std::atomic<bool> wait_at_end{false};
   explicit TorchPlan(c10::cuda::CUDAStream s) : home(s) {}
+  void record_borrowed(c10::cuda::CUDAStream stream) {
+    namespace alloc = c10::cuda::CUDACachingAllocator;
+    for (const auto& weak : borrowed) {
+      const auto memory = weak.lock();
+      if (!memory) continue;
+      if (memory->data_ptr().get_deleter() == alloc::get()->raw_deleter()) alloc::recordStream(memory->data_ptr(), stream);
+      else wait_at_end.store(true, std::memory_order_relaxed);
+    }
+  }
   ~TorchPlan() {
+    try {
+      record_borrowed(home);
+    } catch (...) {
+      wait_at_end.store(true);
+    }
+    if (wait_at_end.load()) {
+      int cur = -1;
+      cudaGetDevice(&cur);
+      cudaSetDevice(home.device_index());
+      if (cudaDeviceSynchronize() != cudaSuccess) (void)cudaGetLastError();
+      if (cur >= 0) cudaSetDevice(cur);
+    }
     if (plan) sk_w2a8_plan_destroy(plan);
     if (filled) cudaEventDestroy(filled);
   }
 };
+
+bool capturing(c10::cuda::CUDAStream stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(stream.stream(), &status) != cudaSuccess || status != cudaStreamCaptureStatusNone;
+}
 
 TorchPlan* as_torch_plan(int64_t handle) {
   TORCH_CHECK(handle != 0, "slimkernels: null plan handle");
@@ -58,7 +93,9 @@ sk_w2a8_plan* plan_on(int64_t handle, c10::cuda::CUDAStream stream) {
       t->waited.store(true, std::memory_order_release);
     }
     t->storage.record_stream(c10::Stream(stream));
+    t->record_borrowed(stream);
   }
+  if (capturing(stream)) t->wait_at_end.store(true, std::memory_order_relaxed);
   return t->plan;
 }
 
@@ -77,11 +114,10 @@ int64_t plan_create(const at::Tensor& w, const at::Tensor& w_scale, int64_t N, i
   }
   c10::cuda::CUDAGuard guard(w.device());
   const auto stream = at::cuda::getCurrentCUDAStream();
-  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-  TORCH_CHECK(cudaStreamIsCapturing(stream.stream(), &capturing) == cudaSuccess && capturing == cudaStreamCaptureStatusNone,
-              "slimkernels::w2a8_plan_create: a plan cannot be made while its stream is being captured");
+  TORCH_CHECK(!capturing(stream), "slimkernels::w2a8_plan_create: a plan cannot be made while its stream is being captured");
   const int layout = tiled ? SK_WEIGHT_TILED : SK_WEIGHT_ROWMAJOR;
   auto t = std::make_unique<TorchPlan>(stream);
+  t->borrowed = {w.storage().getWeakStorageImpl(), w_scale.storage().getWeakStorageImpl()};
   // (arguments the plan refuses are refused before the storage is asked for)
   const int64_t bytes = std::max<int64_t>(256, sk_w2a8_plan_storage_bytes(w.get_device(), N, K, static_cast<int>(group_size), layout));
   t->storage = at::empty({bytes}, w.options().dtype(at::kByte));     // caching allocator: 512-byte aligned
@@ -92,6 +128,7 @@ int64_t plan_create(const at::Tensor& w, const at::Tensor& w_scale, int64_t N, i
   TORCH_CHECK(cudaEventCreateWithFlags(&t->filled, cudaEventDisableTiming) == cudaSuccess &&
                   cudaEventRecord(t->filled, stream.stream()) == cudaSuccess,
               "slimkernels::w2a8_plan_create: recording an event failed");
+  t->record_borrowed(stream);
   return static_cast<int64_t>(reinterpret_cast<intptr_t>(t.release()));
 }
 
@@ -416,6 +453,7 @@ int64_t cached_plan(const at::Tensor& w_packed, const at::Tensor& w_scale, int64
   TORCH_CHECK(w_packed.is_cuda() && w_packed.scalar_type() == at::kByte && w_packed.is_contiguous() && w_packed.dim() == 2,
               "w_packed must be a contiguous 2-D CUDA uint8 tensor [N, K/4]");
   const int64_t N = w_packed.size(0), K = w_packed.size(1) * 4;
+  const bool in_capture = capturing(at::cuda::getCurrentCUDAStream(w_packed.get_device()));   // (dropping a plan may wait for the device)
   std::lock_guard<std::mutex> lock(g_cache_mu);
   int64_t hit = 0;
   for (size_t i = 0; i < g_cache.size();) {
@@ -425,6 +463,10 @@ int64_t cached_plan(const at::Tensor& w_packed, const at::Tensor& w_scale, int64
                       e.w.lock().get() == w_packed.unsafeGetTensorImpl() && e.s.lock().get() == w_scale.unsafeGetTensorImpl() &&
                       e.group_size == group_size && e.zero_point == zero_point && e.bf16 == bf16;
     const bool stale = same && (e.w_version != w_packed._version() || e.s_version != w_scale._version());
+    if ((dead || stale) && in_capture) {
+      ++i;
+      continue;
+    }
     if (dead || stale) {
       plan_destroy(e.plan);
       g_cache[i] = g_cache.back();

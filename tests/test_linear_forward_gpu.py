@@ -71,8 +71,7 @@ def test_plan_used_on_another_stream_and_dropped_there():
     for i in range(6):
         lin = _linear(4096, 4096, seed=3)
         with torch.cuda.stream(side):
-            for w in (lin.w_packed, lin.w_scale, x):
-                w.record_stream(side)
+            x.record_stream(side)
             side.wait_stream(torch.cuda.default_stream())
             ys = [lin(x) for _ in range(8)]
         del lin
@@ -82,6 +81,63 @@ def test_plan_used_on_another_stream_and_dropped_there():
             want = ys[0].clone()
         assert all(torch.equal(y, want) for y in ys)
         del junk
+
+
+def _spin(stream):
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(400_000_000)                             # about 0.2 s
+
+
+@pytest.mark.parametrize("made_on", ["default", "third"])
+@pytest.mark.parametrize("tiled", [False, True])
+@pytest.mark.parametrize("M,G", [(8, 64), (200, 128)])
+def test_a_dropped_plan_keeps_its_borrowed_weights_from_being_handed_out(M, G, tiled, made_on):
+    """Launches on another stream than the weights' are still waiting when plan and weights are dropped: their memory must not
+    go to the next allocations.  (The allocations are never written, so that nothing races if they get it.)"""
+    from slimkernels_b200.torch import W2A8Plan, repack_weight
+    N, K = 1000, 2048
+    lin = _linear(N, K, G)
+    codes, scales = lin.w_packed.clone(), lin.w_scale.clone()
+    if tiled:
+        codes = repack_weight(codes)
+    x_q = torch.randint(-127, 128, (M, K), device="cuda", dtype=torch.int8)
+    x_s = torch.full((M,), 0.01, device="cuda")
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    # either the launches are on another stream than the plan was made on, or both are on another than the weights
+    with torch.cuda.stream(side if made_on == "third" else torch.cuda.default_stream()):
+        plan = W2A8Plan(codes, scales, N=N, K=K, group_size=G, tiled=tiled)
+    want = plan.gemm(x_q, x_s)
+    torch.cuda.synchronize()
+    sizes = [t.untyped_storage().nbytes() for t in (codes, scales)]
+    held = [t.data_ptr() for t in ((codes, scales) if tiled else (scales,))]
+    _spin(side)
+    with torch.cuda.stream(side):
+        y = plan.gemm(x_q, x_s)
+    del plan, codes, scales
+    taken = [torch.empty(n, dtype=torch.uint8, device="cuda") for n in sizes * 4]
+    assert not side.query()
+    for p in held:
+        assert all(not t.data_ptr() <= p < t.data_ptr() + t.numel() for t in taken)
+    side.synchronize()
+    assert torch.equal(y, want)
+
+
+def test_dropping_a_captured_plan_waits_for_the_graphs_that_use_it():
+    lin = _linear(512, 1024)
+    x = torch.randn(4, 1024, device="cuda").half()
+    want = lin(x)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = lin(x)
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    _spin(side)
+    with torch.cuda.stream(side):
+        graph.replay()
+    assert not side.query()
+    del lin
+    assert side.query() and torch.equal(y, want)
 
 
 def test_plan_is_refused_under_capture():

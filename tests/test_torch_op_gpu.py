@@ -136,3 +136,22 @@ def test_sum_row_blocks_adds_in_block_order_in_fp32(dtype):
         torch.ops.slimkernels.sum_row_blocks(blocks[:, :, :260])          # not contiguous
     with pytest.raises(RuntimeError):
         torch.ops.slimkernels.sum_row_blocks(blocks[:, :, :4].contiguous())   # N % 8 != 0
+
+
+def test_a_dead_cached_plan_is_left_alone_while_its_caller_captures():
+    """Dropping a plan whose launches were captured waits for the device, which a capture does not survive."""
+    probs = [random_problem(8, 256, 512, 128, seed=s) for s in (5, 6)]
+    first, second = (_dev(*p) for p in probs)
+    op = torch.ops.slimkernels.w2a8_gemm
+    want = op(*second)
+    op(*first)
+    graphs = [torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()]
+    with torch.cuda.graph(graphs[0]):
+        op(*first)
+    del first, graphs[0]
+    gc.collect()
+    with torch.cuda.graph(graphs[0]):
+        y = op(*second)
+    graphs[0].replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
