@@ -117,6 +117,14 @@ int64_t plan_create(const at::Tensor& w, const at::Tensor& w_scale, int64_t N, i
   TORCH_CHECK(!capturing(stream), "slimkernels::w2a8_plan_create: a plan cannot be made while its stream is being captured");
   const int layout = tiled ? SK_WEIGHT_TILED : SK_WEIGHT_ROWMAJOR;
   auto t = std::make_unique<TorchPlan>(stream);
+  TORCH_CHECK(cudaEventCreateWithFlags(&t->filled, cudaEventDisableTiming) == cudaSuccess, "slimkernels::w2a8_plan_create: no event");
+  // The copies read what the default stream has produced up to here, whichever stream is current (they used to be made on
+  // it): a weight quantised there and first used under a side stream needs no wait of the caller's.
+  const auto default_stream = c10::cuda::getDefaultCUDAStream(stream.device_index());
+  if (stream != default_stream)
+    TORCH_CHECK(cudaEventRecord(t->filled, default_stream.stream()) == cudaSuccess &&
+                    cudaStreamWaitEvent(stream.stream(), t->filled, 0) == cudaSuccess,
+                "slimkernels::w2a8_plan_create: waiting for the default stream failed");
   t->borrowed = {w.storage().getWeakStorageImpl(), w_scale.storage().getWeakStorageImpl()};
   // (arguments the plan refuses are refused before the storage is asked for)
   const int64_t bytes = std::max<int64_t>(256, sk_w2a8_plan_storage_bytes(w.get_device(), N, K, static_cast<int>(group_size), layout));
@@ -125,9 +133,7 @@ int64_t plan_create(const at::Tensor& w, const at::Tensor& w_scale, int64_t N, i
                                w.data_ptr<uint8_t>(), layout, w_scale.data_ptr(), bf16_out ? SK_OUT_BF16 : SK_OUT_F16,
                                t->storage.data_ptr(), bytes, stream.stream()),
         "w2a8_plan_create");
-  TORCH_CHECK(cudaEventCreateWithFlags(&t->filled, cudaEventDisableTiming) == cudaSuccess &&
-                  cudaEventRecord(t->filled, stream.stream()) == cudaSuccess,
-              "slimkernels::w2a8_plan_create: recording an event failed");
+  TORCH_CHECK(cudaEventRecord(t->filled, stream.stream()) == cudaSuccess, "slimkernels::w2a8_plan_create: recording an event failed");
   t->record_borrowed(stream);
   return static_cast<int64_t>(reinterpret_cast<intptr_t>(t.release()));
 }

@@ -83,6 +83,27 @@ def test_plan_used_on_another_stream_and_dropped_there():
         del junk
 
 
+@pytest.mark.parametrize("M", [4, 200])
+def test_plan_made_under_a_side_stream_sees_the_default_streams_weights(M):
+    """A weight is still being produced on the default stream when its first use, under a side stream, makes the plan."""
+    from slimkernels_b200.torch import W2A8Plan
+    N, K, G = 1000, 2048, 128
+    lin = _linear(N, K, G)
+    x_q = torch.randint(-127, 128, (M, K), device="cuda", dtype=torch.int8)
+    x_s = torch.full((M,), 0.01, device="cuda")
+    want = W2A8Plan(lin.w_packed, lin.w_scale, group_size=G).gemm(x_q, x_s)
+    codes, scales = torch.zeros_like(lin.w_packed), torch.zeros_like(lin.w_scale)
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    torch.cuda._sleep(100_000_000)
+    codes.copy_(lin.w_packed)
+    scales.copy_(lin.w_scale)
+    with torch.cuda.stream(side):
+        y = W2A8Plan(codes, scales, group_size=G).gemm(x_q, x_s)
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
+
+
 def _spin(stream):
     with torch.cuda.stream(stream):
         torch.cuda._sleep(400_000_000)                             # about 0.2 s
