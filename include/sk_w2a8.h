@@ -115,6 +115,7 @@ int sk_w2a8_plan_create(sk_w2a8_plan** plan, int device, int64_t N, int64_t K, i
 /* The same plan in device memory the caller provides (sk_w2a8_plan_storage_bytes(...) bytes, 256-byte aligned, kept until
  * the plan is destroyed and every launch made with it has completed) and without synchronising: the copies are made on
  * `stream`, and the plan may be used there at once.  Use on another stream must be ordered after it by the caller.
+ * (So must sk_w2a8_last_device_status, which reads outside any stream: wait for `stream` first.)
  * Creation and destruction neither allocate nor free device memory. */
 int64_t sk_w2a8_plan_storage_bytes(int device, int64_t N, int64_t K, int group_size, int w_layout);
 int sk_w2a8_plan_create_in(sk_w2a8_plan** plan, int device, int64_t N, int64_t K, int group_size, int zero_point,

@@ -24,7 +24,7 @@ void check(int rc, const char* what) {
 // What a plan handle points to.  The plan's device buffers are one tensor from PyTorch's caching allocator and are filled
 // on the stream that is current at creation, so making and dropping a plan neither calls cudaMalloc / cudaFree nor
 // synchronises (both did, several times per plan: about 0.6 ms of a checkpoint layer's load).  Use on that stream is ordered by itself.
-// The first use on another stream waits for the filling on the host (once).
+// The first use on another stream, or look at the status word, waits for the filling on the host (once).
 //
 // Dropping a plan does not wait for its launches either, so the memory that they read must not be handed out before they
 // are done: every use on another stream records that stream with the allocator, for the plan's own buffers and for the
@@ -41,6 +41,15 @@ struct TorchPlan {
   std::atomic<bool> waited{false};
   std::atomic<bool> wait_at_end{false};
   explicit TorchPlan(c10::cuda::CUDAStream s) : home(s) {}
+  void wait_until_filled() {                       // on the host, once
+    if (waited.load(std::memory_order_acquire)) return;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;      // a capture elsewhere must not forbid the wait
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t e = cudaEventSynchronize(filled);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    TORCH_CHECK(e == cudaSuccess, "slimkernels: waiting for a plan failed: ", cudaGetErrorString(e));
+    waited.store(true, std::memory_order_release);
+  }
   void record_borrowed(c10::cuda::CUDAStream stream) {
     namespace alloc = c10::cuda::CUDACachingAllocator;
     for (const auto& weak : borrowed) {
@@ -84,14 +93,7 @@ sk_w2a8_plan* as_plan(int64_t handle) { return as_torch_plan(handle)->plan; }
 sk_w2a8_plan* plan_on(int64_t handle, c10::cuda::CUDAStream stream) {
   TorchPlan* t = as_torch_plan(handle);
   if (stream != t->home) {
-    if (!t->waited.load(std::memory_order_acquire)) {
-      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;    // a capture elsewhere must not forbid the wait
-      cudaThreadExchangeStreamCaptureMode(&mode);
-      const cudaError_t e = cudaEventSynchronize(t->filled);
-      cudaThreadExchangeStreamCaptureMode(&mode);
-      TORCH_CHECK(e == cudaSuccess, "slimkernels: waiting for a plan failed: ", cudaGetErrorString(e));
-      t->waited.store(true, std::memory_order_release);
-    }
+    t->wait_until_filled();
     t->storage.record_stream(c10::Stream(stream));
     t->record_borrowed(stream);
   }
@@ -409,6 +411,7 @@ void launch_floor_probe(int64_t handle, const at::Tensor& on_device_of, int64_t 
 
 int64_t device_status(int64_t handle) {
   int v = 0;
+  as_torch_plan(handle)->wait_until_filled();      // (the status word, too, is set in stream order; it is read outside the stream)
   int rc = sk_w2a8_last_device_status(as_plan(handle), &v);
   TORCH_CHECK(rc == SK_OK || rc == SK_ERR_DEVICE_TIMEOUT, "slimkernels::w2a8_device_status failed: ", sk_status_string(rc));
   return v;

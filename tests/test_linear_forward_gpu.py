@@ -144,6 +144,24 @@ def test_a_dropped_plan_keeps_its_borrowed_weights_from_being_handed_out(M, G, t
     assert torch.equal(y, want)
 
 
+def test_device_status_of_a_plan_whose_stream_has_not_got_to_it():
+    """The status word lies in memory that held something else, and is cleared in stream order."""
+    from slimkernels_b200 import capi
+    from slimkernels_b200.torch import W2A8Plan
+    N, K = 1024, 2048
+    lin = _linear(N, K)
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        nbytes = capi.load().sk_w2a8_plan_storage_bytes(0, N, K, 128, capi.SK_WEIGHT_ROWMAJOR)
+        junk = torch.full((nbytes,), 0xFF, dtype=torch.uint8, device="cuda")
+        side.synchronize()
+        del junk
+        _spin(side)
+        plan = W2A8Plan(lin.w_packed, lin.w_scale)
+        assert plan.device_status() == 0
+
+
 def test_dropping_a_captured_plan_waits_for_the_graphs_that_use_it():
     lin = _linear(512, 1024)
     x = torch.randn(4, 1024, device="cuda").half()
