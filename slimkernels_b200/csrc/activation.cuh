@@ -19,6 +19,8 @@ constexpr int kActThreads = 256;
 // stream may start its own set-up now -- the decode GEMM that follows a quantiser uses that to stream its first
 // weights --, and this kernel's inputs, which the previous kernel wrote, are read only after that kernel is complete.
 __device__ __forceinline__ void act_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// (The kernels' inputs are plain pointers: loads through const __restrict__ ones count as invariant, and a compiler may move
+// those above the wait.)
 __device__ __forceinline__ void act_wait_for_inputs() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <int THREADS = kActThreads>
@@ -82,7 +84,7 @@ __device__ __forceinline__ uint4 as_half8(uint4 v) {
 // (a layer of 96 tokens x 11008 features -> 4096: 22.6 us a call with 256 threads, 19.3 with 1024).
 template <int kMaxVec, bool BF16, int THREADS = kActThreads>
 __global__ void __launch_bounds__(THREADS)
-quantize_activation_kernel(const uint16_t* __restrict__ x, long long ld_x, int8_t* __restrict__ x_q, long long ld_q,
+quantize_activation_kernel(const uint16_t* x, long long ld_x, int8_t* __restrict__ x_q, long long ld_q,
                            float* __restrict__ x_scale, int K) {
   __shared__ float red[THREADS / 32];
   act_launch_dependents();
@@ -158,7 +160,7 @@ constexpr int kClusterVecs = 2;
 // (eight CTAs per SM: 32 registers per thread instead of 40 cost a few spilled words and gain 13 % -- the kernel's
 // phases -- load, SiLU, barriers, quantise, store -- overlap only across the CTAs of an SM)
 __global__ void __launch_bounds__(kActThreads, 8)
-silu_mul_quantize_cluster_kernel(const __half* __restrict__ gate_up, long long ld_gu, int8_t* __restrict__ h_q,
+silu_mul_quantize_cluster_kernel(const __half* gate_up, long long ld_gu, int8_t* __restrict__ h_q,
                                  long long ld_q, float* __restrict__ h_scale, int I) {
   __shared__ float red[kActThreads / 32];
   __shared__ float part[8];                     // partial maxima of the cluster's CTAs
@@ -224,7 +226,7 @@ silu_mul_quantize_cluster_kernel(const __half* __restrict__ gate_up, long long l
 // read twice instead (the second pass is an L2 hit) and SiLU(gate) * up is recomputed, which gives the identical
 // fp32 values; no dynamic shared memory, so eight CTAs fit an SM.
 __global__ void __launch_bounds__(kActThreads)
-silu_mul_quantize_twopass_kernel(const __half* __restrict__ gate_up, long long ld_gu, int8_t* __restrict__ h_q,
+silu_mul_quantize_twopass_kernel(const __half* gate_up, long long ld_gu, int8_t* __restrict__ h_q,
                                  long long ld_q, float* __restrict__ h_scale, int I) {
   __shared__ float red[kActThreads / 32];
   act_launch_dependents();

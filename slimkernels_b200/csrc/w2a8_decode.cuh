@@ -446,7 +446,7 @@ w2a8_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParams 
           // dependent global load per stored row would serialise the tail
           float xs[TOK];
 #pragma unroll
-          for (int t = 0; t < TOK; ++t) xs[t] = (m0 + t < p.M) ? __ldg(p.x_scale + m0 + t) * kScaleDown : 0.f;
+          for (int t = 0; t < TOK; ++t) xs[t] = (m0 + t < p.M) ? ld_global_f32(p.x_scale + m0 + t) * kScaleDown : 0.f;
           for (int d = 0; d <= p.n_extra; ++d) {
             uint16_t* outp = reinterpret_cast<uint16_t*>(d == 0 ? p.out : p.out_extra[d - 1]) +
                              static_cast<size_t>(m0) * p.ld_out + n;
@@ -495,7 +495,7 @@ w2a8_decode_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParams 
       for (int it = 0; it < kMaxIter; ++it) {
         const int idx = threadIdx.x + it * T::kThreads;
         const int m = m0 + my_rank + (idx >> 7) * num_splits;
-        xs[it] = (idx < rows * kTileN && m < p.M) ? __ldg(p.x_scale + m) * kScaleDown : 0.f;
+        xs[it] = (idx < rows * kTileN && m < p.M) ? ld_global_f32(p.x_scale + m) * kScaleDown : 0.f;
       }
       __syncwarp();
       cluster_sync_all();

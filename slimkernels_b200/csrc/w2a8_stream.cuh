@@ -327,7 +327,7 @@ w2a8_stream_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParams 
       // dependent global load per stored row would serialise the tail
       float xs[TOK];
 #pragma unroll
-      for (int t = 0; t < TOK; ++t) xs[t] = (t < p.M) ? __ldg(p.x_scale + t) * kScaleDown : 0.f;
+      for (int t = 0; t < TOK; ++t) xs[t] = (t < p.M) ? ld_global_f32(p.x_scale + t) * kScaleDown : 0.f;
       for (int d = 0; d <= p.n_extra; ++d) {
         uint16_t* outp = reinterpret_cast<uint16_t*>(d == 0 ? p.out : p.out_extra[d - 1]) + n;
 #pragma unroll

@@ -775,10 +775,10 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     // A load that misses L2 would still stall the loop one group later (the ring is shifted by register moves), so
     // every row is pulled into L2 kScalePrefetchGroups groups earlier with a prefetch, which occupies no register.
     const unsigned short* sp =
-        reinterpret_cast<const unsigned short*>(p.w_scale) + static_cast<size_t>(g_begin) * p.N + (n_ok ? n : 0);
+        pointer_from_here(reinterpret_cast<const unsigned short*>(p.w_scale)) + static_cast<size_t>(g_begin) * p.N + (n_ok ? n : 0);
     int g_load = g_begin;                       // next group whose scale is fetched
     auto load_scale = [&]() -> unsigned short {
-      const unsigned short r = (n_ok && g_load < g_end) ? __ldg(sp) : static_cast<unsigned short>(0);
+      const unsigned short r = (n_ok && g_load < g_end) ? *sp : static_cast<unsigned short>(0);
 #ifndef SK_NO_SCALE_PREFETCH
       if (g_load + kScalePrefetchGroups < g_end)
         asm volatile("prefetch.global.L2 [%0];" ::"l"(sp + static_cast<size_t>(kScalePrefetchGroups) * p.N));
