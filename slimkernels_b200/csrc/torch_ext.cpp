@@ -340,11 +340,12 @@ at::Tensor mlp_forward(int64_t gate_up_plan, int64_t down_plan, const at::Tensor
 }
 
 // Activations of any leading shape as the 2-D matrix a quantiser reads: fp16, or bf16 whose rows it can read as they are;
-// anything else is converted to fp16 first.
-at::Tensor activation_rows(const at::Tensor& x, bool* is_bf16) {
+// anything else is converted to fp16 first.  (Rows of another width are converted, too, which makes them contiguous: a
+// slice of wider rows must not pass for rows of `features`.)
+at::Tensor activation_rows(const at::Tensor& x, int64_t features, bool* is_bf16) {
   TORCH_CHECK(x.is_cuda() && x.dim() >= 1, "x must be a CUDA tensor [..., K]");
   at::Tensor x2 = x.dim() == 2 ? x : x.reshape({-1, x.size(-1)});
-  *is_bf16 = x2.scalar_type() == at::kBFloat16 && x2.stride(1) == 1 && x2.stride(0) >= x2.size(1) && x2.stride(0) % 8 == 0 &&
+  *is_bf16 = x2.scalar_type() == at::kBFloat16 && x2.size(1) == features && x2.stride(1) == 1 && x2.stride(0) >= features && x2.stride(0) % 8 == 0 &&
              (reinterpret_cast<uintptr_t>(x2.data_ptr()) & 15) == 0;
   if (!*is_bf16) x2 = x2.to(at::kHalf);
   TORCH_CHECK(x2.stride(1) == 1, "x must have unit inner stride");
@@ -362,7 +363,7 @@ at::Tensor with_leading_shape(const at::Tensor& y, const at::Tensor& x) {
 // one call: at decode sizes the host work of its pieces took longer than the GPU's.
 at::Tensor linear_forward(int64_t handle, const at::Tensor& x, int64_t N, int64_t K, bool bf16_out) {
   bool x_bf16 = false;
-  const at::Tensor x2 = activation_rows(x, &x_bf16);
+  const at::Tensor x2 = activation_rows(x, K, &x_bf16);
   const int64_t M = x2.size(0);
   TORCH_CHECK(x2.size(1) == K, "x must have ", K, " features, got ", x2.size(1));
   int64_t plan_n = 0, plan_k = 0;
@@ -386,8 +387,10 @@ at::Tensor linear_forward(int64_t handle, const at::Tensor& x, int64_t N, int64_
 
 // x [..., hidden] -> [..., hidden]: the MLP block, from activations as linear_forward takes them.
 at::Tensor mlp_block(int64_t gate_up_plan, int64_t down_plan, const at::Tensor& x, int64_t hidden_out, bool bf16_out) {
+  int64_t hidden = 0;
+  check(sk_w2a8_plan_info(as_plan(gate_up_plan), nullptr, &hidden, nullptr, nullptr, nullptr, nullptr), "w2a8_plan_info");
   bool x_bf16 = false;
-  const at::Tensor x2 = activation_rows(x, &x_bf16);
+  const at::Tensor x2 = activation_rows(x, hidden, &x_bf16);
   return with_leading_shape(mlp_run(gate_up_plan, down_plan, x2, x_bf16, hidden_out, bf16_out), x);
 }
 

@@ -83,6 +83,19 @@ def test_plan_used_on_another_stream_and_dropped_there():
         del junk
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_a_narrow_slice_of_wide_rows_is_refused(dtype):
+    from slimkernels_b200.torch import W2A8LlamaMLP
+    mlp = W2A8LlamaMLP(_linear(768, 256), _linear(256, 384, seed=1))
+    wide = torch.randn(5, 512, device="cuda").to(dtype)
+    assert mlp(wide[:, :256]).shape == (5, 256)
+    for x in (wide[:, :128], wide.view(1, 5, 512)[..., :248]):
+        with pytest.raises(RuntimeError):
+            mlp(x)
+        with pytest.raises(RuntimeError):
+            mlp.gate_up(x)
+
+
 @pytest.mark.parametrize("M", [4, 200])
 def test_plan_made_under_a_side_stream_sees_the_default_streams_weights(M):
     """A weight is still being produced on the default stream when its first use, under a side stream, makes the plan."""
