@@ -101,10 +101,10 @@ int sk_w2a8_unrepack(const uint8_t* w_tiled, int64_t N, int64_t K, uint8_t* w_pa
  * Binds one weight matrix to a device: validates shapes/alignment, builds the tiled weight copy (or
  * borrows one), allocates a 4-byte device status word.  Stands where gemm_tn builds its tilers, smem
  * layouts and tensor maps on every call (wgmma_sm90_W2A8.cu:448-466).  Synchronises `device` once.
- * With group size 128 the plan also makes a private copy of the scales in the order its split decode kernel (3) streams
- * them, and -- for weight matrices large enough that the balanced-split decode kernel is their default, or
- * on the first SK_OPT_KERNEL = 5 / SK_OPT_STREAM_CTAS request -- a scratch buffer for that kernel's partial sums
- * (3-20 MiB).
+ * With group size 128 the plan also makes a private copy of the scales in the order its decode kernels (3, 6) stream
+ * them.  An option that leads to the balanced-split decode kernel (SK_OPT_KERNEL = 5, SK_OPT_STREAM_CTAS; on weights of 64 K
+ * blocks per SM or more also a forced token tile of 16, a split of 1 or a persistent launch) makes a scratch buffer for that
+ * kernel's partial sums (3-20 MiB).
  * w_scale_f16 (and w, when it is tiled) must outlive the plan: the kernels read them as they are when a launch runs.  A
  * change of their contents in stream order is seen by every launch of group sizes other than 128 and of more than 32
  * tokens; launches of up to 32 tokens with group size 128 may use the copy of the scales and may read tiled codes before

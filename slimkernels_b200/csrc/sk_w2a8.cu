@@ -246,12 +246,12 @@ struct sk_w2a8_plan {
   const __half* w_scale = nullptr;      // borrowed
   __half* w_scale_tiled = nullptr;      // in the plan's storage, group size 128: [n_tiles][k_blocks][128] copy of the scales
   int* status = nullptr;                // device; first in the plan's storage, one block that also holds the tiled copies
-  bool external_storage = false;        // the buffers below live in the caller's storage (sk_w2a8_plan_create_in)
-  bool stream_owned = false;            // stream_scratch / stream_counters are the plan's own allocations
+  bool external_storage = false;        // that block is the caller's (sk_w2a8_plan_create_in)
   // balanced-split decode kernel: scratch for the partial sums of tiles shared between CTAs, and their counters
-  float* stream_scratch = nullptr;      // device, owned (null: that kernel is not available for this plan)
+  float* stream_scratch = nullptr;      // device, owned; allocated when an option asks for that kernel (stream_setup)
   int* stream_counters = nullptr;       // device, owned; zero between launches
   int stream_ctas = 0, stream_slots = 0;
+  bool stream_failed = false;           // there was no memory for them: the split decode kernel takes those calls
   int last_cuda_error = 0;
   int opt_kernel = 0, opt_token_tile = 0, opt_split_k = 0, opt_persistent = 0, opt_pdl = 0, opt_tma_store = 0;
   long long opt_wait_limit = 0;         // 0: the default limit
@@ -285,19 +285,27 @@ struct LaunchChoice {
   int mix_tiles1 = 0, mix_split = 0;   // decode kernel 3, mixed launch (see w2a8_decode.cuh); split_k then reports mix_split
 };
 
+// Options that take calls away from the direct kernel.
+static bool options_force_tcgen05(const sk_w2a8_plan* plan) {
+  return plan->opt_kernel || plan->opt_token_tile || plan->opt_split_k || plan->opt_persistent || plan->opt_skip_copy;
+}
+// Measured on B200 (M = 16): of the tcgen05 decode kernels the balanced split wins once every SM has ~64 K blocks or more to
+// stream (70B-class projections: 53 against 70 us on 57344 x 8192); below that its longer tail -- partial sums meet in L2,
+// three global round trips -- costs more than the even load saves.  Its 32-token variant is slower throughout.
+static bool stream_pays_from(const sk_w2a8_plan* plan) {
+  return static_cast<long long>(plan->n_tiles) * plan->k_blocks >= 64LL * plan->sm_count;
+}
+
 static LaunchChoice choose(const sk_w2a8_plan* plan, long long M) {
   LaunchChoice c;
   if (plan->opt_token_tile) c.token_tile = plan->opt_token_tile;
   else c.token_tile = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
   const bool decode_ok = plan->G == 128 && c.token_tile <= 32;
-  // Decode sizes that are one token tile go to the balanced-split kernel (5) when the plan has its scratch buffer;
-  // a forced split (SK_OPT_SPLIT_K) or several token tiles go to the kernel that splits over clusters (3).
-  const bool stream_ok = decode_ok && M <= c.token_tile && plan->stream_scratch != nullptr && plan->opt_split_k <= 1;
-  // Measured on B200 (M = 16): the balanced split wins once every SM has ~64 K blocks or more to stream (70B-class
-  // projections: 53 against 70 us on 57344 x 8192); below that its longer tail -- partial sums meet in L2, three
-  // global round trips -- costs more than the even load saves.  Its 32-token variant is slower throughout.
-  const bool stream_pays = stream_ok && c.token_tile == 16 &&
-                           static_cast<long long>(plan->n_tiles) * plan->k_blocks >= 64LL * plan->sm_count;
+  // Decode sizes that are one token tile go to the balanced-split kernel (5) where it pays; a forced split (SK_OPT_SPLIT_K) or
+  // several token tiles go to the kernel that splits over clusters (3).  Small calls without options are the direct kernel's
+  // (choose_direct), so kernel 5 runs only under options, and those that lead here have its scratch allocated (stream_wanted).
+  const bool stream_ok = decode_ok && M <= c.token_tile && plan->opt_split_k <= 1 && plan->K % 256 == 0 && !plan->stream_failed;
+  const bool stream_pays = stream_ok && c.token_tile == 16 && stream_pays_from(plan);
   c.kernel = plan->opt_kernel && plan->opt_kernel != 6 ? plan->opt_kernel : (stream_pays ? 5 : decode_ok ? 3 : 1);
   if (c.kernel == 5 && !stream_ok) c.kernel = 3;
   if (c.kernel == 3 && !decode_ok) c.kernel = 1;
@@ -305,7 +313,8 @@ static LaunchChoice choose(const sk_w2a8_plan* plan, long long M) {
   if (c.kernel == 5) {
     c.split_k = 1;
     c.persistent = 0;
-    c.ctas = plan->stream_ctas;
+    const long long units = static_cast<long long>(plan->n_tiles) * (plan->k_blocks / 2);
+    c.ctas = plan->stream_scratch ? plan->stream_ctas : static_cast<int>(units < 2 * plan->sm_count ? units : 2 * plan->sm_count);
     return c;
   }
   if (plan->opt_split_k) c.split_k = plan->opt_split_k;
@@ -496,17 +505,13 @@ static void stream_geometry(const sk_w2a8_plan* plan, int want_ctas, int* ctas_o
   *slots_out = slots;
 }
 
-// (Re)allocates the scratch buffer and the counters of the balanced-split decode kernel.  Not on the call path: plan
-// creation and sk_w2a8_set_option only.  The device of the plan is current.
+// (Re)allocates the scratch buffer and the counters of the balanced-split decode kernel.  Not on the call path:
+// sk_w2a8_set_option only.  The device of the plan is current.
 static int stream_setup(sk_w2a8_plan* plan, int want_ctas) {
-  if (plan->stream_owned) {
-    if (plan->stream_scratch) cudaFree(plan->stream_scratch);
-    if (plan->stream_counters) cudaFree(plan->stream_counters);
-  }
-  plan->stream_scratch = nullptr;
-  plan->stream_counters = nullptr;
-  plan->stream_owned = false;
+  if (plan->stream_scratch) { cudaFree(plan->stream_scratch); plan->stream_scratch = nullptr; }
+  if (plan->stream_counters) { cudaFree(plan->stream_counters); plan->stream_counters = nullptr; }
   plan->stream_ctas = plan->stream_slots = 0;
+  plan->stream_failed = true;
   if (plan->G != 128 || (plan->K % 256) != 0) return SK_OK;   // whole half stages only: the other decode kernel serves the rest
   int ctas = 0, slots = 0;
   stream_geometry(plan, want_ctas, &ctas, &slots);
@@ -516,24 +521,37 @@ static int stream_setup(sk_w2a8_plan* plan, int want_ctas) {
   const size_t cbytes = static_cast<size_t>(plan->n_tiles) * StreamTraits<32>::kEpiWarps * sizeof(int);
   e = cudaMalloc(&plan->stream_counters, cbytes);
   if (e == cudaSuccess) e = cudaMemset(plan->stream_counters, 0, cbytes);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);     // (launches on non-blocking streams are not ordered after it)
   if (e != cudaSuccess) {
     cudaFree(plan->stream_scratch);
     plan->stream_scratch = nullptr;
     if (plan->stream_counters) { cudaFree(plan->stream_counters); plan->stream_counters = nullptr; }
     return cuda_fail(plan, e);
   }
-  plan->stream_owned = true;
   plan->stream_ctas = ctas;
   plan->stream_slots = slots;
+  plan->stream_failed = false;
   return SK_OK;
+}
+
+// An option that leads calls of up to 16 tokens to choose(), where large weights get the balanced-split kernel.
+static void stream_wanted(sk_w2a8_plan* plan) {
+  if (plan->stream_scratch || plan->stream_failed || plan->G != 128 || plan->K % 256 != 0 || !stream_pays_from(plan)) return;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  int cur = -1;
+  cudaGetDevice(&cur);
+  (void)cudaSetDevice(plan->device);
+  (void)stream_setup(plan, 0);
+  if (cur >= 0 && cur != plan->device) (void)cudaSetDevice(cur);
+  cudaThreadExchangeStreamCaptureMode(&mode);
 }
 
 // Where a plan's buffers sit in one block of storage (256-byte aligned offsets; -1: the plan has no such buffer).
 struct PlanLayout {
-  long long status, w_tiled, w_scale_tiled, stream_scratch, stream_counters, total;
-  size_t counter_bytes;
+  long long status, w_tiled, w_scale_tiled, total;
 };
-static PlanLayout plan_layout(sk_w2a8_plan* plan, int w_layout) {
+static PlanLayout plan_layout(const sk_w2a8_plan* plan, int w_layout) {
   PlanLayout l;
   long long o = 0;
   auto take = [&o](long long bytes) {
@@ -545,17 +563,6 @@ static PlanLayout plan_layout(sk_w2a8_plan* plan, int w_layout) {
   l.status = take(sizeof(int));
   l.w_tiled = w_layout == SK_WEIGHT_ROWMAJOR ? take(blocks * kWpBytes) : -1;
   l.w_scale_tiled = plan->G == 128 ? take(blocks * kTileN * static_cast<long long>(sizeof(__half))) : -1;
-  l.stream_scratch = l.stream_counters = -1;
-  l.counter_bytes = 0;
-  // The balanced-split decode kernel's scratch is part of it only where that kernel is the default (large weight
-  // matrices, see choose()); elsewhere it is allocated on request (SK_OPT_KERNEL = 5 / SK_OPT_STREAM_CTAS, set-up calls).
-  if (plan->G == 128 && (plan->K % 256) == 0 && blocks >= 64LL * plan->sm_count) {
-    stream_geometry(plan, 0, &plan->stream_ctas, &plan->stream_slots);
-    l.counter_bytes = static_cast<size_t>(plan->n_tiles) * StreamTraits<32>::kEpiWarps * sizeof(int);
-    l.stream_scratch = take(static_cast<long long>(plan->n_tiles) * plan->stream_slots * StreamTraits<32>::kSlotFloats *
-                            static_cast<long long>(sizeof(float)));
-    l.stream_counters = take(static_cast<long long>(l.counter_bytes));
-  }
   l.total = o;
   return l;
 }
@@ -633,8 +640,7 @@ static int launch_direct(sk_w2a8_plan* plan, const DirectParams& prm, int split,
 //     11008 in two halves 5.9, but 1 x 4096 x 4096 whole 2.7, in halves 3.7 (the cluster barriers cost more).
 static bool choose_direct(const sk_w2a8_plan* plan, long long M, DirectChoice* out) {
   const bool forced = plan->opt_kernel == 6;
-  if (!forced && (plan->opt_kernel || plan->opt_token_tile || plan->opt_split_k || plan->opt_persistent || plan->opt_skip_copy || M > 128))
-    return false;
+  if (!forced && (options_force_tcgen05(plan) || M > 128)) return false;
   if ((reinterpret_cast<uintptr_t>(plan->w_scale) & 3) && !direct_reads_copy(plan, M)) return false;
   DirectChoice c;
   c.nt = M <= 8 ? 1 : M <= 16 ? 2 : M <= 24 ? 3 : 4;
@@ -1296,11 +1302,6 @@ static int plan_create_common(sk_w2a8_plan** out, int device, int64_t N, int64_t
       sk::tile_scales_kernel<<<blocks, 256, 0, stream>>>(plan->w_scale, plan->w_scale_tiled, N, plan->k_blocks, total);
       e = cudaGetLastError();
     }
-    if (rc == SK_OK && e == cudaSuccess && l.stream_counters >= 0) {
-      plan->stream_scratch = reinterpret_cast<float*>(base + l.stream_scratch);
-      plan->stream_counters = reinterpret_cast<int*>(base + l.stream_counters);
-      e = cudaMemsetAsync(plan->stream_counters, 0, l.counter_bytes, stream);
-    }
     // Last, and not only for its own sake: decode kernels are dependent launches that read the copies before they wait for the
     // kernel in front of them.  Were that a kernel above, they could start when its last CTA exits, before its stores are
     // sure to be visible; this operation starts only after those kernels are complete.
@@ -1383,11 +1384,11 @@ int sk_w2a8_plan_create_in(sk_w2a8_plan** out, int device, int64_t N, int64_t K,
 
 int sk_w2a8_plan_destroy(sk_w2a8_plan* plan) {
   if (!plan) return SK_ERR_NULL_POINTER;
-  if (!plan->external_storage || plan->stream_owned) {
+  if (!plan->external_storage || plan->stream_scratch) {
     int cur = -1;
     cudaGetDevice(&cur);
     (void)cudaSetDevice(plan->device);
-    if (plan->stream_owned) {
+    if (plan->stream_scratch) {
       cudaFree(plan->stream_scratch);
       cudaFree(plan->stream_counters);
     }
@@ -1416,7 +1417,7 @@ int sk_w2a8_set_option(sk_w2a8_plan* plan, int key, int64_t value) {
     case SK_OPT_KERNEL:
       if (value < 0 || value > 6) return SK_ERR_BAD_ARGUMENT;
       if (value == 2 && !plan->w_rowmajor) return SK_ERR_UNAVAILABLE;
-      if (value == 5 && !plan->stream_scratch) {   // first request on a plan that did not get the scratch at creation
+      if (value == 5 && !plan->stream_scratch) {   // first request
         int cur = -1;
         cudaGetDevice(&cur);
         (void)cudaSetDevice(plan->device);
@@ -1432,10 +1433,12 @@ int sk_w2a8_set_option(sk_w2a8_plan* plan, int key, int64_t value) {
     case SK_OPT_TOKEN_TILE:
       if (value != 0 && value != 16 && value != 32 && value != 64 && value != 128 && value != 192 && value != 256)
         return SK_ERR_BAD_ARGUMENT;
+      if (value == 16) sk::stream_wanted(plan);
       plan->opt_token_tile = static_cast<int>(value);
       return SK_OK;
     case SK_OPT_SPLIT_K:
       if (value != 0 && value != 1 && value != 2 && value != 4 && value != 8) return SK_ERR_BAD_ARGUMENT;
+      if (value == 1) sk::stream_wanted(plan);
       plan->opt_split_k = static_cast<int>(value);
       return SK_OK;
     case SK_OPT_DEPENDENT_LAUNCH:
@@ -1448,6 +1451,7 @@ int sk_w2a8_set_option(sk_w2a8_plan* plan, int key, int64_t value) {
       return SK_OK;
     case SK_OPT_PERSISTENT:
       if (value < 0 || value > 2) return SK_ERR_BAD_ARGUMENT;
+      if (value != 0) sk::stream_wanted(plan);
       plan->opt_persistent = static_cast<int>(value);
       return SK_OK;
     case SK_OPT_WAIT_LIMIT_CYCLES:
@@ -1466,6 +1470,7 @@ int sk_w2a8_set_option(sk_w2a8_plan* plan, int key, int64_t value) {
     }
     case SK_OPT_TEST_SKIP_COPY:
       if (value < 0 || value > (1 << 20)) return SK_ERR_BAD_ARGUMENT;
+      if (value != 0) sk::stream_wanted(plan);
       plan->opt_skip_copy = static_cast<int>(value);
       return SK_OK;
     default: return SK_ERR_BAD_ARGUMENT;
@@ -1590,7 +1595,7 @@ int sk_w2a8_launch_floor_probe(sk_w2a8_plan* plan, int64_t M, sk_stream_t stream
   if (e == cudaSuccess) {
     cudaLaunchConfig_t cfg = {};
     const int m_tiles = static_cast<int>((M + ch.token_tile - 1) / ch.token_tile);
-    cfg.gridDim = ch.kernel == 5 ? dim3(plan->stream_ctas, 1, 1)
+    cfg.gridDim = ch.kernel == 5 ? dim3(ch.ctas, 1, 1)
                   : ch.mix_split ? dim3(ch.ctas, 1, 1) : dim3(plan->n_tiles, m_tiles, ch.split_k);
     cfg.blockDim = dim3(sk::DecodeTraits<16>::kThreads, 1, 1);
     cfg.dynamicSmemBytes = dyn - 1024;

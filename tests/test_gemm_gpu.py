@@ -143,8 +143,9 @@ def test_balanced_split_kernel_falls_back_where_it_does_not_apply():
         dp.plan.set_option(capi.SK_OPT_KERNEL, capi.KERNEL_TCGEN05_DECODE_BALANCED)
 
 
-def test_balanced_split_is_the_default_for_large_decode_problems():
-    """From 64 K blocks per SM on (16-token tile) the balanced split is the default; 32-token tiles stay with clusters."""
+def test_balanced_split_is_the_tcgen05_choice_for_large_decode_problems():
+    """From 64 K blocks per SM on (16-token tile) the balanced split is what the tcgen05 kernels take (under options; without
+    any the direct kernel runs); 32-token tiles stay with clusters.  Its scratch is not the plan's until an option asks."""
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     N = 448 * 128
     for K in (2048, 4096):      # 48 and 97 K blocks per SM on 148 SMs
@@ -154,10 +155,18 @@ def test_balanced_split_is_the_default_for_large_decode_problems():
         want = capi.KERNEL_TCGEN05_DECODE_BALANCED if big else capi.KERNEL_TCGEN05_DECODE
         assert dp.plan.query_launch(16)["kernel"] == want
         assert dp.plan.query_launch(32)["kernel"] == capi.KERNEL_TCGEN05_DECODE
-        y = to_np(dp.gemm())
+        assert dp.plan.query_route(16)["kernel"] == capi.KERNEL_DIRECT
+        up = lambda n: (n + 255) // 256 * 256
+        assert capi.load().sk_w2a8_plan_storage_bytes(0, N, K, 128, capi.SK_WEIGHT_ROWMAJOR) == \
+            256 + up(N * K // 4) + up(N * (K // 128) * 2)
         cols = np.arange(0, N, 997)
         y_ref = O.w2a8_gemm_dequant_path(x_q, xs, wp[cols], ws[:, cols])
-        assert np.abs(y[:, cols] - y_ref).max() <= TOL
+        assert np.abs(to_np(dp.gemm())[:, cols] - y_ref).max() <= TOL
+        for force in ({"token_tile": 16}, {"split_k": 1}, {"persistent": 1}):
+            fresh = DeviceProblem(x_q, xs, wp, ws).force(**force)
+            q = fresh.plan.query_route(16)
+            assert q["kernel"] == want and (q["ctas"] == 2 * sms or not big)
+            assert np.abs(to_np(fresh.gemm())[:, cols] - y_ref).max() <= TOL
 
 
 @pytest.mark.parametrize("extra,K,M", [(2, 2048, 16), (9, 2048, 13), (36, 4096, 29), (44, 1024, 16), (60, 2048, 32), (41, 2048, 16)])
