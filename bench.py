@@ -246,7 +246,7 @@ def decode_sweep(dev, peaks):
                 # single launches of one plan, back to back (L2-warm, launch-bound): reported for context
                 ms_single = time_events(lambda: plans[0].gemm(x_q, xs, out=outs[0]), 50, st)
                 # the floor of this launch geometry: the same chain with an empty kernel (same grid, cluster, block,
-                # shared memory, dependent launch; barrier set-up, tensor-memory allocation, the barriers; no bytes)
+                # shared memory, dependent launch; the kernel's barriers and tensor-memory allocation, if any; no bytes)
                 for i in range(4):
                     plans[i % ncopies].launch_floor_probe(M)
                 st.synchronize()

@@ -582,17 +582,32 @@ constexpr long long kDirectQuantElements = 8192;
 // caller who rewrites the scales in stream order finds them read live everywhere else, as the general kernel does.
 static bool direct_reads_copy(const sk_w2a8_plan* plan, long long M) { return plan->G == 128 && M <= 32; }
 
+// The launch-floor probe of the direct kernel: its grid, cluster, threads and dynamic shared memory, and its barriers; nothing
+// else (it has no tensor memory to allocate; its registers, which bound the CTAs of an SM, are not imitated).
+__global__ void __launch_bounds__(256) direct_floor_kernel(const DirectParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  grid_dep_launch_dependents();
+  grid_dep_wait();
+  __syncthreads();
+  if (gridDim.z > 1) {
+    cluster_sync_all();
+    cluster_sync_all();
+  }
+  if (p.out && smem_raw[threadIdx.x] == 0xff) *static_cast<uint8_t*>(p.out) = 1;   // (never: keeps the allocation referenced)
+}
+
 template <int MT, int NT, int WARPS, int DEPTH, int MIN_CTAS, int GPB, bool LIVE, bool QUANT = false>
 static int launch_direct(sk_w2a8_plan* plan, const DirectParams& prm, int split, cudaStream_t stream) {
   using T = DirectTraits<MT, NT, WARPS, DEPTH, GPB, LIVE>;
-  auto kern = w2a8_direct_kernel<MT, NT, WARPS, DEPTH, MIN_CTAS, GPB, LIVE, QUANT>;
+  auto kern = prm.floor_probe ? direct_floor_kernel : w2a8_direct_kernel<MT, NT, WARPS, DEPTH, MIN_CTAS, GPB, LIVE, QUANT>;
   constexpr int kMaxQuant = QUANT ? static_cast<int>(kDirectQuantElements) + 8 * (128 + 16) : 0;   // (a rank's range rounds up to a block)
   if constexpr (T::kQuantOffset + kMaxQuant > 48 * 1024) {
-    static int configured_device_mask[64] = {0};
-    if (plan->device < 64 && !configured_device_mask[plan->device]) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, T::kQuantOffset + kMaxQuant);
+    static int configured_device_mask[64][2] = {};
+    if (plan->device < 64 && !configured_device_mask[plan->device][prm.floor_probe]) {
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           prm.floor_probe ? 227 * 1024 : T::kQuantOffset + kMaxQuant);
       if (e != cudaSuccess) return cuda_fail(plan, e);
-      configured_device_mask[plan->device] = 1;
+      configured_device_mask[plan->device][prm.floor_probe] = 1;
     }
   }
   cudaLaunchConfig_t cfg = {};
@@ -1581,10 +1596,18 @@ int sk_w2a8_launch_floor_probe(sk_w2a8_plan* plan, int64_t M, sk_stream_t stream
   sk::LaunchChoice ch;
   int rc = sk::resolve_launch(plan, M, false, &ch);
   if (rc != SK_OK) return rc;
-  if (ch.kernel != 3 && ch.kernel != 5) return SK_ERR_UNAVAILABLE;   // the probe mirrors the decode kernels' launch
+  if (ch.kernel != 3 && ch.kernel != 5) return SK_ERR_UNAVAILABLE;   // decode-sized calls only
   int cur = -1;
   if (cudaGetDevice(&cur) != cudaSuccess) return sk::cuda_fail(plan, cudaGetLastError());
   if (cur != plan->device && cudaSetDevice(plan->device) != cudaSuccess) return sk::cuda_fail(plan, cudaGetLastError());
+  sk::DirectChoice dc;
+  if (sk::choose_direct(plan, M, &dc)) {
+    sk::DirectParams prm = sk::direct_params(plan, M, nullptr, 0);
+    prm.floor_probe = 1;
+    rc = sk::dispatch_direct(plan, dc, prm, static_cast<cudaStream_t>(stream));
+    if (cur != plan->device) (void)cudaSetDevice(cur);
+    return rc;
+  }
   const int dyn = ch.token_tile == 16 ? sk::DecodeTraits<16>::kDynamicBytes : sk::DecodeTraits<32>::kDynamicBytes;
   static int configured[64] = {0};
   cudaError_t e = cudaSuccess;

@@ -54,6 +54,7 @@ struct DirectParams {
   int blocks_per_group;       // G / 128 (group sizes 64 and 32 are the kernel's GPB = 128 / G instead)
   int zero_point;
   int out_bf16;
+  int floor_probe;            // host: launch an empty kernel of this geometry instead
   // kernels that quantise their activations themselves (x_q, ld_x and x_scale are not used then)
   const uint16_t* x_float;    // [M, ld_float] fp16 or bf16, rows 16-byte aligned
   long long ld_float;

@@ -91,3 +91,37 @@ def test_route_keeps_what_the_tensor_memory_kernels_refuse():
                        np.ones((K // 128, 128), np.float16)).force(kernel=capi.KERNEL_DIRECT)
     with pytest.raises(capi.SkError):
         dp.gemm()
+
+
+def _captured_launches(fn):
+    """(grid, block, dynamic shared memory) of the kernels that fn launches, from a captured graph."""
+    from cuda.bindings import driver
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        fn()
+    handle = driver.CUgraph(init_value=graph.raw_cuda_graph())
+    _, _, count = driver.cuGraphGetNodes(handle)
+    _, nodes, count = driver.cuGraphGetNodes(handle, count)
+    out = []
+    for node in nodes[:count]:
+        err, p = driver.cuGraphKernelNodeGetParams(node)
+        assert int(err) == 0
+        out.append(((p.gridDimX, p.gridDimY, p.gridDimZ), p.blockDimX, p.sharedMemBytes))
+    return out
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 4096, 11008), (8, 4096, 4096), (16, 12288, 4096), (24, 4096, 4096), (8, 57344, 512),
+                                   (16, 57344, 512)])
+def test_launch_floor_probe_has_the_geometry_of_the_launch_it_stands_for(M, N, K):
+    from slimkernels_b200.torch import W2A8Plan
+    x_q = torch.zeros(M, K, dtype=torch.int8, device="cuda")
+    xs = torch.ones(M, device="cuda")
+    out = torch.empty(M, N, dtype=torch.float16, device="cuda")
+    plan = W2A8Plan(torch.zeros(N, K // 4, dtype=torch.uint8, device="cuda"), torch.ones(K // 128, N, dtype=torch.float16, device="cuda"))
+    assert plan.query_route(M)["kernel"] == capi.KERNEL_DIRECT
+    plan.gemm(x_q, xs, out=out)
+    plan.launch_floor_probe(M)
+    torch.cuda.synchronize()
+    assert _captured_launches(lambda: plan.launch_floor_probe(M)) == _captured_launches(lambda: plan.gemm(x_q, xs, out=out))
+    with pytest.raises(RuntimeError):
+        plan.launch_floor_probe(4096)
