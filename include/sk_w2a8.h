@@ -116,7 +116,7 @@ int sk_w2a8_plan_create(sk_w2a8_plan** plan, int device, int64_t N, int64_t K, i
  * the plan is destroyed and every launch made with it has completed) and without synchronising: the copies are made on
  * `stream`, and the plan may be used there at once.  Use on another stream must be ordered after it by the caller.
  * (So must sk_w2a8_last_device_status, which reads outside any stream: wait for `stream` first.)
- * Creation and destruction neither allocate nor free device memory. */
+ * Creation and destruction neither allocate nor free device memory.  The size is 0 for shapes that a plan refuses. */
 int64_t sk_w2a8_plan_storage_bytes(int device, int64_t N, int64_t K, int group_size, int w_layout);
 int sk_w2a8_plan_create_in(sk_w2a8_plan** plan, int device, int64_t N, int64_t K, int group_size, int zero_point,
                            const uint8_t* w, int w_layout, const void* w_scale_f16, int out_dtype, void* storage,

@@ -1237,6 +1237,12 @@ static int repack_common(bool forward, const uint8_t* src, long long N, long lon
 // ================================================================================================
 // extern "C"
 // ================================================================================================
+static bool plan_shape_ok(int64_t N, int64_t K, int group_size) {
+  if (N <= 0 || K <= 0 || N > (1LL << 30) || K > (1LL << 30)) return false;
+  if (group_size <= 0 || (group_size % 32) != 0 || (K % group_size) != 0 || (K % 32) != 0) return false;
+  return (group_size % 128) == 0 || (128 % group_size) == 0;
+}
+
 // Plan creation behind both entry points.  storage == nullptr: one cudaMalloc'ed block, the work on the legacy default
 // stream, and the device synchronised before it returns.  Otherwise the caller's block, the work ordered on `stream`, and
 // no synchronisation.
@@ -1246,9 +1252,7 @@ static int plan_create_common(sk_w2a8_plan** out, int device, int64_t N, int64_t
   if (!out) return SK_ERR_NULL_POINTER;
   *out = nullptr;
   if (!w || !w_scale_f16) return SK_ERR_NULL_POINTER;
-  if (N <= 0 || K <= 0 || N > (1LL << 30) || K > (1LL << 30)) return SK_ERR_BAD_SHAPE;
-  if (group_size <= 0 || (group_size % 32) != 0 || (K % group_size) != 0 || (K % 32) != 0) return SK_ERR_BAD_SHAPE;
-  if (!((group_size % 128) == 0 || (128 % group_size) == 0)) return SK_ERR_BAD_SHAPE;
+  if (!plan_shape_ok(N, K, group_size)) return SK_ERR_BAD_SHAPE;
   if (zero_point < 0 || zero_point > 3) return SK_ERR_BAD_ARGUMENT;
   if (out_dtype != SK_OUT_F16 && out_dtype != SK_OUT_BF16) return SK_ERR_BAD_ARGUMENT;
   if (w_layout != SK_WEIGHT_ROWMAJOR && w_layout != SK_WEIGHT_TILED) return SK_ERR_BAD_ARGUMENT;
@@ -1375,7 +1379,7 @@ int sk_w2a8_plan_create(sk_w2a8_plan** out, int device, int64_t N, int64_t K, in
 }
 
 int64_t sk_w2a8_plan_storage_bytes(int device, int64_t N, int64_t K, int group_size, int w_layout) {
-  if (N <= 0 || K <= 0 || N > (1LL << 30) || K > (1LL << 30) || group_size <= 0) return 0;
+  if (!plan_shape_ok(N, K, group_size)) return 0;
   sk_w2a8_plan probe;
   if (cudaDeviceGetAttribute(&probe.sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
     (void)cudaGetLastError();

@@ -129,7 +129,7 @@ int64_t plan_create(const at::Tensor& w, const at::Tensor& w_scale, int64_t N, i
                     cudaStreamWaitEvent(stream.stream(), t->filled, 0) == cudaSuccess,
                 "slimkernels::w2a8_plan_create: waiting for the default stream failed");
   t->borrowed = {w.storage().getWeakStorageImpl(), w_scale.storage().getWeakStorageImpl()};
-  // (arguments the plan refuses are refused before the storage is asked for)
+  // (0 for shapes that a plan refuses: the call below does, and no storage to speak of is asked for)
   const int64_t bytes = std::max<int64_t>(256, sk_w2a8_plan_storage_bytes(w.get_device(), N, K, static_cast<int>(group_size), layout));
   t->storage = at::empty({bytes}, w.options().dtype(at::kByte));     // caching allocator: 512-byte aligned
   check(sk_w2a8_plan_create_in(&t->plan, w.get_device(), N, K, static_cast<int>(group_size), static_cast<int>(zero_point),

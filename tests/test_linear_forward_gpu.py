@@ -192,6 +192,18 @@ def test_dropping_a_captured_plan_waits_for_the_graphs_that_use_it():
     assert side.query() and torch.equal(y, want)
 
 
+def test_shapes_a_plan_refuses_need_no_storage():
+    from slimkernels_b200 import capi
+    from slimkernels_b200.torch import W2A8Plan
+    size = capi.load().sk_w2a8_plan_storage_bytes
+    assert size(0, 128, 192, 64, capi.SK_WEIGHT_ROWMAJOR) > 0
+    for K, G in ((192, 96), (192, 48), (192, 128), (192, 0), (192, -64), (0, 64)):
+        assert size(0, 128, K, G, capi.SK_WEIGHT_ROWMAJOR) == 0
+    with pytest.raises(RuntimeError):
+        W2A8Plan(torch.zeros(128, 48, dtype=torch.uint8, device="cuda"), torch.ones(2, 128, dtype=torch.float16, device="cuda"),
+                 group_size=96)
+
+
 def test_plan_is_refused_under_capture():
     lin = _linear(256, 256)
     x = torch.randn(2, 256, device="cuda").half()
