@@ -26,18 +26,25 @@ from gpu_util import DeviceProblem, random_problem, to_np  # noqa: E402
                                  (32, 32), (32, 352), (32, 1120)])
 @pytest.mark.parametrize("M,N", [(1, 5), (8, 130), (9, 64), (16, 392), (17, 128), (24, 257), (32, 1000), (33, 40), (70, 200)])
 def test_exact_integers(G, K, M, N):
-    """Scales 1 and small activations: every output is an integer that fp16 holds exactly, so the comparison is exact."""
+    """Scales 1 and 2 and small activations: every output is an integer that fp16 holds exactly, so the comparison is exact.
+    Deep K has 340 activations of -1 or 1 per token, anywhere in it and some in its last group."""
     rng = np.random.default_rng(M * N + K + G)
-    lim = max(1, min(127, 2048 // (3 * K)))
+    lim = max(1, min(127, 2048 // (6 * K)))                        # |sum| <= 6 K lim or 6 * 340, below 2048
     x_q = rng.integers(-lim, lim + 1, size=(M, K), dtype=np.int8)
-    if lim == 1:
-        x_q[:, 600:] = 0                                           # keep |sum| below 2048
+    if 6 * K * lim > 2048:
+        x_q[:] = 0
+        for row in x_q:
+            at = rng.permutation(K)[:332]
+            row[at] = rng.choice([-1, 1], size=332)
+            row[K - G + rng.permutation(G)[:8]] = rng.choice([-1, 1], size=8)
     wp = rng.integers(0, 256, size=(N, K // 4), dtype=np.uint8)
-    ws = np.ones((K // G, N), dtype=np.float16)
+    ws = rng.integers(1, 3, size=(K // G, N)).astype(np.float16)
     zp = int(rng.integers(0, 4))
     dp = DeviceProblem(x_q, np.ones(M, dtype=np.float32), wp, ws, G, zp).force(kernel=capi.KERNEL_DIRECT)
     assert dp.plan.query_route(M)["kernel"] == capi.KERNEL_DIRECT
-    want = x_q.astype(np.int64) @ (O.unpack_matrix(wp).astype(np.int64) - zp).T
+    weights = (O.unpack_matrix(wp).astype(np.int64) - zp) * ws.astype(np.int64).repeat(G, axis=0).T
+    want = x_q.astype(np.int64) @ weights.T
+    assert np.abs(want).max() <= 2048
     y = to_np(dp.gemm(ld_out=N + 3))
     np.testing.assert_array_equal(y[:, :N], want.astype(np.float32))
     assert np.isnan(y[:, N:]).all(), "wrote outside the N columns"
@@ -53,6 +60,22 @@ def test_scales_against_the_oracle_and_repeated_launches(G, M, N, K):
     ref = O.w2a8_gemm_int_path(x_q, xs, wp, ws, G)
     assert np.abs(to_np(y) - ref).max() <= 2.0 ** -10 * max(1.0, np.abs(ref).max())      # an fp16 ulp at the largest value
     assert torch.equal(dp.gemm(), y) and torch.equal(dp.force(kernel=capi.KERNEL_DIRECT, dependent_launch=1).gemm(), y)
+
+
+@pytest.mark.parametrize("G,K", [(64, 4160), (64, 11072), (32, 4128), (32, 11040), (128, 8320), (256, 8448)])
+@pytest.mark.parametrize("M,N", [(1, 72), (13, 136), (24, 40), (31, 200)])
+def test_deep_ragged_k_and_every_split(G, K, M, N):
+    """K that ends inside a block (group sizes 64 and 32) or leaves the warps and CTAs of a split uneven shares, every ring slot
+    used several times: full-range activations and random scales, the K split chosen and forced."""
+    x_q, xs, wp, ws = random_problem(M, N, K, G, seed=K + M)
+    ref = O.w2a8_gemm_int_path(x_q, xs, wp, ws, G)
+    bound = 2.0 ** -10 * max(1.0, np.abs(ref).max())               # an fp16 ulp at the largest value, as above
+    dp = DeviceProblem(x_q, xs, wp, ws, G)
+    for split in (0, 1, 2, 4, 8):
+        dp.force(kernel=capi.KERNEL_DIRECT, split_k=split)
+        q = dp.plan.query_route(M)
+        assert q["kernel"] == capi.KERNEL_DIRECT and (q["split_k"] == split if split else q["split_k"] > 1)
+        assert np.abs(to_np(dp.gemm()) - ref).max() <= bound
 
 
 def test_extreme_operands_and_bf16():

@@ -169,7 +169,8 @@ def test_balanced_split_is_the_tcgen05_choice_for_large_decode_problems():
             assert np.abs(to_np(fresh.gemm())[:, cols] - y_ref).max() <= TOL
 
 
-@pytest.mark.parametrize("extra,K,M", [(2, 2048, 16), (9, 2048, 13), (36, 4096, 29), (44, 1024, 16), (60, 2048, 32), (41, 2048, 16)])
+@pytest.mark.parametrize("extra,K,M", [(2, 2048, 16), (9, 2048, 13), (36, 4096, 29), (44, 1024, 16), (60, 2048, 32), (41, 2048, 16),
+                                       (60, 4096, 32)])
 def test_decode_kernel_mixed_launch_when_there_are_more_tiles_than_sms(extra, K, M):
     """More feature tiles than SMs (but fewer than CTA slots): one CTA per tile for one tile per SM, the tiles beyond
     that split 4 ways (few of them) or 2 ways (an even number of them) inside clusters of four."""
@@ -189,6 +190,13 @@ def test_decode_kernel_mixed_launch_when_there_are_more_tiles_than_sms(extra, K,
         want = 1
     assert q["kernel"] == capi.KERNEL_TCGEN05_DECODE and q["split_k"] == want
     assert q["ctas"] == (tiles1 + extra * want if want > 1 else n_tiles)
+    # without options this kernel runs 25 .. 32 tokens on large weights, the direct kernel the rest
+    default = M > 24 and n_tiles * (K // 128) >= 24 * sms
+    assert (dp.plan.query_route(M) == q) == default
+    if not default:
+        assert dp.plan.query_route(M)["kernel"] == capi.KERNEL_DIRECT
+        dp.force(kernel=capi.KERNEL_TCGEN05_DECODE)
+        assert dp.plan.query_route(M) == q
     y = dp.gemm()
     cols = np.unique(np.concatenate([np.arange(0, N, 701), np.arange(tiles1 * 128 - 64, N)]))   # incl. every split tile
     y_ref = O.w2a8_gemm_dequant_path(x_q, xs, wp[cols], ws[:, cols])
@@ -199,11 +207,14 @@ def test_decode_kernel_mixed_launch_when_there_are_more_tiles_than_sms(extra, K,
     assert np.abs(to_np(y) - to_np(y_plain)).max() <= 4e-3 * max(1.0, float(np.abs(y_ref).max()))
 
 
-def test_decode_kernel_is_the_default_for_small_batches():
+def test_decode_kernel_is_the_tcgen05_choice_for_small_batches():
     x_q, xs, wp, ws = random_problem(8, 512, 2048, 128, seed=3)
     dp = DeviceProblem(x_q, xs, wp, ws)
     assert dp.plan.query_launch(8)["kernel"] == capi.KERNEL_TCGEN05_DECODE
     assert dp.plan.query_launch(64)["kernel"] == capi.KERNEL_TCGEN05
+    assert dp.plan.query_route(8)["kernel"] == capi.KERNEL_DIRECT  # which runs when nothing is forced
+    dp.force(kernel=capi.KERNEL_TCGEN05_DECODE)
+    assert dp.plan.query_route(8)["kernel"] == capi.KERNEL_TCGEN05_DECODE
     y = to_np(dp.gemm())
     y_general = to_np(dp.force(kernel=capi.KERNEL_TCGEN05).gemm())
     y_ref = O.w2a8_gemm_dequant_path(x_q, xs, wp, ws)
