@@ -490,11 +490,11 @@ int64_t cached_plan(const at::Tensor& w_packed, const at::Tensor& w_scale, int64
     ++i;
   }
   if (hit) return hit;
-  if (g_cache.size() >= kMaxCachedPlans) {      // oldest first
+  const int64_t handle = plan_create(w_packed, w_scale, N, K, group_size, zero_point, bf16, /*tiled=*/false);
+  if (g_cache.size() >= kMaxCachedPlans) {      // oldest first (not before plan_create has refused a capture)
     plan_destroy(g_cache.front().plan);
     g_cache.erase(g_cache.begin());
   }
-  const int64_t handle = plan_create(w_packed, w_scale, N, K, group_size, zero_point, bf16, /*tiled=*/false);
   CachedPlan e{c10::weak_intrusive_ptr<c10::TensorImpl>(w_packed.getIntrusivePtr()),
                c10::weak_intrusive_ptr<c10::TensorImpl>(w_scale.getIntrusivePtr()),
                w_packed.data_ptr(), w_scale.data_ptr(), w_packed._version(), w_scale._version(),
