@@ -20,6 +20,8 @@
 
 namespace sk {
 
+constexpr int kChipSms = 148;    // a B200's SMs, for grids and rules that no plan (which asks the device) belongs to
+
 // ------------------------------------------------------------------------------------------------
 // Tiled weight order.  Block (tile T, k-block B) is 4096 bytes at ((T * k_blocks + B) * 4096); inside it the
 // 32-bit word for (row r, 16-code chunk c) sits at byte (c / 4) * 2048 + r * 16 + (c % 4) * 4 and holds
@@ -240,7 +242,7 @@ struct sk_w2a8_plan {
   int device = 0;
   long long N = 0, K = 0;
   int G = 128, zero_point = 1, out_dtype = SK_OUT_F16;
-  int k_blocks = 0, n_tiles = 0, sm_count = 148;
+  int k_blocks = 0, n_tiles = 0, sm_count = sk::kChipSms;
   const uint8_t* w_rowmajor = nullptr;  // borrowed (may be null when created from a tiled buffer)
   const uint8_t* w_tiled = nullptr;     // in the plan's storage, or borrowed
   const __half* w_scale = nullptr;      // borrowed
@@ -1184,7 +1186,7 @@ static int run_gemm(sk_w2a8_plan* plan, long long M, const int8_t* x_q, long lon
         else rc = dispatch_umma_dump(plan, ch.token_tile, map, extra_maps, prm, m_tiles, stream);
         if (rc == SK_OK) {
           const long long mn = M * plan->N;
-          const int blocks = static_cast<int>(mn / 256 + 1 < 148 * 8 ? mn / 256 + 1 : 148 * 8);
+          const int blocks = static_cast<int>(mn / 256 + 1 < sk::kChipSms * 8 ? mn / 256 + 1 : sk::kChipSms * 8);
           diff_partials_kernel<<<blocks, 256, 0, stream>>>(partials, prm.groups, mn, acc_bufs_of(ch.token_tile, ch.kernel));
           e = cudaGetLastError();
           if (e != cudaSuccess) rc = cuda_fail(plan, e);
@@ -1221,7 +1223,7 @@ static int repack_common(bool forward, const uint8_t* src, long long N, long lon
   const long long total_words = n_tiles * k_blocks * 1024;
   const int threads = 256;
   const long long want = (total_words + threads - 1) / threads;
-  const int blocks = static_cast<int>(want < 148 * 16 ? want : 148 * 16);
+  const int blocks = static_cast<int>(want < sk::kChipSms * 16 ? want : sk::kChipSms * 16);
   if (forward)
     repack_kernel<<<blocks, threads, 0, stream>>>(src, reinterpret_cast<uint32_t*>(dst), N, K, k_blocks, total_words);
   else
@@ -1317,7 +1319,7 @@ static int plan_create_common(sk_w2a8_plan** out, int device, int64_t N, int64_t
     }
     if (rc == SK_OK && e == cudaSuccess && !scales_tiled) {
       const long long total = static_cast<long long>(plan->n_tiles) * plan->k_blocks * sk::kTileN;
-      const int blocks = static_cast<int>(total / 256 + 1 < 148 * 8 ? total / 256 + 1 : 148 * 8);
+      const int blocks = static_cast<int>(total / 256 + 1 < sk::kChipSms * 8 ? total / 256 + 1 : sk::kChipSms * 8);
       sk::tile_scales_kernel<<<blocks, 256, 0, stream>>>(plan->w_scale, plan->w_scale_tiled, N, plan->k_blocks, total);
       e = cudaGetLastError();
     }
@@ -1788,7 +1790,7 @@ int sk_quantize_activation_int8_from(const void* x, int x_bf16, int64_t ld_x, in
                                                                                         : sk::quantize_activation_kernel<8, true>)
                      : (vecs == 2 ? sk::quantize_activation_kernel<2, false> : vecs == 4 ? sk::quantize_activation_kernel<4, false>
                                                                                          : sk::quantize_activation_kernel<8, false>);
-  if (M <= 2 * 148 && K > 8 * sk::kActThreads) {      // few rows: more threads per row
+  if (M <= 2 * sk::kChipSms && K > 8 * sk::kActThreads) {      // few rows: more threads per row
     const bool half = K <= 8 * 512;
     cfg.blockDim = dim3(half ? 512 : 1024, 1, 1);
     kern = x_bf16 ? (half ? sk::quantize_activation_kernel<1, true, 512> : sk::quantize_activation_kernel<2, true, 1024>)
@@ -1815,7 +1817,7 @@ int sk_silu_mul_quantize_int8(const void* gate_up_f16, int64_t ld_gu, int64_t M,
   // idle instead: then up to eight CTAs, one vector per thread.
   const long long per_cta = 8LL * sk::kActThreads * sk::kClusterVecs;
   int csize = static_cast<int>(I / per_cta < 8 ? (I + per_cta - 1) / per_cta : 9);
-  if (csize <= 8 && M * 8 <= 148) csize = static_cast<int>((I + 8LL * sk::kActThreads - 1) / (8LL * sk::kActThreads));
+  if (csize <= 8 && M * 8 <= sk::kChipSms) csize = static_cast<int>((I + 8LL * sk::kActThreads - 1) / (8LL * sk::kActThreads));
   if (csize > 8) csize = 8;
   if (I <= per_cta * csize) {
     for (int64_t m0 = 0; m0 < M; m0 += 65535) {       // gridDim.y holds at most 65535 rows per launch
@@ -2018,7 +2020,7 @@ int sk_sum_row_blocks(const void* blocks, int n_blocks, int64_t block_stride, in
   const long long total = rows * (N / 8);
   const int threads = 256;
   const long long want = (total + threads - 1) / threads;
-  const int grid = static_cast<int>(want < 148 * 16 ? want : 148 * 16);
+  const int grid = static_cast<int>(want < sk::kChipSms * 16 ? want : sk::kChipSms * 16);
   const auto st = static_cast<cudaStream_t>(stream);
   if (out_dtype == SK_OUT_BF16)
     sk::sum_row_blocks_kernel<true><<<grid, threads, 0, st>>>(static_cast<const uint16_t*>(blocks), block_stride, ld, n_blocks,

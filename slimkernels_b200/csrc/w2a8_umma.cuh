@@ -182,12 +182,13 @@ struct KernelTraits {
   // so the budgets must add up to no more than the pool or the kernel hangs:
   //   BLOCK_M 256, 4 expander warps: 512 threads, 128 at launch -> epilogue 224, expanders 32, control 32
   //   BLOCK_M 256, 2 expander warps: 384 threads, 168 at launch -> epilogue 224, expanders + control 56
-  //   BLOCK_M 128:                   512 threads, 128 at launch -> epilogue 168, others 88
+  //   BLOCK_M 128, 8 expander warps: 640 threads, 96 at launch -> epilogue 168, others 48
+  //   BLOCK_M 128, 4 (persistent):   512 threads, 128 at launch -> epilogue 168, others 88
   static constexpr bool kUseSetMaxNReg = (EPI_WGS == 2);
   static constexpr int kLaunchRegs = (65536 / kThreads) / 8 * 8;
   static constexpr bool kBig = kColsPerWg > 96;
   static constexpr int kEpiRegs = kBig ? 224 : 168;
-  static constexpr int kOtherRegs = EXP_WARPS == 8 ? 48 : 88;             // (640 threads, 96 at launch -> epilogue 168, others 48)
+  static constexpr int kOtherRegs = EXP_WARPS == 8 ? 48 : 88;
   static constexpr int kExpRegs = kBig ? 32 : kOtherRegs;                 // warpgroup holding the expander warps
   static constexpr int kCtlRegs = kBig ? (kThreads == 384 ? 56 : 32) : kOtherRegs;   // warpgroup holding producer + MMA warps
   static constexpr int kExpWgThreads = (EXP_WARPS == 4) ? 128 : 0;        // expanders have a warpgroup of their own
