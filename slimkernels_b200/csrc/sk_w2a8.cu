@@ -1668,7 +1668,6 @@ const char* sk_device_status_string(int device_status) {
     case sk::kStMmaAccEmpty: return "MMA issuer: an accumulator buffer was never released by the epilogue";
     case sk::kStEpilogueAccFull: return "epilogue: the MMAs of a scale group never completed";
     case sk::kStEpilogueScales: return "epilogue: the copy of the group scales never landed";
-    case sk::kStScalesEmpty: return "scale warp: a half of the coefficient ring was never released by the epilogue";
     case sk::kStDrain: return "producer: a copy in flight did not land while the CTA was giving up";
     case sk::kStStreamSlots: return "epilogue: a tile is shared by more CTAs than the scratch buffer has slots for";
     default: return "unknown device status";

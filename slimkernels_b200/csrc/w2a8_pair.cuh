@@ -92,8 +92,6 @@ __device__ __forceinline__ bool wait_bounded_cluster(uint32_t bar, uint32_t pari
   return ok;
 }
 
-constexpr int kScalePrefetchGroups = 8;   // group scales are pulled into L2 this many groups before they are loaded
-
 template <int STAGES>
 struct PairTraits {
   static constexpr int kTokens = 256;                 // tokens of the pair's tile (MMA N)

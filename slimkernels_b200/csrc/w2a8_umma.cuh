@@ -52,8 +52,7 @@ constexpr int kBlockK = 128;         // K codes per pipeline stage (= one 128-by
 constexpr int kWpBytes = kTileN * kBlockK / 4;   // 4096: tiled 2-bit block
 constexpr int kWxBytes = kTileN * kBlockK;       // 16384: expanded int8 block
 constexpr long long kWaitLimitCycles = 1000000000ll;  // default: every mbarrier wait gives up after 1e9 SM cycles (0.5-0.8 s)
-constexpr int kScaleHalf = 8;         // scale groups per half of the coefficient ring
-constexpr int kScaleSlots = 2 * kScaleHalf;
+constexpr int kScalePrefetchGroups = 8;   // group scales are pulled into L2 this many groups before they are loaded
 constexpr int kBiasFlushGroups = 16;  // the bias term is subtracted from the accumulators this often
 
 // device status codes: role * 16 + barrier kind
@@ -63,7 +62,6 @@ enum : int {
   kStMmaLdFull = 0x31, kStMmaExFull = 0x32, kStMmaAccEmpty = 0x33,
   kStEpilogueAccFull = 0x41, kStEpilogueScales = 0x42,
   kStDrain = 0x51,
-  kStScalesEmpty = 0x71,
   kStStreamSlots = 0x61   // balanced-split decode kernel: host and device disagree on how a tile is cut (never expected)
 };
 
@@ -129,7 +127,7 @@ template <int BLOCK_M, int EPI_WGS, int EXP_WARPS, int LSTAGES, int ESTAGES, int
           bool PERSIST = false>
 struct KernelTraits {
   static constexpr int kEpiWarps = EPI_WGS * 4;
-  static constexpr int kWarps = ((kEpiWarps + EXP_WARPS + 4 + 3) / 4) * 4;   // whole warpgroups
+  static constexpr int kWarps = ((kEpiWarps + EXP_WARPS + 2 + 3) / 4) * 4;   // whole warpgroups
   static constexpr int kThreads = kWarps * 32;
   static constexpr int kEpiThreads = EPI_WGS * 128;
   static constexpr int kExpThreads = EXP_WARPS * 32;
@@ -159,11 +157,10 @@ struct KernelTraits {
   static constexpr int kStageBytes = kStageTokens * kTileN * 2;                  // 16 KB per warpgroup
   static constexpr int kOffStage = kOffWp + LSTAGES * kWpBytes;
   static constexpr int kOffBar = kOffStage + (PERSIST ? EPI_WGS * kStageBytes : 0);
-  static constexpr int kNumBars = 2 * LSTAGES + 2 * ESTAGES + 2 * ACC_BUFS + 4;
+  static constexpr int kNumBars = 2 * LSTAGES + 2 * ESTAGES + 2 * ACC_BUFS;
   static constexpr int kOffMisc = kOffBar + kNumBars * 8;
   static constexpr int kOffXs = kOffMisc + 16;                   // fp32 [2][BLOCK_M]: x_scale of the tile's tokens
-  static constexpr int kOffCoef = kOffXs + 2 * BLOCK_M * 4;      // fp32 [kScaleSlots][128]: the groups' coefficients
-  static constexpr int kTotal = kOffCoef + kScaleSlots * kTileN * 4;
+  static constexpr int kTotal = kOffXs + 2 * BLOCK_M * 4;
   static constexpr int kDynamicBytes = kTotal + 1024;            // slack for 1024-byte alignment of the base
   // After the main loop the operand ring is dead and is reused for the output tile
   // (fp32 [BLOCK_M][128] for the split-K reduction, 16-bit [BLOCK_M][128] otherwise).
@@ -206,8 +203,7 @@ struct KernelTraits {
   static constexpr bool kDoubleBuf = (kNumChunks > 1);
   static constexpr int kMinBlocks = (BLOCK_M <= 32) ? 2 : 1;
   static_assert(kMinBlocks * kThreads <= 2048, "threads per SM");
-  static_assert(kEpiWarps + EXP_WARPS + 4 <= kWarps, "room for the producer, two MMA-issuing warps and the scale warp");
-  static_assert(kOffCoef % 16 == 0 && kMinBlocks * kDynamicBytes <= 227 * 1024, "shared memory");
+  static_assert(kEpiWarps + EXP_WARPS + 3 <= kWarps, "room for the producer warp and two MMA-issuing warps");
 };
 
 struct WaitCtx {
@@ -344,7 +340,6 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
   constexpr int kExpWarp0 = T::kEpiWarps;       // first expander warp
   constexpr int kProducerWarp = kExpWarp0 + EXP_WARPS;
   constexpr int kMmaWarp = kProducerWarp + 1;
-  constexpr int kScaleWarp = kMmaWarp + 2;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -357,8 +352,6 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
   const uint32_t bar_ex_empty = bar_ex_full + 8u * ESTAGES;      // used only when the rings are not tied
   const uint32_t bar_acc_full = bar_ex_empty + 8u * ESTAGES;
   const uint32_t bar_acc_empty = bar_acc_full + 8u * ACC_BUFS;
-  const uint32_t bar_sc_full = bar_acc_empty + 8u * ACC_BUFS;    // halves of the coefficient ring
-  const uint32_t bar_sc_empty = bar_sc_full + 16u;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + T::kOffMisc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + T::kOffMisc + 4);
   const WaitCtx ctx{abort_flag, p.status, p.wait_limit};
@@ -408,7 +401,6 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       mbar_init(bar_ex_empty + 8 * i, readers);    // commit of the MMAs that read them (untied rings only)
     }
     for (int i = 0; i < ACC_BUFS; ++i) { mbar_init(bar_acc_full + 8 * i, 1); mbar_init(bar_acc_empty + 8 * i, T::kEpiWarps); }
-    for (int i = 0; i < 2; ++i) { mbar_init(bar_sc_full + 8 * i, 1); mbar_init(bar_sc_empty + 8 * i, T::kEpiWarps); }
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -646,59 +638,6 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         }
       }
       __syncwarp();
-    } else if (warp == kScaleWarp) {
-      // ============================================================ scale coefficients
-      // What the epilogue multiplies group g's running sums by, (s_g - s_{g+ACC_BUFS}) * 2^100 (s = 0 past the end of the
-      // range and past N), into a ring of two halves of kScaleHalf groups.  A lane takes four features.
-      // With the epilogue's threads loading their own scales a group ahead, every group waited for an L2 round trip
-      // (shifting a register ring moves the register that the load is still to fill).
-      const float kScaleUp = 1.2676506002282294e30f;     // 2^100
-      uint32_t fill = 0;                                 // halves filled so far
-      bool ok = true;
-      for (int tile = tile_first; tile < tile_end && ok; tile += tile_step) {
-        const int n = tile_coord(tile, p.n_tiles, p.num_tiles).n_tile * kTileN + 4 * lane;
-        const __half* col = p.w_scale + n;
-        const bool vec = (p.N & 3) == 0 && (reinterpret_cast<uintptr_t>(p.w_scale) & 7) == 0;
-        auto row = [&](int g) -> uint2 {
-          uint2 v = make_uint2(0u, 0u);
-          if (g < g_end && n < p.N) {
-            const __half* src = col + static_cast<size_t>(g) * p.N;
-            if (vec) {
-              v = ld_global_v2(src);
-            } else {
-              uint32_t h[4];
-#pragma unroll
-              for (int i = 0; i < 4; ++i) h[i] = n + i < p.N ? ld_global_u16(src + i) : 0u;
-              v = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
-            }
-          }
-          return v;
-        };
-        for (int g0 = g_begin; g0 < g_end && ok; g0 += kScaleHalf, ++fill) {
-          const uint32_t half = fill & 1;
-          // (twice the limit: where copies never come, a role that waits for them says so first)
-          ok = wait_bounded_relaxed(bar_sc_empty + 8 * half, ((fill >> 1) & 1) ^ 1, WaitCtx{abort_flag, p.status, 2 * p.wait_limit},
-                                    kStScalesEmpty, 200);
-          if (!ok) break;
-          float* dst = reinterpret_cast<float*>(smem + T::kOffCoef) + half * kScaleHalf * kTileN + 4 * lane;
-#pragma unroll 1
-          for (int i = 0; i < kScaleHalf && g0 + i < g_end; i += 2) {
-            uint2 a[2], b[2];
-#pragma unroll
-            for (int j = 0; j < 2; ++j) { a[j] = row(g0 + i + j); b[j] = row(g0 + i + j + ACC_BUFS); }
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-              const float2 a0 = __half22float2(*reinterpret_cast<const __half2*>(&a[j].x)), a1 = __half22float2(*reinterpret_cast<const __half2*>(&a[j].y));
-              const float2 b0 = __half22float2(*reinterpret_cast<const __half2*>(&b[j].x)), b1 = __half22float2(*reinterpret_cast<const __half2*>(&b[j].y));
-              *reinterpret_cast<float4*>(dst + (i + j) * kTileN) =
-                  make_float4((a0.x - b0.x) * kScaleUp, (a0.y - b0.y) * kScaleUp, (a1.x - b1.x) * kScaleUp, (a1.y - b1.y) * kScaleUp);
-            }
-          }
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar_sc_full + 8 * half);
-        }
-      }
-      __syncwarp();
     } else if (warp < kProducerWarp) {
       // ============================================================ expanders (one or two weight rows per thread)
       const int exp_group = (warp - kExpWarp0) / (EXP_WARPS / T::kExpGroups);
@@ -799,6 +738,7 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     const int row = (warp & 3) * 32 + lane;      // output feature within the tile == TMEM lane
     const int col0 = wg * kCols;                 // first token column of this thread
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + col0;
+    const float kScaleUp = 1.2676506002282294e30f;     // 2^100
     const float bias_f = __uint_as_float(bias);        // bias * 2^-149
 
     // pre-set every accumulator buffer to the bias and hand them to the MMA issuer
@@ -815,7 +755,7 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       for (int a = 0; a < ACC_BUFS; ++a) mbar_arrive(bar_acc_empty + 8 * a);
     }
     int ab = 0, tile_parity = 0;
-    uint32_t aph = 0, sc_fill = 0;
+    uint32_t aph = 0;
     bool epi_ok = true;
 
     for (int tile = tile_first; tile < tile_end && epi_ok; tile += tile_step) {
@@ -838,7 +778,27 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       tile_parity ^= 1;
     }
 
-    const uint32_t coef = smem_base + T::kOffCoef + 4 * row;     // this feature's coefficients, see the scale warp
+    // group scales s_g .. s_{g+ACC_BUFS} in a register ring, loaded one group ahead of their first use (0 past the
+    // end).  The ring keeps the raw fp16 bits: converting at load time would stall on the global load right away.
+    // A load that misses L2 would still stall the loop one group later (the ring is shifted by register moves), so
+    // every row is pulled into L2 kScalePrefetchGroups groups earlier with a prefetch, which occupies no register.
+    const unsigned short* sp =
+        pointer_from_here(reinterpret_cast<const unsigned short*>(p.w_scale)) + static_cast<size_t>(g_begin) * p.N + (n_ok ? n : 0);
+    int g_load = g_begin;                       // next group whose scale is fetched
+    auto load_scale = [&]() -> unsigned short {
+      const unsigned short r = (n_ok && g_load < g_end) ? *sp : static_cast<unsigned short>(0);
+#ifndef SK_NO_SCALE_PREFETCH
+      if (g_load + kScalePrefetchGroups < g_end)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(sp + static_cast<size_t>(kScalePrefetchGroups) * p.N));
+#endif
+      sp += p.N; ++g_load;
+      return r;
+    };
+    for (int i = ACC_BUFS + 1; i < kScalePrefetchGroups && g_begin + i < g_end; ++i)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(sp + static_cast<size_t>(i) * p.N));
+    unsigned short sr[ACC_BUFS + 1];
+#pragma unroll
+    for (int i = 0; i <= ACC_BUFS; ++i) sr[i] = load_scale();
     float s_sum = 0.f;   // sum of the coefficients since the last bias flush
     int flush = 0;
     // TMEM loads are software-pipelined across the chunks of a group: while chunk c is consumed the load of chunk
@@ -850,17 +810,10 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
 #pragma unroll 1
     for (int g = g_begin; g < g_end && epi_ok; ++g) {
       // coefficient of this group's running sum
-      const int sc = (g - g_begin) & (kScaleHalf - 1);
-      if (sc == 0) {
-        epi_ok = wait_bounded(bar_sc_full + 8 * (sc_fill & 1), (sc_fill >> 1) & 1, ctx, kStEpilogueScales);
-        if (!epi_ok) break;
-      }
-      const float s2 = ld_shared_f32(coef + ((sc_fill & 1) * kScaleHalf + sc) * (kTileN * 4));
-      if (sc == kScaleHalf - 1 || g == g_end - 1) {        // the half is read: hand it back
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar_sc_empty + 8 * (sc_fill & 1));
-        ++sc_fill;
-      }
+      const float s2 = (__half2float(__ushort_as_half(sr[0])) - __half2float(__ushort_as_half(sr[ACC_BUFS]))) * kScaleUp;
+#pragma unroll
+      for (int i = 0; i < ACC_BUFS; ++i) sr[i] = sr[i + 1];
+      sr[ACC_BUFS] = load_scale();
       const uint32_t buf = lane_addr + ab * BLOCK_M;
       // the last groups of a tile keep their buffers until these are back at the bias for the next tile (below)
       const bool keep_buf = more_tiles && g >= g_end - ACC_BUFS;
