@@ -41,8 +41,6 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
-#include <type_traits>
-
 #include "ptx_sm100.cuh"
 
 namespace sk {
@@ -725,11 +723,6 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         if (++e == ESTAGES) { e = 0; eph ^= 1; }
       }
     }
-    if constexpr (!DUMP && SPLIT) {   // the epilogue's two
-      __syncwarp();
-      cluster_sync_all();
-      cluster_sync_all();
-    }
   } else {
     // ============================================================ epilogue
     // warp w: TMEM lanes 32 (w % 4) .. +31 (hardware rule), token columns of warpgroup w / 4
@@ -996,46 +989,41 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     if constexpr (PERSIST) {
       if ((threadIdx.x & 127) == 0) bulk_wait_group0();   // this thread's TMA stores are complete
     }
-    if constexpr (!DUMP && SPLIT) {
-      // split-K: fixed-order reduction over the cluster through distributed shared memory.  A warp takes token rows, a lane
-      // four of their features: 16-byte remote loads, every CTA's, in rank order (deterministic).  A warp's whole share
-      // (BLOCK_M / kEpiWarps loads, whatever the split) is in flight at once, and the token scales are fetched before the
-      // cluster barrier: the phase is one remote round trip.  (Two rows at a time, their scales behind them, it was two or
-      // more.  It is in the epilogue's branch because the code behind the roles has the registers of the smallest role.)
+  }
+
+  if constexpr (!DUMP && SPLIT) {
+    {
+      // split-K: fixed-order reduction over the cluster through distributed shared memory
       const float kScaleDown = 5.62949953421312e14f;
-      const TileCoord tc = tile_coord(tile_first, p.n_tiles, p.num_tiles);   // split-K CTAs own exactly one tile
-      const int n = tc.n_tile * kTileN + 4 * lane;
-      const int m0 = tc.m_tile * BLOCK_M;
-      const int j0 = static_cast<int>(cluster_ctarank()) * T::kEpiWarps + warp;     // the warp's rows: j0, j0 + step, ...
-      const int step = num_splits * T::kEpiWarps;
-      float xs_lane = 0.f;
-      if (j0 + lane * step < BLOCK_M && m0 + j0 + lane * step < p.M)
-        xs_lane = ld_global_f32(p.x_scale + m0 + j0 + lane * step) * kScaleDown;
       __syncwarp();
       cluster_sync_all();
-      auto reduce = [&](auto splits) {
-        constexpr int kSplits = decltype(splits)::value;
-        constexpr int kRows = BLOCK_M / T::kEpiWarps / kSplits > 0 ? BLOCK_M / T::kEpiWarps / kSplits : 1;
-        const uint32_t red = smem_base + (j0 * kTileN + 4 * lane) * 4;
-        float4 part[kRows][kSplits];
-#pragma unroll
-        for (int i = 0; i < kRows; ++i)
-#pragma unroll
-          for (int r = 0; r < kSplits; ++r)
-            if (j0 + i * step < BLOCK_M) part[i][r] = ld_dsmem_f32x4(map_to_cta(red + i * step * kTileN * 4, r));
+      if (warp < T::kEpiWarps) {
+        // A warp takes a token row, a lane four of its features: 16-byte remote loads, every CTA's in flight before the
+        // first is added, in rank order (deterministic).  (One float per thread and load left this phase latency-bound:
+        // 128 tokens over 4 CTAs were 16 dependent round trips of ~700 cycles.)
+        const float* red = reinterpret_cast<const float*>(smem);
+        const int my_rank = static_cast<int>(cluster_ctarank());
+        const TileCoord tc = tile_coord(tile_first, p.n_tiles, p.num_tiles);   // split-K CTAs own exactly one tile
+        const int n = tc.n_tile * kTileN + 4 * lane;
+        const int m0 = tc.m_tile * BLOCK_M;
         const bool vec_ok = n + 4 <= p.N && (p.ld_out % 4) == 0;
+#pragma unroll 2
+        for (int j = my_rank * T::kEpiWarps + warp; j < BLOCK_M; j += num_splits * T::kEpiWarps) {
+          const int m = m0 + j;
+          if (m >= p.M) break;
+          const uint32_t local = smem_u32(red + j * kTileN + 4 * lane);
+          float4 part[8];
 #pragma unroll
-        for (int i = 0; i < kRows; ++i) {
-          const float xs = __shfl_sync(0xffffffffu, xs_lane, i);
-          const int m = m0 + j0 + i * step;
-          if (j0 + i * step >= BLOCK_M || m >= p.M) break;
+          for (int r = 0; r < 8; ++r)
+            part[r] = r < num_splits ? ld_dsmem_f32x4(map_to_cta(local, r)) : make_float4(0.f, 0.f, 0.f, 0.f);
+          const float xs = ld_global_f32(p.x_scale + m) * kScaleDown;
           float y[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-          for (int r = 0; r < kSplits; ++r) { y[0] += part[i][r].x; y[1] += part[i][r].y; y[2] += part[i][r].z; y[3] += part[i][r].w; }
+          for (int r = 0; r < 8; ++r) { y[0] += part[r].x; y[1] += part[r].y; y[2] += part[r].z; y[3] += part[r].w; }
           uint16_t bits[4];
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            bits[k] = p.out_bf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(y[k] * xs)) : __half_as_ushort(__float2half_rn(y[k] * xs));
+          for (int i = 0; i < 4; ++i)
+            bits[i] = p.out_bf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(y[i] * xs)) : __half_as_ushort(__float2half_rn(y[i] * xs));
           int d_first = 0, d_last = p.n_extra, m_dst = m;
           if (p.scatter_rows > 0) {                  // row scatter: the row's one destination, and its place there
             d_first = d_last = m / p.scatter_rows;
@@ -1048,15 +1036,12 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
                                                         bits[2] | (static_cast<uint32_t>(bits[3]) << 16));
             } else {
 #pragma unroll
-              for (int k = 0; k < 4; ++k)
-                if (n + k < p.N) o[k] = bits[k];
+              for (int i = 0; i < 4; ++i)
+                if (n + i < p.N) o[i] = bits[i];
             }
           }
         }
-      };
-      if (num_splits == 2) reduce(std::integral_constant<int, 2>{});
-      else if (num_splits == 4) reduce(std::integral_constant<int, 4>{});
-      else reduce(std::integral_constant<int, 8>{});
+      }
       __syncwarp();
       cluster_sync_all();   // peers may still be reading this CTA's shared memory until here
     }
