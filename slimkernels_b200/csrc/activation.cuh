@@ -11,6 +11,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "ptx_sm100.cuh"
+
 namespace sk {
 
 constexpr int kActThreads = 256;
@@ -218,6 +220,77 @@ silu_mul_quantize_cluster_kernel(const __half* gate_up, long long ld_gu, int8_t*
       for (int j = 0; j < 8; ++j)
         w[j >> 2] |= quantize_one_fast(h[i][j], s, r) << (8 * (j & 3));
       qrow[v] = make_uint2(w[0], w[1]);
+    }
+  }
+}
+
+// The same for many rows: CTAs that stay, two to four to an SM, each taking every gridDim.x-th row.  A thread copies its vectors of the
+// next row into shared memory of its own (nobody else reads them: no barrier) as soon as it has this row's values in registers,
+// so the loads run under the row maximum, the quantising and the stores, and there is one CTA barrier per row; the cluster
+// kernel above starts a CTA and pays a cluster barrier for a third of a row.
+constexpr int kRowsThreads = 512;
+constexpr int rows_ctas_per_sm(int vecs) { return vecs == 1 ? 4 : vecs == 2 ? 3 : 2; }   // what the values in registers leave room for
+template <int VECS>
+__global__ void __launch_bounds__(kRowsThreads, rows_ctas_per_sm(VECS))
+silu_mul_quantize_rows_kernel(const __half* gate_up, long long ld_gu, int8_t* __restrict__ h_q, long long ld_q,
+                              float* __restrict__ h_scale, long long M, int I) {
+  extern __shared__ uint4 row_buf[];            // gate [I / 8], up [I / 8]
+  __shared__ float red[2][kRowsThreads / 32];
+  act_launch_dependents();
+  act_wait_for_inputs();
+  const int nvec = I / 8;
+  auto fetch = [&](long long m) {
+    const uint4* g = reinterpret_cast<const uint4*>(gate_up + m * ld_gu) + threadIdx.x;
+    const uint4* u = reinterpret_cast<const uint4*>(gate_up + m * ld_gu + I) + threadIdx.x;
+#pragma unroll
+    for (int i = 0; i < VECS; ++i)
+      if (threadIdx.x + i * kRowsThreads < nvec) {
+        cp_async16(smem_u32(row_buf + i * kRowsThreads + threadIdx.x), g + i * kRowsThreads);
+        cp_async16(smem_u32(row_buf + nvec + i * kRowsThreads + threadIdx.x), u + i * kRowsThreads);
+      }
+  };
+  if (blockIdx.x < M) fetch(blockIdx.x);
+  int turn = 0;
+  for (long long m = blockIdx.x; m < M; m += gridDim.x, turn ^= 1) {
+    cp_async_wait_all();
+    float h[VECS][8];
+    float amax = 0.f;
+#pragma unroll
+    for (int i = 0; i < VECS; ++i) {
+      if (threadIdx.x + i * kRowsThreads < nvec) {
+        const uint4 gv = row_buf[i * kRowsThreads + threadIdx.x], uv = row_buf[nvec + i * kRowsThreads + threadIdx.x];
+        const __half2* gh = reinterpret_cast<const __half2*>(&gv);
+        const __half2* uh = reinterpret_cast<const __half2*>(&uv);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 gf = __half22float2(gh[j]), uf = __half22float2(uh[j]);
+          h[i][2 * j] = silu_mul(gf.x, uf.x);
+          h[i][2 * j + 1] = silu_mul(gf.y, uf.y);
+          amax = fmaxf(amax, fmaxf(fabsf(h[i][2 * j]), fabsf(h[i][2 * j + 1])));
+        }
+      }
+    }
+    if (m + gridDim.x < M) fetch(m + gridDim.x);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    if ((threadIdx.x & 31) == 0) red[turn][threadIdx.x >> 5] = amax;
+    __syncthreads();                            // (the other half of red is the next row's: a thread is at most one row ahead)
+    amax = red[turn][threadIdx.x & 15];
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    const float s = amax > 0.f ? amax / 127.f : 1.f;
+    const float r = 1.f / s;
+    if (threadIdx.x == 0) h_scale[m] = s;
+    uint2* qrow = reinterpret_cast<uint2*>(h_q + m * ld_q);
+#pragma unroll
+    for (int i = 0; i < VECS; ++i) {
+      const int v = threadIdx.x + i * kRowsThreads;
+      if (v < nvec) {
+        uint32_t w[2] = {0u, 0u};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) w[j >> 2] |= quantize_one_fast(h[i][j], s, r) << (8 * (j & 3));
+        qrow[v] = make_uint2(w[0], w[1]);
+      }
     }
   }
 }

@@ -292,6 +292,13 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, const uint4& v) {
                : "memory");
 }
 
+// Per-thread asynchronous copies.
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {   // through L2 only: for data read once
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // What a kernel before this one wrote, read after grid_dep_wait: volatile, so that the load stays behind it.
 __device__ __forceinline__ float ld_global_f32(const float* p) {
   float v;

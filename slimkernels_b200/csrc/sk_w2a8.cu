@@ -1811,6 +1811,37 @@ int sk_silu_mul_quantize_int8(const void* gate_up_f16, int64_t ld_gu, int64_t M,
     return SK_ERR_BAD_ALIGNMENT;
   const auto st = static_cast<cudaStream_t>(stream);
   const __half* gu = static_cast<const __half*>(gate_up_f16);
+  // From 64 rows on CTAs that stay and take a row each at a time (the cluster kernel / this one, us: 64 x 11008 4.8 / 4.8,
+  // 128 x 11008 6.7 / 5.4, 592 x 11008 12.9 / 9.7, 4096 x 11008 66.8 / 51.4; 64 x 4096 2.7 / 2.4; but 32 x 14336 3.7 / 4.4: a row is one
+  // CTA's work here, up to eight's there).
+  if (M >= 64 && I <= 8LL * sk::kRowsThreads * 4) {
+    const int vecs = static_cast<int>((I / 8 + sk::kRowsThreads - 1) / sk::kRowsThreads);
+    auto kern = vecs == 1   ? sk::silu_mul_quantize_rows_kernel<1>
+                : vecs == 2 ? sk::silu_mul_quantize_rows_kernel<2>
+                : vecs == 3 ? sk::silu_mul_quantize_rows_kernel<3>
+                            : sk::silu_mul_quantize_rows_kernel<4>;
+    const int smem = static_cast<int>(I) * 4, grid = sk::kChipSms * sk::rows_ctas_per_sm(vecs);
+    if (smem > 47 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return SK_ERR_CUDA;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(M < grid ? M : grid));
+    cfg.blockDim = dim3(sk::kRowsThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see sk_quantize_activation_int8
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, kern, gu, static_cast<long long>(ld_gu), h_q, static_cast<long long>(ld_q), h_scale,
+                           static_cast<long long>(M), static_cast<int>(I)) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return SK_ERR_CUDA;
+    }
+    return SK_OK;
+  }
   // one pass over HBM: the row split over a cluster of 1..8 CTAs whose threads keep their fp32 values in registers
   // As many CTAs as the row needs, whether or not that is a power of two: 11008 features are 3 x 1.8 vectors per thread, in
   // four CTAs a third of the second vectors' threads would idle (12 us of 697 of the MLP block of 4096 tokens).  Few rows leave SMs

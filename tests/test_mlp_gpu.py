@@ -58,6 +58,31 @@ def test_silu_mul_quantize(M, I):
     assert diff.max() <= 1 and (diff != 0).mean() < 2e-3
 
 
+@pytest.mark.parametrize("M,I,pad", [(64, 8, 0), (64, 4096, 0), (65, 4104, 8), (700, 264, 16), (64, 8192, 0), (450, 8200, 0), (300, 11008, 0),
+                                     (64, 12288, 8), (64, 12296, 0), (310, 16384, 0), (64, 16392, 0)])
+def test_silu_many_rows_equal_few_rows(M, I, pad):
+    """64 rows and more go through the kernel of resident CTAs (up to 16384 features), fewer through clusters: the same bits."""
+    lib = capi.load()
+    g = torch.Generator(device="cuda").manual_seed(M + I)
+    gu = (torch.randn(M, 2 * I + pad, generator=g, device="cuda") * 3).half()
+    gu[1] = 0
+    gu[2, 3] = float("inf")
+    gu[3, I] = float("nan")
+    gu[4, :8] = 65504
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def run(lo, hi, q, s):
+        assert lib.sk_silu_mul_quantize_int8(gu[lo:].data_ptr(), 2 * I + pad, hi - lo, I, q[lo:].data_ptr(), I + pad, s[lo:].data_ptr(), stream) == 0
+
+    q = [torch.full((M, I + pad), 99, dtype=torch.int8, device="cuda") for _ in range(2)]
+    s = [torch.zeros(M, device="cuda") for _ in range(2)]
+    run(0, M, q[0], s[0])
+    for lo in range(0, M, 50):
+        run(lo, min(M, lo + 50), q[1], s[1])
+    assert torch.equal(q[0], q[1]) and torch.equal(s[0].view(torch.int32), s[1].view(torch.int32))
+    assert pad == 0 or bool((q[0][:, I:] == 99).all())
+
+
 def _mlp_problem(M, hidden, inter, seed=0):
     rng = np.random.default_rng(seed)
     x = rng.standard_normal((M, hidden)).astype(np.float16)
