@@ -234,6 +234,26 @@ __device__ __forceinline__ bool wait_bounded(uint32_t bar, uint32_t parity, cons
   return wait_slow(bar, parity, ctx.abort_flag, ctx.status, code, ctx.limit);
 }
 
+// Bounded wait for two barriers: where both are complete already, as they mostly are, the two polls overlap and there is one
+// branch.
+__device__ __forceinline__ bool wait_bounded_two(uint32_t bar_a, uint32_t parity_a, uint32_t bar_b, uint32_t parity_b, const WaitCtx& ctx,
+                                                 int code_a, int code_b) {
+  long long t0 = 0;
+  for (uint32_t spins = 0;; ++spins) {
+    const bool a = mbar_try_wait(bar_a, parity_a), b = mbar_try_wait(bar_b, parity_b);
+    if (a && b) return true;
+    if ((spins & 63u) == 0) {
+      if (spins == 0) t0 = clock64();
+      if (*ctx.abort_flag) return false;
+      if (clock64() - t0 > ctx.limit) {
+        *ctx.abort_flag = 1;
+        atomicCAS(ctx.status, 0, a ? code_b : code_a);
+        return false;
+      }
+    }
+  }
+}
+
 // Bounded wait for a role that is not on the critical path of a K block: sleeps between polls, so that it does not
 // take issue slots and integer-pipe cycles from the warps that expand (the expansion saturates the integer pipe).
 __device__ __forceinline__ bool wait_bounded_relaxed(uint32_t bar, uint32_t parity, const WaitCtx& ctx, int code,
@@ -338,6 +358,7 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
   constexpr int kExpWarp0 = T::kEpiWarps;       // first expander warp
   constexpr int kProducerWarp = kExpWarp0 + EXP_WARPS;
   constexpr int kMmaWarp = kProducerWarp + 1;
+  constexpr bool kBlockTurns = ACC_BUFS == 4;   // group size 64: the MMA issuers take K blocks, not groups, in turn
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -389,7 +410,7 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
   // Every mbarrier counts ONE arrival per participating warp (lane 0, after __syncwarp): arrivals on one
   // barrier are serialised shared-memory atomics.
   if (threadIdx.x == 0) {
-    const int readers = OTHER_G && p.steps_per_group < 4 ? 2 : 1;   // issuing warps that read a stage
+    const int readers = OTHER_G && p.steps_per_group < 4 && !(kBlockTurns && p.steps_per_group == 2) ? 2 : 1;   // issuing warps that read a stage
     for (int i = 0; i < LSTAGES; ++i) {
       mbar_init(bar_ld_full + 8 * i, 1);           // TMA transaction bytes
       mbar_init(bar_ld_empty + 8 * i, readers);    // tcgen05.commit of the MMAs that read the stage
@@ -490,20 +511,25 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         // phase can succeed one phase early.  (For the same reason the rings have even lengths where the issuers take blocks
         // in turn.)  Both issuers read a block, so its "free" barriers count both.
         // 256, 384, ...: a group spans blocks; one issuer.
+        // Where a block's groups and the next block's fill different buffers (two groups, four buffers) the issuers take blocks
+        // in turn instead, as with group size 128: half the iterations for each.
         const int steps = p.steps_per_group;                  // 1, 2 or a multiple of 8 (in blocks: 4)
         const int per_block = steps < 4 ? 4 / steps : 1;      // groups per block
         const int blocks = steps < 4 ? 1 : steps / 4;         // blocks per group
-        if (per_block > 1 || mma_id == 0)
-        for (int kb = kb_begin, buf = mma_id & (per_block > 1 ? 1 : 0), pos = 0; kb < kb_end; ++kb) {
-          ok = wait_bounded(bar_ld_full + 8 * l, lph, ctx, kStMmaLdFull) &&
-               wait_bounded(bar_ex_full + 8 * e, eph, ctx, kStMmaExFull);
-          const int n_groups = per_block > 1 ? min(per_block, g_end - kb * per_block) : 1;    // (the last block may be short)
-          for (int i = per_block > 1 ? mma_id : 0; i < n_groups && ok; i += 2) {
-            if (pos == 0) ok = wait_bounded(bar_acc_empty + 8 * buf, aph, ctx, kStMmaAccEmpty);
-            if (!ok) break;
-            tcgen05_fence_after_sync();
-            const bool last = pos == blocks - 1;
-            if (elect_one()) {
+        const bool by_block = kBlockTurns && per_block == 2;
+        const int step = by_block ? 2 : 1;                    // blocks an issuer advances by
+        if ((per_block > 1 || mma_id == 0) && elect_one()) {
+          int buf = by_block ? 2 * mma_id : per_block > 1 ? mma_id : 0, pos = 0;
+          if (by_block) l = e = mma_id;
+#pragma unroll 1
+          for (int kb = kb_begin + (by_block ? mma_id : 0); kb < kb_end && ok; kb += step) {
+            const int n_groups = per_block > 1 ? min(per_block, g_end - kb * per_block) : 1;    // (the last block may be short)
+            ok = wait_bounded(bar_ex_full + 8 * e, eph, ctx, kStMmaExFull);     // (for the copies, too: the expanders waited for them)
+            for (int i = per_block > 1 && !by_block ? mma_id : 0; i < n_groups && ok; i += by_block ? 1 : 2) {
+              if (pos == 0) ok = wait_bounded(bar_acc_empty + 8 * buf, aph, ctx, kStMmaAccEmpty);
+              if (!ok) break;
+              tcgen05_fence_after_sync();
+              const bool last = pos == blocks - 1;
               const uint64_t a_desc = a_desc0 + static_cast<uint64_t>(e * (kWxBytes >> 4) + 2 * i * steps);
               const uint64_t b_desc = b_desc0 + static_cast<uint64_t>(l * (T::kXBytes >> 4) + 2 * i * steps);
               const uint32_t d = tmem_base + buf * BLOCK_M;
@@ -511,50 +537,39 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
               for (int s = 0; s < 4; ++s)
                 if (s < steps) umma_i8(d, a_desc + 2 * s, b_desc + 2 * s, idesc, 1u);
               if (last) umma_commit(bar_acc_full + 8 * buf);
+              pos = last ? 0 : pos + 1;
+              if (last) {                                     // the issuer's next buffer
+                if (by_block) {
+                  buf ^= 1;
+                  if ((buf & 1) == 0) aph ^= 1;               // (its two buffers are this block's)
+                } else {
+                  buf += per_block > 1 ? 2 : 1;
+                  if (buf >= ACC_BUFS) { buf -= ACC_BUFS; aph ^= 1; }
+                }
+              }
             }
-            __syncwarp();
-            pos = last ? 0 : pos + 1;
-            if (last) {                                       // the issuer's next buffer
-              buf += per_block > 1 ? 2 : 1;
-              if (buf >= ACC_BUFS) { buf -= ACC_BUFS; aph ^= 1; }
-            }
-          }
-          if (!ok) break;
-          if (elect_one()) {
+            if (!ok) break;
             umma_commit(bar_ld_empty + 8 * l);
             if constexpr (!T::kTied) umma_commit(bar_ex_empty + 8 * e);
+            if ((l += step) >= LSTAGES) l -= LSTAGES;
+            if ((e += step) >= ESTAGES) { e -= ESTAGES; eph ^= 1; }
           }
-          __syncwarp();
-          if (++l == LSTAGES) { l = 0; lph ^= 1; }
-          if (++e == ESTAGES) { e = 0; eph ^= 1; }
         }
+        __syncwarp();
       } else if (p.steps_per_group == 4) {
-        // one K block == one scale group: four MMAs and three commits per iteration, nothing else
-        int turn = 0;                             // whose group this is (alternates over all K blocks of all tiles)
-        for (int tile = tile_first; tile < tile_end && ok; tile += tile_step)
-        for (int kb = kb_begin; kb < kb_end; ++kb, turn ^= 1) {
-          if (turn != mma_id) {                   // the other warp's group: only keep the ring state in step
-            if (++l == LSTAGES) { l = 0; lph ^= 1; }
-            if (++e == ESTAGES) { e = 0; eph ^= 1; }
-            if (++ab == ACC_BUFS) { ab = 0; aph ^= 1; }
-            continue;
-          }
-#ifdef SK_TRACE_MMA_FINE
-          if (lane == 0 && kb - kb_begin >= 8 && kb - kb_begin < 16) SK_TRACE_EVENT(5, (kb - kb_begin - 8) * 8 + 0);
-          ok = wait_bounded(bar_ld_full + 8 * l, lph, ctx, kStMmaLdFull);
-          if (lane == 0 && kb - kb_begin >= 8 && kb - kb_begin < 16) SK_TRACE_EVENT(5, (kb - kb_begin - 8) * 8 + 1);
-          ok = ok && wait_bounded(bar_ex_full + 8 * e, eph, ctx, kStMmaExFull);
-          if (lane == 0 && kb - kb_begin >= 8 && kb - kb_begin < 16) SK_TRACE_EVENT(5, (kb - kb_begin - 8) * 8 + 2);
-          ok = ok && wait_bounded(bar_acc_empty + 8 * ab, aph, ctx, kStMmaAccEmpty);
-          if (lane == 0 && kb - kb_begin >= 8 && kb - kb_begin < 16) SK_TRACE_EVENT(5, (kb - kb_begin - 8) * 8 + 3);
-#else
-          ok = wait_bounded(bar_ld_full + 8 * l, lph, ctx, kStMmaLdFull) &&
-               wait_bounded(bar_ex_full + 8 * e, eph, ctx, kStMmaExFull) &&
-               wait_bounded(bar_acc_empty + 8 * ab, aph, ctx, kStMmaAccEmpty);
-#endif
-          if (!ok) break;
-          tcgen05_fence_after_sync();
-          if (elect_one()) {
+        // One K block == one scale group: four MMAs and two commits per iteration, nothing else.  What an iteration costs
+        // around them paces the small tiles (and, with the expanders, the large one): one lane runs the loop, its stages
+        // and buffers advance by two, the barrier of the expanded weights stands for the copies too (the expanders waited
+        // for them), and the two polls overlap.  ISSUE_FIGURES
+        const int per_cta = PERSIST ? (tile_end - tile_first + tile_step - 1) / tile_step : 1;
+        const int blocks = per_cta * (kb_end - kb_begin);
+        if (elect_one()) {
+          l = e = mma_id;
+          ab = mma_id;
+#pragma unroll 1
+          for (int i = mma_id; i < blocks; i += 2) {
+            if (!wait_bounded_two(bar_ex_full + 8 * e, eph, bar_acc_empty + 8 * ab, aph, ctx, kStMmaExFull, kStMmaAccEmpty)) break;
+            tcgen05_fence_after_sync();
             const uint64_t a_desc = a_desc0 + static_cast<uint64_t>(e * (kWxBytes >> 4));
             const uint64_t b_desc = b_desc0 + static_cast<uint64_t>(l * (T::kXBytes >> 4));
             const uint32_t d = tmem_base + ab * BLOCK_M;
@@ -571,22 +586,15 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
               umma_i8(d, a_desc + 4, b_desc + 4, idesc, 1u);
               umma_i8(d, a_desc + 6, b_desc + 6, idesc, 1u);
             }
-#ifdef SK_TRACE_MMA_FINE
-            if (kb - kb_begin >= 8 && kb - kb_begin < 16) SK_TRACE_EVENT(5, (kb - kb_begin - 8) * 8 + 4);
-#endif
             umma_commit(bar_acc_full + 8 * ab);
             umma_commit(bar_ld_empty + 8 * l);
             if constexpr (!T::kTied) umma_commit(bar_ex_empty + 8 * e);
-#ifdef SK_TRACE_MMA_FINE
-            if (kb - kb_begin >= 8 && kb - kb_begin < 16) SK_TRACE_EVENT(5, (kb - kb_begin - 8) * 8 + 5);
-#endif
-            SK_TRACE_EVENT(2, SK_TRACE_BASE + kb - kb_begin);
+            if ((l += 2) >= LSTAGES) l -= LSTAGES;                       // (even rings)
+            if ((e += 2) >= ESTAGES) { e -= ESTAGES; eph ^= 1; }
+            if ((ab += 2) >= ACC_BUFS) { ab -= ACC_BUFS; aph ^= 1; }
           }
-          __syncwarp();
-          if (++l == LSTAGES) { l = 0; lph ^= 1; }
-          if (++e == ESTAGES) { e = 0; eph ^= 1; }
-          if (++ab == ACC_BUFS) { ab = 0; aph ^= 1; }
         }
+        __syncwarp();
       } else {
         // other group sizes in the debug, persistent and 192-token kernels: one issuer, tracking the position inside the group
         // per 32-wide K step
