@@ -143,71 +143,6 @@ quantize_activation_kernel(const uint16_t* x, long long ld_x, int8_t* __restrict
   for (int v = threadIdx.x + kMaxVec * THREADS; v < nvec; v += THREADS) emit(v, as_half8<BF16>(row[v]));
 }
 
-// The same for many rows: CTAs that stay and take every gridDim.x-th row, with a thread's part of the next row copied into shared
-// memory of its own while this row is reduced, quantised and stored (see silu_mul_quantize_rows_kernel).
-constexpr int kRowsThreads = 512;
-constexpr int kQuantRowsCtas = 4;               // per SM
-template <int VECS, bool BF16>
-__global__ void __launch_bounds__(kRowsThreads, kQuantRowsCtas)
-quantize_activation_rows_kernel(const uint16_t* x, long long ld_x, int8_t* __restrict__ x_q, long long ld_q,
-                                float* __restrict__ x_scale, long long M, int K) {
-  extern __shared__ uint4 row_buf[];            // [K / 8]
-  __shared__ float red[2][kRowsThreads / 32];
-  act_launch_dependents();
-  act_wait_for_inputs();
-  const int nvec = K / 8;
-  auto fetch = [&](long long m) {
-    const uint4* row = reinterpret_cast<const uint4*>(x + m * ld_x) + threadIdx.x;
-#pragma unroll
-    for (int i = 0; i < VECS; ++i)
-      if (threadIdx.x + i * kRowsThreads < nvec) cp_async16(smem_u32(row_buf + i * kRowsThreads + threadIdx.x), row + i * kRowsThreads);
-  };
-  if (blockIdx.x < M) fetch(blockIdx.x);
-  int turn = 0;
-  for (long long m = blockIdx.x; m < M; m += gridDim.x, turn ^= 1) {
-    cp_async_wait_all();
-    uint4 keep[VECS];
-    float amax = 0.f;
-#pragma unroll
-    for (int i = 0; i < VECS; ++i)
-      if (threadIdx.x + i * kRowsThreads < nvec) {
-        keep[i] = as_half8<BF16>(row_buf[i * kRowsThreads + threadIdx.x]);
-        const __half2* h = reinterpret_cast<const __half2*>(&keep[i]);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 f = __half22float2(h[j]);
-          amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
-        }
-      }
-    if (m + gridDim.x < M) fetch(m + gridDim.x);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    if ((threadIdx.x & 31) == 0) red[turn][threadIdx.x >> 5] = amax;
-    __syncthreads();                            // (the other half of red is the next row's: a thread is at most one row ahead)
-    amax = red[turn][threadIdx.x & 15];
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    const float s = amax > 0.f ? amax / 127.f : 1.f;
-    const float r = 1.f / s;
-    if (threadIdx.x == 0) x_scale[m] = s;
-    uint2* qrow = reinterpret_cast<uint2*>(x_q + m * ld_q);
-#pragma unroll
-    for (int i = 0; i < VECS; ++i) {
-      const int v = threadIdx.x + i * kRowsThreads;
-      if (v < nvec) {
-        const __half2* h = reinterpret_cast<const __half2*>(&keep[i]);
-        uint32_t w[2] = {0u, 0u};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 f = __half22float2(h[j]);
-          w[j >> 1] |= (quantize_one_fast(f.x, s, r) | (quantize_one_fast(f.y, s, r) << 8)) << (16 * (j & 1));
-        }
-        qrow[v] = make_uint2(w[0], w[1]);
-      }
-    }
-  }
-}
-
 // gate_up fp16 [M, ld_gu] with gate = columns [0, I), up = columns [I, 2I)  ->  h = SiLU(gate) * up (fp32),
 // h_q int8 [M, ld_q], h_scale fp32 [M].  I % 8 == 0.
 // SiLU(g) * u = g * u / (1 + exp(-g)) in fp32.  The exponential and the reciprocal are the hardware approximations
@@ -293,6 +228,7 @@ silu_mul_quantize_cluster_kernel(const __half* gate_up, long long ld_gu, int8_t*
 // next row into shared memory of its own (nobody else reads them: no barrier) as soon as it has this row's values in registers,
 // so the loads run under the row maximum, the quantising and the stores, and there is one CTA barrier per row; the cluster
 // kernel above starts a CTA and pays a cluster barrier for a third of a row.
+constexpr int kRowsThreads = 512;
 constexpr int rows_ctas_per_sm(int vecs) { return vecs == 1 ? 4 : vecs == 2 ? 3 : 2; }   // what the values in registers leave room for
 template <int VECS>
 __global__ void __launch_bounds__(kRowsThreads, rows_ctas_per_sm(VECS))

@@ -1785,26 +1785,6 @@ int sk_quantize_activation_int8_from(const void* x, int x_bf16, int64_t ld_x, in
   const uint16_t* src = static_cast<const uint16_t*>(x);
   const long long ldx = ld_x, ldq = ld_q;
   const int k = static_cast<int>(K);
-  if (M >= 64 && K <= 8LL * sk::kRowsThreads * 4) {
-    const int v = (k / 8 + sk::kRowsThreads - 1) / sk::kRowsThreads;
-    auto rows = x_bf16 ? (v == 1   ? sk::quantize_activation_rows_kernel<1, true>
-                          : v == 2 ? sk::quantize_activation_rows_kernel<2, true>
-                          : v == 3 ? sk::quantize_activation_rows_kernel<3, true>
-                                   : sk::quantize_activation_rows_kernel<4, true>)
-                       : (v == 1   ? sk::quantize_activation_rows_kernel<1, false>
-                          : v == 2 ? sk::quantize_activation_rows_kernel<2, false>
-                          : v == 3 ? sk::quantize_activation_rows_kernel<3, false>
-                                   : sk::quantize_activation_rows_kernel<4, false>);
-    const long long grid = sk::kChipSms * sk::kQuantRowsCtas;
-    cfg.gridDim = dim3(static_cast<unsigned>(M < grid ? M : grid));
-    cfg.blockDim = dim3(sk::kRowsThreads, 1, 1);
-    cfg.dynamicSmemBytes = static_cast<size_t>(k) * 2;           // (32 KB at most)
-    if (cudaLaunchKernelEx(&cfg, rows, src, ldx, x_q, ldq, x_scale, static_cast<long long>(M), k) != cudaSuccess) {
-      (void)cudaGetLastError();
-      return SK_ERR_CUDA;
-    }
-    return SK_OK;
-  }
   const int vecs = K <= 8 * sk::kActThreads * 2 ? 2 : K <= 8 * sk::kActThreads * 4 ? 4 : 8;
   auto kern = x_bf16 ? (vecs == 2 ? sk::quantize_activation_kernel<2, true> : vecs == 4 ? sk::quantize_activation_kernel<4, true>
                                                                                         : sk::quantize_activation_kernel<8, true>)
