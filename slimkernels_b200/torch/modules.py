@@ -60,11 +60,13 @@ class W2A8Linear(nn.Module):
     def plan(self) -> W2A8Plan:
         """The plan of the CURRENT weight buffers: it holds a tiled copy of w_packed and a pointer to w_scale, so it
         is rebuilt when the buffers were written in place (load_state_dict) or replaced (.to(), .cuda())."""
-        key = (self.w_packed.data_ptr(), self.w_packed._version, self.w_scale.data_ptr(), self.w_scale._version,
-               self.w_packed.device)
+        # Asked on every call, so the buffers are looked up once and where they are kept: five look-ups through
+        # nn.Module.__getattr__ took longer than all the rest of the check (a one-token call HOST_FIGURES us).
+        buffers = self._buffers
+        w, s = buffers["w_packed"], buffers["w_scale"]
+        key = (w.data_ptr(), w._version, s.data_ptr(), s._version, w.device)
         if self._plan is None or self._plan_key != key:
-            self._plan = W2A8Plan(self.w_packed, self.w_scale, group_size=self.group_size, zero_point=self.zero_point,
-                                  out_dtype=self.out_dtype)
+            self._plan = W2A8Plan(w, s, group_size=self.group_size, zero_point=self.zero_point, out_dtype=self.out_dtype)
             self._plan_key = key
         return self._plan
 
@@ -87,5 +89,6 @@ class W2A8LlamaMLP(nn.Module):
         self.gate_up, self.down = gate_up, down
 
     def forward(self, x):
-        gate_up_plan, down_plan = self.gate_up.plan(), self.down.plan()      # also loads the extension
+        modules = self._modules                                              # (see W2A8Linear.plan)
+        gate_up_plan, down_plan = modules["gate_up"].plan(), modules["down"].plan()      # also loads the extension
         return torch.ops.slimkernels.w2a8_mlp_block.default(gate_up_plan._h, down_plan._h, x, down_plan.N, down_plan._bf16)
