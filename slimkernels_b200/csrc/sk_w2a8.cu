@@ -1814,7 +1814,8 @@ int sk_silu_mul_quantize_int8(const void* gate_up_f16, int64_t ld_gu, int64_t M,
   // From 64 rows on CTAs that stay and take a row each at a time (the cluster kernel / this one, us: 64 x 11008 4.8 / 4.8,
   // 128 x 11008 6.7 / 5.4, 592 x 11008 12.9 / 9.7, 4096 x 11008 66.8 / 51.4; 64 x 4096 2.7 / 2.4; but 32 x 14336 3.7 / 4.4: a row is one
   // CTA's work here, up to eight's there).
-  if (M >= 64 && I <= 8LL * sk::kRowsThreads * 4) {
+  // One vector per thread keeps pace only for a few rows per CTA (4096 x 4096 21.2 / 23.1).
+  if (M >= 64 && I <= 8LL * sk::kRowsThreads * 4 && (I > 8LL * sk::kRowsThreads || M <= 4 * sk::kChipSms)) {
     const int vecs = static_cast<int>((I / 8 + sk::kRowsThreads - 1) / sk::kRowsThreads);
     auto kern = vecs == 1   ? sk::silu_mul_quantize_rows_kernel<1>
                 : vecs == 2 ? sk::silu_mul_quantize_rows_kernel<2>
