@@ -358,6 +358,13 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
   constexpr int kExpWarp0 = T::kEpiWarps;       // first expander warp
   constexpr int kProducerWarp = kExpWarp0 + EXP_WARPS;
   constexpr int kMmaWarp = kProducerWarp + 1;
+  // Accumulator buffers that change hands together.  What the epilogue does around a group's FMAs -- poll, fence, first load,
+  // arrival, loop -- is a serial chain of about 450 cycles, more than the MMAs of a group up to 128 tokens (256), so with four
+  // buffers it takes two groups at a time.  Cycles per K block, before (with the issuers' shorter loop) and after: 128 tokens 650 (684)
+  // -> 619, 64 tokens 588 (575) -> 539, group size 64 1239 (1181) -> 1017 and 1107 (1080) -> 831: each alone moved little, the three
+  // roles were equally slow.  333 x 5000 x 4160 with group size 64 26.3 -> 22.9 us.
+  constexpr int kPair = ACC_BUFS == 4 && BLOCK_M >= 64 && !DUMP && !PERSIST ? 2 : 1;
+  auto acc_bar = [](int buf) { return 8u * static_cast<uint32_t>(buf / kPair); };      // offset of a buffer's barrier
   constexpr bool kBlockTurns = ACC_BUFS == 4;   // group size 64: the MMA issuers take K blocks, not groups, in turn
 
   extern __shared__ uint8_t smem_raw[];
@@ -419,7 +426,10 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       mbar_init(bar_ex_full + 8 * i, EXP_WARPS / T::kExpGroups);   // expanded weights of the stage are in place
       mbar_init(bar_ex_empty + 8 * i, readers);    // commit of the MMAs that read them (untied rings only)
     }
-    for (int i = 0; i < ACC_BUFS; ++i) { mbar_init(bar_acc_full + 8 * i, 1); mbar_init(bar_acc_empty + 8 * i, T::kEpiWarps); }
+    for (int i = 0; i < ACC_BUFS / kPair; ++i) {
+      mbar_init(bar_acc_full + 8 * i, kPair);      // a commit per group
+      mbar_init(bar_acc_empty + 8 * i, T::kEpiWarps);
+    }
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -504,6 +514,12 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       int l = 0, e = 0, ab = 0;                 // load stage, expanded stage, accumulator buffer
       uint32_t lph = 0, eph = 0, aph = 0;       // their phases
       bool ok = true;
+      // An odd number of groups leaves the last pair of buffers one commit short: the issuer whose turn it would be arrives for
+      // it, once the pair is free (before that the arrival would count for the pair's groups before these).
+      auto fill_pair = [&](int buf, uint32_t phase) {
+        if (((g_end - g_begin) & 1) && wait_bounded(bar_acc_empty + acc_bar(buf), phase, ctx, kStMmaAccEmpty))
+          mbar_arrive(bar_acc_full + acc_bar(buf));
+      };
       if constexpr (OTHER_G) {
         // Group sizes other than 128 (a kernel of its own: the issuing warps of the 256-token tile have 32 registers).
         // 64 and 32: a 128-wide K block holds two or four groups, and an issuer takes those whose accumulator buffers have its
@@ -526,7 +542,7 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
             const int n_groups = per_block > 1 ? min(per_block, g_end - kb * per_block) : 1;    // (the last block may be short)
             ok = wait_bounded(bar_ex_full + 8 * e, eph, ctx, kStMmaExFull);     // (for the copies, too: the expanders waited for them)
             for (int i = per_block > 1 && !by_block ? mma_id : 0; i < n_groups && ok; i += by_block ? 1 : 2) {
-              if (pos == 0) ok = wait_bounded(bar_acc_empty + 8 * buf, aph, ctx, kStMmaAccEmpty);
+              if (pos == 0) ok = wait_bounded(bar_acc_empty + acc_bar(buf), aph, ctx, kStMmaAccEmpty);
               if (!ok) break;
               tcgen05_fence_after_sync();
               const bool last = pos == blocks - 1;
@@ -536,7 +552,7 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
 #pragma unroll
               for (int s = 0; s < 4; ++s)
                 if (s < steps) umma_i8(d, a_desc + 2 * s, b_desc + 2 * s, idesc, 1u);
-              if (last) umma_commit(bar_acc_full + 8 * buf);
+              if (last) umma_commit(bar_acc_full + acc_bar(buf));
               pos = last ? 0 : pos + 1;
               if (last) {                                     // the issuer's next buffer
                 if (by_block) {
@@ -554,47 +570,98 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
             if ((l += step) >= LSTAGES) l -= LSTAGES;
             if ((e += step) >= ESTAGES) { e -= ESTAGES; eph ^= 1; }
           }
+          if (kPair == 2 && ok && (by_block ? (buf & 1) == 1 : mma_id == (per_block > 1 ? 1 : 0))) fill_pair(buf, aph);
         }
         __syncwarp();
       } else if (p.steps_per_group == 4) {
-        // One K block == one scale group: four MMAs and two commits per iteration, nothing else.  What an iteration costs
-        // around them paces the small tiles (and, with the expanders, the large one): one lane runs the loop, its stages
-        // and buffers advance by two, the barrier of the expanded weights stands for the copies too (the expanders waited
-        // for them), and the two polls overlap.  ISSUE_FIGURES
-        const int per_cta = PERSIST ? (tile_end - tile_first + tile_step - 1) / tile_step : 1;
-        const int blocks = per_cta * (kb_end - kb_begin);
-        if (elect_one()) {
-          l = e = mma_id;
-          ab = mma_id;
-#pragma unroll 1
-          for (int i = mma_id; i < blocks; i += 2) {
-            if (!wait_bounded_two(bar_ex_full + 8 * e, eph, bar_acc_empty + 8 * ab, aph, ctx, kStMmaExFull, kStMmaAccEmpty)) break;
-            tcgen05_fence_after_sync();
-            const uint64_t a_desc = a_desc0 + static_cast<uint64_t>(e * (kWxBytes >> 4));
-            const uint64_t b_desc = b_desc0 + static_cast<uint64_t>(l * (T::kXBytes >> 4));
-            const uint32_t d = tmem_base + ab * BLOCK_M;
-            // +2 in the (address >> 4) field advances 32 bytes along K inside the 128-byte swizzle row
-            if constexpr (A_TMEM) {
-              const uint32_t a_t = tmem_base + T::kATmemCol0 + e * 32;   // 8 columns per 32-wide K step
-              umma_i8_ts(d, a_t, b_desc, idesc, 1u);
-              umma_i8_ts(d, a_t + 8, b_desc + 2, idesc, 1u);
-              umma_i8_ts(d, a_t + 16, b_desc + 4, idesc, 1u);
-              umma_i8_ts(d, a_t + 24, b_desc + 6, idesc, 1u);
-            } else {
-              umma_i8(d, a_desc, b_desc, idesc, 1u);
-              umma_i8(d, a_desc + 2, b_desc + 2, idesc, 1u);
-              umma_i8(d, a_desc + 4, b_desc + 4, idesc, 1u);
-              umma_i8(d, a_desc + 6, b_desc + 6, idesc, 1u);
+        if constexpr (ACC_BUFS == 2) {
+          // (the large tiles wait for their expanders; the loop below took 795 cycles a K block there, this one 785)
+          // one K block == one scale group: four MMAs and their commits per iteration, nothing else
+          int turn = 0;                             // whose group this is (alternates over all K blocks of all tiles)
+          for (int tile = tile_first; tile < tile_end && ok; tile += tile_step)
+          for (int kb = kb_begin; kb < kb_end; ++kb, turn ^= 1) {
+            if (turn != mma_id) {                   // the other warp's group: only keep the ring state in step
+              if (++l == LSTAGES) { l = 0; lph ^= 1; }
+              if (++e == ESTAGES) { e = 0; eph ^= 1; }
+              if (++ab == ACC_BUFS) { ab = 0; aph ^= 1; }
+              continue;
             }
-            umma_commit(bar_acc_full + 8 * ab);
-            umma_commit(bar_ld_empty + 8 * l);
-            if constexpr (!T::kTied) umma_commit(bar_ex_empty + 8 * e);
-            if ((l += 2) >= LSTAGES) l -= LSTAGES;                       // (even rings)
-            if ((e += 2) >= ESTAGES) { e -= ESTAGES; eph ^= 1; }
-            if ((ab += 2) >= ACC_BUFS) { ab -= ACC_BUFS; aph ^= 1; }
+            ok = wait_bounded(bar_ld_full + 8 * l, lph, ctx, kStMmaLdFull) &&
+                 wait_bounded(bar_ex_full + 8 * e, eph, ctx, kStMmaExFull) &&
+                 wait_bounded(bar_acc_empty + 8 * ab, aph, ctx, kStMmaAccEmpty);
+            if (!ok) break;
+            tcgen05_fence_after_sync();
+            if (elect_one()) {
+              const uint64_t a_desc = a_desc0 + static_cast<uint64_t>(e * (kWxBytes >> 4));
+              const uint64_t b_desc = b_desc0 + static_cast<uint64_t>(l * (T::kXBytes >> 4));
+              const uint32_t d = tmem_base + ab * BLOCK_M;
+              // +2 in the (address >> 4) field advances 32 bytes along K inside the 128-byte swizzle row
+              if constexpr (A_TMEM) {
+                const uint32_t a_t = tmem_base + T::kATmemCol0 + e * 32;   // 8 columns per 32-wide K step
+                umma_i8_ts(d, a_t, b_desc, idesc, 1u);
+                umma_i8_ts(d, a_t + 8, b_desc + 2, idesc, 1u);
+                umma_i8_ts(d, a_t + 16, b_desc + 4, idesc, 1u);
+                umma_i8_ts(d, a_t + 24, b_desc + 6, idesc, 1u);
+              } else {
+                umma_i8(d, a_desc, b_desc, idesc, 1u);
+                umma_i8(d, a_desc + 2, b_desc + 2, idesc, 1u);
+                umma_i8(d, a_desc + 4, b_desc + 4, idesc, 1u);
+                umma_i8(d, a_desc + 6, b_desc + 6, idesc, 1u);
+              }
+              umma_commit(bar_acc_full + 8 * ab);
+              umma_commit(bar_ld_empty + 8 * l);
+              if constexpr (!T::kTied) umma_commit(bar_ex_empty + 8 * e);
+              SK_TRACE_EVENT(2, SK_TRACE_BASE + kb - kb_begin);
+            }
+            __syncwarp();
+            if (++l == LSTAGES) { l = 0; lph ^= 1; }
+            if (++e == ESTAGES) { e = 0; eph ^= 1; }
+            if (++ab == ACC_BUFS) { ab = 0; aph ^= 1; }
           }
+        } else {
+          // One K block == one scale group: four MMAs and two commits per iteration, nothing else.  What an iteration costs
+          // around them paces the small tiles: one lane runs the loop, its stages
+          // and buffers advance by two, the barrier of the expanded weights stands for the copies too (the expanders waited
+          // for them), and the two polls overlap.  An iteration was 1150 cycles with every barrier complete, of which the MMAs 140.
+          const int per_cta = PERSIST ? (tile_end - tile_first + tile_step - 1) / tile_step : 1;
+          const int blocks = per_cta * (kb_end - kb_begin);
+          if (elect_one()) {
+            l = e = mma_id;
+            ab = mma_id;
+#pragma unroll 1
+            for (int i = mma_id; i < blocks; i += 2) {
+              if (!wait_bounded_two(bar_ex_full + 8 * e, eph, bar_acc_empty + acc_bar(ab), aph, ctx, kStMmaExFull, kStMmaAccEmpty)) {
+                ok = false;
+                break;
+              }
+              tcgen05_fence_after_sync();
+              const uint64_t a_desc = a_desc0 + static_cast<uint64_t>(e * (kWxBytes >> 4));
+              const uint64_t b_desc = b_desc0 + static_cast<uint64_t>(l * (T::kXBytes >> 4));
+              const uint32_t d = tmem_base + ab * BLOCK_M;
+              // +2 in the (address >> 4) field advances 32 bytes along K inside the 128-byte swizzle row
+              if constexpr (A_TMEM) {
+                const uint32_t a_t = tmem_base + T::kATmemCol0 + e * 32;   // 8 columns per 32-wide K step
+                umma_i8_ts(d, a_t, b_desc, idesc, 1u);
+                umma_i8_ts(d, a_t + 8, b_desc + 2, idesc, 1u);
+                umma_i8_ts(d, a_t + 16, b_desc + 4, idesc, 1u);
+                umma_i8_ts(d, a_t + 24, b_desc + 6, idesc, 1u);
+              } else {
+                umma_i8(d, a_desc, b_desc, idesc, 1u);
+                umma_i8(d, a_desc + 2, b_desc + 2, idesc, 1u);
+                umma_i8(d, a_desc + 4, b_desc + 4, idesc, 1u);
+                umma_i8(d, a_desc + 6, b_desc + 6, idesc, 1u);
+              }
+              umma_commit(bar_acc_full + acc_bar(ab));
+              umma_commit(bar_ld_empty + 8 * l);
+              if constexpr (!T::kTied) umma_commit(bar_ex_empty + 8 * e);
+              if ((l += 2) >= LSTAGES) l -= LSTAGES;                       // (even rings)
+              if ((e += 2) >= ESTAGES) { e -= ESTAGES; eph ^= 1; }
+              if ((ab += 2) >= ACC_BUFS) { ab -= ACC_BUFS; aph ^= 1; }
+            }
+            if (kPair == 2 && ok && mma_id == 1) fill_pair(ab, aph);
+          }
+          __syncwarp();
         }
-        __syncwarp();
       } else {
         // other group sizes in the debug, persistent and 192-token kernels: one issuer, tracking the position inside the group
         // per 32-wide K step
@@ -667,6 +734,7 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       }
       bool ok = true;
       int turn = 0;                                            // whose K block this is
+      bool ready = false;                                      // the next block's copies have been seen to land
       for (int tile = tile_first; tile < tile_end && ok; tile += tile_step)
       for (int kb = kb_begin; kb < kb_end; ++kb) {
         if constexpr (T::kExpGroups > 1) {
@@ -679,7 +747,7 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         }
         // The loads below must not be issued before the wait has been seen to succeed: a load that does not depend
         // on the poll's predicate can be served before the barrier state is sampled and return stale bytes.
-        ok = wait_bounded(bar_ld_full + 8 * l, lph, ctx, kStExpanderFull);
+        if (!ready) ok = wait_bounded(bar_ld_full + 8 * l, lph, ctx, kStExpanderFull);
         if (!ok) break;
         if constexpr (!T::kTied) {
           ok = wait_bounded(bar_ex_empty + 8 * e, eph ^ 1, ctx, kStExpanderEmpty);
@@ -688,6 +756,11 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         const uint32_t wp = smem_base + wp_off[0] + l * kWpBytes;
         const uint4 q0 = ld_shared_v4(wp);
         const uint4 q1 = kHalfRows ? make_uint4(0, 0, 0, 0) : ld_shared_v4(wp + 2048);
+        if constexpr (T::kExpGroups > 1) {
+          // this group's next block: polled here, so that the poll's latency is under the expansion
+          const int ln = l + T::kExpGroups;
+          ready = mbar_try_wait(bar_ld_full + 8 * (ln >= LSTAGES ? ln - LSTAGES : ln), lph ^ (ln >= LSTAGES ? 1u : 0u));
+        }
         if constexpr (A_TMEM) {
           // this thread's row (= its TMEM lane): 32 bytes of codes in, 128 int8 bytes out as 32 TMEM columns
           const uint32_t words[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
@@ -753,7 +826,7 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     __syncwarp();
     if (lane == 0) {
 #pragma unroll
-      for (int a = 0; a < ACC_BUFS; ++a) mbar_arrive(bar_acc_empty + 8 * a);
+      for (int a = 0; a < ACC_BUFS / kPair; ++a) mbar_arrive(bar_acc_empty + 8 * a);
     }
     int ab = 0, tile_parity = 0;
     uint32_t aph = 0;
@@ -795,11 +868,8 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       sp += p.N; ++g_load;
       return r;
     };
-    for (int i = ACC_BUFS + 1; i < kScalePrefetchGroups && g_begin + i < g_end; ++i)
+    for (int i = kPair == 2 ? 2 * ACC_BUFS : ACC_BUFS + 1; i < kScalePrefetchGroups && g_begin + i < g_end; ++i)
       asm volatile("prefetch.global.L2 [%0];" ::"l"(sp + static_cast<size_t>(i) * p.N));
-    unsigned short sr[ACC_BUFS + 1];
-#pragma unroll
-    for (int i = 0; i <= ACC_BUFS; ++i) sr[i] = load_scale();
     float s_sum = 0.f;   // sum of the coefficients since the last bias flush
     int flush = 0;
     // TMEM loads are software-pipelined across the chunks of a group: while chunk c is consumed the load of chunk
@@ -808,62 +878,135 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     constexpr bool kDB = T::kDoubleBuf && !DUMP;
     constexpr int kBufMask = kDB ? 1 : 0;
     uint32_t v[kBufMask + 1][kChunk];
+    if constexpr (kPair == 2) {
+      // cur[u]: the scale of the group that buffer u holds next; raw[u]: the fp16 bits of the one after it (ACC_BUFS groups on),
+      // fetched when the buffer was last read.  Unrolled over the buffers, nothing is shifted from register to register.
+      // A group past the end has the coefficient 0: its buffer's sums, whatever they are, are finite.
+      unsigned short raw[2 * ACC_BUFS];
+#pragma unroll
+      for (int i = 0; i < 2 * ACC_BUFS; ++i) raw[i] = load_scale();
+      float cur[ACC_BUFS];
+#pragma unroll
+      for (int i = 0; i < ACC_BUFS; ++i) { cur[i] = __half2float(__ushort_as_half(raw[i])); raw[i] = raw[ACC_BUFS + i]; }
+      auto coefficient = [&](int u) {
+        const float after = __half2float(__ushort_as_half(raw[u]));
+        const float c = (cur[u] - after) * kScaleUp;
+        cur[u] = after;
+        raw[u] = load_scale();
+        return c;
+      };
+      float s2[2] = {coefficient(0), coefficient(1)};
+      bool ready = false;                       // the pair's barrier has been seen to complete
+      int g = g_begin;
 #pragma unroll 1
-    for (int g = g_begin; g < g_end && epi_ok; ++g) {
-      // coefficient of this group's running sum
-      const float s2 = (__half2float(__ushort_as_half(sr[0])) - __half2float(__ushort_as_half(sr[ACC_BUFS]))) * kScaleUp;
+      while (g < g_end && epi_ok) {
 #pragma unroll
-      for (int i = 0; i < ACC_BUFS; ++i) sr[i] = sr[i + 1];
-      sr[ACC_BUFS] = load_scale();
-      const uint32_t buf = lane_addr + ab * BLOCK_M;
-      // the last groups of a tile keep their buffers until these are back at the bias for the next tile (below)
-      const bool keep_buf = more_tiles && g >= g_end - ACC_BUFS;
-      if (threadIdx.x == 0) SK_TRACE_EVENT(7, (g - g_begin) * 8 + 0);
-      epi_ok = wait_bounded(bar_acc_full + 8 * ab, aph, ctx, kStEpilogueAccFull);
-      if (!epi_ok) break;
-      if (threadIdx.x == 0) SK_TRACE_EVENT(7, (g - g_begin) * 8 + 1);
-      tcgen05_fence_after_sync();
-      if constexpr (kDB) tmem_ld_chunk<kChunk>(buf, v[0]);
-      int ab_next = ab + 1;
-      uint32_t aph_next = aph;
-      if (ab_next == ACC_BUFS) { ab_next = 0; aph_next ^= 1; }
+        for (int u = 0; u < ACC_BUFS; u += 2) {
+          if (g >= g_end) break;
+          const uint32_t bar = acc_bar(u);
+          if (!ready) epi_ok = wait_bounded(bar_acc_full + bar, aph, ctx, kStEpilogueAccFull);
+          if (!epi_ok) break;
+          tcgen05_fence_after_sync();
+          const uint32_t buf = lane_addr + u * BLOCK_M;
+          if constexpr (kDB) tmem_ld_chunk<kChunk>(buf, v[0]);
+          float s2_next[2] = {0.f, 0.f};
 #pragma unroll
-      for (int c = 0; c < kNumChunks; ++c) {
-        if constexpr (!kDB) tmem_ld_chunk<kChunk>(buf + c * kChunk, v[0]);
-        tmem_ld_wait();
-        if (threadIdx.x == 0 && c < 4) SK_TRACE_EVENT(7, (g - g_begin) * 8 + 2 + c);
-        if constexpr (kDB) {
-          if (c + 1 < kNumChunks) tmem_ld_chunk<kChunk>(buf + (c + 1) * kChunk, v[(c + 1) & kBufMask]);
+          for (int k = 0; k < 2 * kNumChunks; ++k) {       // the first group's chunks, then the second's
+            const int c = k % kNumChunks;
+            if constexpr (!kDB) tmem_ld_chunk<kChunk>(buf + (k / kNumChunks) * BLOCK_M + c * kChunk, v[0]);
+            tmem_ld_wait();
+            if constexpr (kDB) {
+              if (k + 1 < 2 * kNumChunks)
+                tmem_ld_chunk<kChunk>(buf + ((k + 1) / kNumChunks) * BLOCK_M + ((k + 1) % kNumChunks) * kChunk, v[(k + 1) & kBufMask]);
+            }
+            if (k == 2 * kNumChunks - 1) {      // both buffers fully read: back to the MMA issuers (they keep accumulating)
+              tcgen05_fence_before_sync();
+              __syncwarp();
+              mbar_arrive_if(bar_acc_empty + bar, lane == 0);
+              ready = mbar_try_wait(bar_acc_full + acc_bar((u + 2) % ACC_BUFS), aph ^ (u + 2 == ACC_BUFS ? 1u : 0u));
+              s2_next[0] = coefficient((u + 2) % ACC_BUFS);
+              s2_next[1] = coefficient((u + 3) % ACC_BUFS);
+            }
+#pragma unroll
+            for (int j = 0; j < kChunk; ++j)
+              acc[c * kChunk + j] = fmaf(s2[k / kNumChunks], __uint_as_float(v[k & kBufMask][j]), acc[c * kChunk + j]);
+          }
+          s_sum += s2[0];
+          s_sum += s2[1];
+          s2[0] = s2_next[0];
+          s2[1] = s2_next[1];
+          g += 2;
+          if (u + 2 == ACC_BUFS) aph ^= 1;
         }
-        if (c == kNumChunks - 1 && !keep_buf) {   // buffer fully read: hand it back to the MMA issuer (it keeps accumulating)
-          tcgen05_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar_acc_empty + 8 * ab);
-        }
-        if constexpr (DUMP) {
-          if (n_ok) {
+        flush += ACC_BUFS;
+        if (flush == kBiasFlushGroups) {
+          const float corr = s_sum * bias_f;
 #pragma unroll
-            for (int j = 0; j < kChunk; ++j) {
-              const int m = m0 + col0 + c * kChunk + j;
-              if (m < p.M)
-                p.partials[(static_cast<size_t>(g) * p.M + m) * p.N + n] =
-                    static_cast<int32_t>(v[c & kBufMask][j]) - static_cast<int32_t>(bias);
+          for (int j = 0; j < kCols; ++j) acc[j] -= corr;
+          s_sum = 0.f; flush = 0;
+        }
+      }
+    } else {
+      unsigned short sr[ACC_BUFS + 1];
+#pragma unroll
+      for (int i = 0; i <= ACC_BUFS; ++i) sr[i] = load_scale();
+#pragma unroll 1
+      for (int g = g_begin; g < g_end && epi_ok; ++g) {
+        // coefficient of this group's running sum
+        const float s2 = (__half2float(__ushort_as_half(sr[0])) - __half2float(__ushort_as_half(sr[ACC_BUFS]))) * kScaleUp;
+#pragma unroll
+        for (int i = 0; i < ACC_BUFS; ++i) sr[i] = sr[i + 1];
+        sr[ACC_BUFS] = load_scale();
+        const uint32_t buf = lane_addr + ab * BLOCK_M;
+        // the last groups of a tile keep their buffers until these are back at the bias for the next tile (below)
+        const bool keep_buf = more_tiles && g >= g_end - ACC_BUFS;
+        if (threadIdx.x == 0) SK_TRACE_EVENT(7, (g - g_begin) * 8 + 0);
+        epi_ok = wait_bounded(bar_acc_full + 8 * ab, aph, ctx, kStEpilogueAccFull);
+        if (!epi_ok) break;
+        if (threadIdx.x == 0) SK_TRACE_EVENT(7, (g - g_begin) * 8 + 1);
+        tcgen05_fence_after_sync();
+        if constexpr (kDB) tmem_ld_chunk<kChunk>(buf, v[0]);
+        int ab_next = ab + 1;
+        uint32_t aph_next = aph;
+        if (ab_next == ACC_BUFS) { ab_next = 0; aph_next ^= 1; }
+#pragma unroll
+        for (int c = 0; c < kNumChunks; ++c) {
+          if constexpr (!kDB) tmem_ld_chunk<kChunk>(buf + c * kChunk, v[0]);
+          tmem_ld_wait();
+          if (threadIdx.x == 0 && c < 4) SK_TRACE_EVENT(7, (g - g_begin) * 8 + 2 + c);
+          if constexpr (kDB) {
+            if (c + 1 < kNumChunks) tmem_ld_chunk<kChunk>(buf + (c + 1) * kChunk, v[(c + 1) & kBufMask]);
+          }
+          if (c == kNumChunks - 1 && !keep_buf) {   // buffer fully read: hand it back to the MMA issuer (it keeps accumulating)
+            tcgen05_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_acc_empty + 8 * ab);
+          }
+          if constexpr (DUMP) {
+            if (n_ok) {
+#pragma unroll
+              for (int j = 0; j < kChunk; ++j) {
+                const int m = m0 + col0 + c * kChunk + j;
+                if (m < p.M)
+                  p.partials[(static_cast<size_t>(g) * p.M + m) * p.N + n] =
+                      static_cast<int32_t>(v[c & kBufMask][j]) - static_cast<int32_t>(bias);
+              }
             }
           }
+#pragma unroll
+          for (int j = 0; j < kChunk; ++j)
+            acc[c * kChunk + j] = fmaf(s2, __uint_as_float(v[c & kBufMask][j]), acc[c * kChunk + j]);
         }
+        if (threadIdx.x == 0) SK_TRACE_EVENT(3, SK_TRACE_BASE + g - g_begin);
+        s_sum += s2;
+        if (++flush == kBiasFlushGroups) {
+          const float corr = s_sum * bias_f;
 #pragma unroll
-        for (int j = 0; j < kChunk; ++j)
-          acc[c * kChunk + j] = fmaf(s2, __uint_as_float(v[c & kBufMask][j]), acc[c * kChunk + j]);
+          for (int j = 0; j < kCols; ++j) acc[j] -= corr;
+          s_sum = 0.f; flush = 0;
+        }
+        ab = ab_next; aph = aph_next;
       }
-      if (threadIdx.x == 0) SK_TRACE_EVENT(3, SK_TRACE_BASE + g - g_begin);
-      s_sum += s2;
-      if (++flush == kBiasFlushGroups) {
-        const float corr = s_sum * bias_f;
-#pragma unroll
-        for (int j = 0; j < kCols; ++j) acc[j] -= corr;
-        s_sum = 0.f; flush = 0;
-      }
-      ab = ab_next; aph = aph_next;
     }
     if (threadIdx.x == 0 && tile == tile_first) SK_TRACE_EVENT(6, 0);
     if (more_tiles && epi_ok) {

@@ -36,6 +36,21 @@ def test_every_tile_split_and_group_size(tile, split, G, K):
     assert torch.isnan(y[:, N:]).all() and torch.equal(dp.gemm(ld_out=N + 5)[:, :N], y[:, :N])
 
 
+# Where the MMA issuers take K blocks (or groups) in turn: one block or group in all, odd numbers of either, less and more than
+# the rings and accumulator buffers hold, a last block with one group.  Tolerance as above.
+@pytest.mark.parametrize("tile,M", [(64, 61), (128, 128), (256, 257)])
+@pytest.mark.parametrize("split", [1, 2])
+@pytest.mark.parametrize("G,K", [(128, 128), (128, 256), (128, 384), (128, 896), (128, 1664), (64, 64), (64, 128), (64, 192), (64, 832),
+                                 (64, 1600), (32, 32), (32, 96), (32, 288), (256, 256), (256, 768)])
+def test_turns_of_the_issuers(tile, M, split, G, K):
+    x_q, xs, wp, ws = random_problem(M, 130, K, G, seed=tile + split + K)
+    dp = DeviceProblem(x_q, xs, wp, ws, G).force(kernel=capi.KERNEL_TCGEN05, token_tile=tile, split_k=split)
+    ref = O.w2a8_gemm_int_path(x_q, xs, wp, ws, G)
+    y = dp.gemm()
+    assert np.abs(to_np(y) - ref).max() <= 4e-3 * max(1.0, np.abs(ref).max())
+    assert dp.plan.device_status() == 0 and torch.equal(dp.gemm(), y)
+
+
 @pytest.mark.parametrize("G", [32, 64, 128, 256])
 @pytest.mark.parametrize("M,N,K", [(40, 512, 4096), (96, 1024, 4096), (130, 300, 11008), (333, 1000, 4096), (512, 2048, 2048),
                                    (600, 4096, 2048)])
