@@ -63,7 +63,9 @@ class W2A8Linear(nn.Module):
         # Asked on every call, so the buffers are looked up once and where they are kept: five look-ups through
         # nn.Module.__getattr__ took 4 us where the check itself takes 1.
         buffers = self._buffers
-        w, s = buffers["w_packed"], buffers["w_scale"]
+        w, s = buffers.get("w_packed"), buffers.get("w_scale")
+        if w is None or s is None:                       # (replaced by something that is not a buffer)
+            w, s = self.w_packed, self.w_scale
         key = (w.data_ptr(), w._version, s.data_ptr(), s._version, w.device)
         if self._plan is None or self._plan_key != key:
             self._plan = W2A8Plan(w, s, group_size=self.group_size, zero_point=self.zero_point, out_dtype=self.out_dtype)
@@ -90,5 +92,6 @@ class W2A8LlamaMLP(nn.Module):
 
     def forward(self, x):
         modules = self._modules                                              # (see W2A8Linear.plan)
-        gate_up_plan, down_plan = modules["gate_up"].plan(), modules["down"].plan()      # also loads the extension
+        gate_up, down = modules.get("gate_up") or self.gate_up, modules.get("down") or self.down
+        gate_up_plan, down_plan = gate_up.plan(), down.plan()                # also loads the extension
         return torch.ops.slimkernels.w2a8_mlp_block.default(gate_up_plan._h, down_plan._h, x, down_plan.N, down_plan._bf16)
