@@ -6,6 +6,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <mutex>
 #include <new>
 #include <vector>
@@ -1822,9 +1823,20 @@ int sk_silu_mul_quantize_int8(const void* gate_up_f16, int64_t ld_gu, int64_t M,
                 : vecs == 3 ? sk::silu_mul_quantize_rows_kernel<3>
                             : sk::silu_mul_quantize_rows_kernel<4>;
     const int smem = static_cast<int>(I) * 4, grid = sk::kChipSms * sk::rows_ctas_per_sm(vecs);
-    if (smem > 47 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
-      (void)cudaGetLastError();
-      return SK_ERR_CUDA;
+    if (vecs >= 3) {                      // more than 48 KB of shared memory with the longest rows
+      // Always the most that the instantiation takes: the attribute belongs to the kernel, so a size of this call's own would be
+      // taken from under another thread's launch with longer rows.
+      static std::atomic<int> configured[2][64];
+      int dev = 0;
+      if (cudaGetDevice(&dev) != cudaSuccess) return SK_ERR_CUDA;
+      const bool known = dev >= 0 && dev < 64;
+      if (!known || !configured[vecs - 3][dev].load(std::memory_order_acquire)) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, vecs * sk::kRowsThreads * 8 * 4) != cudaSuccess) {
+          (void)cudaGetLastError();
+          return SK_ERR_CUDA;
+        }
+        if (known) configured[vecs - 3][dev].store(1, std::memory_order_release);
+      }
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(M < grid ? M : grid));

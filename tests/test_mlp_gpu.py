@@ -1,5 +1,6 @@
 """Activation quantiser, SiLU*up re-quantiser and the W2A8 Llama MLP block (benchmark config 4) against the oracle."""
 import ctypes
+import threading
 
 import numpy as np
 import pytest
@@ -81,6 +82,38 @@ def test_silu_many_rows_equal_few_rows(M, I, pad):
         run(lo, min(M, lo + 50), q[1], s[1])
     assert torch.equal(q[0], q[1]) and torch.equal(s[0].view(torch.int32), s[1].view(torch.int32))
     assert pad == 0 or bool((q[0][:, I:] == 99).all())
+
+
+# Two widths that share an instantiation of the kernel of resident CTAs and need more than the default 48 KB of shared memory.
+@pytest.mark.parametrize("widths", [(12800, 14336)])
+def test_silu_from_two_threads(widths):
+    """Calls with different widths from two host threads: none is refused, and the results are those of a single thread."""
+    lib = capi.load()
+    M, calls = 296, 5000
+    g = torch.Generator(device="cuda").manual_seed(1)
+    gus = [torch.randn(M, 2 * I, generator=g, device="cuda").half() for I in widths]
+
+    def run(gu, stream, n):
+        I = gu.shape[1] // 2
+        q, s = torch.empty(M, I, dtype=torch.int8, device="cuda"), torch.empty(M, device="cuda")
+        torch.cuda.synchronize()
+        rcs = {lib.sk_silu_mul_quantize_int8(gu.data_ptr(), 2 * I, M, I, q.data_ptr(), I, s.data_ptr(), stream.cuda_stream) for _ in range(n)}
+        stream.synchronize()
+        return rcs, q, s
+
+    alone = [run(gu, torch.cuda.Stream(), 1) for gu in gus]
+    both = [None, None]
+
+    def work(i):
+        both[i] = run(gus[i], torch.cuda.Stream(), calls)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for a, b in zip(alone, both):
+        assert b[0] == {0} and torch.equal(a[1], b[1]) and torch.equal(a[2], b[2])
 
 
 def _mlp_problem(M, hidden, inter, seed=0):
