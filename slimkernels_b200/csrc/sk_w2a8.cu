@@ -1812,12 +1812,23 @@ int sk_silu_mul_quantize_int8(const void* gate_up_f16, int64_t ld_gu, int64_t M,
     return SK_ERR_BAD_ALIGNMENT;
   const auto st = static_cast<cudaStream_t>(stream);
   const __half* gu = static_cast<const __half*>(gate_up_f16);
-  // From 64 rows on CTAs that stay and take a row each at a time (the cluster kernel / this one, us: 64 x 11008 4.8 / 4.8,
-  // 128 x 11008 6.7 / 5.4, 592 x 11008 12.9 / 9.7, 4096 x 11008 66.8 / 51.4; 64 x 4096 2.7 / 2.4; but 32 x 14336 3.7 / 4.4: a row is one
-  // CTA's work here, up to eight's there).
-  // One vector per thread keeps pace only for a few rows per CTA (4096 x 4096 21.2 / 23.1).
-  if (M >= 64 && I <= 8LL * sk::kRowsThreads * 4 && (I > 8LL * sk::kRowsThreads || M <= 4 * sk::kChipSms)) {
-    const int vecs = static_cast<int>((I / 8 + sk::kRowsThreads - 1) / sk::kRowsThreads);
+  // Many rows: CTAs that stay and take a row each at a time.  A row is one CTA's work here and up to eight CTAs' in the cluster kernel
+  // below.  Measured between the two GEMMs of a block, where the calls are, in us by which a block is shorter with resident CTAs:
+  //   * from 64 rows on: 64 x 4096 .7, 64 x 11008 .7, 128 x 8192 1.9, 296 x 11008 2.1, 592 x 11008 2.8, 4096 x 11008 19, 4096 x 5504 8;
+  //     under 64 rows nothing to 1 at most (32 x 14336 -.4).  The gain is not the same everywhere: 128 x 12288 -.6;
+  //   * four vectors per thread from 104 rows on: 72 to 96 x 14336 up to -1.3, 148 x 14336 +.5 (by themselves, one after another, 96 x
+  //     14336 7 % slower and 104 x 14336 7 % faster);
+  //   * not up to 2048 features, where half the threads have nothing (128 x 1024 -.6, 256 x 256 -.6);
+  //   * up to 4096, where the cluster kernel has one CTA per row too, only while every row has a CTA of its own: 592 x 4096 +.5, 592 x
+  //     3072 1.5, but 768 x 3072 -1.0, 4096 x 4096 -2.8;
+  //   * with two vectors, a wave holds 444 resident CTAs but 592 clusters of two: 528 to 592 rows of 5504 and 6144 features -1.1 to -2.1,
+  //     of 7168 and more +.2 to +1.1; 512 x 5504 +.8, 608 x 5504 -.2 to -.9, 1024 x 5504 +1.4.
+  const int vecs = static_cast<int>(I <= 8LL * sk::kRowsThreads * 4 ? (I / 8 + sk::kRowsThreads - 1) / sk::kRowsThreads : 5);
+  const bool resident = vecs == 1   ? M >= 64 && M <= 4 * sk::kChipSms && I > 4 * sk::kRowsThreads
+                        : vecs == 2 ? M >= 64 && (I > 12 * sk::kRowsThreads || M <= 512 || M > 4 * sk::kChipSms)
+                        : vecs == 3 ? M >= 64
+                                    : vecs == 4 && M >= 104;
+  if (resident) {
     auto kern = vecs == 1   ? sk::silu_mul_quantize_rows_kernel<1>
                 : vecs == 2 ? sk::silu_mul_quantize_rows_kernel<2>
                 : vecs == 3 ? sk::silu_mul_quantize_rows_kernel<3>

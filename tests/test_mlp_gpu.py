@@ -1,5 +1,9 @@
 """Activation quantiser, SiLU*up re-quantiser and the W2A8 Llama MLP block (benchmark config 4) against the oracle."""
 import ctypes
+import json
+import os
+import subprocess
+import sys
 import threading
 
 import numpy as np
@@ -60,9 +64,11 @@ def test_silu_mul_quantize(M, I):
 
 
 @pytest.mark.parametrize("M,I,pad", [(64, 8, 0), (64, 4096, 0), (65, 4104, 8), (700, 264, 16), (64, 8192, 0), (450, 8200, 0), (300, 11008, 0),
-                                     (64, 12288, 8), (64, 12296, 0), (310, 16384, 0), (64, 16392, 0)])
+                                     (64, 12288, 8), (64, 12296, 0), (310, 16384, 0), (64, 16392, 0),
+                                     (64, 2056, 8), (592, 4096, 0), (104, 12296, 8), (512, 6144, 0), (593, 4104, 0)])
 def test_silu_many_rows_equal_few_rows(M, I, pad):
-    """64 rows and more go through the kernel of resident CTAs (up to 16384 features), fewer through clusters: the same bits."""
+    """Many rows go through the kernel of resident CTAs, 50 at a time through clusters: the same bits.  (64, 8), (700, 264), (64, 12296) and
+    (64, 16392) lie beyond the lines of the dispatch and take clusters both times."""
     lib = capi.load()
     g = torch.Generator(device="cuda").manual_seed(M + I)
     gu = (torch.randn(M, 2 * I + pad, generator=g, device="cuda") * 3).half()
@@ -82,6 +88,39 @@ def test_silu_many_rows_equal_few_rows(M, I, pad):
         run(lo, min(M, lo + 50), q[1], s[1])
     assert torch.equal(q[0], q[1]) and torch.equal(s[0].view(torch.int32), s[1].view(torch.int32))
     assert pad == 0 or bool((q[0][:, I:] == 99).all())
+
+
+# Both sides of every line of the re-quantiser's dispatch: which kernel a call of that size launches.
+_SILU_LINES = [(63, 4096, "cluster"), (64, 4096, "rows"), (64, 2048, "cluster"), (64, 2056, "rows"), (592, 256, "cluster"), (592, 4096, "rows"),
+               (593, 4096, "cluster"), (444, 4104, "rows"), (512, 6144, "rows"), (513, 6144, "cluster"), (592, 4104, "cluster"), (592, 6152, "rows"),
+               (593, 6144, "rows"), (63, 11008, "cluster"), (64, 12288, "rows"), (64, 12296, "cluster"), (103, 16384, "cluster"),
+               (104, 12296, "rows"), (104, 16384, "rows"), (104, 16392, "cluster")]
+_SILU_LAUNCHES = """
+import json, sys
+import torch
+from torch.profiler import ProfilerActivity, profile
+from slimkernels_b200 import capi
+lib = capi.load()
+cases = json.loads(sys.argv[1])
+gu, q, s = torch.zeros(600 * 2 * 16392, dtype=torch.half, device="cuda"), torch.zeros(600 * 16392, dtype=torch.int8, device="cuda"), torch.zeros(600, device="cuda")
+with profile(activities=[ProfilerActivity.CUDA]) as prof:
+    for M, I in cases:
+        assert lib.sk_silu_mul_quantize_int8(gu.data_ptr(), 2 * I, M, I, q.data_ptr(), I, s.data_ptr(), 0) == 0
+    torch.cuda.synchronize()
+kernels = sorted((e.time_range.start, e.name) for e in prof.events() if "silu_mul_quantize" in e.name)
+print(json.dumps([n for _, n in kernels]))
+"""
+
+
+def test_silu_dispatch():
+    """Calls on which the kernel of resident CTAs was measured to be the slower one go through clusters, the others do not."""
+    cases = json.dumps([c[:2] for c in _SILU_LINES])
+    run = subprocess.run([sys.executable, "-c", _SILU_LAUNCHES, cases], capture_output=True, text=True, timeout=300,
+                         cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert run.returncode == 0, run.stderr[-2000:]
+    names = json.loads(run.stdout.splitlines()[-1])
+    assert len(names) == len(_SILU_LINES)
+    assert [(c[0], c[1], "rows" if "rows" in n else "cluster") for c, n in zip(_SILU_LINES, names)] == _SILU_LINES
 
 
 # Two widths that share an instantiation of the kernel of resident CTAs and need more than the default 48 KB of shared memory.
