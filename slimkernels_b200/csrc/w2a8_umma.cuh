@@ -363,7 +363,11 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
   // buffers it takes two groups at a time.  Cycles per K block, before (with the issuers' shorter loop) and after: 128 tokens 650 (684)
   // -> 619, 64 tokens 588 (575) -> 539, group size 64 1239 (1181) -> 1017 and 1107 (1080) -> 831: each alone moved little, the three
   // roles were equally slow.  333 x 5000 x 4160 with group size 64 26.3 -> 22.9 us.
-  constexpr int kPair = ACC_BUFS == 4 && BLOCK_M >= 64 && !DUMP && !PERSIST ? 2 : 1;
+  // Not the K split of 64 tokens with group size 128: the reduction leaves no registers for the second group's scales there (24 bytes
+  // spilled), and a call took 2.3 to 2.9 % longer than with one group at a time, now 1.0 % shorter (medians over 83 calls of 33 to 512
+  // tokens in 2, 4 and 8 splits: 64 x 4096 x 4096 in four 9.45, with pairs 9.72, now 9.43 us).  With other group sizes the same spill costs less than
+  // the pairs give (64: .90 of the time in two splits, 256: .95, 32: .975).
+  constexpr int kPair = ACC_BUFS == 4 && BLOCK_M >= 64 && !DUMP && !PERSIST && !(SPLIT && !OTHER_G && BLOCK_M == 64) ? 2 : 1;
   auto acc_bar = [](int buf) { return 8u * static_cast<uint32_t>(buf / kPair); };      // offset of a buffer's barrier
   constexpr bool kBlockTurns = ACC_BUFS == 4;   // group size 64: the MMA issuers take K blocks, not groups, in turn
 
