@@ -6,8 +6,8 @@
 //      memory stages guarded by mbarriers;
 //   2. expander warps turn the 2-bit codes into int8 bytes (code - zero_point) with a byte-permute look-up
 //      (prmt), written straight into the 128-byte-swizzled K-major layout the tensor core reads;
-//   3. two MMA warps, taking the scale groups in turn, issue tcgen05.mma kind::i8 (128 x BLOCK_M x 32 per
-//      instruction): the weights are the "A"/M operand, the tokens the "B"/N operand, int32 accumulators live in
+//   3. two MMA warps, taking the scale groups (or the K blocks) in turn, issue tcgen05.mma kind::i8 (128 x BLOCK_M x 32
+//      per instruction): the weights are the "A"/M operand, the tokens the "B"/N operand, int32 accumulators live in
 //      tensor memory, one accumulator buffer per scale group (ACC_BUFS buffers, so later groups accumulate while
 //      earlier ones drain);
 //   4. one or two epilogue warpgroups read each finished group from tensor memory (lane = output feature,
@@ -27,10 +27,11 @@
 // Re-setting a buffer per group instead (tcgen05.st) costs more tensor-memory write bandwidth than the whole
 // epilogue has to spare.  The debug entry point stores the running sums; the host differences them into P.
 //
-// The producer and MMA warps run their loops warp-uniformly (all lanes wait, one elected lane issues) and keep
-// the loop bodies short: a single warp retires dependent instructions several cycles apart.  Even so one issuing
-// thread needs longer for its commits, barrier polls and loop between two groups than the tensor core needs for a
-// group, hence the two issuers.  mbarriers count one arrival per warp.
+// The producer warp runs its loop warp-uniformly (all lanes wait, one elected lane issues), and so do the MMA warps of the tiles
+// with two accumulator buffers at group size 128; elsewhere one elected lane runs the MMA warps' whole loop.  The loop
+// bodies are short: a single warp retires dependent instructions several cycles apart.  Even so one issuing thread
+// needs longer for its commits, barrier polls and loop between two groups than the tensor core needs for a group, hence
+// the two issuers.  mbarriers count one arrival per warp.
 //
 // With SPLIT_K > 1 the CTAs of one thread-block cluster split the groups of a tile and reduce their fp32
 // accumulators through distributed shared memory in a fixed order (deterministic, no global scratch).
@@ -77,6 +78,16 @@ enum : int {
 #else
 #define SK_TRACE_EVENT(role, idx) do { } while (0)
 #define SK_TRACE_BASE 0
+#endif
+
+// The issuers' way through K blocks 8 to 15: before and after their waits, before and after their commits (-DSK_TRACE_MMA_FINE too).
+#if defined(SK_TRACE) && defined(SK_TRACE_MMA_FINE)
+#define SK_TRACE_FINE(kb, step)                                                          \
+  do {                                                                                   \
+    if ((kb) >= 8 && (kb) < 16) SK_TRACE_EVENT(5, ((kb) - 8) * 8 + (step));              \
+  } while (0)
+#else
+#define SK_TRACE_FINE(kb, step) do { } while (0)
 #endif
 
 // Tensor maps of the further destinations of an output tile (peer GPUs' buffers): [M][N] 16-bit, box 128 x BLOCK_M.
@@ -505,12 +516,13 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       }
       __syncwarp();
     } else if (warp == kMmaWarp || warp == kMmaWarp + 1) {
-      // ============================================================ MMA issuers (whole warp loops, one lane issues)
-      // TWO warps take the scale groups in turn.  Between the MMAs of one group and those of the next a single
-      // issuing thread spends ~800 cycles on its commits, loop and barrier polls -- longer than the tensor core
-      // needs for what is queued -- so with one issuer the tensor pipe idles about half the time; with two, one
-      // warp's overhead overlaps the other's issue.  Consecutive groups use different accumulator buffers and
-      // different stages, and tcgen05.commit tracks the issuing thread's own MMAs, so the two streams are independent.
+      // ============================================================ MMA issuers
+      // TWO warps take turns.  Between the MMAs of one group and those of the next a single issuing thread spends ~800
+      // cycles on its commits, loop and barrier polls -- longer than the tensor core needs for what is queued -- so
+      // with one issuer the tensor pipe idles about half the time; with two, one warp's overhead overlaps the
+      // other's issue.  What one takes and what the other takes use different accumulator buffers (and, where they take
+      // whole K blocks, different stages), and tcgen05.commit tracks the issuing thread's own MMAs, so the two streams are
+      // independent.  Which turns they take, and whether the warp or one lane runs the loop, is said at each loop below.
       const int mma_id = warp - kMmaWarp;
       constexpr uint32_t idesc = make_idesc_i8(kTileN, BLOCK_M, /*a_signed=*/true, /*b_signed=*/true);
       const uint64_t a_desc0 = make_kmajor_sw128_desc(smem_base + T::kOffWx);
@@ -533,6 +545,9 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         // 256, 384, ...: a group spans blocks; one issuer.
         // Where a block's groups and the next block's fill different buffers (two groups, four buffers) the issuers take blocks
         // in turn instead, as with group size 128: half the iterations for each.
+        // Time of a call against a loop of the whole warp with, up to 128 tokens, one group at a time in the epilogue (medians over 33
+        // to 4096 tokens, no split): group size 64 .82 with 64 tokens, .86 with 128, .99 with 256; 32 .82 / .90 / .99; 256 .89 / .90 / .88.
+        static_assert(!A_TMEM && T::kTied, "weights in shared memory, tied rings");
         const int steps = p.steps_per_group;                  // 1, 2 or a multiple of 8 (in blocks: 4)
         const int per_block = steps < 4 ? 4 / steps : 1;      // groups per block
         const int blocks = steps < 4 ? 1 : steps / 4;         // blocks per group
@@ -569,8 +584,8 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
               }
             }
             if (!ok) break;
-            umma_commit(bar_ld_empty + 8 * l);
-            if constexpr (!T::kTied) umma_commit(bar_ex_empty + 8 * e);
+            umma_commit(bar_ld_empty + 8 * l);                // (tied rings: the expanded weights are free with it)
+            SK_TRACE_EVENT(2, kb - kb_begin);
             if ((l += step) >= LSTAGES) l -= LSTAGES;
             if ((e += step) >= ESTAGES) { e -= ESTAGES; eph ^= 1; }
           }
@@ -590,10 +605,12 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
               if (++ab == ACC_BUFS) { ab = 0; aph ^= 1; }
               continue;
             }
+            if (lane == 0) SK_TRACE_FINE(kb - kb_begin, 0);
             ok = wait_bounded(bar_ld_full + 8 * l, lph, ctx, kStMmaLdFull) &&
                  wait_bounded(bar_ex_full + 8 * e, eph, ctx, kStMmaExFull) &&
                  wait_bounded(bar_acc_empty + 8 * ab, aph, ctx, kStMmaAccEmpty);
             if (!ok) break;
+            if (lane == 0) SK_TRACE_FINE(kb - kb_begin, 1);
             tcgen05_fence_after_sync();
             if (elect_one()) {
               const uint64_t a_desc = a_desc0 + static_cast<uint64_t>(e * (kWxBytes >> 4));
@@ -612,9 +629,11 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
                 umma_i8(d, a_desc + 4, b_desc + 4, idesc, 1u);
                 umma_i8(d, a_desc + 6, b_desc + 6, idesc, 1u);
               }
+              SK_TRACE_FINE(kb - kb_begin, 2);
               umma_commit(bar_acc_full + 8 * ab);
               umma_commit(bar_ld_empty + 8 * l);
               if constexpr (!T::kTied) umma_commit(bar_ex_empty + 8 * e);
+              SK_TRACE_FINE(kb - kb_begin, 3);
               SK_TRACE_EVENT(2, SK_TRACE_BASE + kb - kb_begin);
             }
             __syncwarp();
@@ -627,6 +646,7 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
           // around them paces the small tiles: one lane runs the loop, its stages
           // and buffers advance by two, the barrier of the expanded weights stands for the copies too (the expanders waited
           // for them), and the two polls overlap.  An iteration was 1150 cycles with every barrier complete, of which the MMAs 140.
+          static_assert(!A_TMEM && T::kTied, "weights in shared memory, tied rings");
           const int per_cta = PERSIST ? (tile_end - tile_first + tile_step - 1) / tile_step : 1;
           const int blocks = per_cta * (kb_end - kb_begin);
           if (elect_one()) {
@@ -634,30 +654,26 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
             ab = mma_id;
 #pragma unroll 1
             for (int i = mma_id; i < blocks; i += 2) {
+              SK_TRACE_FINE(i, 0);
               if (!wait_bounded_two(bar_ex_full + 8 * e, eph, bar_acc_empty + acc_bar(ab), aph, ctx, kStMmaExFull, kStMmaAccEmpty)) {
                 ok = false;
                 break;
               }
+              SK_TRACE_FINE(i, 1);
               tcgen05_fence_after_sync();
               const uint64_t a_desc = a_desc0 + static_cast<uint64_t>(e * (kWxBytes >> 4));
               const uint64_t b_desc = b_desc0 + static_cast<uint64_t>(l * (T::kXBytes >> 4));
               const uint32_t d = tmem_base + ab * BLOCK_M;
               // +2 in the (address >> 4) field advances 32 bytes along K inside the 128-byte swizzle row
-              if constexpr (A_TMEM) {
-                const uint32_t a_t = tmem_base + T::kATmemCol0 + e * 32;   // 8 columns per 32-wide K step
-                umma_i8_ts(d, a_t, b_desc, idesc, 1u);
-                umma_i8_ts(d, a_t + 8, b_desc + 2, idesc, 1u);
-                umma_i8_ts(d, a_t + 16, b_desc + 4, idesc, 1u);
-                umma_i8_ts(d, a_t + 24, b_desc + 6, idesc, 1u);
-              } else {
-                umma_i8(d, a_desc, b_desc, idesc, 1u);
-                umma_i8(d, a_desc + 2, b_desc + 2, idesc, 1u);
-                umma_i8(d, a_desc + 4, b_desc + 4, idesc, 1u);
-                umma_i8(d, a_desc + 6, b_desc + 6, idesc, 1u);
-              }
+              umma_i8(d, a_desc, b_desc, idesc, 1u);
+              umma_i8(d, a_desc + 2, b_desc + 2, idesc, 1u);
+              umma_i8(d, a_desc + 4, b_desc + 4, idesc, 1u);
+              umma_i8(d, a_desc + 6, b_desc + 6, idesc, 1u);
+              SK_TRACE_FINE(i, 2);
               umma_commit(bar_acc_full + acc_bar(ab));
-              umma_commit(bar_ld_empty + 8 * l);
-              if constexpr (!T::kTied) umma_commit(bar_ex_empty + 8 * e);
+              umma_commit(bar_ld_empty + 8 * l);                           // (and the expanded weights' stage: tied rings)
+              SK_TRACE_FINE(i, 3);
+              SK_TRACE_EVENT(2, i);
               if ((l += 2) >= LSTAGES) l -= LSTAGES;                       // (even rings)
               if ((e += 2) >= ESTAGES) { e -= ESTAGES; eph ^= 1; }
               if ((ab += 2) >= ACC_BUFS) { ab -= ACC_BUFS; aph ^= 1; }
@@ -883,6 +899,7 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     constexpr int kBufMask = kDB ? 1 : 0;
     uint32_t v[kBufMask + 1][kChunk];
     if constexpr (kPair == 2) {
+      static_assert(kBiasFlushGroups % ACC_BUFS == 0, "the bias is taken off after whole rounds of the buffers");
       // cur[u]: the scale of the group that buffer u holds next; raw[u]: the fp16 bits of the one after it (ACC_BUFS groups on),
       // fetched when the buffer was last read.  Unrolled over the buffers, nothing is shifted from register to register.
       // A group past the end has the coefficient 0: its buffer's sums, whatever they are, are finite.
@@ -908,8 +925,10 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         for (int u = 0; u < ACC_BUFS; u += 2) {
           if (g >= g_end) break;
           const uint32_t bar = acc_bar(u);
+          if (threadIdx.x == 0) SK_TRACE_EVENT(7, (g - g_begin) * 8 + 0);
           if (!ready) epi_ok = wait_bounded(bar_acc_full + bar, aph, ctx, kStEpilogueAccFull);
           if (!epi_ok) break;
+          if (threadIdx.x == 0) SK_TRACE_EVENT(7, (g - g_begin) * 8 + 1);
           tcgen05_fence_after_sync();
           const uint32_t buf = lane_addr + u * BLOCK_M;
           if constexpr (kDB) tmem_ld_chunk<kChunk>(buf, v[0]);
@@ -919,6 +938,7 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
             const int c = k % kNumChunks;
             if constexpr (!kDB) tmem_ld_chunk<kChunk>(buf + (k / kNumChunks) * BLOCK_M + c * kChunk, v[0]);
             tmem_ld_wait();
+            if (threadIdx.x == 0) SK_TRACE_EVENT(7, (g - g_begin) * 8 + 2 + k);
             if constexpr (kDB) {
               if (k + 1 < 2 * kNumChunks)
                 tmem_ld_chunk<kChunk>(buf + ((k + 1) / kNumChunks) * BLOCK_M + ((k + 1) % kNumChunks) * kChunk, v[(k + 1) & kBufMask]);
@@ -935,6 +955,7 @@ w2a8_umma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
             for (int j = 0; j < kChunk; ++j)
               acc[c * kChunk + j] = fmaf(s2[k / kNumChunks], __uint_as_float(v[k & kBufMask][j]), acc[c * kChunk + j]);
           }
+          if (threadIdx.x == 0) SK_TRACE_EVENT(3, SK_TRACE_BASE + g - g_begin);
           s_sum += s2[0];
           s_sum += s2[1];
           s2[0] = s2_next[0];
