@@ -831,10 +831,16 @@ static int resolve_launch(const sk_w2a8_plan* plan, long long M, bool debug_part
 // The token tile and K split the general kernel runs M > 32 tokens with: of the tiles up to the heuristic one's size and
 // the splits the K range allows, the pair that a simple model gives the least time,
 //     waves x (set-up and output + K blocks per CTA x time per K block + cluster reduction),
-// with the constants below fitted to sweeps on B200 (one CTA per SM; they hold within 10 % from 32 to 1376 CTAs).  It replaces "the smallest tile that holds
-// M", which left most SMs idle wherever there are few tiles: 96 x 4096 x 11008 38.4 us on 32 CTAs, 15.3 as 128 tokens split 4
-// ways; 256 x 4096 x 4096 22.4, 13.7 as 64-token tiles; 512 x 4096 x 11008 50.7, 35.2 as 128-token tiles (in part the
-// expanders' second group, see w2a8_umma.cuh).
+// with the constants below (one CTA per SM), fitted to sweeps on B200 before the issuers' shorter loop and the epilogue's pairs.
+// Against the kernels as they are it is right to 8 % for whole tiles with group size 128 and high elsewhere (medians over 33 to 4096
+// tokens, tiles of 64 / 128 / 256 tokens: group size 64 by 22 / 19 / 5 %, 32 by 21 / 8 / 15 %, 256 by 12 / 15 / 20 %), for splits
+// 19 % low to 23 % high.  What it is for, the choice, holds: of 280 calls (33 to 4096 tokens, six weights, four group sizes) the launch chosen
+// takes within 3 % of the best forced one in all but two kinds.  Where it splits 8 ways into 128 CTAs (96 to 256 x 1024 x 8192) a call
+// takes 1.4 to 1.6 times the best launch, as it did before: of these clusters of eight the chip holds 15 at a time.  And 333 x 22016 x 4096
+// with group size 128 takes 94.7 us as 256 tokens, 87.1 as 128.
+// It replaces "the smallest tile that holds M", which left most SMs idle wherever there are few tiles: 96 x 4096 x 11008
+// 38.4 us on 32 CTAs, 15.3 as 128 tokens split 4 ways; 256 x 4096 x 4096 22.4, 13.7 as 64-token tiles; 512 x 4096 x 11008 50.7, 35.2 as
+// 128-token tiles (in part the expanders' second group, see w2a8_umma.cuh).
 // The launch that resolve_launch names stays where the model sees less than 5 % in it, where its depth check moved it to
 // another tile, and where an option forces any part of it.  What is refused is decided before, on that launch.
 static void refine_launch(const sk_w2a8_plan* plan, long long M, LaunchChoice* ch) {

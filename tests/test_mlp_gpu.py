@@ -65,10 +65,12 @@ def test_silu_mul_quantize(M, I):
 
 @pytest.mark.parametrize("M,I,pad", [(64, 8, 0), (64, 4096, 0), (65, 4104, 8), (700, 264, 16), (64, 8192, 0), (450, 8200, 0), (300, 11008, 0),
                                      (64, 12288, 8), (64, 12296, 0), (310, 16384, 0), (64, 16392, 0),
-                                     (64, 2056, 8), (592, 4096, 0), (104, 12296, 8), (512, 6144, 0), (593, 4104, 0)])
+                                     (64, 2056, 8), (592, 4096, 0), (104, 12296, 8), (512, 6144, 0), (593, 4104, 0),
+                                     (2000, 4104, 8), (1400, 8184, 0), (1000, 11008, 8), (1000, 16376, 0)])
 def test_silu_many_rows_equal_few_rows(M, I, pad):
     """Many rows go through the kernel of resident CTAs, 50 at a time through clusters: the same bits.  (64, 8), (700, 264), (64, 12296) and
-    (64, 16392) lie beyond the lines of the dispatch and take clusters both times."""
+    (64, 16392) lie beyond the lines of the dispatch and take clusters both times.  In the last four every CTA takes three to five rows, so that
+    both halves of its reduction buffer and the copies of the next row are used again; all end in a part of a vector per thread."""
     lib = capi.load()
     g = torch.Generator(device="cuda").manual_seed(M + I)
     gu = (torch.randn(M, 2 * I + pad, generator=g, device="cuda") * 3).half()
