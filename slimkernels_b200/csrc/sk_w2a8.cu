@@ -1819,21 +1819,26 @@ int sk_silu_mul_quantize_int8(const void* gate_up_f16, int64_t ld_gu, int64_t M,
   const auto st = static_cast<cudaStream_t>(stream);
   const __half* gu = static_cast<const __half*>(gate_up_f16);
   // Many rows: CTAs that stay and take a row each at a time.  A row is one CTA's work here and up to eight CTAs' in the cluster kernel
-  // below.  Measured between the two GEMMs of a block, where the calls are, in us by which a block is shorter with resident CTAs:
-  //   * from 64 rows on: 64 x 4096 .7, 64 x 11008 .7, 128 x 8192 1.9, 296 x 11008 2.1, 592 x 11008 2.8, 4096 x 11008 19, 4096 x 5504 8;
-  //     under 64 rows nothing to 1 at most (32 x 14336 -.4).  The gain is not the same everywhere: 128 x 12288 -.6;
-  //   * four vectors per thread from 104 rows on: 72 to 96 x 14336 up to -1.3, 148 x 14336 +.5 (by themselves, one after another, 96 x
-  //     14336 7 % slower and 104 x 14336 7 % faster);
-  //   * not up to 2048 features, where half the threads have nothing (128 x 1024 -.6, 256 x 256 -.6);
-  //   * up to 4096, where the cluster kernel has one CTA per row too, only while every row has a CTA of its own: 592 x 4096 +.5, 592 x
-  //     3072 1.5, but 768 x 3072 -1.0, 4096 x 4096 -2.8;
-  //   * with two vectors, a wave holds 444 resident CTAs but 592 clusters of two: 528 to 592 rows of 5504 and 6144 features -1.1 to -2.1,
-  //     of 7168 and more +.2 to +1.1; 512 x 5504 +.8, 608 x 5504 -.2 to -.9, 1024 x 5504 +1.4.
+  // below.  Where which is the faster one, in us by which an MLP block of 512 to 8192 hidden features gets shorter with resident CTAs
+  // (a range: with the hidden size):
+  //   * from 64 rows on: 64 x 14336 .3 to 1.0, 64 x 8320 1.6 to 2.0, 128 x 8320 1.7 to 2.0, 444 x 5504 1.4 to 1.7, 1024 x 6144 1.0 to 1.9, 2048 x
+  //     11008 8, 4096 x 11008 19.  Under 64 rows it is nothing or less (48 x 13312 -.2 to -.8).  Single sizes lose a little still (88 x
+  //     13824 -.3 to -.9, 128 x 12288 up to -.6, 960 x 4224 -.2 to -.6, with 8192 hidden features -2.4);
+  //   * up to 2048 features, where half the threads or more have nothing, with more than 384 Ki values: 192 x 2048 -.6, 208 x 2048 up to .7,
+  //     256 x 1536 -.4 to -.8, 272 x 1536 .2 to .7, 256 x 1024 -.9 to .3, 416 x 1024 .2 to .5, 592 x 512 .1;
+  //   * up to 4096 features, where a cluster is one CTA too, only while every row has a CTA of its own: 592 x 3072 .5 to 1.1, 640 x 3072 -1.3 to
+  //     -1.9, 4096 x 4096 -2.8;
+  //   * with two vectors a wave holds 444 resident CTAs or 592 clusters of two.  Between and somewhat above the cluster is the better one:
+  //     up to 4608 features for 445 to 600 rows (480 x 4224 -.5 to -1.3, 576 x 4480 -.4 to -2.9, 640 x 4224 -.6 to 1.5), up to 6144 for 513 to 768
+  //     (512 x 5504 .7 to 1.0, 520 x 5504 -.7 to -4.2, 720 x 5504 .2 to -1.9, 832 x 5504 1.2 to 2.2), above 7168 for 481 to 512 (512 x 8192 -.3 to -2.2,
+  //     520 x 8192 1.0; 512 x 7168 .7 to -1.1).
   const int vecs = static_cast<int>(I <= 8LL * sk::kRowsThreads * 4 ? (I / 8 + sk::kRowsThreads - 1) / sk::kRowsThreads : 5);
-  const bool resident = vecs == 1   ? M >= 64 && M <= 4 * sk::kChipSms && I > 4 * sk::kRowsThreads
-                        : vecs == 2 ? M >= 64 && (I > 12 * sk::kRowsThreads || M <= 512 || M > 4 * sk::kChipSms)
-                        : vecs == 3 ? M >= 64
-                                    : vecs == 4 && M >= 104;
+  bool resident = vecs <= 4 && M >= 64;
+  if (vecs == 1) resident = resident && M <= 4 * sk::kChipSms && (I > 2048 || M * I > (384 << 10));
+  if (vecs == 2)
+    resident = resident && !(I <= 4608   ? M > 3 * sk::kChipSms && M <= 600
+                             : I <= 6144 ? M > 512 && M <= 768
+                                         : I > 7168 && M > 480 && M <= 512);
   if (resident) {
     auto kern = vecs == 1   ? sk::silu_mul_quantize_rows_kernel<1>
                 : vecs == 2 ? sk::silu_mul_quantize_rows_kernel<2>

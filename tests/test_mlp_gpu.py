@@ -65,11 +65,11 @@ def test_silu_mul_quantize(M, I):
 
 @pytest.mark.parametrize("M,I,pad", [(64, 8, 0), (64, 4096, 0), (65, 4104, 8), (700, 264, 16), (64, 8192, 0), (450, 8200, 0), (300, 11008, 0),
                                      (64, 12288, 8), (64, 12296, 0), (310, 16384, 0), (64, 16392, 0),
-                                     (64, 2056, 8), (592, 4096, 0), (104, 12296, 8), (512, 6144, 0), (593, 4104, 0),
+                                     (64, 2056, 8), (592, 4096, 0), (64, 16384, 8), (512, 6144, 0), (601, 4104, 0),
                                      (2000, 4104, 8), (1400, 8184, 0), (1000, 11008, 8), (1000, 16376, 0)])
 def test_silu_many_rows_equal_few_rows(M, I, pad):
-    """Many rows go through the kernel of resident CTAs, 50 at a time through clusters: the same bits.  (64, 8), (700, 264), (64, 12296) and
-    (64, 16392) lie beyond the lines of the dispatch and take clusters both times.  In the last four every CTA takes three to five rows, so that
+    """Many rows go through the kernel of resident CTAs, 50 at a time through clusters: the same bits.  (64, 8), (700, 264) and (64, 16392) lie
+    beyond the lines of the dispatch and take clusters both times.  In the last four every CTA takes three to five rows, so that
     both halves of its reduction buffer and the copies of the next row are used again; all end in a part of a vector per thread."""
     lib = capi.load()
     g = torch.Generator(device="cuda").manual_seed(M + I)
@@ -93,10 +93,12 @@ def test_silu_many_rows_equal_few_rows(M, I, pad):
 
 
 # Both sides of every line of the re-quantiser's dispatch: which kernel a call of that size launches.
-_SILU_LINES = [(63, 4096, "cluster"), (64, 4096, "rows"), (64, 2048, "cluster"), (64, 2056, "rows"), (592, 256, "cluster"), (592, 4096, "rows"),
-               (593, 4096, "cluster"), (444, 4104, "rows"), (512, 6144, "rows"), (513, 6144, "cluster"), (592, 4104, "cluster"), (592, 6152, "rows"),
-               (593, 6144, "rows"), (63, 11008, "cluster"), (64, 12288, "rows"), (64, 12296, "cluster"), (103, 16384, "cluster"),
-               (104, 12296, "rows"), (104, 16384, "rows"), (104, 16392, "cluster")]
+_SILU_LINES = [(63, 4096, "cluster"), (64, 4096, "rows"), (64, 2048, "cluster"), (64, 2056, "rows"), (192, 2048, "cluster"), (193, 2048, "rows"),
+               (384, 1024, "cluster"), (385, 1024, "rows"), (592, 256, "cluster"), (592, 4096, "rows"), (593, 4096, "cluster"),
+               (444, 4104, "rows"), (445, 4608, "cluster"), (600, 4104, "cluster"), (601, 4608, "rows"), (512, 4616, "rows"),
+               (513, 4616, "cluster"), (768, 6144, "cluster"), (769, 6144, "rows"), (600, 6152, "rows"), (512, 7168, "rows"), (480, 7176, "rows"),
+               (481, 7176, "cluster"), (512, 8192, "cluster"), (513, 8192, "rows"), (512, 8200, "rows"), (63, 11008, "cluster"),
+               (64, 12288, "rows"), (64, 16384, "rows"), (63, 16384, "cluster"), (104, 16392, "cluster")]
 _SILU_LAUNCHES = """
 import json, sys
 import torch
@@ -104,7 +106,8 @@ from torch.profiler import ProfilerActivity, profile
 from slimkernels_b200 import capi
 lib = capi.load()
 cases = json.loads(sys.argv[1])
-gu, q, s = torch.zeros(600 * 2 * 16392, dtype=torch.half, device="cuda"), torch.zeros(600 * 16392, dtype=torch.int8, device="cuda"), torch.zeros(600, device="cuda")
+most = max(M * I for M, I in cases)
+gu, q, s = torch.zeros(2 * most, dtype=torch.half, device="cuda"), torch.zeros(most, dtype=torch.int8, device="cuda"), torch.zeros(1024, device="cuda")
 with profile(activities=[ProfilerActivity.CUDA]) as prof:
     for M, I in cases:
         assert lib.sk_silu_mul_quantize_int8(gu.data_ptr(), 2 * I, M, I, q.data_ptr(), I, s.data_ptr(), 0) == 0
